@@ -108,6 +108,8 @@ int  wr_cuda_ctx_last_device_error(wr_cuda_ctx *ctx);
  * destroy.  64-byte aligned.  WR_CUDA_ERR_NOMEM when the host cannot pin. */
 int  wr_cuda_host_alloc(wr_cuda_ctx *ctx, uint64_t bytes, void **out);
 void wr_cuda_host_free(wr_cuda_ctx *ctx, void *p);
+/* The same for a buffer that no call is using, without its context (which may be gone). */
+void wr_cuda_host_release(void *p);
 
 /* Number of kernels this library has launched on the context so far. */
 uint64_t wr_cuda_ctx_launch_count(wr_cuda_ctx *ctx);

@@ -164,6 +164,13 @@ extern "C" void wr_cuda_host_free(wr_cuda_ctx *ctx, void *p)
     (void)cudaGetLastError();
 }
 
+extern "C" void wr_cuda_host_release(void *p)
+{
+    if (!p) return;
+    (void)cudaFreeHost(p);
+    (void)cudaGetLastError();
+}
+
 extern "C" uint64_t wr_cuda_ctx_launch_count(wr_cuda_ctx *ctx)
 {
     if (!ctx) return 0;

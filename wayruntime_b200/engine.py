@@ -103,7 +103,9 @@ class Engine:
             if argmax:
                 out[i] = int(res["argmax"][j])
             elif j in asked:
-                out[i] = res["logits"][asked.index(j)][None, :].repeat(len(want[i]), axis=0)
+                at = asked.index(j)
+                row = res["logits"][at:at + 1]           # (its own row: nothing is copied for one place)
+                out[i] = row if len(want[i]) == 1 else row.repeat(len(want[i]), axis=0)
             else:
                 out[i] = np.empty((0, m.vocab), np.float32)
 
@@ -128,7 +130,7 @@ class Engine:
             return int(res["argmax"][0])
         if not parts:
             return np.empty((0, m.vocab), np.float32)
-        rows = np.concatenate(parts)
+        rows = parts[0] if len(parts) == 1 else np.concatenate(parts)
         return rows if order == list(want) else rows[[order.index(w) for w in want]]
 
     # ---- scheduling
