@@ -4,6 +4,8 @@
 // of the mixed stack's F32 models.
 #include <math.h>
 
+#include <algorithm>
+
 #include "gemv.cuh"
 #include "warp_reduce.cuh"
 
@@ -25,14 +27,14 @@ __device__ __forceinline__ float4 ldg_stream(const float *p)
 // ---- the GEMV pair ---------------------------------------------------------
 //
 // y[r][n] = sum_k W[n][k] * x[r][k], optionally with RMSNorm fused on x, and a
-// residual add or SiLU(gate)*up on the way out.  Two kernels, one arithmetic:
+// residual add or SiLU(gate)*up on the way out.  Three kernels, one arithmetic:
 // K is cut into four quarters; inside a quarter lane l takes the 16-byte
 // vectors l, l+32, ... in ascending order with fused multiply-adds, starting
 // from zero; lane l then adds its four quarter sums in order; the 32 lane sums
 // are added by the xor butterfly (offsets 16, 8, 4, 2, 1).  The fused norm
 // multiplies x by the norm weight first and the finished sum by
 // 1/sqrt(mean(x^2)+eps) last, the sum of squares following the same quarter /
-// lane / butterfly order.  Because both kernels compute every output by exactly
+// lane / butterfly order.  Because all kernels compute every output by exactly
 // this recipe, a row's bits do not depend on how many rows share the call or on
 // which kernel served it.
 //
@@ -41,7 +43,8 @@ __device__ __forceinline__ float4 ldg_stream(const float *p)
 //     flight at once and nothing is staged; x comes straight from L2.  With few
 //     rows the weights are all the traffic, and one warp per weight row would
 //     leave most of the device idle on a narrow output (1024 rows = 7 warps/SM).
-//   gemv_rows_kernel (up to 16 rows per CTA): each warp owns NW weight rows
+//   gemv_batch_kernel (5 to 16 activation rows): the same split, with the activations resident in shared memory.
+//   gemv_rows_kernel (more rows, or rows too long to be resident; up to 16 rows per CTA): each warp owns NW weight rows
 //     and walks the four quarters itself; the activation rows of the current
 //     piece of a quarter sit in shared memory for all four warps, so x costs
 //     RG/(4*NW) of the weight bytes instead of RG/C.
@@ -217,6 +220,182 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_splitk_kernel(const GemvPar
     }
 }
 
+// The same recipe for five to sixteen rows, with the activations resident.  16 rows of the Qwen3-0.6B shape, us per launch: o and
+// down projections 32 -> 10.4, gate / up 47 -> 23, q / k / v 27 -> 16, head 446 -> 215; a step 7.75 -> 5.07 ms.
+//  What bounded gemv_rows_kernel was latency:
+// every 512 values of x were staged between two block-wide barriers, with two weight vectors in flight per lane (16 rows,
+// 1024 x 3072: 32 us where HBM takes 1.9).  Here a CTA keeps RG rows of x in shared memory for good and walks tiles of
+// 4 groups x 4 weight rows; a group's four warps take one quarter of K each, as in gemv_splitk_kernel, so that narrow
+// outputs fill the device too, and no barrier stands between a warp's loads.  Row groups beyond RG rows are other CTAs
+// that walk the same tiles at the same time: their weights come from L2.
+// x lies as pairs of rows (two K-values of rows 2j and 2j + 1 to 16 bytes), so that one packed fused multiply-add serves
+// two rows; shared memory is read RG * 4 bytes per four weights of each of four rows: at most 7 us per 16 million weights
+// of 16 rows, under the 9.6 that HBM takes.
+constexpr int kBatchThreads = 512, kBatchGroups = 4, kBatchC = 4;
+
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint64_t &acc, uint64_t a, uint64_t b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+template <int RG> constexpr size_t batch_smem(uint32_t k) { return (size_t)RG * k * 4 + (size_t)kBatchGroups * 4 * kBatchC * RG * 128; }
+
+template <int RG>
+__global__ void __launch_bounds__(kBatchThreads, 1) gemv_batch_kernel(const GemvParams p, uint32_t tiles, uint32_t row_groups)
+{
+    constexpr int C = kBatchC, J = RG / 2, kVecs = 2;        // weight rows of a warp, row pairs, vectors in flight
+    extern __shared__ float4 xs[];                            // [J][2][vec], then the quarters' sums
+    __shared__ float inv_rms[RG];
+    pdl_trigger();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, group = warp >> 2, quarter = warp & 3;
+    const KQuarters kq(p.k);
+    float *parts = reinterpret_cast<float *>(xs + (size_t)RG * kq.vec);
+    const uint32_t r0 = (blockIdx.x % row_groups) * RG;       // (the grid is a multiple of row_groups)
+    const uint32_t units = tiles * row_groups, v_lo = kq.lo(quarter) + lane, v_hi = kq.hi(quarter);
+
+    const float *wrow[C];
+    uint32_t s = 0, n0 = 0;
+    auto find = [&](uint32_t unit) {
+        uint32_t cta = unit / row_groups;
+        s = 0;
+        if (!p.swiglu) {
+            while (s + 1 < p.n_seg && cta >= p.cta_end[s]) ++s;
+            if (s > 0) cta -= p.cta_end[s - 1];
+        }
+        n0 = (cta * kBatchGroups + group) * (p.swiglu ? C / 2 : C);
+        weight_rows<C>(p, p.seg[s], n0, wrow);
+    };
+    float4 w[kVecs][C];
+    auto load = [&](uint32_t v) {
+#pragma unroll
+        for (int u = 0; u < kVecs; ++u)
+            if (v + 32 * u < v_hi) {
+#pragma unroll
+                for (int c = 0; c < C; ++c) w[u][c] = ldg_stream(wrow[c] + 4 * (v + 32 * u));
+            }
+    };
+    find(blockIdx.x);
+    load(v_lo);                                               // weights need no kernel before this one
+    pdl_wait();
+
+    // x (times the norm weight) into shared memory: a warp per row pair and quarter, which also has the quarter's lane
+    // sums of squares in the recipe's order
+    if (warp < 4 * J) {
+        const int j = warp >> 2;
+        const float *xa = p.x + (size_t)(r0 + 2 * j) * p.x_stride, *xb = xa + p.x_stride;
+        const bool a_in = r0 + 2 * j < p.rows, b_in = r0 + 2 * j + 1 < p.rows;
+        float sa = 0.f, sb = 0.f;
+#pragma unroll 4
+        for (uint32_t v = v_lo; v < v_hi; v += 32) {
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+            if (a_in) a = *reinterpret_cast<const float4 *>(xa + 4 * v);
+            if (b_in) b = *reinterpret_cast<const float4 *>(xb + 4 * v);
+            if (p.norm_w) {
+                const float4 nw = *reinterpret_cast<const float4 *>(p.norm_w + 4 * v);
+                sa = sumsq4(sa, a);
+                sb = sumsq4(sb, b);
+                a = mul4(a, nw);
+                b = mul4(b, nw);
+            }
+            xs[(size_t)(2 * j) * kq.vec + v] = make_float4(a.x, b.x, a.y, b.y);
+            xs[(size_t)(2 * j + 1) * kq.vec + v] = make_float4(a.z, b.z, a.w, b.w);
+        }
+        parts[((2 * j) * 4 + quarter) * 32 + lane] = sa;
+        parts[((2 * j + 1) * 4 + quarter) * 32 + lane] = sb;
+    }
+    __syncthreads();
+    if (p.norm_w && warp < RG) {
+        float t = parts[(warp * 4) * 32 + lane];
+#pragma unroll
+        for (int q = 1; q < 4; ++q) t = __fadd_rn(t, parts[(warp * 4 + q) * 32 + lane]);
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) t = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
+        if (lane == 0) inv_rms[warp] = inv_rms_of(t, p.k, p.eps);
+    }
+    __syncthreads();
+
+    float *mine = parts + (size_t)group * 4 * C * RG * 32;    // this group's [quarter][c][r][lane]
+    for (uint32_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        uint64_t acc[C][J];
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int j = 0; j < J; ++j) acc[c][j] = 0;
+        const uint32_t seg_at = s, n_at = n0;
+        for (uint32_t v = v_lo; v < v_hi; v += 32 * kVecs) {
+#pragma unroll
+            for (int u = 0; u < kVecs; ++u) {
+                const uint32_t at = v + 32 * u;
+                if (at >= v_hi) break;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint64_t w0[C], w1[C];
+#pragma unroll
+                    for (int c = 0; c < C; ++c) {
+                        w0[c] = h ? pack2(w[u][c].z, w[u][c].z) : pack2(w[u][c].x, w[u][c].x);
+                        w1[c] = h ? pack2(w[u][c].w, w[u][c].w) : pack2(w[u][c].y, w[u][c].y);
+                    }
+#pragma unroll
+                    for (int j = 0; j < J; ++j) {
+                        const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(&xs[(size_t)(2 * j + h) * kq.vec + at]);
+#pragma unroll
+                        for (int c = 0; c < C; ++c) fma2(acc[c][j], w0[c], x.x);
+#pragma unroll
+                        for (int c = 0; c < C; ++c) fma2(acc[c][j], w1[c], x.y);
+                    }
+                }
+            }
+            if (v + 32 * kVecs < v_hi) load(v + 32 * kVecs);
+        }
+        if (unit + gridDim.x < units) {                       // the next tile's first vectors, ahead of this one's reduction
+            find(unit + gridDim.x);
+            load(v_lo);
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                float *to = mine + (((size_t)quarter * C + c) * RG + 2 * j) * 32 + lane;
+                to[0] = __uint_as_float((uint32_t)acc[c][j]);
+                to[32] = __uint_as_float((uint32_t)(acc[c][j] >> 32));
+            }
+        asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");
+        // RG of the C * RG sums per warp: one weight row, or (swiglu) half the rows of a gate row and its up row
+        float v[RG];
+#pragma unroll
+        for (int i = 0; i < RG; ++i) {
+            const int c = !p.swiglu ? quarter : (quarter >> 1) + (i < RG / 2 ? 0 : C / 2);
+            const int r = !p.swiglu ? i : (quarter & 1) * (RG / 2) + i % (RG / 2);
+            const float *from = mine + (size_t)(c * RG + r) * 32 + lane;
+            v[i] = from[0];
+#pragma unroll
+            for (int q = 1; q < 4; ++q) v[i] = __fadd_rn(v[i], from[(size_t)q * C * RG * 32]);
+        }
+        const uint32_t at = warp_reduce_many<RG>(v, lane);
+        const GemvSeg seg = p.seg[seg_at];
+        if (!p.swiglu) {
+            const uint32_t n = n_at + quarter, row = r0 + at;
+            if (reduce_writer<RG>(lane) && n < seg.n && row < p.rows)
+                seg.out[(size_t)row * seg.out_stride + n] =
+                    finish(p, seg_at, n, row, __fmul_rn(v[0], p.norm_w ? inv_rms[at] : 1.0f));
+        } else {
+            const float up = __shfl_xor_sync(0xffffffffu, v[0], 16);      // (the index's highest bit is lane bit 4)
+            const uint32_t n = n_at + (quarter >> 1), r = (quarter & 1) * (RG / 2) + at, row = r0 + r;
+            if (reduce_writer<RG>(lane) && at < (uint32_t)RG / 2 && n < seg.n && row < p.rows) {
+                const float inv = p.norm_w ? inv_rms[r] : 1.0f;
+                seg.out[(size_t)row * seg.out_stride + n] = silu_mul(__fmul_rn(v[0], inv), __fmul_rn(up, inv));
+            }
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");   // the sums have been read
+    }
+}
+
 // RG: activation rows per CTA (row group); NW: weight rows per warp.
 template <int RG, int NW>
 __global__ void __launch_bounds__(kGemvThreads) gemv_rows_kernel(const GemvParams p)
@@ -375,11 +554,7 @@ void launch_splitk(const GemvParams &p, uint32_t ctas, cudaStream_t st)
 template <int NW>
 void launch_gemv_rg(const GemvParams &p, uint32_t ctas, cudaStream_t st)
 {
-    const uint32_t r = p.rows;
-    if (r == 1) launch_gemv_t<1, NW>(p, ctas, st);
-    else if (r == 2) launch_gemv_t<2, NW>(p, ctas, st);
-    else if (r <= 4) launch_gemv_t<4, NW>(p, ctas, st);
-    else if (r <= 8) launch_gemv_t<8, NW>(p, ctas, st);
+    if (p.rows <= 8) launch_gemv_t<8, NW>(p, ctas, st);
     else launch_gemv_t<16, NW>(p, ctas, st);
 }
 
@@ -394,6 +569,35 @@ int weight_rows_per_warp(uint32_t n_total)
 
 
 constexpr uint32_t kSplitKRowsMax = 4;
+constexpr size_t kSmemMax = 232448 - 1024;               // dynamic shared memory beside the kernel's own
+
+// CTAs and running ends of the segments for tiles of `cols` output columns
+uint32_t count_tiles(GemvParams &p, uint32_t cols)
+{
+    if (p.swiglu) return (p.seg[0].n + cols - 1) / cols;
+    uint32_t ctas = 0;
+    for (uint32_t s = 0; s < p.n_seg; ++s) {
+        ctas += (p.seg[s].n + cols - 1) / cols;
+        p.cta_end[s] = ctas;
+    }
+    return ctas;
+}
+
+template <int RG>
+int launch_batch(wr_cuda_ctx *ctx, GemvParams &p)
+{
+    constexpr uint32_t flag = RG == 8 ? 1u << 19 : 1u << 20;
+    if (!(ctx->attr_flags & flag)) {
+        WR_CUDA_TRY(cudaFuncSetAttribute(gemv_batch_kernel<RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+        ctx->attr_flags |= flag;
+    }
+    const uint32_t tiles = count_tiles(p, kBatchGroups * (p.swiglu ? kBatchC / 2 : kBatchC));
+    const uint32_t row_groups = (p.rows + RG - 1) / RG, most = std::max(1u, (uint32_t)ctx->sm_count / row_groups);
+    WR_CUDA_TRY(wr_launch_pdl(gemv_batch_kernel<RG>, dim3(std::min(tiles, most) * row_groups), dim3(kBatchThreads),
+                              batch_smem<RG>(p.k), ctx->stream, p, tiles, row_groups));
+    WR_CUDA_TRY(cudaGetLastError());
+    return WR_CUDA_OK;
+}
 
 }  // namespace
 
@@ -402,32 +606,19 @@ int wr_gemv_launch(wr_cuda_ctx *ctx, GemvParams &p, uint32_t n_total_for_width)
     if (p.rows <= kSplitKRowsMax) {
         // weight rows per CTA: 2 for narrow outputs (more CTAs), 4 otherwise
         const int c = (p.swiglu || n_total_for_width >= 4096) ? 4 : 2;
-        const uint32_t cols_per_cta = p.swiglu ? (uint32_t)c / 2 : (uint32_t)c;
-        uint32_t ctas = 0;
-        if (p.swiglu) {
-            ctas = (p.seg[0].n + cols_per_cta - 1) / cols_per_cta;
-        } else {
-            for (uint32_t s = 0; s < p.n_seg; ++s) {
-                ctas += (p.seg[s].n + cols_per_cta - 1) / cols_per_cta;
-                p.cta_end[s] = ctas;
-            }
-        }
+        const uint32_t ctas = count_tiles(p, p.swiglu ? (uint32_t)c / 2 : (uint32_t)c);
         if (c == 4) launch_splitk<4>(p, ctas, ctx->stream);
         else launch_splitk<2>(p, ctas, ctx->stream);
         WR_CUDA_TRY(cudaGetLastError());
         return WR_CUDA_OK;
     }
-    const int nw = p.swiglu ? 2 : weight_rows_per_warp(n_total_for_width);
-    const uint32_t cols_per_cta = (p.swiglu ? 1u : (uint32_t)nw) * kGemvWarps;
-    uint32_t ctas = 0;
-    if (p.swiglu) {
-        ctas = (p.seg[0].n + cols_per_cta - 1) / cols_per_cta;
-    } else {
-        for (uint32_t s = 0; s < p.n_seg; ++s) {
-            ctas += (p.seg[s].n + cols_per_cta - 1) / cols_per_cta;
-            p.cta_end[s] = ctas;
-        }
+    // up to a decode batch: activations resident, eight rows to a CTA, or four where eight are too long
+    if (p.rows <= WR_CUDA_BATCH_MAX) {
+        if (batch_smem<8>(p.k) <= kSmemMax) return launch_batch<8>(ctx, p);
+        if (batch_smem<4>(p.k) <= kSmemMax) return launch_batch<4>(ctx, p);
     }
+    const int nw = p.swiglu ? 2 : weight_rows_per_warp(n_total_for_width);
+    const uint32_t ctas = count_tiles(p, (p.swiglu ? 1u : (uint32_t)nw) * kGemvWarps);
     cudaStream_t st = ctx->stream;
     if (nw == 4) launch_gemv_rg<4>(p, ctas, st);
     else if (nw == 2) launch_gemv_rg<2>(p, ctas, st);
