@@ -215,7 +215,14 @@ int wr_append_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
                      const uint32_t *positions, uint32_t n_tokens, const float *dk,
                      const float *dv, float *dq, uint32_t n_q_heads, float theta_base,
                      uint32_t n_rot_pairs, uint32_t flags,
-                     const float *dq_in /* null: rotate dq in place */);
+                     const float *dq_in /* null: rotate dq in place */, const struct wr_append_extra *extra = nullptr);
+// What the append of a prompt's rows (head_dim 128, rows 16-byte aligned) can do on the way: RMSNorm of every Q and K
+// head first, and the rotated queries as F16 rows elsewhere (dq then stays as it is).
+struct wr_append_extra {
+    const float *q_norm, *k_norm;    // or both null
+    float eps;
+    __half *q16;
+};
 
 // One-kernel layer-step for short contexts (attn_step_small.cu): QK-norm, RoPE, append and the
 // new token's attention, for sessions of head_dim 128 with at most WR_STEP_SMALL_MAX_KEYS keys.
