@@ -1,0 +1,103 @@
+"""GPU: the dense stack's products for more rows than a decode batch (gemm_f32.cu), against float64.
+
+One layer; the attention rows that the call reports (attn_tap_out) are the fixed point in the middle:
+    hidden_out = embed + attn @ wo^T + FFN(RMSNorm(.))
+checks the split of plain and normed rows, the gate / up pairs and the sums in parts, and the V rows that reach the
+cache check the three-segment product (to one F16 step: the cache truncates).
+
+Tolerance (2-norm): each product sees both operands within 2^-24 and drops lo lo (2^-24 at most); 64 K-values add up in
+the tensor core, at most 12 additions that may each lose a unit of 2^-23, and the sums of 64 are added in F32.  That is
+under 16 * 2^-23 = 1.9e-6 for a product, and the rows pass through three of them; SiLU's slope is at most 1.1.
+"""
+import numpy as np
+import pytest
+
+import _gen
+from test_gpu_model_glue import _after_attention, _model, _rms, _weights
+
+pytestmark = pytest.mark.gpu
+REL = 3 * 1.1 * 16 * 2.0 ** -23
+
+SHAPES = [  # rows, hidden, q heads, kv heads, ffn
+    (17, 132, 2, 1, 20),              # nothing aligns: one K block and a bit, eight-row groups half full
+    (128, 256, 4, 2, 520), (129, 256, 4, 2, 524),
+    (300, 1024, 8, 4, 1536),          # parts of K in both sums, several tiles
+    (257, 2052, 16, 8, 4100),         # tiles of 256 columns, K beyond a row's kept values
+    (40, 512, 10, 2, 2052),           # short prompt, four parts
+]
+
+
+def _run(shape, rows, w, max_rows, tokens):
+    import wayruntime_b200 as wr
+    ctx = wr.Context(0)
+    dm = _model(ctx, w, shape, max_rows=max_rows)
+    kv = ctx.kv_create(1, shape["n_kv_heads"], 128, rows)
+    res = dm.forward(dm.FWD_PREFILL, [kv], [0], tokens, hidden=True, attn_tap=True)
+    v = kv.read_rows(0, 1, 0, rows).reshape(rows, -1).view(np.float16).astype(np.float64)
+    kv.close()
+    dm.close()
+    ctx.close()
+    return res, v
+
+
+def _check(res, v, w, tokens):
+    emb = w["embed"][tokens]
+    want = _after_attention(w, emb, res["attn"][0]) - emb
+    got = res["hidden"].astype(np.float64) - emb
+    assert np.linalg.norm(got - want) <= REL * (np.linalg.norm(want) + np.linalg.norm(emb))
+    want = _rms(emb, w["l0.attn_norm"]) @ w["l0.wv"].astype(np.float64).T
+    assert np.abs(v - want).max() <= 2.0 ** -10 * np.abs(want).max() * (1 + 1e-3)
+
+
+@pytest.mark.parametrize("rows,hidden,n_q,n_kv,ffn", SHAPES)
+def test_rows_match_float64(rows, hidden, n_q, n_kv, ffn):
+    shape = dict(n_layers=1, hidden=hidden, n_q_heads=n_q, n_kv_heads=n_kv, head_dim=128, vocab=515, ffn=ffn)
+    w = _weights(shape, 1200 + rows)
+    tokens = [(29 * r + 3) % shape["vocab"] for r in range(rows)]
+    res, v = _run(shape, rows, w, max(rows, 64), tokens)
+    _check(res, v, w, tokens)
+
+
+def test_rows_of_very_different_scale_keep_their_precision():
+    """Weight rows from 1e-18 to 1e9, a row of zeros, large values beside small ones, a channel that the next weight undoes:
+    every column of the result by its own norm."""
+    shape = dict(n_layers=1, hidden=256, n_q_heads=4, n_kv_heads=2, head_dim=128, vocab=64, ffn=256)
+    w = _weights(shape, 1300, tied=False)
+    for name in ("l0.w_gate", "l0.w_up", "l0.wv"):
+        w[name][3] *= 1e-18
+        w[name][5] = 0.0
+        w[name][7, 1] = 64.0
+    w["l0.w_down"][9] *= 1e9
+    w["l0.wo"][11] *= 1e-30
+    w["l0.w_up"][13] *= 1024.0
+    w["l0.w_down"][:, 13] /= 1024.0
+    w["embed"][8] *= 1e-3
+    tokens = [r % 64 for r in range(33)]
+    res, v = _run(shape, 33, w, 64, tokens)
+    emb = w["embed"][tokens]
+    want = _after_attention(w, emb, res["attn"][0]) - emb
+    err = np.linalg.norm(res["hidden"] - emb - want, axis=0)
+    # (a column's sums are its terms' root sum of squares or less, the bound is by their size: a factor of 4)
+    assert (err <= 4 * REL * (np.linalg.norm(want, axis=0) + np.linalg.norm(emb, axis=0))).all()
+
+
+def test_a_row_with_an_infinity_ends_not_finite_and_leaves_the_rows_before_it():
+    """(The attention kernel masks by a weight of zero, so rows of the same 128-row tile are not finite either.)"""
+    shape = dict(n_layers=1, hidden=256, n_q_heads=4, n_kv_heads=2, head_dim=128, vocab=64, ffn=260)
+    w = _weights(shape, 1301, tied=False)
+    clean = [1 + r % 60 for r in range(150)]
+    good, _ = _run(shape, 150, w, 256, clean)
+    w["embed"][0, 5] = np.inf
+    bad, _ = _run(shape, 150, w, 256, clean[:149] + [0])
+    assert not np.isfinite(bad["hidden"][149]).any()
+    assert np.array_equal(bad["hidden"][:128], good["hidden"][:128])
+
+
+def test_a_rows_bits_do_not_depend_on_how_many_follow():
+    shape = dict(n_layers=1, hidden=1024, n_q_heads=8, n_kv_heads=4, head_dim=128, vocab=300, ffn=1024)
+    w = _weights(shape, 1302)
+    tokens = [(7 * r + 1) % 300 for r in range(400)]
+    many, _ = _run(shape, 400, w, 512, tokens)
+    few, _ = _run(shape, 140, w, 512, tokens[:140])
+    assert np.array_equal(many["attn"][0][:128], few["attn"][0][:128])
+    assert np.array_equal(many["hidden"][:128], few["hidden"][:128])

@@ -1,6 +1,7 @@
 // model.cuh — wr_cuda_model: the F32 layer stack of model_glue.cu or the mixed stack of model_mixed.cu.
 #pragma once
 
+#include "gemm_f32.cuh"
 #include "wr_internal.cuh"
 
 struct wr_cuda_layer_dev {
@@ -24,6 +25,12 @@ struct wr_cuda_model {
     float *normed = nullptr, *logits = nullptr;
     uint32_t *tokens = nullptr, *best = nullptr, *part_i = nullptr;
     float *part_v = nullptr;             // arg-max partials [16][kArgmaxParts]
+    // prompts on the tensor cores (gemm_f32.cuh): one layer's weights and one product's input, split, and the parts of
+    // a product that adds to the residual; null when max_rows is no more than a decode batch, or memory did not suffice
+    char *prompt = nullptr;
+    wr_split_weight split[4];            // q | k | v, o, gate / up, down (blocks and unscale; n and k per layer)
+    __half *split_rows = nullptr;
+    float *row_scale = nullptr, *parts = nullptr;
     uint32_t *h_tokens = nullptr;        // pinned: token ids in, arg-max ids out
     uint32_t ffn_max = 0;
     uint64_t launches = 0;

@@ -26,8 +26,11 @@
 #include <math.h>
 #include <stdlib.h>
 
+#include <algorithm>
 #include <chrono>
 
+#include "gemm_bf16.cuh"
+#include "gemm_f32.cuh"
 #include "gemv.cuh"
 #include "model.cuh"
 #include "wr_internal.cuh"
@@ -171,6 +174,108 @@ int gemv(wr_cuda_model *m, GemvParams &p, uint32_t n_total_for_width)
 
 size_t up256(size_t n) { return (n + 255u) & ~(size_t)255u; }
 
+// Scratch of the prompt path.  A model that cannot have it keeps the GEMV for prompts too.
+void take_prompt_scratch(wr_cuda_model *m)
+{
+    if (m->max_rows <= WR_CUDA_BATCH_MAX) return;
+    const uint32_t nq = m->n_q * m->hd, nkv = m->n_kv * m->hd, gate_up = (m->ffn_max + 7u) / 8u * 16u;
+    const uint32_t n[4] = {nq + 2 * nkv, m->hidden, gate_up, m->hidden}, k[4] = {m->hidden, nq, m->hidden, m->ffn_max};
+    const size_t R = m->max_rows, widest = std::max({m->hidden, nq, m->ffn_max});
+    size_t parts = 1, total = 0;
+    for (int i = 0; i < 4; ++i) total += up256(wr_split_weight_bytes(n[i], k[i])) + up256((size_t)n[i] * 4);
+    for (const wr_cuda_layer_dev &l : m->layers)
+        parts = std::max<size_t>({parts, wr_f32_gemm_k_parts(m->hidden, nq), wr_f32_gemm_k_parts(m->hidden, l.ffn)});
+    const size_t rows = up256(2 * R * ((widest + 7) & ~(size_t)7) * 2), sums = up256(parts * R * m->hidden * 4);
+    total += rows + up256(R * 4) + sums;
+    if (cudaMalloc((void **)&m->prompt, total) != cudaSuccess) {
+        (void)cudaGetLastError();
+        m->prompt = nullptr;
+        return;
+    }
+    m->slab_bytes += total;
+    char *cur = m->prompt;
+    for (int i = 0; i < 4; ++i) {
+        m->split[i].blocks = cur;
+        cur += up256(wr_split_weight_bytes(n[i], k[i]));
+        m->split[i].unscale = reinterpret_cast<float *>(cur);
+        cur += up256((size_t)n[i] * 4);
+    }
+    m->split_rows = reinterpret_cast<__half *>(cur);
+    cur += rows;
+    m->row_scale = reinterpret_cast<float *>(cur);
+    cur += up256(R * 4);
+    m->parts = reinterpret_cast<float *>(cur);
+}
+
+// Split rows of x (the residual takes the parts of the product before first), and their tensor map.
+int split_rows(wr_cuda_model *m, CUtensorMap *map, float *x, uint32_t x_stride, uint32_t k, uint32_t rows,
+               uint32_t n_parts, const float *norm_w)
+{
+    wr_split_rows_args a{};
+    a.x = x; a.x_stride = x_stride; a.k = k; a.rows = rows;
+    a.parts = n_parts ? m->parts : nullptr; a.n_parts = n_parts;
+    a.norm_w = norm_w; a.eps = m->eps;
+    a.out = map ? m->split_rows : nullptr; a.ld = (k + 7u) & ~7u; a.pad = rows;
+    a.row_scale = m->row_scale;
+    ++m->launches;
+    const int rc = wr_split_rows_launch(m->ctx, a);
+    return rc != WR_CUDA_OK || !map ? rc : wr_gemm_map_rows(map, m->split_rows, 2 * rows, k, a.ld);
+}
+
+// The products of a layer for the rows of a prompt: before (q, k, v) and after (o, feed-forward) attention.  A product
+// that adds to the residual leaves its sums in m->parts; whoever reads the residual next adds them: *n_parts.
+int prompt_before(wr_cuda_model *m, const wr_cuda_layer_dev &l, uint32_t rows, uint32_t *n_parts)
+{
+    const uint32_t hid = m->hidden, nq = m->n_q * m->hd, nkv = m->n_kv * m->hd;
+    auto weight = [&](int i, uint32_t n, uint32_t k) {
+        wr_split_weight w = m->split[i];
+        w.n = n;
+        w.k = k;
+        return w;
+    };
+    const wr_split_source list[4] = {
+        {weight(0, nq + 2 * nkv, hid), {l.wq, l.wk, l.wv}, {nq, nkv, nkv}, 0},
+        {weight(1, hid, nq), {l.wo, nullptr, nullptr}, {hid, 0, 0}, 0},
+        {weight(2, (l.ffn + 7u) / 8u * 16u, hid), {l.w_gate, l.w_up, nullptr}, {l.ffn, l.ffn, 0}, 1},
+        {weight(3, hid, l.ffn), {l.w_down, nullptr, nullptr}, {hid, 0, 0}, 0}};
+    int rc = wr_split_weights_launch(m->ctx, list, 4);
+    if (rc != WR_CUDA_OK) return rc;
+    for (int i = 0; i < 4; ++i) m->split[i] = list[i].to;
+    CUtensorMap map;
+    rc = split_rows(m, &map, m->resid, hid, hid, rows, *n_parts, l.attn_norm);
+    if (rc != WR_CUDA_OK) return rc;
+    *n_parts = 0;
+    wr_f32_gemm_args a{};
+    a.m = a.pad = rows; a.row_scale = m->row_scale; a.k_parts = 1;
+    a.seg[0] = {m->q, nq, nq}; a.seg[1] = {m->k, nkv, nkv}; a.seg[2] = {m->v, nkv, nkv}; a.n_seg = 3;
+    m->launches += 2;
+    return wr_f32_gemm_launch(m->ctx, map, m->split[0], a);
+}
+
+int prompt_after(wr_cuda_model *m, const wr_cuda_layer_dev &l, uint32_t rows, uint32_t *n_parts)
+{
+    const uint32_t hid = m->hidden, nq = m->n_q * m->hd;
+    CUtensorMap map;
+    auto to_residual = [&](const wr_split_weight &w) {
+        wr_f32_gemm_args a{};
+        a.m = a.pad = rows; a.row_scale = m->row_scale; a.k_parts = wr_f32_gemm_k_parts(w.n, w.k);
+        a.seg[0] = {m->parts, hid, hid}; a.n_seg = 1;
+        *n_parts = a.k_parts;
+        return wr_f32_gemm_launch(m->ctx, map, w, a);
+    };
+    m->launches += 3;
+    int rc = split_rows(m, &map, m->attn, nq, nq, rows, 0, nullptr);
+    if (rc != WR_CUDA_OK || (rc = to_residual(m->split[1])) != WR_CUDA_OK) return rc;
+    rc = split_rows(m, &map, m->resid, hid, hid, rows, *n_parts, l.ffn_norm);
+    if (rc != WR_CUDA_OK) return rc;
+    wr_f32_gemm_args a{};
+    a.m = a.pad = rows; a.row_scale = m->row_scale; a.k_parts = 1;
+    a.seg[0] = {m->gate, l.ffn, m->ffn_max}; a.n_seg = 1; a.pair = 1;
+    if ((rc = wr_f32_gemm_launch(m->ctx, map, m->split[2], a)) != WR_CUDA_OK) return rc;
+    rc = split_rows(m, &map, m->gate, m->ffn_max, l.ffn, rows, 0, nullptr);
+    return rc != WR_CUDA_OK ? rc : to_residual(m->split[3]);
+}
+
 }  // namespace
 
 extern "C" int wr_cuda_model_create(wr_cuda_ctx *ctx, const wr_cuda_model_desc *d, wr_cuda_model **out)
@@ -283,6 +388,7 @@ extern "C" int wr_cuda_model_create(wr_cuda_ctx *ctx, const wr_cuda_model_desc *
         delete m;
         return WR_CUDA_ERR_INTERNAL;
     }
+    take_prompt_scratch(m);
     *out = m;
     return WR_CUDA_OK;
 }
@@ -296,6 +402,7 @@ extern "C" void wr_cuda_model_destroy(wr_cuda_model *m)
         cudaStreamSynchronize(m->ctx->stream);
         if (m->mixed) wr_mixed_destroy(m->mixed);
         cudaFree(m->slab);
+        cudaFree(m->prompt);
         cudaFreeHost(m->h_tokens);
     }
     delete m;
@@ -368,22 +475,39 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
         ++m->launches;
         WR_CUDA_TRY(cudaGetLastError());
     }
+    // More rows than a decode batch go through the tensor cores.  The line: 17 rows are two passes of the GEMV over the
+    // weights, which take longer than splitting the weights and one product.
+    const bool wide = mode == WR_CUDA_FWD_PREFILL && n_rows > WR_CUDA_BATCH_MAX && m->prompt;
+    const bool fused = wide && m->hd == 128;
+    uint32_t n_parts = 0;
     for (uint32_t L = 0; L < m->n_layers; ++L) {
         const wr_cuda_layer_dev &l = m->layers[L];
         int rc;
         {
             std::lock_guard<std::mutex> g(ctx->lock);
-            GemvParams p{};
-            p.seg[0] = {l.wq, m->q, nq, nq};
-            p.seg[1] = {l.wk, m->k, nkv, nkv};
-            p.seg[2] = {l.wv, m->v, nkv, nkv};
-            p.n_seg = 3;
-            p.x = m->resid; p.x_stride = hid; p.k = hid; p.rows = n_rows;
-            p.norm_w = l.attn_norm; p.eps = m->eps;
-            rc = gemv(m, p, nq + 2 * nkv);
+            if (wide) {
+                rc = prompt_before(m, l, n_rows, &n_parts);
+            } else {
+                GemvParams p{};
+                p.seg[0] = {l.wq, m->q, nq, nq};
+                p.seg[1] = {l.wk, m->k, nkv, nkv};
+                p.seg[2] = {l.wv, m->v, nkv, nkv};
+                p.n_seg = 3;
+                p.x = m->resid; p.x_stride = hid; p.k = hid; p.rows = n_rows;
+                p.norm_w = l.attn_norm; p.eps = m->eps;
+                rc = gemv(m, p, nq + 2 * nkv);
+            }
             if (rc != WR_CUDA_OK) return rc;
+            if (fused) {                     // head norms, rotation, cache rows and F16 queries in one
+                rc = wr_append_validate(ctx, 1, kv, L, positions, n_rows, m->k, m->v, m->q, m->n_q, WR_CUDA_MEM_DEVICE);
+                if (rc != WR_CUDA_OK) return rc;
+                const wr_append_extra extra = {l.q_norm, l.k_norm, m->eps, m->split_rows};
+                rc = wr_append_launch(ctx, 1, kv, L, positions, n_rows, m->k, m->v, m->q, m->n_q, m->theta, m->n_rot,
+                                      WR_CUDA_APPEND_ROPE, nullptr, &extra);
+                if (rc != WR_CUDA_OK) return rc;
+            }
             const uint32_t r_lo = (mode == WR_CUDA_FWD_DECODE) ? n_short : 0;    // rows of the three-kernel path
-            if (l.q_norm && r_lo < n_rows) {
+            if (l.q_norm && r_lo < n_rows && !fused) {
                 const uint32_t n_a = (n_rows - r_lo) * m->n_q, n_b = (n_rows - r_lo) * m->n_kv;
                 head_rmsnorm_kernel<<<(n_a + n_b + 3) / 4, 128, 0, st>>>(m->q + (size_t)r_lo * nq, l.q_norm, n_a,
                                                                        m->k + (size_t)r_lo * nkv, l.k_norm, n_b,
@@ -406,11 +530,13 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
                 if (rc != WR_CUDA_OK) return rc;
             }
         } else {
-            rc = wr_cuda_kv_append(ctx, 1, kv, L, positions, n_rows, m->k, m->v, m->q, m->n_q, m->theta,
-                                   m->n_rot, WR_CUDA_APPEND_ROPE, WR_CUDA_MEM_DEVICE);
-            if (rc != WR_CUDA_OK) return rc;
-            rc = wr_cuda_attn_prefill(ctx, kv[0], L, positions[0], n_rows, m->q, WR_CUDA_F32, m->attn,
-                                      m->n_q, m->scale, 0, WR_CUDA_MEM_DEVICE);
+            if (!fused) {
+                rc = wr_cuda_kv_append(ctx, 1, kv, L, positions, n_rows, m->k, m->v, m->q, m->n_q, m->theta,
+                                       m->n_rot, WR_CUDA_APPEND_ROPE, WR_CUDA_MEM_DEVICE);
+                if (rc != WR_CUDA_OK) return rc;
+            }
+            rc = wr_cuda_attn_prefill(ctx, kv[0], L, positions[0], n_rows, fused ? (const void *)m->split_rows : m->q,
+                                      fused ? WR_CUDA_F16 : WR_CUDA_F32, m->attn, m->n_q, m->scale, 0, WR_CUDA_MEM_DEVICE);
             if (rc != WR_CUDA_OK) return rc;
         }
         {
@@ -424,6 +550,11 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
                         WR_CUDA_TRY(cudaMemcpyAsync(dst + (size_t)perm[i] * nq, m->attn + (size_t)i * nq,
                                                     (size_t)nq * 4, cudaMemcpyDeviceToHost, st));
                 }
+            }
+            if (wide) {
+                rc = prompt_after(m, l, n_rows, &n_parts);
+                if (rc != WR_CUDA_OK) return rc;
+                continue;
             }
             GemvParams p{};
             p.seg[0] = {l.wo, m->resid, hid, hid};
@@ -453,6 +584,10 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
         }
     }
     std::lock_guard<std::mutex> g(ctx->lock);
+    if (n_parts) {
+        const int rc = split_rows(m, nullptr, m->resid, hid, hid, n_rows, n_parts, nullptr);
+        if (rc != WR_CUDA_OK) return rc;
+    }
     // Device rows [o_lo, n_rows) are finished (final norm, LM head); device row i is the caller's row
     // perm[i] when the decode rows were reordered, and then every row is finished and only the asked
     // ones are copied out.
