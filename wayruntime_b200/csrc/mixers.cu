@@ -470,8 +470,19 @@ template <> struct States<1> {
 
 // NS: states a thread carries; LG: log2 of the threads that share a channel.  U tokens go through the state at a
 // time; their partial sums are then exchanged so that each of the channel's threads finishes tokens of its own.
-template <typename T, typename TO, int NS, int LG>
-__global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, const wr_scan_args a)
+//
+// A sequence is one chain, and with one state per thread the instructions around a state's four (addresses, loads, the sums'
+// exchange) are most of the work.  A long portion is therefore cut into pieces of kScanPiece tokens, which gives enough threads
+// for four states each: SCAN_ENDS works out what every piece but the last leaves of nothing, and the sum of its step
+// sizes; SCAN_PIECE starts every piece from the state before the portion, brought forward over the pieces before it
+// (2^(a2 * their step sizes) times it, plus what they left).  The decays are worked out twice.
+// 2048 tokens x 4096 channels x 16 states, us alone: 147 -> 45 + 86; a prompt through four such layers and four of attention
+// (where the clock is lower): 4135 -> 3589.
+enum { SCAN_WHOLE = 0, SCAN_ENDS = 1, SCAN_PIECE = 2 };
+constexpr uint32_t kScanPiece = 256;
+
+template <typename T, typename TO, int NS, int LG, int MODE>
+__global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, const wr_scan_args a, float *ends, float *steps)
 {
     constexpr uint32_t TPC = 1u << LG, CB = kScanThreads >> LG, HELD = NS * TPC;            // channels per block, states held
     constexpr uint32_t BST = (HELD + 3) & ~3u;                                              // a token's B (or C) in shared memory
@@ -496,12 +507,22 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, co
     const float D = c < a.inner ? a.d[c] : 0.f;
     pdl_wait();
     const wr_seq_dev s = rw.seqs[seq];
-    const uint32_t row0 = row0_of(rw, seq), n_tok = s.n;
+    const uint32_t piece = MODE == SCAN_WHOLE ? 0u : blockIdx.z, tok0 = piece * kScanPiece;
+    const uint32_t row0 = row0_of(rw, seq) + tok0, n_tok = MODE == SCAN_WHOLE ? s.n : min(s.n - tok0, kScanPiece);
     const float *st_in = reinterpret_cast<const float *>(s.st_in + a.state_off);
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
         const uint32_t n = part * NS + j;
-        S.set(j, (!s.fresh && c < a.inner && n < a.state) ? st_in[(size_t)c * a.state + n] : 0.f);
+        S.set(j, (MODE != SCAN_ENDS && !s.fresh && c < a.inner && n < a.state) ? st_in[(size_t)c * a.state + n] : 0.f);
+    }
+    float dt_sum = 0.f;                                          // (SCAN_ENDS)
+    if (MODE == SCAN_PIECE && c < ld) {
+        States<NS> e, b;
+        for (uint32_t i = 0; i < piece; ++i) {
+            e.decay(steps[(size_t)i * ld + c], A2);
+            b.load(ends + ((size_t)i * ld + c) * HELD + part * NS);
+            S.advance(e, b);
+        }
     }
     __syncthreads();
     auto request = [&](uint32_t tile) {
@@ -512,14 +533,14 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, co
             const size_t row = row0 + t0 + t;
             const uint32_t at = (st * TILE + t) * CB + 4 * q;
             cp_async<4 * sizeof(T)>(xs + at, static_cast<const T *>(a.x) + row * a.x_ld + ch);
-            cp_async<4 * sizeof(T)>(zs + at, static_cast<const T *>(a.z) + row * a.z_ld + ch);
+            if (MODE != SCAN_ENDS) cp_async<4 * sizeof(T)>(zs + at, static_cast<const T *>(a.z) + row * a.z_ld + ch);
             cp_async<16>(dts + at, a.dt + row * ld + ch);
         }
         for (uint32_t i = tid; i < nt * bc4; i += kScanThreads) {
             const uint32_t t = i / bc4, q = i % bc4;
             const float *src = a.bc + (size_t)(row0 + t0 + t) * a.bc_ld + 4 * q;
             cp_async<16>(bs + (st * TILE + t) * BST + 4 * q, src + a.b_off);
-            cp_async<16>(cs + (st * TILE + t) * BST + 4 * q, src + a.c_off);
+            if (MODE != SCAN_ENDS) cp_async<16>(cs + (st * TILE + t) * BST + 4 * q, src + a.c_off);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -543,7 +564,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, co
                 const uint32_t t = st * TILE + t0 + i;
                 const float dt = dts[t * CB + cl], dx = dt * to_f32(xs[t * CB + cl]);
                 g.b[i].load(bs + t * BST + part * NS);
-                g.c[i].load(cs + t * BST + part * NS);
+                if (MODE != SCAN_ENDS) g.c[i].load(cs + t * BST + part * NS);
+                else dt_sum += dt;
                 g.e[i].decay(dt, A2);
                 g.b[i].scale(dx);
             }
@@ -551,7 +573,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, co
         float y[U];
         auto chain = [&](const Group &g, int i, int u) {
             S.advance(g.e[i], g.b[i]);
-            y[u] = S.dot(g.c[i]);
+            if (MODE != SCAN_ENDS) y[u] = S.dot(g.c[i]);
         };
         // the channel's threads exchange their parts of U tokens' sums and finish some tokens each
         auto finish = [&](uint32_t tb) {
@@ -595,7 +617,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, co
                 if (tb + U < TILE) fetch(ga, tb + U, All());
 #pragma unroll
                 for (int i = 0; i < NT; ++i) chain(gb, i, NT + i);
-                finish(tb);
+                if (MODE != SCAN_ENDS) finish(tb);
             }
         } else {
 #pragma unroll 1
@@ -608,15 +630,23 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, co
                         chain(ga, 0, u);
                     }
                 }
-                finish(tb);
+                if (MODE != SCAN_ENDS) finish(tb);
             }
         }
         __syncthreads();
-        for (uint32_t i = tid; i < nt * (CB / 4); i += kScanThreads) {
+        for (uint32_t i = tid; MODE != SCAN_ENDS && i < nt * (CB / 4); i += kScanThreads) {
             const uint32_t t = i / (CB / 4), q = i % (CB / 4), ch = c_base + 4 * q;
             if (ch < ld) Out<TO>(a.out, row0 + t0 + t, ld).put4(ch, load4(ys + t * CB + 4 * q));
         }
     }
+    if (MODE == SCAN_ENDS) {
+        if (c >= ld) return;
+#pragma unroll
+        for (int j = 0; j < NS; ++j) ends[((size_t)piece * ld + c) * HELD + part * NS + j] = S.get(j);
+        if (part == 0) steps[(size_t)piece * ld + c] = dt_sum;
+        return;
+    }
+    if (MODE == SCAN_PIECE && tok0 + n_tok < s.n) return;        // (the last piece leaves the state)
     float *st_out = reinterpret_cast<float *>(s.st_out + a.state_off);
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
@@ -701,21 +731,42 @@ template <typename TO> int scan_step(wr_cuda_ctx *ctx, const wr_rows &rw, const 
     return scan_step_one<TO, 5>(ctx, rw, a);                     // (128 states at most)
 }
 
-template <typename T, typename TO, int NS, int LG> int scan_one(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a)
+template <typename T, typename TO, int NS, int LG, int MODE = SCAN_WHOLE>
+int scan_one(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a, uint32_t pieces = 1, float *ends = nullptr, float *steps = nullptr)
 {
     constexpr uint32_t CB = kScanThreads >> LG, HELD = NS << LG, BST = (HELD + 3) & ~3u, TILE = HELD > 128 ? 16 : 32;
     constexpr size_t smem = (size_t)(4 * TILE * BST + 3 * TILE * CB) * 4 + (size_t)4 * TILE * CB * sizeof(T);
-    auto k = scan_kernel<T, TO, NS, LG>;
+    auto k = scan_kernel<T, TO, NS, LG, MODE>;
     if (smem > 48 * 1024)
         WR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    WR_CUDA_TRY(wr_launch_pdl(k, dim3((wr_ld(a.inner) + CB - 1) / CB, rw.n_seq), dim3(kScanThreads), smem, ctx->stream, rw, a));
+    WR_CUDA_TRY(wr_launch_pdl(k, dim3((wr_ld(a.inner) + CB - 1) / CB, rw.n_seq, pieces), dim3(kScanThreads), smem, ctx->stream, rw, a,
+                              ends, steps));
     return finish_launch(ctx);
+}
+
+template <typename T, typename TO, int LG> int scan_pieces(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a)
+{
+    const uint32_t pieces = (rw.n_rows + kScanPiece - 1) / kScanPiece;
+    const size_t held = 4u << LG, n_ends = (size_t)(pieces - 1) * wr_ld(a.inner) * held, n_steps = (size_t)(pieces - 1) * wr_ld(a.inner);
+    const int rc = wr_ctx_reserve_ws(ctx, (n_ends + n_steps) * 4, 0);
+    if (rc != WR_CUDA_OK) return rc;
+    float *ends = ctx->ws, *steps = ends + n_ends;
+    const int first = scan_one<T, TO, 4, LG, SCAN_ENDS>(ctx, rw, a, pieces - 1, ends, steps);
+    return first != WR_CUDA_OK ? first : scan_one<T, TO, 4, LG, SCAN_PIECE>(ctx, rw, a, pieces, ends, steps);
 }
 
 // One state per thread while that is what it takes to fill the device, two above; a choice by the model's sizes
 // alone, so that a session's sums are added in one order whatever the step looks like.
 template <typename T, typename TO> int scan_launch(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a)
 {
+    // The line to pieces: from three of them on the second pass over the decays is less than what four states per thread save
+    // (and the last sum of a session's state is formed piece by piece, whatever else is in the step).
+    if (!rw.decode && rw.n_seq == 1 && rw.n_rows > 2 * kScanPiece && a.state > 4 && a.state <= 32) {
+        const int rc = a.state <= 8    ? scan_pieces<T, TO, 1>(ctx, rw, a)
+                       : a.state <= 16 ? scan_pieces<T, TO, 2>(ctx, rw, a)
+                                       : scan_pieces<T, TO, 3>(ctx, rw, a);
+        if (rc != WR_CUDA_ERR_NOMEM) return rc;
+    }
     const bool few = (uint64_t)a.inner * a.state < 131072;
     if (a.state <= 1) return scan_one<T, TO, 1, 0>(ctx, rw, a);
     if (a.state <= 2) return scan_one<T, TO, 1, 1>(ctx, rw, a);
