@@ -6,6 +6,8 @@
 
 #include <algorithm>
 
+#include "gemm_bf16.cuh"
+#include "gemm_f32.cuh"
 #include "gemv.cuh"
 #include "warp_reduce.cuh"
 
@@ -601,8 +603,82 @@ int launch_batch(wr_cuda_ctx *ctx, GemvParams &p)
 
 }  // namespace
 
+namespace {
+
+// out = act(sum of the parts + bias) mul + add for one product of many rows
+__global__ void __launch_bounds__(256) finish_rows_kernel(const GemvParams p, const float *parts, uint32_t n_parts, uint32_t ld)
+{
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t row = blockIdx.y, n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= p.seg[0].n) return;
+    float y = parts[(size_t)row * ld + n];
+    for (uint32_t j = 1; j < n_parts; ++j) y = __fadd_rn(y, parts[((size_t)j * p.rows + row) * ld + n]);
+    p.seg[0].out[(size_t)row * p.seg[0].out_stride + n] = finish(p, 0, n, row, y);
+}
+
+// More rows than a decode batch: the tensor-core product of gemm_f32.cu, weights and rows split into the context's
+// workspace on the way.  17 rows are two passes of the GEMV over the weights; this is three (in, out and in again, the
+// last two in L2) whatever the rows, and the products at the tensor cores' rate.  WR_CUDA_ERR_NOMEM: no workspace.
+int launch_wide(wr_cuda_ctx *ctx, GemvParams &p)
+{
+    auto up256 = [](size_t n) { return (n + 255u) & ~(size_t)255u; };
+    uint32_t n = 0;
+    for (uint32_t s = 0; s < p.n_seg; ++s) n += p.seg[s].n;
+    bool direct = !p.bias && p.act == WR_GEMV_ACT_NONE && p.mul == 1.f && !p.add;
+    for (uint32_t s = 0; s < (p.swiglu ? 1u : p.n_seg); ++s)
+        direct = direct && !(p.seg[s].n & 3u) && !(p.seg[s].out_stride & 3u) && !((uintptr_t)p.seg[s].out & 15u);
+    if (!direct && (p.swiglu || p.n_seg > 1)) return WR_CUDA_ERR_UNSUPPORTED;
+    wr_split_source src{};
+    wr_split_weight &w = src.to;
+    w.n = p.swiglu ? (p.seg[0].n + 7u) / 8u * 16u : (n + 3u) & ~3u;
+    w.k = p.k;
+    for (uint32_t s = 0; s < p.n_seg; ++s) {
+        src.src[s] = p.seg[s].w;
+        src.n[s] = p.seg[s].n;
+    }
+    src.pair = p.swiglu;
+    const uint32_t parts = direct ? 1u : wr_f32_gemm_k_parts(w.n, w.k), ld = (p.k + 7u) & ~7u;
+    const size_t b_blocks = up256(wr_split_weight_bytes(w.n, w.k)), b_unscale = up256((size_t)w.n * 4);
+    const size_t b_rows = up256((size_t)2 * p.rows * ld * 2), b_scale = up256((size_t)p.rows * 4);
+    const size_t b_parts = direct ? 0 : (size_t)parts * p.rows * w.n * 4;
+    int rc = wr_ctx_reserve_ws(ctx, b_blocks + b_unscale + b_rows + b_scale + b_parts, 0);
+    if (rc != WR_CUDA_OK) return rc;
+    char *at = reinterpret_cast<char *>(ctx->ws);
+    w.blocks = at;
+    w.unscale = reinterpret_cast<float *>(at += b_blocks);
+    wr_split_rows_args r{};
+    r.x = const_cast<float *>(p.x); r.x_stride = p.x_stride; r.k = p.k; r.rows = p.rows;      // (no parts: x is only read)
+    r.norm_w = p.norm_w; r.eps = p.eps;
+    r.out = reinterpret_cast<__half *>(at += b_unscale); r.ld = ld; r.pad = p.rows;
+    r.row_scale = reinterpret_cast<float *>(at += b_rows);
+    float *sums = reinterpret_cast<float *>(at += b_scale);
+    CUtensorMap map;
+    if ((rc = wr_split_weights_launch(ctx, &src, 1)) != WR_CUDA_OK || (rc = wr_split_rows_launch(ctx, r)) != WR_CUDA_OK ||
+        (rc = wr_gemm_map_rows(&map, r.out, 2 * p.rows, p.k, ld)) != WR_CUDA_OK)
+        return rc;
+    wr_f32_gemm_args a{};
+    a.m = a.pad = p.rows; a.row_scale = r.row_scale; a.k_parts = parts; a.pair = p.swiglu; a.n_seg = p.swiglu ? 1u : p.n_seg;
+    if (direct)
+        for (uint32_t s = 0; s < a.n_seg; ++s) a.seg[s] = {p.seg[s].out, p.seg[s].n, p.seg[s].out_stride};
+    else
+        a.seg[0] = {sums, w.n, w.n};
+    if ((rc = wr_f32_gemm_launch(ctx, map, w, a)) != WR_CUDA_OK || direct) return rc;
+    WR_CUDA_TRY(wr_launch_pdl(finish_rows_kernel, dim3((n + 255) / 256, p.rows), dim3(256), 0, ctx->stream, p, (const float *)sums,
+                              parts, w.n));
+    ctx->launches++;
+    WR_CUDA_TRY(cudaGetLastError());
+    return WR_CUDA_OK;
+}
+
+}  // namespace
+
 int wr_gemv_launch(wr_cuda_ctx *ctx, GemvParams &p, uint32_t n_total_for_width)
 {
+    if (p.rows > WR_CUDA_BATCH_MAX && p.rows <= 65535 && !(p.x_stride & 3u) && !((uintptr_t)p.x & 15u)) {
+        const int rc = launch_wide(ctx, p);
+        if (rc != WR_CUDA_ERR_NOMEM && rc != WR_CUDA_ERR_UNSUPPORTED) return rc;
+    }
     if (p.rows <= kSplitKRowsMax) {
         // weight rows per CTA: 2 for narrow outputs (more CTAs), 4 otherwise
         const int c = (p.swiglu || n_total_for_width >= 4096) ? 4 : 2;
