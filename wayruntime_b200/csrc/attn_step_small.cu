@@ -19,22 +19,35 @@
 // softmax is the materialised form (all scores, one maximum, one sum) in F32
 // with exp from the hardware; the reference's online form differs from it by
 // float associativity only (kernels.c:1466-1470).
+#include <algorithm>
+
 #include "mathx_dev.cuh"
 #include "wr_internal.cuh"
 
 namespace {
 
-constexpr int kSmallThreads = 256;
-constexpr int kSmallWarps = kSmallThreads / 32;
+// What bounds the kernel is round trips to L2: one per 256 keys for the scores and one per 128 for the values with 256 threads.
+// A CTA has SETS times as many; sixteen groups of keys share the values as before, and each thread takes 8 / SETS dimensions, so
+// every sum runs over the same terms in the same order whatever SETS is (the longest session of the launch decides).
+// 48 CTAs, sessions of 200 to 1000 keys, 2 q heads per kv head: 34.4 -> 29.4 us.
+constexpr uint32_t kSetThreads = 256;
+__host__ __device__ constexpr uint32_t max_sets(uint32_t group) { return group > 4 ? 2u : 4u; }     // (registers)
+inline uint32_t sets_for(uint32_t n_keys, uint32_t group)
+{
+    const uint32_t sets = n_keys <= 256 ? 1u : n_keys <= 512 ? 2u : 4u;
+    return sets < max_sets(group) ? sets : max_sets(group);
+}
 constexpr uint32_t kSmallMaxKeys = WR_STEP_SMALL_MAX_KEYS;
 constexpr uint32_t kSmallMaxGroup = 8;     // q heads per kv head
 constexpr uint32_t kHd = 128;
 
 struct step_small_params {
     wr_batch_desc b;                 // b.seq_len[s] = position of the new token of session s
-    float *q;                        // [n_sess][n_q][128]: raw projections in, (normed, rotated) rows out
-    const float *k, *v;              // [n_sess][n_kv][128] raw projections
-    float *out;                      // [n_sess][n_q][128]
+    uint32_t row[WR_CUDA_BATCH_MAX]; // session s is row `row[s]` of
+    const float *q;                  // [rows][n_q][128]: raw projections
+    float *q_out;                    // (normed, rotated) rows, maybe the same buffer; or null
+    const float *k, *v;              // [rows][n_kv][128] raw projections; or null: the cache has the new row already
+    float *out;                      // [rows][n_q][128]
     const float *q_norm, *k_norm;    // [128] each, or both null
     uint32_t n_kv, n_q, n_rot;
     float eps, theta, scale;
@@ -48,9 +61,12 @@ __device__ __forceinline__ const char *row_chunk(const char *block, uint32_t tok
 
 // GM: upper bound of q heads per kv head this instantiation is unrolled for (the kernel runs its code
 // once, on a handful of warps, so code size is time: a cold instruction line costs as much as a load).
-template <int GM>
-__global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const step_small_params p)
+template <int GM, int SETS>
+__global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(const step_small_params p)
 {
+    constexpr uint32_t kSmallThreads = kSetThreads * SETS, kSmallWarps = kSmallThreads / 32;
+    constexpr uint32_t kRaw = SETS == 4 ? 8 : 16;                // 16-byte pieces of a key row in flight per thread
+
     __shared__ __align__(16) float sq[GM][kHd];                  // this kv head's q rows
     __shared__ __align__(16) float sk[kHd], sv[kHd];
     __shared__ __align__(16) __half nk[kHd], nv[kHd];            // the new row as the cache holds it
@@ -63,7 +79,8 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
     const uint32_t s = blockIdx.x / p.n_kv, kvh = blockIdx.x % p.n_kv;
     const uint32_t G = p.n_q / p.n_kv;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t pos = p.b.seq_len[s], n_keys = pos + 1;
+    const uint32_t pos = p.b.seq_len[s], n_keys = pos + 1, row = p.row[s];
+    const bool append = p.k != nullptr;
     constexpr uint32_t half = kHd / 2;
 
     // ---- what does not depend on the kernel before this one (the projections): norm weights, the
@@ -84,10 +101,10 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
     }
     pdl_wait();
     // ---- rows in
-    float *qrows = p.q + ((size_t)s * p.n_q + (size_t)kvh * G) * kHd;
-    for (uint32_t i = tid; i < G * kHd; i += kSmallThreads) sq[i / kHd][i % kHd] = qrows[i];
-    if (tid < kHd) sk[tid] = p.k[((size_t)s * p.n_kv + kvh) * kHd + tid];
-    else if (tid < 2 * kHd) sv[tid - kHd] = p.v[((size_t)s * p.n_kv + kvh) * kHd + tid - kHd];
+    const size_t q_at = ((size_t)row * p.n_q + (size_t)kvh * G) * kHd;
+    for (uint32_t i = tid; i < G * kHd; i += kSmallThreads) sq[i / kHd][i % kHd] = p.q[q_at + i];
+    if (append && tid < kHd) sk[tid] = p.k[((size_t)row * p.n_kv + kvh) * kHd + tid];
+    else if (append && tid < 2 * kHd) sv[tid - kHd] = p.v[((size_t)row * p.n_kv + kvh) * kHd + tid - kHd];
     __syncthreads();
 
     // ---- per-head RMSNorm of K and of the G q heads (one warp per vector), as head_rmsnorm_kernel
@@ -120,7 +137,7 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
 
     // ---- append: the new K / V row into its page (truncating convert), and kept for this CTA's own use;
     //      the rotated q rows go back to the caller's buffer
-    if (tid < kHd) {
+    if (append && tid < kHd) {
         char *page = const_cast<char *>(s_page[pos / kPageTokens]);
         const uint32_t tk = pos % kPageTokens, off = wr_elem_off(tk, tid, kHd);
         const uint16_t kb = wr_f32_to_f16_trunc(sk[tid]), vb = wr_f32_to_f16_trunc(sv[tid]);
@@ -129,7 +146,8 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
         nk[tid] = __ushort_as_half(kb);
         nv[tid] = __ushort_as_half(vb);
     }
-    for (uint32_t i = tid; i < G * kHd; i += kSmallThreads) qrows[i] = sq[i / kHd][i % kHd];
+    if (p.q_out)
+        for (uint32_t i = tid; i < G * kHd; i += kSmallThreads) p.q_out[q_at + i] = sq[i / kHd][i % kHd];
     __syncthreads();
 
     // ---- scores: one thread per key, all G heads at once.  The sixteen 16-byte loads of a key row are
@@ -140,15 +158,17 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
         for (uint32_t g = 0; g < (uint32_t)GM; ++g) dot[g] = 0.f;
         const char *kb = s_page[key / kPageTokens] + wr_block_off(kvh, 0, kHd);
         const uint32_t tok = key % kPageTokens;
-        uint4 raw[kHd / 8];
 #pragma unroll
-        for (uint32_t c = 0; c < kHd / 8; ++c) {
-            if (key == pos) raw[c] = *reinterpret_cast<const uint4 *>(&nk[8 * c]);
-            else raw[c] = __ldg(reinterpret_cast<const uint4 *>(row_chunk(kb, tok, c)));
+        for (uint32_t c0 = 0; c0 < kHd / 8; c0 += kRaw) {
+        uint4 raw[kRaw];
+#pragma unroll
+        for (uint32_t i = 0; i < kRaw; ++i) {
+            if (append && key == pos) raw[i] = *reinterpret_cast<const uint4 *>(&nk[8 * (c0 + i)]);
+            else raw[i] = __ldg(reinterpret_cast<const uint4 *>(row_chunk(kb, tok, c0 + i)));
         }
 #pragma unroll
-        for (uint32_t c = 0; c < kHd / 8; ++c) {
-            const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw[c]);
+        for (uint32_t c = c0; c < c0 + kRaw; ++c) {
+            const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw[c - c0]);
             float kf[8];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -167,6 +187,7 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
                     dot[g] = d;
                 }
             }
+        }
         }
 #pragma unroll
         for (uint32_t g = 0; g < (uint32_t)GM; ++g)
@@ -192,39 +213,41 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
     }
     __syncthreads();
 
-    // ---- P.V: thread = (16-byte chunk c of the row, key group kg of 16); all G heads at once
+    // ---- P.V: thread = (W dimensions of the row, key group kg of 16); all G heads at once
     {
-        const uint32_t kg = lane & 15u, c = warp * 2u + (lane >> 4);
-        float acc[(uint32_t)GM][8];
+        constexpr uint32_t W = 8 / SETS;
+        const uint32_t kg = lane & 15u, d0 = (warp * 2u + (lane >> 4)) * W;
+        float acc[(uint32_t)GM][W];
 #pragma unroll
         for (uint32_t g = 0; g < (uint32_t)GM; ++g)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
-        constexpr uint32_t kBatch = 8;               // V rows whose loads are in flight together
+            for (uint32_t i = 0; i < W; ++i) acc[g][i] = 0.f;
+        constexpr uint32_t kBatch = SETS == 4 ? 16 : 8;  // V rows whose loads are in flight together
         for (uint32_t key0 = kg; key0 < n_keys; key0 += 16 * kBatch) {
-            uint4 raw[kBatch];
+            __align__(16) uint32_t raw[kBatch][W / 2];
 #pragma unroll
             for (uint32_t u = 0; u < kBatch; ++u) {
                 const uint32_t key = key0 + 16 * u;
-                raw[u] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (uint32_t i = 0; i < W / 2; ++i) raw[u][i] = 0u;
                 if (key < n_keys) {
-                    if (key == pos) {
-                        raw[u] = *reinterpret_cast<const uint4 *>(&nv[8 * c]);
-                    } else {
-                        const char *vb = s_page[key / kPageTokens] + wr_block_off(kvh, 1, kHd);
-                        raw[u] = __ldg(reinterpret_cast<const uint4 *>(row_chunk(vb, key % kPageTokens, c)));
-                    }
+                    const char *from = reinterpret_cast<const char *>(&nv[d0]);
+                    if (!append || key != pos)
+                        from = row_chunk(s_page[key / kPageTokens] + wr_block_off(kvh, 1, kHd), key % kPageTokens, d0 / 8) +
+                               d0 % 8 * 2;
+                    if constexpr (W == 8) *reinterpret_cast<uint4 *>(raw[u]) = *reinterpret_cast<const uint4 *>(from);
+                    else if constexpr (W == 4) *reinterpret_cast<uint2 *>(raw[u]) = *reinterpret_cast<const uint2 *>(from);
+                    else raw[u][0] = *reinterpret_cast<const uint32_t *>(from);
                 }
             }
 #pragma unroll
             for (uint32_t u = 0; u < kBatch; ++u) {
                 const uint32_t key = key0 + 16 * u;
                 if (key >= n_keys) break;
-                const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw[u]);
-                float vf[8];
+                float vf[W];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 f = __half22float2(h2[i]);
+                for (uint32_t i = 0; i < W / 2; ++i) {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&raw[u][i]));
                     vf[2 * i] = f.x;
                     vf[2 * i + 1] = f.y;
                 }
@@ -233,7 +256,7 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
                     if (g < G) {
                         const float pw = sc[g][key];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) acc[g][i] = fmaf(pw, vf[i], acc[g][i]);
+                        for (uint32_t i = 0; i < W; ++i) acc[g][i] = fmaf(pw, vf[i], acc[g][i]);
                     }
                 }
             }
@@ -243,7 +266,7 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
         for (uint32_t g = 0; g < (uint32_t)GM; ++g) {
             if (g < G) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (uint32_t i = 0; i < W; ++i) {
                     float a = acc[g][i];
                     a += __shfl_xor_sync(0xffffffffu, a, 8);
                     a += __shfl_xor_sync(0xffffffffu, a, 4);
@@ -253,60 +276,72 @@ __global__ void __launch_bounds__(kSmallThreads) attn_step_small_kernel(const st
                 }
                 if (kg == 0) {
                     const float inv = s_inv_l[g];
-                    float *o = p.out + ((size_t)s * p.n_q + (size_t)kvh * G + g) * kHd + 8 * c;
-                    *reinterpret_cast<float4 *>(o) =
-                        make_float4(acc[g][0] * inv, acc[g][1] * inv, acc[g][2] * inv, acc[g][3] * inv);
-                    *reinterpret_cast<float4 *>(o + 4) =
-                        make_float4(acc[g][4] * inv, acc[g][5] * inv, acc[g][6] * inv, acc[g][7] * inv);
+                    float *o = p.out + q_at + (size_t)g * kHd + d0;
+#pragma unroll
+                    for (uint32_t i = 0; i < W; i += 2)
+                        *reinterpret_cast<float2 *>(o + i) = make_float2(acc[g][i] * inv, acc[g][i + 1] * inv);
                 }
             }
         }
     }
 }
 
-}  // namespace
-
-bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t n_q_heads, uint32_t position)
+template <int GM>
+cudaError_t launch_small(uint32_t sets, uint32_t grid, cudaStream_t st, const step_small_params &p)
 {
-    return kv->hd_at(0) == kHd && kv->n_kv_at(0) > 0 && n_q_heads % kv->n_kv_at(0) == 0 && n_q_heads / kv->n_kv_at(0) <= kSmallMaxGroup &&
-           position + 1 <= kSmallMaxKeys;
+    if (sets == 1) return wr_launch_pdl(attn_step_small_kernel<GM, 1>, dim3(grid), dim3(kSetThreads), 0, st, p);
+    if (sets == 2) return wr_launch_pdl(attn_step_small_kernel<GM, 2>, dim3(grid), dim3(2 * kSetThreads), 0, st, p);
+    if constexpr (max_sets(GM) == 4) return wr_launch_pdl(attn_step_small_kernel<GM, 4>, dim3(grid), dim3(4 * kSetThreads), 0, st, p);
+    return cudaErrorInvalidValue;
 }
 
-// Enqueue on device-resident rows.  Caller holds ctx->lock; every session must pass
-// wr_step_small_covers and wr_kv_batch_check, and positions[s] < max_ctx.
+}  // namespace
+
+bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t layer, uint32_t n_q_heads, uint32_t position)
+{
+    return kv->hd_at(layer) == kHd && kv->n_kv_at(layer) > 0 && n_q_heads % kv->n_kv_at(layer) == 0 &&
+           n_q_heads / kv->n_kv_at(layer) <= kSmallMaxGroup && position + 1 <= kSmallMaxKeys;
+}
+
+// Enqueue on rows the device can reach.  Caller holds ctx->lock; every session must pass wr_step_small_covers and
+// wr_kv_batch_check, and positions[s] < max_ctx.
 int wr_step_small_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
-                         const uint32_t *positions, float *dq, const float *dk, const float *dv, float *dout,
-                         uint32_t n_q_heads, float theta_base, uint32_t n_rot_pairs, const float *q_norm,
-                         const float *k_norm, float eps, float scale_override)
+                         const uint32_t *positions, const wr_step_small_args &a)
 {
     if (n_sess == 0 || n_sess > WR_CUDA_BATCH_MAX) return WR_CUDA_ERR_LIMIT;
     step_small_params p;
     for (uint32_t s = 0; s < n_sess; ++s) {
-        if (!wr_step_small_covers(kv[s], n_q_heads, positions[s])) return WR_CUDA_ERR_UNSUPPORTED;
+        if (!wr_step_small_covers(kv[s], layer, a.n_q_heads, positions[s])) return WR_CUDA_ERR_UNSUPPORTED;
         if (positions[s] >= kv[s]->max_ctx) return WR_CUDA_ERR_CTX_FULL;
         p.b.pages[s] = kv[s]->d_pages + (size_t)layer * kv[s]->n_pages;
         p.b.seq_len[s] = positions[s];
+        p.row[s] = a.rows ? a.rows[s] : s;
     }
     constexpr uint32_t half = kHd / 2u;
-    p.q = dq;
-    p.k = dk;
-    p.v = dv;
-    p.out = dout;
-    p.q_norm = q_norm;
-    p.k_norm = k_norm;
-    p.n_kv = kv[0]->n_kv_at(0);
-    p.n_q = n_q_heads;
-    p.n_rot = (n_rot_pairs >= 1 && n_rot_pairs < half) ? n_rot_pairs : half;     // kernels.c:1381-1383
-    p.eps = eps;
-    p.theta = (theta_base < 1.0f) ? 10000.0f : theta_base;                       // kernels.c:1374
-    p.scale = (scale_override > 0.0f) ? scale_override : 1.0f / sqrtf((float)kHd);
-    const uint32_t group = n_q_heads / p.n_kv, grid = n_sess * p.n_kv;
-    const dim3 g3(grid), b3(kSmallThreads);
-    if (group == 1) WR_CUDA_TRY(wr_launch_pdl(attn_step_small_kernel<1>, g3, b3, 0, ctx->stream, p));
-    else if (group == 2) WR_CUDA_TRY(wr_launch_pdl(attn_step_small_kernel<2>, g3, b3, 0, ctx->stream, p));
-    else if (group <= 4) WR_CUDA_TRY(wr_launch_pdl(attn_step_small_kernel<4>, g3, b3, 0, ctx->stream, p));
-    else WR_CUDA_TRY(wr_launch_pdl(attn_step_small_kernel<8>, g3, b3, 0, ctx->stream, p));
+    p.q = a.q;
+    p.q_out = a.q_out;
+    p.k = a.k;
+    p.v = a.v;
+    p.out = a.out;
+    p.q_norm = a.q_norm;
+    p.k_norm = a.k_norm;
+    p.n_kv = kv[0]->n_kv_at(layer);
+    p.n_q = a.n_q_heads;
+    p.n_rot = !a.rope ? 0u : (a.n_rot_pairs >= 1 && a.n_rot_pairs < half) ? a.n_rot_pairs : half;     // kernels.c:1381-1383
+    p.eps = a.eps;
+    p.theta = (a.theta_base < 1.0f) ? 10000.0f : a.theta_base;                       // kernels.c:1374
+    p.scale = (a.scale_override > 0.0f) ? a.scale_override : 1.0f / sqrtf((float)kHd);
+    const uint32_t group = a.n_q_heads / p.n_kv, grid = n_sess * p.n_kv;
+    uint32_t sets = 1;                                           // the most that a session of this launch has
+    for (uint32_t i = 0; i < n_sess; ++i) sets = std::max(sets, sets_for(positions[i] + 1, group));
+    if (group == 1) WR_CUDA_TRY(launch_small<1>(sets, grid, ctx->stream, p));
+    else if (group == 2) WR_CUDA_TRY(launch_small<2>(sets, grid, ctx->stream, p));
+    else if (group <= 4) WR_CUDA_TRY(launch_small<4>(sets, grid, ctx->stream, p));
+    else WR_CUDA_TRY(launch_small<8>(sets, grid, ctx->stream, p));
     ctx->launches++;
+    // (it writes cache rows and lets its successor start: no kernel may read tiles before it has waited)
+    ctx->pdl_kind = WR_PDL_DECODE_PART;
+    ctx->pdl_index = ctx->launches;
     WR_CUDA_TRY(cudaGetLastError());
     return WR_CUDA_OK;
 }

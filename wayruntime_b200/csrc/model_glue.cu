@@ -453,14 +453,14 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
         uint32_t n = 0;
         for (int pass = 0; pass < 2; ++pass)
             for (uint32_t r = 0; r < n_rows; ++r) {
-                const bool small = use_small && wr_step_small_covers(kv[r], m->n_q, positions[r]);
+                const bool small = use_small && wr_step_small_covers(kv[r], 0, m->n_q, positions[r]);
                 if (small == (pass == 0)) perm[n++] = r;
             }
         for (uint32_t i = 0; i < n_rows; ++i) {
             if (perm[i] != i) permuted = true;
             kv_p[i] = kv[perm[i]];
             pos_p[i] = positions[perm[i]];
-            if (use_small && wr_step_small_covers(kv_p[i], m->n_q, pos_p[i])) n_short = i + 1;
+            if (use_small && wr_step_small_covers(kv_p[i], 0, m->n_q, pos_p[i])) n_short = i + 1;
             if (pos_p[i] >= kv_p[i]->max_ctx) return WR_CUDA_ERR_CTX_FULL;
         }
     }
@@ -516,8 +516,11 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
                 WR_CUDA_TRY(cudaGetLastError());
             }
             if (mode == WR_CUDA_FWD_DECODE && n_short) {
-                rc = wr_step_small_launch(ctx, n_short, kv_p, L, pos_p, m->q, m->k, m->v, m->attn, m->n_q,
-                                          m->theta, m->n_rot, l.q_norm, l.k_norm, m->eps, m->scale);
+                wr_step_small_args a{};
+                a.q = m->q; a.q_out = m->q; a.k = m->k; a.v = m->v; a.out = m->attn;
+                a.n_q_heads = m->n_q; a.rope = 1; a.n_rot_pairs = m->n_rot; a.theta_base = m->theta;
+                a.q_norm = l.q_norm; a.k_norm = l.k_norm; a.eps = m->eps; a.scale_override = m->scale;
+                rc = wr_step_small_launch(ctx, n_short, kv_p, L, pos_p, a);
                 if (rc != WR_CUDA_OK) return rc;
             }
         }

@@ -199,7 +199,7 @@ int wr_decode_validate(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv,
 int wr_decode_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
                      const uint32_t *seq_lens, const float *dq, float *dout, uint32_t n_q,
                      float scale_override, uint32_t window, int emit_triples, wr_decode_xchg *xchg,
-                     bool early_tiles = false);
+                     bool early_tiles = false, const uint32_t *rows = nullptr /* session s is row rows[s] */);
 
 int wr_ctx_reserve_stage(wr_cuda_ctx *ctx, size_t dev_bytes, size_t host_bytes);
 // Wait for the context's stream and report (and clear) the device-side error
@@ -227,11 +227,20 @@ struct wr_append_extra {
 // One-kernel layer-step for short contexts (attn_step_small.cu): QK-norm, RoPE, append and the
 // new token's attention, for sessions of head_dim 128 with at most WR_STEP_SMALL_MAX_KEYS keys.
 #define WR_STEP_SMALL_MAX_KEYS 1024u
-bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t n_q_heads, uint32_t position);
+bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t layer, uint32_t n_q_heads, uint32_t position);
+struct wr_step_small_args {
+    const float *q;                  // [rows][n_q_heads][128]
+    float *q_out;                    // normed, rotated rows (may be q); null: not wanted
+    const float *k, *v;              // [rows][n_kv][128] new rows; null: they are in the cache
+    float *out;
+    const uint32_t *rows;            // session s is row rows[s] of all these; null: s
+    uint32_t n_q_heads, rope, n_rot_pairs;
+    float theta_base;
+    const float *q_norm, *k_norm;
+    float eps, scale_override;
+};
 int wr_step_small_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
-                         const uint32_t *positions, float *dq, const float *dk, const float *dv, float *dout,
-                         uint32_t n_q_heads, float theta_base, uint32_t n_rot_pairs, const float *q_norm,
-                         const float *k_norm, float eps, float scale_override);
+                         const uint32_t *positions, const wr_step_small_args &args);
 
 // Resolve the device addresses of the allocation-free decode path's scratch
 // arrays and set its kernels' attributes, once per device (that device current).
