@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kBatchThreads, 1) gemv_batch_kernel(const Gemv
     }
     __syncthreads();
 
-    float *mine = parts + (size_t)group * 4 * C * RG * 32;    // this group's [quarter][c][r][lane]
+    uint64_t *mine = reinterpret_cast<uint64_t *>(parts) + (size_t)group * 4 * C * J * 32;    // this group's [quarter][c][row pair][lane]
     for (uint32_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
         uint64_t acc[C][J];
 #pragma unroll
@@ -362,22 +362,21 @@ __global__ void __launch_bounds__(kBatchThreads, 1) gemv_batch_kernel(const Gemv
 #pragma unroll
         for (int c = 0; c < C; ++c)
 #pragma unroll
-            for (int j = 0; j < J; ++j) {
-                float *to = mine + (((size_t)quarter * C + c) * RG + 2 * j) * 32 + lane;
-                to[0] = __uint_as_float((uint32_t)acc[c][j]);
-                to[32] = __uint_as_float((uint32_t)(acc[c][j] >> 32));
-            }
+            for (int j = 0; j < J; ++j) mine[((quarter * C + c) * J + j) * 32 + lane] = acc[c][j];
         asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");
-        // RG of the C * RG sums per warp: one weight row, or (swiglu) half the rows of a gate row and its up row
+        // RG of the C * RG sums per warp, two rows to a pair: one weight row, or (swiglu) half the rows of a gate row and
+        // its up row
         float v[RG];
 #pragma unroll
-        for (int i = 0; i < RG; ++i) {
-            const int c = !p.swiglu ? quarter : (quarter >> 1) + (i < RG / 2 ? 0 : C / 2);
-            const int r = !p.swiglu ? i : (quarter & 1) * (RG / 2) + i % (RG / 2);
-            const float *from = mine + (size_t)(c * RG + r) * 32 + lane;
-            v[i] = from[0];
+        for (int i = 0; i < J; ++i) {
+            const int c = !p.swiglu ? quarter : (quarter >> 1) + (i < J / 2 ? 0 : C / 2);
+            const int j = !p.swiglu ? i : (quarter & 1) * (J / 2) + i % (J / 2);
+            const uint64_t *from = mine + (c * J + j) * 32 + lane;
+            uint64_t t = from[0];
 #pragma unroll
-            for (int q = 1; q < 4; ++q) v[i] = __fadd_rn(v[i], from[(size_t)q * C * RG * 32]);
+            for (int q = 1; q < 4; ++q) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(t) : "l"(from[q * C * J * 32]));
+            v[2 * i] = __uint_as_float((uint32_t)t);
+            v[2 * i + 1] = __uint_as_float((uint32_t)(t >> 32));
         }
         const uint32_t at = warp_reduce_many<RG>(v, lane);
         const GemvSeg seg = p.seg[seg_at];
