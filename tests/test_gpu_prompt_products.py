@@ -31,7 +31,7 @@ def _run(shape, rows, w, max_rows, tokens):
     import wayruntime_b200 as wr
     ctx = wr.Context(0)
     dm = _model(ctx, w, shape, max_rows=max_rows)
-    kv = ctx.kv_create(1, shape["n_kv_heads"], 128, rows)
+    kv = ctx.kv_create(shape["n_layers"], shape["n_kv_heads"], 128, rows)
     res = dm.forward(dm.FWD_PREFILL, [kv], [0], tokens, hidden=True, attn_tap=True)
     v = kv.read_rows(0, 1, 0, rows).reshape(rows, -1).view(np.float16).astype(np.float64)
     kv.close()
@@ -101,3 +101,18 @@ def test_a_rows_bits_do_not_depend_on_how_many_follow():
     few, _ = _run(shape, 140, w, 512, tokens[:140])
     assert np.array_equal(many["attn"][0][:128], few["attn"][0][:128])
     assert np.array_equal(many["hidden"][:128], few["hidden"][:128])
+
+
+def test_weights_are_split_for_each_call_where_memory_is_short():
+    """Split weights are kept when they take a sixteenth of the free memory or less; the results are the same."""
+    import torch
+    shape = dict(n_layers=2, hidden=1024, n_q_heads=8, n_kv_heads=4, head_dim=128, vocab=300, ffn=4096)
+    w = _weights(shape, 1303)
+    tokens = [(7 * r + 1) % 300 for r in range(150)]
+    kept, v = _run(shape, 150, w, 256, tokens)
+    free = torch.cuda.mem_get_info()[0]
+    hold = torch.empty(free - (3 << 29), dtype=torch.uint8, device="cuda")       # 1.5 GB stay free, the weights are 128 MB
+    short, _ = _run(shape, 150, w, 256, tokens)
+    del hold
+    torch.cuda.empty_cache()
+    assert np.array_equal(kept["hidden"], short["hidden"])

@@ -25,10 +25,11 @@ struct wr_cuda_model {
     float *normed = nullptr, *logits = nullptr;
     uint32_t *tokens = nullptr, *best = nullptr, *part_i = nullptr;
     float *part_v = nullptr;             // arg-max partials [16][kArgmaxParts]
-    // prompts on the tensor cores (gemm_f32.cuh): one layer's weights and one product's input, split, and the parts of
+    // prompts on the tensor cores (gemm_f32.cuh): split weights, one product's input, split, and the parts of
     // a product that adds to the residual; null when max_rows is no more than a decode batch, or memory did not suffice
     char *prompt = nullptr;
-    wr_split_weight split[4];            // q | k | v, o, gate / up, down (blocks and unscale; n and k per layer)
+    bool split_kept = false;             // every layer has split weights of its own (else all use the same memory in turn)
+    std::vector<wr_split_weight> split;  // per layer: q | k | v, o, gate / up, down
     __half *split_rows = nullptr;
     float *row_scale = nullptr, *parts = nullptr;
     uint32_t *h_tokens = nullptr;        // pinned: token ids in, arg-max ids out

@@ -14,13 +14,13 @@
 // x * (1/sqrt(mean(x^2)+eps)) * w; :1318-1350 SiLU(a)*b).  Sums run in a
 // different order than the host's SIMD loops, so results agree to F32 rounding,
 // not bit for bit.  A row's result does not depend on how many other rows
-// share the call (same lanes, same order), which keeps batched logits
-// byte-equal to serial ones as the reference promises (src/core/batch.c:1-40).
+// share the call (same lanes, same order) among up to sixteen, which keeps batched logits
+// byte-equal to serial ones as the reference promises (src/core/batch.c:1-40), nor, beyond
+// sixteen, on how many more there are.
 //
-// Kernels: a row-block GEMV (gemv.cu: each warp owns 1-4 weight rows, the activation
-// rows sit in shared memory, the weights stream from HBM exactly once per group
-// of up to 16 activation rows) with optional fused RMSNorm on the input, fused
-// residual add or SiLU*up on the output; per-head RMSNorm; embedding gather;
+// Kernels: a GEMV for up to 16 activation rows (gemv.cu: weights stream from HBM once) with optional fused RMSNorm on the
+// input, fused residual add or SiLU*up on the output; for the rows of a prompt the split tensor-core product of
+// gemm_f32.cu, whose sums are added to the residual by the kernel that reads it next; per-head RMSNorm; embedding gather;
 // row RMSNorm; a two-step arg-max with the reference's tie rule (first maximum wins,
 // src/cli/wayrt.c:805-812).
 #include <math.h>
@@ -174,37 +174,70 @@ int gemv(wr_cuda_model *m, GemvParams &p, uint32_t n_total_for_width)
 
 size_t up256(size_t n) { return (n + 255u) & ~(size_t)255u; }
 
-// Scratch of the prompt path.  A model that cannot have it keeps the GEMV for prompts too.
-void take_prompt_scratch(wr_cuda_model *m)
+// What the rows of a prompt need beside the weights.  Splitting a layer's weights for each call moves them three times (a
+// prompt of 1000 rows of the Qwen3-0.6B shape: 0.6 of 6.6 ms; of 17 rows most of its time), so split weights are kept where
+// they take little: a sixteenth of the memory that is free.  Otherwise all layers use the same memory in turn.  A model that
+// cannot have even that keeps the GEMV for prompts.
+void take_prompt_memory(wr_cuda_model *m)
 {
     if (m->max_rows <= WR_CUDA_BATCH_MAX) return;
-    const uint32_t nq = m->n_q * m->hd, nkv = m->n_kv * m->hd, gate_up = (m->ffn_max + 7u) / 8u * 16u;
-    const uint32_t n[4] = {nq + 2 * nkv, m->hidden, gate_up, m->hidden}, k[4] = {m->hidden, nq, m->hidden, m->ffn_max};
-    const size_t R = m->max_rows, widest = std::max({m->hidden, nq, m->ffn_max});
-    size_t parts = 1, total = 0;
-    for (int i = 0; i < 4; ++i) total += up256(wr_split_weight_bytes(n[i], k[i])) + up256((size_t)n[i] * 4);
-    for (const wr_cuda_layer_dev &l : m->layers)
-        parts = std::max<size_t>({parts, wr_f32_gemm_k_parts(m->hidden, nq), wr_f32_gemm_k_parts(m->hidden, l.ffn)});
+    const uint32_t nq = m->n_q * m->hd, nkv = m->n_kv * m->hd;
+    const size_t R = m->max_rows, widest = std::max({m->hidden, nq, m->ffn_max}), n_layers = m->layers.size();
+    size_t parts = 1, all = 0, most = 0;
+    std::vector<size_t> at(n_layers);                    // a layer's split weights, from the first one's
+    m->split.resize(4 * n_layers);
+    for (size_t L = 0; L < n_layers; ++L) {
+        const uint32_t ffn = m->layers[L].ffn, gate_up = (ffn + 7u) / 8u * 16u;
+        const uint32_t n[4] = {nq + 2 * nkv, m->hidden, gate_up, m->hidden}, k[4] = {m->hidden, nq, m->hidden, ffn};
+        size_t bytes = 0;
+        for (int i = 0; i < 4; ++i) {
+            m->split[4 * L + i].n = n[i];
+            m->split[4 * L + i].k = k[i];
+            bytes += up256(wr_split_weight_bytes(n[i], k[i])) + up256((size_t)n[i] * 4);
+        }
+        parts = std::max<size_t>({parts, wr_f32_gemm_k_parts(m->hidden, nq), wr_f32_gemm_k_parts(m->hidden, ffn)});
+        at[L] = all;
+        all += bytes;
+        most = std::max(most, bytes);
+    }
     const size_t rows = up256(2 * R * ((widest + 7) & ~(size_t)7) * 2), sums = up256(parts * R * m->hidden * 4);
-    total += rows + up256(R * 4) + sums;
-    if (cudaMalloc((void **)&m->prompt, total) != cudaSuccess) {
-        (void)cudaGetLastError();
-        m->prompt = nullptr;
-        return;
-    }
-    m->slab_bytes += total;
+    const size_t rest = rows + up256(R * 4) + sums;
+    size_t free_bytes = 0, total_bytes = 0;
+    if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) (void)cudaGetLastError();
+    m->split_kept = all <= free_bytes / 16 && cudaMalloc((void **)&m->prompt, all + rest) == cudaSuccess;
+    if (!m->split_kept && cudaMalloc((void **)&m->prompt, most + rest) != cudaSuccess) m->prompt = nullptr;
+    (void)cudaGetLastError();
+    if (!m->prompt) return;
+    m->slab_bytes += (m->split_kept ? all : most) + rest;
     char *cur = m->prompt;
-    for (int i = 0; i < 4; ++i) {
-        m->split[i].blocks = cur;
-        cur += up256(wr_split_weight_bytes(n[i], k[i]));
-        m->split[i].unscale = reinterpret_cast<float *>(cur);
-        cur += up256((size_t)n[i] * 4);
+    for (size_t L = 0; L < n_layers; ++L) {
+        cur = m->prompt + (m->split_kept ? at[L] : 0);
+        for (int i = 0; i < 4; ++i) {
+            wr_split_weight &w = m->split[4 * L + i];
+            w.blocks = cur;
+            cur += up256(wr_split_weight_bytes(w.n, w.k));
+            w.unscale = reinterpret_cast<float *>(cur);
+            cur += up256((size_t)w.n * 4);
+        }
     }
+    cur = m->prompt + (m->split_kept ? all : most);
     m->split_rows = reinterpret_cast<__half *>(cur);
     cur += rows;
     m->row_scale = reinterpret_cast<float *>(cur);
     cur += up256(R * 4);
     m->parts = reinterpret_cast<float *>(cur);
+}
+
+int split_layer(wr_cuda_model *m, uint32_t L)
+{
+    const wr_cuda_layer_dev &l = m->layers[L];
+    const uint32_t hid = m->hidden, nq = m->n_q * m->hd, nkv = m->n_kv * m->hd;
+    const wr_split_weight *w = &m->split[4 * L];
+    const wr_split_source list[4] = {{w[0], {l.wq, l.wk, l.wv}, {nq, nkv, nkv}, 0},
+                                     {w[1], {l.wo, nullptr, nullptr}, {hid, 0, 0}, 0},
+                                     {w[2], {l.w_gate, l.w_up, nullptr}, {l.ffn, l.ffn, 0}, 1},
+                                     {w[3], {l.w_down, nullptr, nullptr}, {hid, 0, 0}, 0}};
+    return wr_split_weights_launch(m->ctx, list, 4);
 }
 
 // Split rows of x (the residual takes the parts of the product before first), and their tensor map.
@@ -224,23 +257,15 @@ int split_rows(wr_cuda_model *m, CUtensorMap *map, float *x, uint32_t x_stride, 
 
 // The products of a layer for the rows of a prompt: before (q, k, v) and after (o, feed-forward) attention.  A product
 // that adds to the residual leaves its sums in m->parts; whoever reads the residual next adds them: *n_parts.
-int prompt_before(wr_cuda_model *m, const wr_cuda_layer_dev &l, uint32_t rows, uint32_t *n_parts)
+int prompt_before(wr_cuda_model *m, uint32_t L, uint32_t rows, uint32_t *n_parts)
 {
+    const wr_cuda_layer_dev &l = m->layers[L];
     const uint32_t hid = m->hidden, nq = m->n_q * m->hd, nkv = m->n_kv * m->hd;
-    auto weight = [&](int i, uint32_t n, uint32_t k) {
-        wr_split_weight w = m->split[i];
-        w.n = n;
-        w.k = k;
-        return w;
-    };
-    const wr_split_source list[4] = {
-        {weight(0, nq + 2 * nkv, hid), {l.wq, l.wk, l.wv}, {nq, nkv, nkv}, 0},
-        {weight(1, hid, nq), {l.wo, nullptr, nullptr}, {hid, 0, 0}, 0},
-        {weight(2, (l.ffn + 7u) / 8u * 16u, hid), {l.w_gate, l.w_up, nullptr}, {l.ffn, l.ffn, 0}, 1},
-        {weight(3, hid, l.ffn), {l.w_down, nullptr, nullptr}, {hid, 0, 0}, 0}};
-    int rc = wr_split_weights_launch(m->ctx, list, 4);
-    if (rc != WR_CUDA_OK) return rc;
-    for (int i = 0; i < 4; ++i) m->split[i] = list[i].to;
+    int rc = WR_CUDA_OK;
+    if (!m->split_kept) {
+        ++m->launches;
+        if ((rc = split_layer(m, L)) != WR_CUDA_OK) return rc;
+    }
     CUtensorMap map;
     rc = split_rows(m, &map, m->resid, hid, hid, rows, *n_parts, l.attn_norm);
     if (rc != WR_CUDA_OK) return rc;
@@ -248,12 +273,14 @@ int prompt_before(wr_cuda_model *m, const wr_cuda_layer_dev &l, uint32_t rows, u
     wr_f32_gemm_args a{};
     a.m = a.pad = rows; a.row_scale = m->row_scale; a.k_parts = 1;
     a.seg[0] = {m->q, nq, nq}; a.seg[1] = {m->k, nkv, nkv}; a.seg[2] = {m->v, nkv, nkv}; a.n_seg = 3;
-    m->launches += 2;
-    return wr_f32_gemm_launch(m->ctx, map, m->split[0], a);
+    ++m->launches;
+    return wr_f32_gemm_launch(m->ctx, map, m->split[4 * L], a);
 }
 
-int prompt_after(wr_cuda_model *m, const wr_cuda_layer_dev &l, uint32_t rows, uint32_t *n_parts)
+int prompt_after(wr_cuda_model *m, uint32_t L, uint32_t rows, uint32_t *n_parts)
 {
+    const wr_cuda_layer_dev &l = m->layers[L];
+    const wr_split_weight *w4 = &m->split[4 * L];
     const uint32_t hid = m->hidden, nq = m->n_q * m->hd;
     CUtensorMap map;
     auto to_residual = [&](const wr_split_weight &w) {
@@ -265,15 +292,15 @@ int prompt_after(wr_cuda_model *m, const wr_cuda_layer_dev &l, uint32_t rows, ui
     };
     m->launches += 3;
     int rc = split_rows(m, &map, m->attn, nq, nq, rows, 0, nullptr);
-    if (rc != WR_CUDA_OK || (rc = to_residual(m->split[1])) != WR_CUDA_OK) return rc;
+    if (rc != WR_CUDA_OK || (rc = to_residual(w4[1])) != WR_CUDA_OK) return rc;
     rc = split_rows(m, &map, m->resid, hid, hid, rows, *n_parts, l.ffn_norm);
     if (rc != WR_CUDA_OK) return rc;
     wr_f32_gemm_args a{};
     a.m = a.pad = rows; a.row_scale = m->row_scale; a.k_parts = 1;
     a.seg[0] = {m->gate, l.ffn, m->ffn_max}; a.n_seg = 1; a.pair = 1;
-    if ((rc = wr_f32_gemm_launch(m->ctx, map, m->split[2], a)) != WR_CUDA_OK) return rc;
+    if ((rc = wr_f32_gemm_launch(m->ctx, map, w4[2], a)) != WR_CUDA_OK) return rc;
     rc = split_rows(m, &map, m->gate, m->ffn_max, l.ffn, rows, 0, nullptr);
-    return rc != WR_CUDA_OK ? rc : to_residual(m->split[3]);
+    return rc != WR_CUDA_OK ? rc : to_residual(w4[3]);
 }
 
 }  // namespace
@@ -388,7 +415,9 @@ extern "C" int wr_cuda_model_create(wr_cuda_ctx *ctx, const wr_cuda_model_desc *
         delete m;
         return WR_CUDA_ERR_INTERNAL;
     }
-    take_prompt_scratch(m);
+    take_prompt_memory(m);
+    for (uint32_t L = 0; m->split_kept && L < m->n_layers; ++L) m->split_kept = split_layer(m, L) == WR_CUDA_OK;
+    if (m->split_kept) m->split_kept = cudaStreamSynchronize(ctx->stream) == cudaSuccess;
     *out = m;
     return WR_CUDA_OK;
 }
@@ -486,7 +515,7 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
         {
             std::lock_guard<std::mutex> g(ctx->lock);
             if (wide) {
-                rc = prompt_before(m, l, n_rows, &n_parts);
+                rc = prompt_before(m, L, n_rows, &n_parts);
             } else {
                 GemvParams p{};
                 p.seg[0] = {l.wq, m->q, nq, nq};
@@ -555,7 +584,7 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
                 }
             }
             if (wide) {
-                rc = prompt_after(m, l, n_rows, &n_parts);
+                rc = prompt_after(m, L, n_rows, &n_parts);
                 if (rc != WR_CUDA_OK) return rc;
                 continue;
             }
