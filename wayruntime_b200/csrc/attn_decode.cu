@@ -217,7 +217,7 @@ void wr_decode_plan(uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer, cons
 int wr_decode_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
                      const uint32_t *seq_lens, const float *dq, float *dout, uint32_t n_q,
                      float scale_override, uint32_t window, int emit_triples, wr_decode_xchg *xchg,
-                     bool early_tiles, const uint32_t *rows)
+                     bool early_tiles)
 {
     const uint32_t n_kv = kv[0]->n_kv_at(layer), hd = kv[0]->hd_at(layer);
     const uint32_t group = n_q / n_kv;
@@ -228,7 +228,6 @@ int wr_decode_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
         params p;
         uint32_t nt = 1, items = 0;
         wr_decode_plan(n_sess, kv, layer, seq_lens, n_q, window, p, nt, items);
-        for (uint32_t i = 0; rows && i < n_sess; ++i) p.row[i] = rows[p.row[i]];
         int rc = wr_ctx_reserve_ws(ctx, (size_t)std::max(items, 1u) * 8 * kTripleStride * sizeof(float),
                                    (size_t)p.n_groups * kTicketsPerGroup + kTicketExtra);
         if (rc != WR_CUDA_OK) return rc;
@@ -315,44 +314,6 @@ int wr_decode_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
     return WR_CUDA_OK;
 }
 
-// Sessions of at most kStepKeys keys go through the one-kernel step (attn_step_small.cu), which has no queue, partial sums or
-// merge, and in a decode step appends too.  A rule on the session alone, in every entry point that gives finished rows.
-// The line: up to 256 keys the scores are one round trip per thread.  One session, 16 q heads over 8, 64 to 192 keys, rows in
-// page-locked memory: 33 -> 29 us a call.
-constexpr uint32_t kStepKeys = 256;
-
-struct wr_decode_split {
-    uint32_t n_short = 0, n_long = 0;
-    uint32_t short_row[WR_CUDA_BATCH_MAX], short_pos[WR_CUDA_BATCH_MAX], long_row[WR_CUDA_BATCH_MAX], long_len[WR_CUDA_BATCH_MAX];
-    wr_cuda_kv *short_kv[WR_CUDA_BATCH_MAX], *long_kv[WR_CUDA_BATCH_MAX];
-
-    wr_decode_split(uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer, const uint32_t *seq_lens, uint32_t n_q, uint32_t window)
-    {
-        for (uint32_t s = 0; s < n_sess; ++s) {
-            if (window == 0 && seq_lens[s] && seq_lens[s] <= kStepKeys && wr_step_small_covers(kv[s], layer, n_q, seq_lens[s] - 1)) {
-                short_row[n_short] = s;
-                short_pos[n_short] = seq_lens[s] - 1;
-                short_kv[n_short++] = kv[s];
-            } else {
-                long_row[n_long] = s;
-                long_len[n_long] = seq_lens[s];
-                long_kv[n_long++] = kv[s];
-            }
-        }
-    }
-    // Attention over cached rows: out[r] for every session.
-    int attend(wr_cuda_ctx *ctx, uint32_t layer, const float *dq, float *dout, uint32_t n_q, float scale, uint32_t window, bool early)
-    {
-        if (n_short) {
-            wr_step_small_args a{};
-            a.q = dq; a.out = dout; a.rows = short_row; a.n_q_heads = n_q; a.scale_override = scale;
-            const int rc = wr_step_small_launch(ctx, n_short, short_kv, layer, short_pos, a);
-            if (rc != WR_CUDA_OK || !n_long) return rc;
-        }
-        return wr_decode_launch(ctx, n_long, long_kv, layer, long_len, dq, dout, n_q, scale, window, 0, nullptr, early && !n_short, long_row);
-    }
-};
-
 static int decode_common(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
                          const uint32_t *seq_lens, const float *q, float *out, uint32_t n_q,
                          float scale_override, uint32_t window, int mem, int emit_triples)
@@ -379,10 +340,8 @@ static int decode_common(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *k
     // written): the second one may request its first tiles while the first one drains.
     const bool early = mem == WR_CUDA_MEM_DEVICE && ctx->pdl_index == ctx->launches &&
                        ctx->pdl_kind == WR_PDL_DECODE_FULL;
-    rc = emit_triples ? wr_decode_launch(ctx, n_sess, kv, layer, seq_lens, dq, dout, n_q, scale_override, window, emit_triples,
-                                         nullptr, early)
-                      : wr_decode_split(n_sess, kv, layer, seq_lens, n_q, window).attend(ctx, layer, dq, dout, n_q, scale_override,
-                                                                                       window, early);
+    rc = wr_decode_launch(ctx, n_sess, kv, layer, seq_lens, dq, dout, n_q, scale_override, window,
+                          emit_triples, nullptr, early);
     if (rc != WR_CUDA_OK) return rc;
     if (mem == WR_CUDA_MEM_HOST) {
         WR_CUDA_TRY(cudaMemcpyAsync(out, dout, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -454,20 +413,11 @@ extern "C" int wr_cuda_decode_step(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv
     // library's early-starting kernels, or is a decode launch that covered every SM.
     const int prev = (ctx->pdl_index == ctx->launches) ? ctx->pdl_kind : WR_PDL_NONE;
     const bool early = prev == WR_PDL_NONE || prev == WR_PDL_DECODE_FULL;
-    wr_decode_split split(n_sess, kv, layer, seq_lens, n_q_heads, window);
-    if (!split.n_long) {                                     // rotation, cache rows and attention in one kernel
-        wr_step_small_args a{};
-        a.q = dq_in ? dq_in : dq;
-        a.q_out = mem == WR_CUDA_MEM_DEVICE && (flags & WR_CUDA_APPEND_ROPE) ? dq : nullptr;
-        a.k = dk; a.v = dv; a.out = dout; a.n_q_heads = n_q_heads;
-        a.rope = (flags & WR_CUDA_APPEND_ROPE) ? 1u : 0u; a.n_rot_pairs = n_rot_pairs; a.theta_base = theta_base;
-        a.scale_override = scale_override;
-        rc = wr_step_small_launch(ctx, n_sess, kv, layer, positions, a);
-    } else {
-        rc = wr_append_launch(ctx, n_sess, kv, layer, positions, 1, dk, dv, dq, n_q_heads, theta_base,
-                              n_rot_pairs, flags, dq_in);
-        if (rc == WR_CUDA_OK) rc = split.attend(ctx, layer, dq, dout, n_q_heads, scale_override, window, early);
-    }
+    rc = wr_append_launch(ctx, n_sess, kv, layer, positions, 1, dk, dv, dq, n_q_heads, theta_base,
+                          n_rot_pairs, flags, dq_in);
+    if (rc != WR_CUDA_OK) return rc;
+    rc = wr_decode_launch(ctx, n_sess, kv, layer, seq_lens, dq, dout, n_q_heads, scale_override,
+                          window, 0, nullptr, early);
     if (rc != WR_CUDA_OK) return rc;
     if (mem == WR_CUDA_MEM_HOST) {
         if (staged_out)

@@ -199,7 +199,7 @@ int wr_decode_validate(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv,
 int wr_decode_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
                      const uint32_t *seq_lens, const float *dq, float *dout, uint32_t n_q,
                      float scale_override, uint32_t window, int emit_triples, wr_decode_xchg *xchg,
-                     bool early_tiles = false, const uint32_t *rows = nullptr /* session s is row rows[s] */);
+                     bool early_tiles = false);
 
 int wr_ctx_reserve_stage(wr_cuda_ctx *ctx, size_t dev_bytes, size_t host_bytes);
 // Wait for the context's stream and report (and clear) the device-side error
