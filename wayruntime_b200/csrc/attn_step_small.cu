@@ -43,11 +43,9 @@ constexpr uint32_t kHd = 128;
 
 struct step_small_params {
     wr_batch_desc b;                 // b.seq_len[s] = position of the new token of session s
-    uint32_t row[WR_CUDA_BATCH_MAX]; // session s is row `row[s]` of
-    const float *q;                  // [rows][n_q][128]: raw projections
-    float *q_out;                    // (normed, rotated) rows, maybe the same buffer; or null
-    const float *k, *v;              // [rows][n_kv][128] raw projections; or null: the cache has the new row already
-    float *out;                      // [rows][n_q][128]
+    float *q;                        // [n_sess][n_q][128]: raw projections in, (normed, rotated) rows out
+    const float *k, *v;              // [n_sess][n_kv][128] raw projections
+    float *out;                      // [n_sess][n_q][128]
     const float *q_norm, *k_norm;    // [128] each, or both null
     uint32_t n_kv, n_q, n_rot;
     float eps, theta, scale;
@@ -79,8 +77,7 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
     const uint32_t s = blockIdx.x / p.n_kv, kvh = blockIdx.x % p.n_kv;
     const uint32_t G = p.n_q / p.n_kv;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t pos = p.b.seq_len[s], n_keys = pos + 1, row = p.row[s];
-    const bool append = p.k != nullptr;
+    const uint32_t pos = p.b.seq_len[s], n_keys = pos + 1;
     constexpr uint32_t half = kHd / 2;
 
     // ---- what does not depend on the kernel before this one (the projections): norm weights, the
@@ -101,10 +98,10 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
     }
     pdl_wait();
     // ---- rows in
-    const size_t q_at = ((size_t)row * p.n_q + (size_t)kvh * G) * kHd;
+    const size_t q_at = ((size_t)s * p.n_q + (size_t)kvh * G) * kHd;
     for (uint32_t i = tid; i < G * kHd; i += kSmallThreads) sq[i / kHd][i % kHd] = p.q[q_at + i];
-    if (append && tid < kHd) sk[tid] = p.k[((size_t)row * p.n_kv + kvh) * kHd + tid];
-    else if (append && tid < 2 * kHd) sv[tid - kHd] = p.v[((size_t)row * p.n_kv + kvh) * kHd + tid - kHd];
+    if (tid < kHd) sk[tid] = p.k[((size_t)s * p.n_kv + kvh) * kHd + tid];
+    else if (tid < 2 * kHd) sv[tid - kHd] = p.v[((size_t)s * p.n_kv + kvh) * kHd + tid - kHd];
     __syncthreads();
 
     // ---- per-head RMSNorm of K and of the G q heads (one warp per vector), as head_rmsnorm_kernel
@@ -137,7 +134,7 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
 
     // ---- append: the new K / V row into its page (truncating convert), and kept for this CTA's own use;
     //      the rotated q rows go back to the caller's buffer
-    if (append && tid < kHd) {
+    if (tid < kHd) {
         char *page = const_cast<char *>(s_page[pos / kPageTokens]);
         const uint32_t tk = pos % kPageTokens, off = wr_elem_off(tk, tid, kHd);
         const uint16_t kb = wr_f32_to_f16_trunc(sk[tid]), vb = wr_f32_to_f16_trunc(sv[tid]);
@@ -146,8 +143,7 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
         nk[tid] = __ushort_as_half(kb);
         nv[tid] = __ushort_as_half(vb);
     }
-    if (p.q_out)
-        for (uint32_t i = tid; i < G * kHd; i += kSmallThreads) p.q_out[q_at + i] = sq[i / kHd][i % kHd];
+    for (uint32_t i = tid; i < G * kHd; i += kSmallThreads) p.q[q_at + i] = sq[i / kHd][i % kHd];
     __syncthreads();
 
     // ---- scores: one thread per key, all G heads at once.  The sixteen 16-byte loads of a key row are
@@ -163,7 +159,7 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
         uint4 raw[kRaw];
 #pragma unroll
         for (uint32_t i = 0; i < kRaw; ++i) {
-            if (append && key == pos) raw[i] = *reinterpret_cast<const uint4 *>(&nk[8 * (c0 + i)]);
+            if (key == pos) raw[i] = *reinterpret_cast<const uint4 *>(&nk[8 * (c0 + i)]);
             else raw[i] = __ldg(reinterpret_cast<const uint4 *>(row_chunk(kb, tok, c0 + i)));
         }
 #pragma unroll
@@ -232,7 +228,7 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
                 for (uint32_t i = 0; i < W / 2; ++i) raw[u][i] = 0u;
                 if (key < n_keys) {
                     const char *from = reinterpret_cast<const char *>(&nv[d0]);
-                    if (!append || key != pos)
+                    if (key != pos)
                         from = row_chunk(s_page[key / kPageTokens] + wr_block_off(kvh, 1, kHd), key % kPageTokens, d0 / 8) +
                                d0 % 8 * 2;
                     if constexpr (W == 8) *reinterpret_cast<uint4 *>(raw[u]) = *reinterpret_cast<const uint4 *>(from);
@@ -286,24 +282,31 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
     }
 }
 
-template <int GM>
-cudaError_t launch_small(uint32_t sets, uint32_t grid, cudaStream_t st, const step_small_params &p)
+template <int GM, int SETS>
+cudaError_t launch_sets(uint32_t grid, cudaStream_t st, bool side, const step_small_params &p)
 {
-    if (sets == 1) return wr_launch_pdl(attn_step_small_kernel<GM, 1>, dim3(grid), dim3(kSetThreads), 0, st, p);
-    if (sets == 2) return wr_launch_pdl(attn_step_small_kernel<GM, 2>, dim3(grid), dim3(2 * kSetThreads), 0, st, p);
-    if constexpr (max_sets(GM) == 4) return wr_launch_pdl(attn_step_small_kernel<GM, 4>, dim3(grid), dim3(4 * kSetThreads), 0, st, p);
+    if (!side) return wr_launch_pdl(attn_step_small_kernel<GM, SETS>, dim3(grid), dim3(kSetThreads * SETS), 0, st, p);
+    attn_step_small_kernel<GM, SETS><<<grid, kSetThreads * SETS, 0, st>>>(p);
+    return cudaGetLastError();
+}
+template <int GM>
+cudaError_t launch_small(uint32_t sets, uint32_t grid, cudaStream_t st, bool side, const step_small_params &p)
+{
+    if (sets == 1) return launch_sets<GM, 1>(grid, st, side, p);
+    if (sets == 2) return launch_sets<GM, 2>(grid, st, side, p);
+    if constexpr (max_sets(GM) == 4) return launch_sets<GM, 4>(grid, st, side, p);
     return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
-bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t layer, uint32_t n_q_heads, uint32_t position)
+bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t n_q_heads, uint32_t position)
 {
-    return kv->hd_at(layer) == kHd && kv->n_kv_at(layer) > 0 && n_q_heads % kv->n_kv_at(layer) == 0 &&
-           n_q_heads / kv->n_kv_at(layer) <= kSmallMaxGroup && position + 1 <= kSmallMaxKeys;
+    return kv->hd_at(0) == kHd && kv->n_kv_at(0) > 0 && n_q_heads % kv->n_kv_at(0) == 0 &&
+           n_q_heads / kv->n_kv_at(0) <= kSmallMaxGroup && position + 1 <= kSmallMaxKeys;
 }
 
-// Enqueue on rows the device can reach.  Caller holds ctx->lock; every session must pass wr_step_small_covers and
+// Enqueue on device-resident rows.  Caller holds ctx->lock; every session must pass wr_step_small_covers and
 // wr_kv_batch_check, and positions[s] < max_ctx.
 int wr_step_small_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
                          const uint32_t *positions, const wr_step_small_args &a)
@@ -311,15 +314,13 @@ int wr_step_small_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *k
     if (n_sess == 0 || n_sess > WR_CUDA_BATCH_MAX) return WR_CUDA_ERR_LIMIT;
     step_small_params p;
     for (uint32_t s = 0; s < n_sess; ++s) {
-        if (!wr_step_small_covers(kv[s], layer, a.n_q_heads, positions[s])) return WR_CUDA_ERR_UNSUPPORTED;
+        if (!wr_step_small_covers(kv[s], a.n_q_heads, positions[s])) return WR_CUDA_ERR_UNSUPPORTED;
         if (positions[s] >= kv[s]->max_ctx) return WR_CUDA_ERR_CTX_FULL;
         p.b.pages[s] = kv[s]->d_pages + (size_t)layer * kv[s]->n_pages;
         p.b.seq_len[s] = positions[s];
-        p.row[s] = a.rows ? a.rows[s] : s;
     }
     constexpr uint32_t half = kHd / 2u;
     p.q = a.q;
-    p.q_out = a.q_out;
     p.k = a.k;
     p.v = a.v;
     p.out = a.out;
@@ -327,21 +328,19 @@ int wr_step_small_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *k
     p.k_norm = a.k_norm;
     p.n_kv = kv[0]->n_kv_at(layer);
     p.n_q = a.n_q_heads;
-    p.n_rot = !a.rope ? 0u : (a.n_rot_pairs >= 1 && a.n_rot_pairs < half) ? a.n_rot_pairs : half;     // kernels.c:1381-1383
+    p.n_rot = (a.n_rot_pairs >= 1 && a.n_rot_pairs < half) ? a.n_rot_pairs : half;     // kernels.c:1381-1383
     p.eps = a.eps;
     p.theta = (a.theta_base < 1.0f) ? 10000.0f : a.theta_base;                       // kernels.c:1374
     p.scale = (a.scale_override > 0.0f) ? a.scale_override : 1.0f / sqrtf((float)kHd);
     const uint32_t group = a.n_q_heads / p.n_kv, grid = n_sess * p.n_kv;
     uint32_t sets = 1;                                           // the most that a session of this launch has
     for (uint32_t i = 0; i < n_sess; ++i) sets = std::max(sets, sets_for(positions[i] + 1, group));
-    if (group == 1) WR_CUDA_TRY(launch_small<1>(sets, grid, ctx->stream, p));
-    else if (group == 2) WR_CUDA_TRY(launch_small<2>(sets, grid, ctx->stream, p));
-    else if (group <= 4) WR_CUDA_TRY(launch_small<4>(sets, grid, ctx->stream, p));
-    else WR_CUDA_TRY(launch_small<8>(sets, grid, ctx->stream, p));
+    const cudaStream_t st = a.side ? a.side : ctx->stream;
+    if (group == 1) WR_CUDA_TRY(launch_small<1>(sets, grid, st, a.side != nullptr, p));
+    else if (group == 2) WR_CUDA_TRY(launch_small<2>(sets, grid, st, a.side != nullptr, p));
+    else if (group <= 4) WR_CUDA_TRY(launch_small<4>(sets, grid, st, a.side != nullptr, p));
+    else WR_CUDA_TRY(launch_small<8>(sets, grid, st, a.side != nullptr, p));
     ctx->launches++;
-    // (it writes cache rows and lets its successor start: no kernel may read tiles before it has waited)
-    ctx->pdl_kind = WR_PDL_DECODE_PART;
-    ctx->pdl_index = ctx->launches;
     WR_CUDA_TRY(cudaGetLastError());
     return WR_CUDA_OK;
 }

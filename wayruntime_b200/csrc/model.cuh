@@ -36,6 +36,9 @@ struct wr_cuda_model {
     uint32_t ffn_max = 0;
     uint64_t launches = 0;
     uint64_t last_enqueue_ns = 0;        // host time the last forward pass spent before it began to wait
+    // Decode steps that hold short and long sessions attend to the short ones on a stream of their own.
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     std::mutex fwd;                      // one forward pass at a time (the scratch rows are shared)
 };
 

@@ -227,17 +227,16 @@ struct wr_append_extra {
 // One-kernel layer-step for short contexts (attn_step_small.cu): QK-norm, RoPE, append and the
 // new token's attention, for sessions of head_dim 128 with at most WR_STEP_SMALL_MAX_KEYS keys.
 #define WR_STEP_SMALL_MAX_KEYS 1024u
-bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t layer, uint32_t n_q_heads, uint32_t position);
+bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t n_q_heads, uint32_t position);
 struct wr_step_small_args {
-    const float *q;                  // [rows][n_q_heads][128]
-    float *q_out;                    // normed, rotated rows (may be q); null: not wanted
-    const float *k, *v;              // [rows][n_kv][128] new rows; null: they are in the cache
+    float *q;                        // [n_sess][n_q_heads][128]: raw rows in, normed and rotated ones out
+    const float *k, *v;              // [n_sess][n_kv][128] new rows
     float *out;
-    const uint32_t *rows;            // session s is row rows[s] of all these; null: s
-    uint32_t n_q_heads, rope, n_rot_pairs;
+    uint32_t n_q_heads, n_rot_pairs;
     float theta_base;
     const float *q_norm, *k_norm;
     float eps, scale_override;
+    cudaStream_t side;               // launched there, in full order, instead of on the context's stream; or null
 };
 int wr_step_small_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
                          const uint32_t *positions, const wr_step_small_args &args);
