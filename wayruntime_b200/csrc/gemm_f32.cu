@@ -348,51 +348,61 @@ __global__ void __launch_bounds__(32 * kSplitWarps) split_weights_kernel(const S
     if (lane == 0 && row < s.to.n) s.to.unscale[row] = pow2(-e);
 }
 
-constexpr uint32_t kRowThreads = 256;
+constexpr uint32_t kRowThreads = 256, kMaxParts = 4;
 
-// One block per activation row: partial sums into the residual, sum of squares and largest magnitude, then the split.
-__global__ void __launch_bounds__(kRowThreads) split_rows_kernel(const wr_split_rows_args p)
+// One block per activation row: partial sums into the residual, sum of squares and largest magnitude, then the split.  What
+// bounds it is one chain of round trips per row: everything a thread reads is requested at once, the norm's weights before the
+// wait, and KEEP (vectors that a thread holds) is no larger than the row asks for, so that rows fit the device in one go.
+template <uint32_t KEEP>
+__global__ void __launch_bounds__(kRowThreads, KEEP == 1 ? 5 : 4) split_rows_kernel(const wr_split_rows_args p)
 {
     __shared__ float part_ss[kRowThreads / 32];
     __shared__ uint32_t part_top[kRowThreads / 32];
     pdl_trigger();
-    pdl_wait();
     const uint32_t row = blockIdx.x, tid = threadIdx.x, vecs = p.k / 4;
     float4 *x = reinterpret_cast<float4 *>(p.x + (size_t)row * p.x_stride);
-    constexpr uint32_t kKeep = 4;                        // vectors that a thread holds
-    float4 kept[kKeep];
+    const float4 *parts = reinterpret_cast<const float4 *>(p.parts + (p.parts ? (size_t)row * p.k : 0));
+    const float4 *weight = reinterpret_cast<const float4 *>(p.norm_w);
+    float4 w[KEEP], kept[KEEP];
+#pragma unroll
+    for (uint32_t u = 0; u < KEEP; ++u)
+        if (weight && u * kRowThreads + tid < vecs) w[u] = __ldg(weight + u * kRowThreads + tid);
+    pdl_wait();
     float ss = 0.f;
     uint32_t top = 0;
     auto take = [&](uint32_t i) {
         float4 v = x[i];
         if (p.parts) {
-            const float4 *part = reinterpret_cast<const float4 *>(p.parts + (size_t)row * p.k) + i;
-            float4 y = part[0];
-            for (uint32_t j = 1; j < p.n_parts; ++j) {
-                const float4 z = part[(size_t)j * p.rows * vecs];
-                y = make_float4(y.x + z.x, y.y + z.y, y.z + z.z, y.w + z.w);
-            }
-            v = make_float4(v.x + y.x, v.y + y.y, v.z + y.z, v.w + y.w);
+            float4 z[kMaxParts];
+#pragma unroll
+            for (uint32_t j = 0; j < kMaxParts; ++j)
+                if (j < p.n_parts) z[j] = parts[(size_t)j * p.rows * vecs + i];
+#pragma unroll
+            for (uint32_t j = 1; j < kMaxParts; ++j)
+                if (j < p.n_parts) z[0] = make_float4(z[0].x + z[j].x, z[0].y + z[j].y, z[0].z + z[j].z, z[0].w + z[j].w);
+            v = make_float4(v.x + z[0].x, v.y + z[0].y, v.z + z[0].z, v.w + z[0].w);
             x[i] = v;
         }
         return v;
     };
-    auto weigh = [&](uint32_t i, float4 v) {
-        if (!p.norm_w) return v;
-        const float4 w = __ldg(reinterpret_cast<const float4 *>(p.norm_w) + i);
+    auto weigh = [&](float4 v, const float4 &w) {
+        if (!weight) return v;
         return make_float4(__fmul_rn(v.x, w.x), __fmul_rn(v.y, w.y), __fmul_rn(v.z, w.z), __fmul_rn(v.w, w.w));
     };
-    auto look = [&](uint32_t i) {
-        float4 v = take(i);
+    auto look = [&](float4 v, const float4 &w) {
         ss = fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, ss))));
-        v = weigh(i, v);
+        v = weigh(v, w);
         top = max(top, abs_bits(v));
         return v;
     };
+    auto weight_at = [&](uint32_t i) { return weight ? __ldg(weight + i) : make_float4(1.f, 1.f, 1.f, 1.f); };
 #pragma unroll
-    for (uint32_t u = 0; u < kKeep; ++u)
-        if (u * kRowThreads + tid < vecs) kept[u] = look(u * kRowThreads + tid);
-    for (uint32_t i = kKeep * kRowThreads + tid; i < vecs; i += kRowThreads) (void)look(i);
+    for (uint32_t u = 0; u < KEEP; ++u)
+        if (u * kRowThreads + tid < vecs) kept[u] = take(u * kRowThreads + tid);
+#pragma unroll
+    for (uint32_t u = 0; u < KEEP; ++u)
+        if (u * kRowThreads + tid < vecs) kept[u] = look(kept[u], w[u]);
+    for (uint32_t i = KEEP * kRowThreads + tid; i < vecs; i += kRowThreads) (void)look(take(i), weight_at(i));
     if (!p.out) return;
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -405,9 +415,9 @@ __global__ void __launch_bounds__(kRowThreads) split_rows_kernel(const wr_split_
     ss = part_ss[0];
     top = part_top[0];
 #pragma unroll
-    for (uint32_t w = 1; w < kRowThreads / 32; ++w) {
-        ss += part_ss[w];
-        top = max(top, part_top[w]);
+    for (uint32_t i = 1; i < kRowThreads / 32; ++i) {
+        ss += part_ss[i];
+        top = max(top, part_top[i]);
     }
     const int e = scale_exponent(top);
     const float scale = pow2(e);
@@ -419,11 +429,11 @@ __global__ void __launch_bounds__(kRowThreads) split_rows_kernel(const wr_split_
         *reinterpret_cast<uint2 *>(lo + 4 * i) = l;
     };
 #pragma unroll
-    for (uint32_t u = 0; u < kKeep; ++u)
+    for (uint32_t u = 0; u < KEEP; ++u)
         if (u * kRowThreads + tid < vecs) store(u * kRowThreads + tid, kept[u]);
-    for (uint32_t i = kKeep * kRowThreads + tid; i < vecs; i += kRowThreads) store(i, weigh(i, x[i]));
+    for (uint32_t i = KEEP * kRowThreads + tid; i < vecs; i += kRowThreads) store(i, weigh(x[i], weight_at(i)));
     if (tid == 0) {
-        const float inv = p.norm_w ? 1.0f / sqrtf(__fadd_rn(__fdiv_rn(ss, (float)p.k), p.eps)) : 1.0f;
+        const float inv = weight ? 1.0f / sqrtf(__fadd_rn(__fdiv_rn(ss, (float)p.k), p.eps)) : 1.0f;
         p.row_scale[row] = inv * pow2(-e);
     }
 }
@@ -479,7 +489,11 @@ int wr_split_weights_launch(wr_cuda_ctx *ctx, const wr_split_source *list, uint3
 int wr_split_rows_launch(wr_cuda_ctx *ctx, const wr_split_rows_args &a)
 {
     if (a.rows == 0 || a.k == 0 || (a.k & 3u) || (a.x_stride & 3u) || (a.ld & 7u)) return WR_CUDA_ERR_INVAL;
-    WR_CUDA_TRY(wr_launch_pdl(split_rows_kernel, dim3(a.rows), dim3(kRowThreads), 0, ctx->stream, a));
+    if (a.parts && (a.n_parts == 0 || a.n_parts > kMaxParts)) return WR_CUDA_ERR_INVAL;
+    const dim3 grid(a.rows), block(kRowThreads);
+    if (a.k <= 4 * kRowThreads) WR_CUDA_TRY(wr_launch_pdl(split_rows_kernel<1>, grid, block, 0, ctx->stream, a));
+    else if (a.k <= 8 * kRowThreads) WR_CUDA_TRY(wr_launch_pdl(split_rows_kernel<2>, grid, block, 0, ctx->stream, a));
+    else WR_CUDA_TRY(wr_launch_pdl(split_rows_kernel<4>, grid, block, 0, ctx->stream, a));
     ctx->launches++;
     WR_CUDA_TRY(cudaGetLastError());
     return WR_CUDA_OK;
