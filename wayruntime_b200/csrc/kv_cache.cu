@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(kAppendThreads) rope_kv_append_kernel(const ap
     }
 }
 
-// The same for more tokens than a decode batch (head_dim 128).  rope_kv_append_kernel spends a prompt's time on starting
+// The same for 64 tokens and more (head_dim 128).  rope_kv_append_kernel spends a prompt's time on starting
 // 256 threads per token and eight Q heads, each with a table of angles of its own, and moves two and four bytes at a
 // time.  Here a CTA has up to four tokens, their angles are worked out once, and a thread moves sixteen values of a head
 // (eight and the eight that they pair with): 64 bytes in, 32 or 64 out.  HBM bounds it from there.  2048 tokens of 8 K
@@ -680,7 +680,7 @@ struct prompt_append_params {
     __half *q16;                     // rotated Q rows as F16 instead of back into a.q_rows, or null
     uint32_t per_cta;                // tokens
 };
-constexpr uint32_t kPromptTokens = 4, kPromptHd = 128, kPromptHalf = kPromptHd / 2;
+constexpr uint32_t kPromptLeast = 64, kPromptTokens = 4, kPromptHd = 128, kPromptHalf = kPromptHd / 2;
 
 __global__ void __launch_bounds__(kAppendThreads) rope_prompt_append_kernel(const prompt_append_params p)
 {
@@ -829,12 +829,13 @@ int wr_append_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
     p.n_rot = (n_rot_pairs >= 1 && n_rot_pairs < half) ? n_rot_pairs : half;  // kernels.c:1381-1383
     p.theta = (theta_base < 1.0f) ? 10000.0f : theta_base;                    // kernels.c:1374
     p.rope = (flags & WR_CUDA_APPEND_ROPE) ? 1u : 0u;
-    // More tokens than a decode batch: the prompt kernel, where its 16-byte pieces are aligned (the line: 16 sessions' tokens
-    // take 4 us in the kernel above, and their cache bytes and rotated rows are the same in both).
+    // Many tokens: the prompt kernel, where its 16-byte pieces are aligned; cache bytes and rotated rows are the same in both.  The
+    // line: an append and attention of 17 tokens take 52.7 us (one kv head) and 21.9 (8, with 32 Q heads) with the kernel
+    // above, 53.5 and 21.9 with this one; of 64 tokens with 40 Q heads 25.2 and 24.1.
     const uint32_t n_tok = n_sess * n_tokens;
     const bool vectors = hd == kPromptHd && p.q_in == p.q_rows && (((uintptr_t)dk | (uintptr_t)dv | (uintptr_t)dq) & 15u) == 0;
     if (extra && !vectors) return WR_CUDA_ERR_UNSUPPORTED;
-    if (vectors && (n_tok > WR_CUDA_BATCH_MAX || extra)) {
+    if (vectors && (n_tok >= kPromptLeast || extra)) {
         prompt_append_params pp{};
         pp.a = p;
         if (extra) {
