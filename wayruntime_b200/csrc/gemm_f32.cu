@@ -135,7 +135,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
                     }
                 }
             }
-            if (!ok) atomicCAS(p.err, 0, 51);
+            if (!ok) atomicCAS(p.err, 0, 61);
             // nothing of this CTA's may be in flight when it leaves (gemm_bf16.cu)
             const uint32_t last = it < T::kStages ? it : T::kStages;
             for (uint32_t i = it - last; i < it; ++i)
@@ -172,7 +172,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
                 if (lead) tc5::commit(&acc_full[acc]);
             }
         }
-        if (!ok && lane == 0) atomicCAS(p.err, 0, 52);
+        if (!ok && lane == 0) atomicCAS(p.err, 0, 62);
     } else {
         const uint32_t quarter = warp & 3, c_lo = (warp - 2) / 4 * T::kCols;     // TMEM lanes and columns of this warp
         uint32_t it = 0;
@@ -245,7 +245,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
             }
             __syncwarp();
         }
-        if (!ok && lane == 0) atomicCAS(p.err, 0, 53);
+        if (!ok && lane == 0) atomicCAS(p.err, 0, 63);
     }
     tc5::fence_before();
     __syncthreads();

@@ -618,7 +618,9 @@ __global__ void __launch_bounds__(256) finish_rows_kernel(const GemvParams p, co
 
 // More rows than a decode batch: the tensor-core product of gemm_f32.cu, weights and rows split into the context's
 // workspace on the way.  17 rows are two passes of the GEMV over the weights; this is three (in, out and in again, the
-// last two in L2) whatever the rows, and the products at the tensor cores' rate.  WR_CUDA_ERR_NOMEM: no workspace.
+// last two in L2) whatever the rows, and the products at the tensor cores' rate.  Two layers of the mixed stack in F32, the whole
+// call: 17 rows of width 4096 2459 -> 1464 us, 40 of 2048 1268 -> 661, 700 of 1024 4568 -> 1172.  WR_CUDA_ERR_NOMEM: no
+// workspace.
 int launch_wide(wr_cuda_ctx *ctx, GemvParams &p)
 {
     auto up256 = [](size_t n) { return (n + 255u) & ~(size_t)255u; };

@@ -520,8 +520,8 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
         ++m->launches;
         WR_CUDA_TRY(cudaGetLastError());
     }
-    // More rows than a decode batch go through the tensor cores.  The line: 17 rows are two passes of the GEMV over the
-    // weights, which take longer than splitting the weights and one product.
+    // More rows than a decode batch go through the tensor cores.  At the line already (two layers, the whole call): 17 rows of width
+    // 1024 445 us with the GEMV and 258, 20 of width 2048 855 and 442, 33 of width 4096 3518 and 806.
     const bool wide = mode == WR_CUDA_FWD_PREFILL && n_rows > WR_CUDA_BATCH_MAX && m->prompt;
     const bool fused = wide && m->hd == 128;
     uint32_t n_parts = 0;
