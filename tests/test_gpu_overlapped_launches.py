@@ -157,3 +157,44 @@ def test_back_to_back_prefill_launches_match_single_launches():
     for kv in kvs:
         kv.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("f16", [False, True])
+def test_decode_step_behind_a_prompts_append_and_a_prefill_of_few_tiles(f16):
+    """A long prompt append, an attention call whose tiles do not cover the device and a full decode step on the same
+    layer: the step's first tiles are rows that the append writes."""
+    import torch
+    import wayruntime_b200 as wr
+    ctx = wr.Context(0)
+    n, rows, hq = 6000, 100, 32                          # 1 row tile x 16 head pairs
+    lens = [n + 1] * 16
+    k, v = (torch.from_numpy(_gen.normal(7100 + i, (n, HKV, HD))).cuda() for i in range(2))
+    q = torch.from_numpy(_gen.normal(7102, (rows, hq, HD))).cuda()
+    q = q.half() if f16 else q
+    step = [torch.from_numpy(_gen.normal(7103 + i, (16, h, HD))).cuda() for i, h in enumerate((hq, HKV, HKV))]
+    kvs = [ctx.kv_create(1, HKV, HD, n + 1) for _ in lens]
+
+    def run(between):
+        """Attention rows of the prefill and of the step; every session but the first is filled before."""
+        for kv in kvs:
+            kv.write_rows(0, 0, 0, np.zeros((n, HKV, HD), np.uint16))
+            kv.write_rows(0, 1, 0, np.zeros((n, HKV, HD), np.uint16))
+        out, got = torch.full((rows, hq, HD), float("nan"), device="cuda"), torch.full((16, hq, HD), float("nan"), device="cuda")
+        sq = step[0].clone()
+        torch.cuda.synchronize()
+        ctx.sync()
+        ctx.kv_append(kvs[:1], 0, [0], k, v, None, 0, theta=THETA, n_tokens=n)
+        between()
+        ctx.attn_prefill(kvs[0], 0, n - rows, rows, q, out, hq)
+        between()
+        ctx.decode_step(kvs, 0, [m - 1 for m in lens], sq, step[1], step[2], got, hq, theta=THETA)
+        ctx.sync()
+        return out.cpu().numpy(), got.cpu().numpy()
+
+    alone = run(ctx.sync)
+    for _ in range(4):
+        for a, b in zip(alone, run(lambda: None)):
+            assert np.isfinite(b).all() and np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    for kv in kvs:
+        kv.close()
+    ctx.close()

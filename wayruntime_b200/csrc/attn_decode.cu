@@ -410,7 +410,8 @@ extern "C" int wr_cuda_decode_step(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv
     // Early first-tile loads in the decode kernel: the append below writes one row per session, into
     // the session's last page, which those loads skip.  Every other page must be settled when the
     // decode kernel's CTAs can start: true when the kernel before the append is not one of this
-    // library's early-starting kernels, or is a decode launch that covered every SM.
+    // library's early-starting kernels, or is a decode launch that covered every SM.  (Behind a prompt's
+    // attention on part of the SMs the prompt's append may still be writing the pages.)
     const int prev = (ctx->pdl_index == ctx->launches) ? ctx->pdl_kind : WR_PDL_NONE;
     const bool early = prev == WR_PDL_NONE || prev == WR_PDL_DECODE_FULL;
     rc = wr_append_launch(ctx, n_sess, kv, layer, positions, 1, dk, dv, dq, n_q_heads, theta_base,

@@ -1140,17 +1140,19 @@ extern "C" int wr_cuda_attn_prefill(wr_cuda_ctx *ctx, wr_cuda_kv *kv, uint32_t l
         dout = (float *)(stage + off);
         WR_CUDA_TRY(cudaMemcpyAsync((void *)dq, q, q_in_bytes, cudaMemcpyHostToDevice, ctx->stream));
     }
+    if (((uintptr_t)(convert ? q16 : dq) & 15u) || ((uintptr_t)dout & 15u)) return WR_CUDA_ERR_INVAL;
     if (convert) {
         const bool vec = ((uintptr_t)dq & 15u) == 0;
         const size_t items = vec ? elems / 8 : elems;
         const uint32_t blocks = (uint32_t)std::min<size_t>((items + 255) / 256, (size_t)ctx->sm_count * 16);
         WR_CUDA_TRY(wr_launch_pdl(q_to_f16_kernel, dim3(blocks), dim3(256), 0, ctx->stream, (const float *)dq, q16, elems, vec));
         ctx->launches++;
+        ctx->pdl_kind = WR_PDL_PREFILL_PART;             // (should nothing follow it: it does not wait before it triggers)
+        ctx->pdl_index = ctx->launches;
         WR_CUDA_TRY(cudaGetLastError());
     } else {
         q16 = (__half *)dq;
     }
-    if (((uintptr_t)q16 & 15u) || ((uintptr_t)dout & 15u)) return WR_CUDA_ERR_INVAL;
 
     CUtensorMap q_map;
     const cuuint64_t dims[2] = {(cuuint64_t)n_q_heads * kHd, (cuuint64_t)n};
@@ -1210,7 +1212,7 @@ extern "C" int wr_cuda_attn_prefill(wr_cuda_ctx *ctx, wr_cuda_kv *kv, uint32_t l
     WR_CUDA_TRY(wr_launch_pdl(attn_prefill_kernel<false>, dim3(grid), dim3(kThreads), kSmemBytes, ctx->stream, q_map,
                               q_map, o_map, p));
     ctx->launches++;
-    ctx->pdl_kind = full ? WR_PDL_PREFILL_FULL : WR_PDL_NONE;
+    ctx->pdl_kind = full ? WR_PDL_PREFILL_FULL : WR_PDL_PREFILL_PART;
     ctx->pdl_index = ctx->launches;
     WR_CUDA_TRY(cudaGetLastError());
     if (host) {

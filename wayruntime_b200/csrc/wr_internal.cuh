@@ -121,7 +121,10 @@ struct wr_cuda_ctx {
     uint64_t pdl_index = ~0ull;
     int pdl_kind = 0;                // WR_PDL_*
 };
-enum { WR_PDL_NONE = 0, WR_PDL_APPEND = 1, WR_PDL_DECODE_FULL = 2, WR_PDL_DECODE_PART = 3, WR_PDL_PREFILL_FULL = 4 };
+// NONE says that nothing before the kernel that asks can still be running; a kernel that lets the next one start early
+// and does not cover every SM (PREFILL_PART) is something else: behind it the prompt append may still be writing pages.
+enum { WR_PDL_NONE = 0, WR_PDL_APPEND = 1, WR_PDL_DECODE_FULL = 2, WR_PDL_DECODE_PART = 3, WR_PDL_PREFILL_FULL = 4,
+       WR_PDL_PREFILL_PART = 5 };
 
 // What one layer of a session keeps: K/V pages, a recurrent state, both or neither.
 struct wr_kv_layer {
