@@ -166,7 +166,7 @@ def test_decode_step_behind_a_prompts_append_and_a_prefill_of_few_tiles(f16):
     import torch
     import wayruntime_b200 as wr
     ctx = wr.Context(0)
-    n, rows, hq = 6000, 100, 32                          # 1 row tile x 16 head pairs
+    n, rows, hq = 4000, 100, 32                          # 1 row tile x 16 head pairs
     lens = [n + 1] * 16
     k, v = (torch.from_numpy(_gen.normal(7100 + i, (n, HKV, HD))).cuda() for i in range(2))
     q = torch.from_numpy(_gen.normal(7102, (rows, hq, HD))).cuda()
