@@ -5,9 +5,10 @@ One layer; the attention rows that the call reports (attn_tap_out) are the fixed
 checks the split of plain and normed rows, the gate / up pairs and the sums in parts, and the V rows that reach the
 cache check the three-segment product (to one F16 step: the cache truncates).
 
-Tolerance (2-norm): each product sees both operands within 2^-24 and drops lo lo (2^-24 at most); 64 K-values add up in
-the tensor core, at most 12 additions that may each lose a unit of 2^-23, and the sums of 64 are added in F32.  That is
-under 16 * 2^-23 = 1.9e-6 for a product, and the rows pass through three of them; SiLU's slope is at most 1.1.
+Tolerance (2-norm): a product rounds its result once, the sums in parts and the residual's additions up to four times more,
+the norm's sum of squares, quotient and root at most eighteen times, SiLU and its product six: under 32 roundings of 2^-24
+for what rows pass through.  The operands are within sqrt(k) 2^-31 of their rows' length and the digit products left out within 2^-28
+of the largest ones (2^-31 in the mean square): below one rounding more for K up to 4096.
 """
 import numpy as np
 import pytest
@@ -16,13 +17,13 @@ import _gen
 from test_gpu_model_glue import _after_attention, _model, _rms, _weights
 
 pytestmark = pytest.mark.gpu
-REL = 3 * 1.1 * 16 * 2.0 ** -23
+REL = 33 * 2.0 ** -24
 
 SHAPES = [  # rows, hidden, q heads, kv heads, ffn
     (17, 132, 2, 1, 20),              # nothing aligns: one K block and a bit, eight-row groups half full
     (128, 256, 4, 2, 520), (129, 256, 4, 2, 524),
     (300, 1024, 8, 4, 1536),          # parts of K in both sums, several tiles
-    (257, 2052, 16, 8, 4100),         # tiles of 256 columns, K beyond a row's kept values
+    (257, 2052, 16, 8, 4100),         # several tiles of 128 columns, K beyond a row's kept values
     (40, 512, 10, 2, 2052),           # short prompt, four parts
 ]
 
@@ -79,6 +80,94 @@ def test_rows_of_very_different_scale_keep_their_precision():
     err = np.linalg.norm(res["hidden"] - emb - want, axis=0)
     # (a column's sums are its terms' root sum of squares or less, the bound is by their size: a factor of 4)
     assert (err <= 4 * REL * (np.linalg.norm(want, axis=0) + np.linalg.norm(emb, axis=0))).all()
+
+
+@pytest.mark.parametrize("rows,hidden,n_q,n_kv,ffn", [(200, 1024, 8, 4, 3072), (100, 2048, 16, 8, 4096), (33, 4096, 16, 8, 2048)])
+def test_rows_are_no_further_from_float64_than_those_of_the_decode_kernels(rows, hidden, n_q, n_kv, ffn):
+    import wayruntime_b200 as wr
+    shape = dict(n_layers=1, hidden=hidden, n_q_heads=n_q, n_kv_heads=n_kv, head_dim=128, vocab=515, ffn=ffn)
+    w = _weights(shape, 1400 + rows)
+    tokens = [(29 * r + 3) % shape["vocab"] for r in range(rows)]
+    emb = w["embed"][tokens]
+    ctx = wr.Context(0)
+    dm = _model(ctx, w, shape, max_rows=256)
+    err = []
+    for portion in (rows, 16):                       # (up to sixteen rows go through the F32 kernels)
+        kv, got, attn = ctx.kv_create(1, n_kv, 128, rows), [], []
+        for at in range(0, rows, portion):
+            res = dm.forward(dm.FWD_PREFILL, [kv], [at], tokens[at:at + portion], hidden=True, attn_tap=True)
+            got.append(res["hidden"])
+            attn.append(res["attn"][0])
+        want = _after_attention(w, emb, np.concatenate(attn))
+        err.append(np.linalg.norm(np.concatenate(got) - want) / np.linalg.norm(want - emb))
+        kv.close()
+    dm.close()
+    ctx.close()
+    assert err[0] <= err[1], err
+
+
+def test_weight_rows_of_one_entry_and_of_small_integers():
+    """Products of one term and sums of whole multiples: nothing but the result's own rounding, and that of the activations
+    to 2^-31 of their row's largest."""
+    shape = dict(n_layers=1, hidden=256, n_q_heads=4, n_kv_heads=2, head_dim=128, vocab=64, ffn=256)
+    w = _weights(shape, 1305, tied=False)
+    w["embed"][:, :128] = 0.0                        # nothing to add the first channels to
+    w["l0.w_down"][:128] = 0.0
+    wo = w["l0.wo"]
+    wo[:128] = 0.0
+    for n in range(64):
+        wo[n, 5 * n] = (3 + n) * 2.0 ** (n % 9 - 4)
+    wo[64:128] = np.random.default_rng(1306).integers(-4, 5, (64, wo.shape[1]))
+    tokens = [(5 * r + 1) % 64 for r in range(150)]
+    res, _ = _run(shape, 150, w, 256, tokens)
+    attn = res["attn"][0].astype(np.float64)
+    want = attn @ wo[:128].astype(np.float64).T
+    top = np.abs(attn).max(axis=1)[:, None] * np.abs(wo[:128].astype(np.float64)).sum(axis=1)
+    assert (np.abs(res["hidden"][:, :128] - want) <= 2.0 ** -24 * np.abs(want) + 2.0 ** -31 * top).all()
+
+
+def test_factors_far_from_one_do_not_overflow_on_the_way():
+    """Feed-forward values near 2^-112 under weights near 2^110: the product is of ordinary size."""
+    shape = dict(n_layers=1, hidden=256, n_q_heads=4, n_kv_heads=2, head_dim=128, vocab=64, ffn=512)
+    w = _weights(shape, 1307, tied=False)
+    w["l0.w_up"] *= np.float32(2.0 ** -112)
+    w["l0.w_down"] *= np.float32(2.0 ** 112)
+    tokens = [(5 * r + 1) % 64 for r in range(40)]
+    res, v = _run(shape, 40, w, 64, tokens)
+    _check(res, v, w, tokens)
+
+
+def test_infinities_are_what_the_decode_kernels_make_of_them():
+    """Infinite weights, and infinite feed-forward values: the same results are infinite, with the same sign, or not numbers."""
+    import wayruntime_b200 as wr
+    shape = dict(n_layers=1, hidden=1024, n_q_heads=16, n_kv_heads=2, head_dim=128, vocab=64, ffn=2052)
+    w = _weights(shape, 1308, tied=False)
+    down = w["l0.w_down"].copy()
+    w["l0.w_down"][5, 2000] = -np.inf                # (sums of K's second part)
+    w["l0.w_down"][6, 41] = np.nan
+    w["l0.w_down"][700, 5], w["l0.w_down"][700, 1900] = np.inf, -np.inf
+    tokens = [(5 * r + 1) % 64 for r in range(48)]
+    ctx = wr.Context(0)
+
+    def both():
+        dm, out = _model(ctx, w, shape, max_rows=64), []
+        for portion in (48, 16):
+            kv = ctx.kv_create(1, 2, 128, 48)
+            out.append(np.concatenate([dm.forward(dm.FWD_PREFILL, [kv], [at], tokens[at:at + portion], hidden=True)["hidden"]
+                                       for at in range(0, 48, portion)]))
+            kv.close()
+        dm.close()
+        kinds = [np.where(np.isnan(o), 2, np.where(np.isinf(o), np.sign(o), 0)) for o in out]
+        assert np.array_equal(kinds[0], kinds[1])
+        return kinds[0]
+
+    kinds = both()
+    assert all((kinds == i).any() for i in (-1, 0, 1, 2))
+    w["l0.w_down"] = down
+    w["l0.w_up"][43, 7] = np.inf
+    kinds = both()
+    assert all((kinds == i).any() for i in (-1, 1))
+    ctx.close()
 
 
 def test_a_row_with_an_infinity_ends_not_finite_and_leaves_the_rows_before_it():

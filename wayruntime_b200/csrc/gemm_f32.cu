@@ -2,20 +2,17 @@
 //
 // What bounds it: F32 FMAs.  The GEMV kernels (gemv.cu) stream the weights once per 16 rows; a prompt of 1000 rows of the
 // Qwen3-0.6B shape took 121 ms = 8 TFLOP/s with them, and the FMA pipes as a whole end near 70.  The tensor cores have no
-// F32 multiplier, but F32 values are two F16 values each (gemm_f32.cuh), and
-//     x w = hi hi + (hi lo + lo hi) + lo lo,      the last term 2^-24 of the first and left out:
-// three F16 products for one F32 product, a third of the tensor rate.
-//
-// Sums: tcgen05 adds into an F32 accumulator and rounds every sum towards zero; a K of thousands would lose hundreds of
-// such roundings, all in one direction.  So an accumulator holds 64 K-values only (cross terms first, while it is small, then
-// four additions of the large ones); eight warps fetch it and add it to F32 registers that keep what rounding loses
-// (Kahan).  What the four roundings take on average is known, kTowardsZero, and put back at the end.  Error of one layer of
-// products against float64 (2-norm), widths 1024 / 2048 / 4096: the GEMV 2.2 / 2.5 / 3.0e-7, accumulators of 64 K-values with plain
-// sums 3.6 / 4.1 / 4.7e-7, this 2.4 / 2.5 / 2.5e-7.
-// Accumulators: four of 128 columns, so that the fetch may lag behind.  A kept remainder in F32 would not fit the registers: with
-// spills the fetch, not the products, set the pace (1000 x 4096 x 1024: 49.7 us, 37.3 without them; nothing fetched: 31.0).
-// 1000 rows, us: 4096 x 1024 37, 6144 x 1024 58, 1024 x 3072 26 (= 660 to 740 TFLOP/s of F16 products, 220 to 245 of F32 ones).
-// Stages: 64 K-values of hi and lo of both operands.  Persistent CTAs, tiles of 128 x BN, m fastest: the tiles in flight
+// F32 multiplier, and in their F32 accumulators every sum is rounded towards zero; but they add integers exactly.  So a row is
+// held as 32-bit integers under one power of two (gemm_f32.cuh), an integer as four signed digits of base 256,
+//     x w = sum over i, j of x_i w_j 256^(6 - i - j),
+// and the ten digit products with i + j <= 3 are summed over K into four S32 accumulators, one for each i + j.  Nothing is
+// rounded until they are put together, once per result, in 64 bits.  The six products left out are below 2^-28 of the product of
+// the two rows' largest values, and 2^-31 of it in the mean square.
+// Error of one product against float64 (2-norm; rounding the exact result to F32 is 2.5e-8), K of 1024 / 2048 / 4096 and Gaussian
+// rows: the GEMV 9.5e-8 / 1.1e-7 / 1.3e-7, this 4.5e-8 / 3.6e-8 / 3.6e-8 (with the rounding of the residual that it is added to).
+// 1000 rows, us: 4096 x 1024 35.6, gate / up of 2 x 3072 x 1024 53.9, 1024 x 3072 26.2: 2300 to 2450 TOP/s of digit products, 230 to
+// 245 TFLOP/s of F32 ones.  Sixteen warps fetch: with eight the gate / up product takes 63.2.
+// Stages: 64 K-values, all digits of both operands.  Persistent CTAs, tiles of 128 x BN, m fastest: the tiles in flight
 // share weight rows in L2.
 #include <math.h>
 
@@ -28,26 +25,26 @@
 namespace {
 
 constexpr uint32_t kBM = 128, kBK = 64;
-constexpr uint32_t kEpiWarps = 8, kThreads = 64 + 32 * kEpiWarps;
-constexpr uint32_t kABytes = kBM * kBK * 2;          // one of hi / lo
-constexpr uint32_t kAccs = 4;
-// Rounding a sum towards zero takes half a unit of its last place on average: 2^-24 times the mean of 1 / mantissa, which
-// is 1 / (2 ln 2) for mantissas spread evenly over their logarithm.  Of four additions of like size the j-th has j / 4 of
-// the final value: 2.5 times that.
-constexpr float kTowardsZero = 2.5f * 0.7213f * 5.9604645e-8f;
+constexpr uint32_t kEpiWarps = 16, kThreads = 64 + 32 * kEpiWarps;
+constexpr uint32_t kABytes = kBM * kBK * 2;          // two digits of a stage's values
+constexpr uint32_t kDiags = 4;
+constexpr uint32_t kPartMost = 32704;                // |one accumulator| <= 4 * 2^14 * K < 2^31
 
 template <uint32_t BN> struct Tile {
     static constexpr uint32_t kBBytes = BN * kBK * 2;
     static constexpr uint32_t kStageBytes = 2 * (kABytes + kBBytes);
     static constexpr uint32_t kStages = 196608 / kStageBytes;        // 3 or 4
     static constexpr uint32_t kSmem = kStages * kStageBytes + 1024;
-    static constexpr uint32_t kTmemCols = kAccs * BN;
-    static constexpr uint32_t kCols = BN / 2;                        // columns a warp finishes
+    static constexpr uint32_t kAccs = 128 / BN;                      // sets of accumulators
+    static constexpr uint32_t kTmemCols = 512;
+    static constexpr uint32_t kCols = BN / 4;                        // columns a warp finishes
 };
+// Sums of i + j = 0, 2, 1, 3 lie side by side in this order: digits q and q + 2 of a weight lie BN rows apart in shared
+// memory, and one instruction of twice the width takes a digit of x with both.
+__host__ __device__ constexpr uint32_t diag_at(uint32_t d) { return d == 1 ? 2u : d == 2 ? 1u : d; }
 
 struct GemmParams {
     wr_f32_gemm_args a;
-    wr_split_weight w;
     uint32_t m_tiles, n_tiles, k_blocks, part_blocks;
     long long wait_limit;
     int *err;
@@ -58,32 +55,63 @@ __device__ __forceinline__ float silu_mul(float g, float u)
     return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u);
 }
 
-__device__ __forceinline__ uint64_t pair2(float lo, float hi)
+__device__ __forceinline__ float pow2(int e) { return __int_as_float((e + 127) << 23); }
+
+// Sixteen results of a thread as they go out: values y of row `row`, columns n on.
+__device__ __forceinline__ void put16(const GemmParams &p, const float (&y)[16], uint32_t part, uint32_t row, uint32_t n_at)
 {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
+    if (p.a.source.pair) {
+        float *o = p.a.seg[0].out + (size_t)row * p.a.seg[0].ld + n_at / 2;
+        float z[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) z[i] = silu_mul(y[i], y[8 + i]);
+        *reinterpret_cast<float4 *>(o) = make_float4(z[0], z[1], z[2], z[3]);
+        if (p.a.seg[0].n - n_at / 2 > 4)                         // (a multiple of 4)
+            *reinterpret_cast<float4 *>(o + 4) = make_float4(z[4], z[5], z[6], z[7]);
+        return;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i += 4) {
+        uint32_t n = n_at + i, s = 0;
+        if (n >= p.a.source.to.n) continue;
+        while (s + 1 < p.a.n_seg && n >= p.a.seg[s].n) n -= p.a.seg[s++].n;
+        float *o = p.a.seg[s].out + ((size_t)part * p.a.m + row) * p.a.seg[s].ld + n;
+        *reinterpret_cast<float4 *>(o) = make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
+    }
 }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+
+// The same where a power of two is not a normal F32 number, or an infinity or a NaN is among the factors.  The latter is what
+// plain F32 arithmetic makes of it (kNotFinite is no exponent's size, and no two exponents' sum).
+__device__ __noinline__ void put16_rare(const GemmParams &p, const float *raw, const wr_split_scale rs, uint32_t part, uint32_t row,
+                                        uint32_t n_at, uint32_t k_lo, uint32_t k_hi)
 {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
+    const wr_f32_gemm_args &a = p.a;
+    float y[16];
+#pragma unroll 1
+    for (uint32_t i = 0; i < 16; ++i) {
+        y[i] = 0.f;
+        if (n_at + i >= a.source.to.n) continue;
+        const int e = rs.exponent + a.source.to.exponent[n_at + i];
+        if (e < kNotFinite / 2) {
+            const int first = min(max(e, -126), 127);
+            y[i] = raw[i] * pow2(first) * pow2(min(max(e - first, -126), 127));
+        } else {
+            const float *w = wr_split_row(a.source, n_at + i), *x = a.x + (size_t)row * a.x_stride;
+            for (uint32_t k = k_lo; k < min(k_hi, a.source.to.k); ++k)
+                y[i] = fmaf(a.norm_w ? __fmul_rn(x[k], a.norm_w[k]) : x[k], w ? w[k] : 0.f, y[i]);
+        }
+        y[i] = __fmul_rn(y[i], rs.factor);
+    }
+    put16(p, y, part, row, n_at);
 }
 
 template <uint32_t BN>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
+gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ GemmParams p)
 {
     using T = Tile<BN>;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full[T::kStages], empty[T::kStages], acc_full[kAccs], acc_empty[kAccs];
+    __shared__ __align__(8) uint64_t full[T::kStages], empty[T::kStages], acc_full[T::kAccs], acc_empty[T::kAccs];
     __shared__ uint32_t tmem_slot;
     uint8_t *stages = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023u) & ~(uintptr_t)1023u);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -93,7 +121,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
         }
-        for (uint32_t i = 0; i < kAccs; ++i) {
+        for (uint32_t i = 0; i < T::kAccs; ++i) {
             mbar_init(&acc_full[i], 1);
             mbar_init(&acc_empty[i], kEpiWarps);
         }
@@ -104,20 +132,21 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
     __syncthreads();
     tc5::fence_after();
     const uint32_t tmem = tmem_slot;
+    const wr_split_weight &w = p.a.source.to;
     pdl_wait();
     // a unit of work: a tile, and a part of K
     const uint32_t tiles = p.m_tiles * p.n_tiles, units = tiles * p.a.k_parts;
 
     if (warp == 0) {
         if (lane == 0) {
-            const size_t lo_off = (size_t)wr_weight_blocks(p.w.n) * p.k_blocks * kWBlockBytes;
+            const size_t lo_off = (size_t)wr_weight_blocks(w.n) * p.k_blocks * kWBlockBytes;
             uint32_t it = 0;
             bool ok = true;
             for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
                 const uint32_t tile = unit % tiles, k_lo = unit / tiles * p.part_blocks;
                 const uint32_t k_hi = min(k_lo + p.part_blocks, p.k_blocks);
                 const uint32_t m0 = (tile % p.m_tiles) * kBM, nb0 = (tile / p.m_tiles) * (BN / kWBlock);
-                const uint32_t nb = min(BN / kWBlock, wr_weight_blocks(p.w.n) - nb0);
+                const uint32_t nb = min(BN / kWBlock, wr_weight_blocks(w.n) - nb0);
                 for (uint32_t kb = k_lo; kb < k_hi; ++kb, ++it) {
                     const uint32_t st = it % T::kStages;
                     if (it >= T::kStages && !mbar_wait(&empty[st], (it / T::kStages - 1) & 1, p.wait_limit)) {
@@ -128,14 +157,14 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
                     mbar_expect_tx(&full[st], 2 * (kABytes + nb * kWBlockBytes));
                     tc5::tma_load_2d(a, &x_map, (int)(kb * kBK), (int)m0, &full[st]);
                     tc5::tma_load_2d(a + kABytes, &x_map, (int)(kb * kBK), (int)(p.a.pad + m0), &full[st]);
-                    const char *w = p.w.blocks + ((size_t)nb0 * p.k_blocks + kb) * kWBlockBytes;
-                    for (uint32_t i = 0; i < nb; ++i, w += (size_t)p.k_blocks * kWBlockBytes) {
-                        bulk_g2s(b + i * kWBlockBytes, w, kWBlockBytes, &full[st]);
-                        bulk_g2s(b + T::kBBytes + i * kWBlockBytes, w + lo_off, kWBlockBytes, &full[st]);
+                    const char *from = w.blocks + ((size_t)nb0 * p.k_blocks + kb) * kWBlockBytes;
+                    for (uint32_t i = 0; i < nb; ++i, from += (size_t)p.k_blocks * kWBlockBytes) {
+                        bulk_g2s(b + i * kWBlockBytes, from, kWBlockBytes, &full[st]);
+                        bulk_g2s(b + T::kBBytes + i * kWBlockBytes, from + lo_off, kWBlockBytes, &full[st]);
                     }
                 }
             }
-            if (!ok) atomicCAS(p.err, 0, 61);
+            if (!ok) atomicCAS(p.err, 0, 71);
             // nothing of this CTA's may be in flight when it leaves (gemm_bf16.cu)
             const uint32_t last = it < T::kStages ? it : T::kStages;
             for (uint32_t i = it - last; i < it; ++i)
@@ -143,109 +172,101 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
         }
     } else if (warp == 1) {
         const bool lead = tc5::elect_one();
-        const uint32_t idesc = tc5::idesc_f16(kBM, BN);
-        uint32_t it = 0;
+        constexpr uint32_t one = tc5::idesc_i8(kBM, BN), two = tc5::idesc_i8(kBM, 2 * BN);
+        uint32_t it = 0, turn = 0;
         bool ok = true;
-        for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+        for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x, ++turn) {
             const uint32_t k_lo = unit / tiles * p.part_blocks, k_hi = min(k_lo + p.part_blocks, p.k_blocks);
+            const uint32_t acc = turn % T::kAccs, d = tmem + acc * kDiags * BN;
+            if (turn >= T::kAccs && !mbar_wait(&acc_empty[acc], (turn / T::kAccs - 1) & 1, p.wait_limit)) {
+                ok = false;
+                break;
+            }
             for (uint32_t kb = k_lo; kb < k_hi; ++kb, ++it) {
-                const uint32_t st = it % T::kStages, acc = it % kAccs;
-                if ((it >= kAccs && !mbar_wait(&acc_empty[acc], (it / kAccs - 1) & 1, p.wait_limit)) ||
-                    !mbar_wait(&full[st], (it / T::kStages) & 1, p.wait_limit)) {
+                const uint32_t st = it % T::kStages;
+                if (!mbar_wait(&full[st], (it / T::kStages) & 1, p.wait_limit)) {
                     ok = false;
                     break;
                 }
                 tc5::fence_after();
                 const uint32_t a_addr = smem_u32(stages + st * T::kStageBytes), b_addr = a_addr + 2 * kABytes;
-                const uint64_t ah = tc5::desc_kmajor(a_addr), al = tc5::desc_kmajor(a_addr + kABytes);
-                const uint64_t bh = tc5::desc_kmajor(b_addr), bl = tc5::desc_kmajor(b_addr + T::kBBytes);
-                const uint32_t d = tmem + acc * BN;
+                // digit i of 32 K-values: 64 bytes in a row for an odd one, the second half of the stage from 2 on
+                auto a_of = [&](uint32_t i, uint32_t kk) { return tc5::desc_kmajor(a_addr + (i >> 1) * kABytes) + 4 * (i & 1) + 2 * kk; };
+                auto b_of = [&](uint32_t i, uint32_t kk) { return tc5::desc_kmajor(b_addr) + 4 * (i & 1) + 2 * kk; };
+                if (lead) {
 #pragma unroll
-                for (uint32_t kk = 0; kk < kBK / 16; ++kk) {
-                    if (lead) tc5::mma_ss(d, al + 2 * kk, bh + 2 * kk, idesc, kk != 0);
-                    if (lead) tc5::mma_ss(d, ah + 2 * kk, bl + 2 * kk, idesc, 1);
+                    for (uint32_t kk = 0; kk < kBK / 32; ++kk) {
+                        const uint32_t more = kb != k_lo || kk != 0;
+                        tc5::mma_i8_ss(d + diag_at(0) * BN, a_of(0, kk), b_of(0, kk), two, more);      // 0 0, 0 2
+                        tc5::mma_i8_ss(d + diag_at(1) * BN, a_of(0, kk), b_of(1, kk), two, more);      // 0 1, 0 3
+                        tc5::mma_i8_ss(d + diag_at(1) * BN, a_of(1, kk), b_of(0, kk), two, 1);         // 1 0, 1 2
+                        tc5::mma_i8_ss(d + diag_at(2) * BN, a_of(1, kk), b_of(1, kk), one, 1);
+                        tc5::mma_i8_ss(d + diag_at(2) * BN, a_of(2, kk), b_of(0, kk), one, 1);
+                        tc5::mma_i8_ss(d + diag_at(3) * BN, a_of(2, kk), b_of(1, kk), one, 1);
+                        tc5::mma_i8_ss(d + diag_at(3) * BN, a_of(3, kk), b_of(0, kk), one, 1);
+                    }
+                    tc5::commit(&empty[st]);
+                    if (kb + 1 == k_hi) tc5::commit(&acc_full[acc]);
                 }
-#pragma unroll
-                for (uint32_t kk = 0; kk < kBK / 16; ++kk)
-                    if (lead) tc5::mma_ss(d, ah + 2 * kk, bh + 2 * kk, idesc, 1);
-                if (lead) tc5::commit(&empty[st]);
-                if (lead) tc5::commit(&acc_full[acc]);
+                __syncwarp();
             }
         }
-        if (!ok && lane == 0) atomicCAS(p.err, 0, 62);
+        if (!ok && lane == 0) atomicCAS(p.err, 0, 72);
     } else {
         const uint32_t quarter = warp & 3, c_lo = (warp - 2) / 4 * T::kCols;     // TMEM lanes and columns of this warp
-        uint32_t it = 0;
+        uint32_t turn = 0;
         bool ok = true;
-        for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
-            const uint32_t tile = unit % tiles, part = unit / tiles, k_lo = part * p.part_blocks;
-            const uint32_t k_hi = min(k_lo + p.part_blocks, p.k_blocks);
+        for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x, ++turn) {
+            const uint32_t tile = unit % tiles, part = unit / tiles, acc = turn % T::kAccs;
+            const uint32_t k_lo = part * p.part_blocks * kBK, k_hi = k_lo + p.part_blocks * kBK;
             const uint32_t row = (tile % p.m_tiles) * kBM + quarter * 32 + lane, n0 = (tile / p.m_tiles) * BN + c_lo;
-            // pairs; `lost` is what the sums' rounding took, itself rounded to two BF16 (2^-33 of the sum: as F32 it
-            // would not fit the registers)
-            uint64_t sum[T::kCols / 2];
-            uint32_t lost[T::kCols / 2];
-#pragma unroll
-            for (uint32_t c = 0; c < T::kCols / 2; ++c) sum[c] = lost[c] = 0;
-            for (uint32_t kb = k_lo; kb < k_hi; ++kb, ++it) {
-                const uint32_t acc = it % kAccs;
-                if (!mbar_wait(&acc_full[acc], (it / kAccs) & 1, p.wait_limit)) {
-                    ok = false;
-                    break;
-                }
-                tc5::fence_after();
-#pragma unroll
-                for (uint32_t c0 = 0; c0 < T::kCols; c0 += 16) {
-                    float v[16];
-                    tc5::ld16(tmem + ((quarter * 32) << 16) + acc * BN + c_lo + c0, v);
-                    tc5::wait_ld();
-#pragma unroll
-                    for (uint32_t c = 0; c < 16; c += 2) {
-                        uint64_t &s = sum[(c0 + c) / 2];
-                        uint32_t &l = lost[(c0 + c) / 2];
-                        const uint64_t old = pair2(__uint_as_float(l << 16), __uint_as_float(l & 0xffff0000u));
-                        const uint64_t y = sub2(pair2(v[c], v[c + 1]), old), t = add2(s, y), e = sub2(sub2(t, s), y);
-                        asm("cvt.rn.bf16x2.f32 %0, %1, %2;"
-                            : "=r"(l) : "f"(__uint_as_float((uint32_t)(e >> 32))), "f"(__uint_as_float((uint32_t)e)));
-                        s = t;
-                    }
-                }
-                tc5::fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[acc]);
+            const bool in = row < p.a.m;
+            const wr_split_scale rs = in ? p.a.row_scale[row] : wr_split_scale{0.f, 0};
+            if (!mbar_wait(&acc_full[acc], (turn / T::kAccs) & 1, p.wait_limit)) {
+                ok = false;
+                break;
             }
-            if (ok && row < p.a.m) {
-                const float rs = p.a.row_scale[row];
-                auto value = [&](uint32_t c) {
-                    const float y = __uint_as_float((uint32_t)(sum[c / 2] >> (32 * (c & 1u))));
-                    return __fmul_rn(__fmul_rn(fmaf(y, kTowardsZero, y), __ldg(p.w.unscale + n0 + c)), rs);
-                };
-                if (p.a.pair) {
+            tc5::fence_after();
+#pragma unroll 1
+            for (uint32_t c = 0; c < T::kCols; c += 16) {
+                int v[kDiags][16];
 #pragma unroll
-                    for (uint32_t c = 0; c < T::kCols; c += 16) {
-                        if (n0 + c >= p.w.n) continue;
-                        float *o = p.a.seg[0].out + (size_t)row * p.a.seg[0].ld + (n0 + c) / 2;
-                        float y[8];
+                for (uint32_t d = 0; d < kDiags; ++d)
+                    tc5::ld16(tmem + ((quarter * 32) << 16) + (acc * kDiags + diag_at(d)) * BN + c_lo + c, reinterpret_cast<float *>(v[d]));
+                tc5::wait_ld();
+                if (c + 16 == T::kCols) {                        // the next tile may have the accumulators
+                    tc5::fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[acc]);
+                }
+                if (!in || n0 + c >= w.n) continue;
+                float y[16];
+                bool odd = false;
 #pragma unroll
-                        for (uint32_t e = 0; e < 8; ++e) y[e] = silu_mul(value(c + e), value(c + 8 + e));
-                        const uint32_t left = p.a.seg[0].n - (n0 + c) / 2;           // (a multiple of 4)
-                        *reinterpret_cast<float4 *>(o) = make_float4(y[0], y[1], y[2], y[3]);
-                        if (left > 4) *reinterpret_cast<float4 *>(o + 4) = make_float4(y[4], y[5], y[6], y[7]);
+                for (uint32_t i = 0; i < 16; i += 4) {
+                    const int4 we = __ldg(reinterpret_cast<const int4 *>(w.exponent + n0 + c + i));
+                    const int es[4] = {we.x, we.y, we.z, we.w};
+#pragma unroll
+                    for (uint32_t j = i; j < i + 4; ++j) {
+                        const long long t = (long long)v[0][j] * (1 << 24) + (long long)v[1][j] * (1 << 16) + (long long)v[2][j] * 256 + v[3][j];
+                        const int e = rs.exponent + es[j - i];
+                        odd = odd || (uint32_t)(e + 126) > 253u;
+                        v[0][j] = __float_as_int(__ll2float_rn(t));
+                        y[j] = __fmul_rn(__int_as_float(v[0][j]) * pow2(e), rs.factor);
                     }
+                }
+                if (!odd) {
+                    put16(p, y, part, row, n0 + c);
                 } else {
+                    float raw[16];
 #pragma unroll
-                    for (uint32_t c = 0; c < T::kCols; c += 4) {
-                        uint32_t n = n0 + c, s = 0;
-                        if (n >= p.w.n) continue;
-                        while (s + 1 < p.a.n_seg && n >= p.a.seg[s].n) n -= p.a.seg[s++].n;
-                        float *o = p.a.seg[s].out + ((size_t)part * p.a.m + row) * p.a.seg[s].ld + n;
-                        *reinterpret_cast<float4 *>(o) = make_float4(value(c), value(c + 1), value(c + 2), value(c + 3));
-                    }
+                    for (uint32_t i = 0; i < 16; ++i) raw[i] = __int_as_float(v[0][i]);
+                    put16_rare(p, raw, rs, part, row, n0 + c, k_lo, k_hi);
                 }
             }
             __syncwarp();
         }
-        if (!ok && lane == 0) atomicCAS(p.err, 0, 63);
+        if (!ok && lane == 0) atomicCAS(p.err, 0, 73);
     }
     tc5::fence_before();
     __syncthreads();
@@ -255,20 +276,39 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
 
 // ---- splitting
 
-// Power of two that puts a row whose largest |x| has these bits into [2^14, 2^15).  Rows of zeros, and rows that hold
-// infinities or NaNs (products of which are not finite either way), stay as they are.
+// What a row whose largest |x| has these bits is multiplied by, as an exponent: the largest power of two that leaves all of it within
+// four signed digits, |x| <= 0x7f7f7f7f.
 __device__ __forceinline__ int scale_exponent(uint32_t max_bits)
 {
-    if (max_bits == 0 || max_bits >= 0x7f800000u) return 0;
-    const int e = (int)(max_bits >> 23) - 127;            // (denormal rows: -127)
-    return min(14 - e, 126);
+    const int e = max(max_bits >> 23, 1u) - 127;          // (denormal rows: -126)
+    return ((max_bits & 0x7fffffu) <= 0x7efefeu ? 30 : 29) - e;
 }
-__device__ __forceinline__ float pow2(int e) { return __int_as_float((e + 127) << 23); }
-
-__device__ __forceinline__ void split4(const float4 v, float scale, uint2 &hi, uint2 &lo)
+// The exponent that undoes it; infinities and NaNs are marked.
+__device__ __forceinline__ int undo_exponent(uint32_t max_bits)
 {
-    split_half2(v.x * scale, v.y * scale, hi.x, lo.x);
-    split_half2(v.z * scale, v.w * scale, hi.y, lo.y);
+    return max_bits >= 0x7f800000u ? kNotFinite : max_bits == 0 ? 0 : -scale_exponent(max_bits);
+}
+struct Scale {
+    float a, b;                                           // two factors: together up to 2^156
+    __device__ __forceinline__ explicit Scale(uint32_t max_bits)
+    {
+        const int s = max_bits >= 0x7f800000u || max_bits == 0 ? 0 : scale_exponent(max_bits);
+        a = pow2(min(s, 126));
+        b = pow2(max(s - 126, 0));
+    }
+};
+
+// Digits of four values: w[i] holds digit i (0 the highest) of each.  x + 0x80808080 has digit + 128 in every byte.
+__device__ __forceinline__ void digits4(const float4 v, const Scale &s, uint32_t (&w)[4])
+{
+    auto bytes = [&](float x) { return ((uint32_t)__float2int_rn(x * s.a * s.b) + 0x80808080u) ^ 0x80808080u; };
+    const uint32_t x = bytes(v.x), y = bytes(v.y), z = bytes(v.z), u = bytes(v.w);
+    const uint32_t xy_lo = __byte_perm(x, y, 0x5140), zu_lo = __byte_perm(z, u, 0x5140);
+    const uint32_t xy_hi = __byte_perm(x, y, 0x7362), zu_hi = __byte_perm(z, u, 0x7362);
+    w[3] = __byte_perm(xy_lo, zu_lo, 0x5410);
+    w[2] = __byte_perm(xy_lo, zu_lo, 0x7632);
+    w[1] = __byte_perm(xy_hi, zu_hi, 0x5410);
+    w[0] = __byte_perm(xy_hi, zu_hi, 0x7632);
 }
 __device__ __forceinline__ uint32_t abs_bits(const float4 v)
 {
@@ -284,8 +324,8 @@ struct SplitWeights {
 
 constexpr uint32_t kSplitWarps = 8;
 
-// A warp per weight row: the largest magnitude, then hi and lo pieces of eight values, 128 bytes of a block row per eight
-// lanes.  HBM: 4 bytes in per weight; the 4 bytes out stay in L2 (a layer at a time) until the product has read them.
+// A warp per weight row: the largest magnitude, then the digits, eight values to a lane: 64 bytes of each digit per eight lanes.
+// HBM bounds it: 4 bytes in per weight and 4 out (which stay in L2 where a few MB are split for the product that follows).
 __global__ void __launch_bounds__(32 * kSplitWarps) split_weights_kernel(const SplitWeights p)
 {
     pdl_trigger();
@@ -294,15 +334,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps) split_weights_kernel(const S
     if (i) g -= p.end[i - 1];
     const wr_split_source &s = p.s[i];
     const uint32_t lane = threadIdx.x & 31, row = g * kSplitWarps + (threadIdx.x >> 5), k = s.to.k;
-    const float *src = nullptr;
-    if (s.pair) {
-        const uint32_t at = row / 16 * 8 + row % 8;
-        if (at < s.n[0]) src = s.src[row / 8 & 1] + (size_t)at * k;
-    } else {
-        uint32_t at = row, j = 0;
-        while (j < 2 && at >= s.n[j]) at -= s.n[j++];
-        if (at < s.n[j]) src = s.src[j] + (size_t)at * k;
-    }
+    const float *src = wr_split_row(s, row);
     // weights are read before the wait: nothing ever writes them
     const uint32_t k_pad = (k + kWBlock - 1) / kWBlock * kWBlock;
     constexpr uint32_t kKeep = 4;                        // pieces of eight values that a lane holds
@@ -324,18 +356,17 @@ __global__ void __launch_bounds__(32 * kSplitWarps) split_weights_kernel(const S
         top = max(top, max(abs_bits(v[0]), abs_bits(v[1])));
     }
     top = __reduce_max_sync(0xffffffffu, top);
-    const int e = scale_exponent(top);
-    const float scale = pow2(e);
+    const Scale scale(top);
     pdl_wait();                                          // the blocks are read by the product before
     if (row >= wr_weight_blocks(s.to.n) * kWBlock) return;
     const size_t lo_off = (size_t)wr_weight_blocks(s.to.n) * (k_pad / kWBlock) * kWBlockBytes;
     auto store = [&](uint32_t at, const float4 (&v)[2]) {
-        uint2 h0, l0, h1, l1;
-        split4(v[0], scale, h0, l0);
-        split4(v[1], scale, h1, l1);
-        char *to = s.to.blocks + wr_weight_off(k, row, at);
-        *reinterpret_cast<uint4 *>(to) = make_uint4(h0.x, h0.y, h1.x, h1.y);
-        *reinterpret_cast<uint4 *>(to + lo_off) = make_uint4(l0.x, l0.y, l1.x, l1.y);
+        uint32_t a[4], b[4];
+        digits4(v[0], scale, a);
+        digits4(v[1], scale, b);
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i)
+            *reinterpret_cast<uint2 *>(s.to.blocks + (i >> 1) * lo_off + wr_split_off(k, row, i & 1, at)) = make_uint2(a[i], b[i]);
     };
 #pragma unroll
     for (uint32_t u = 0; u < kKeep; ++u)
@@ -345,7 +376,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps) split_weights_kernel(const S
         load(at, v);
         store(at, v);
     }
-    if (lane == 0 && row < s.to.n) s.to.unscale[row] = pow2(-e);
+    if (lane == 0 && row < s.to.n) s.to.exponent[row] = undo_exponent(top) + 24;     // (digit products are in units of 2^24)
 }
 
 constexpr uint32_t kRowThreads = 256, kMaxParts = 4;
@@ -359,7 +390,7 @@ __global__ void __launch_bounds__(kRowThreads, KEEP == 1 ? 5 : 4) split_rows_ker
     __shared__ float part_ss[kRowThreads / 32];
     __shared__ uint32_t part_top[kRowThreads / 32];
     pdl_trigger();
-    const uint32_t row = blockIdx.x, tid = threadIdx.x, vecs = p.k / 4;
+    const uint32_t row = blockIdx.x, tid = threadIdx.x, vecs = p.k / 4, padded = (p.k + kWBlock - 1) / kWBlock * kWBlock / 4;
     float4 *x = reinterpret_cast<float4 *>(p.x + (size_t)row * p.x_stride);
     const float4 *parts = reinterpret_cast<const float4 *>(p.parts + (p.parts ? (size_t)row * p.k : 0));
     const float4 *weight = reinterpret_cast<const float4 *>(p.norm_w);
@@ -419,27 +450,29 @@ __global__ void __launch_bounds__(kRowThreads, KEEP == 1 ? 5 : 4) split_rows_ker
         ss += part_ss[i];
         top = max(top, part_top[i]);
     }
-    const int e = scale_exponent(top);
-    const float scale = pow2(e);
-    __half *hi = p.out + (size_t)row * p.ld, *lo = p.out + (size_t)(p.pad + row) * p.ld;
+    const Scale scale(top);
+    char *out = reinterpret_cast<char *>(p.out) + (size_t)row * p.ld * 2;
+    const size_t lo_off = (size_t)p.pad * p.ld * 2;
     auto store = [&](uint32_t i, float4 v) {
-        uint2 h, l;
-        split4(v, scale, h, l);
-        *reinterpret_cast<uint2 *>(hi + 4 * i) = h;
-        *reinterpret_cast<uint2 *>(lo + 4 * i) = l;
+        uint32_t w[4];
+        digits4(v, scale, w);
+        char *to = out + i / 16 * 128 + i % 16 * 4;              // (64 K-values: 64 bytes of each digit)
+#pragma unroll
+        for (uint32_t d = 0; d < 4; ++d) *reinterpret_cast<uint32_t *>(to + (d >> 1) * lo_off + (d & 1) * 64) = w[d];
     };
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (uint32_t u = 0; u < KEEP; ++u)
-        if (u * kRowThreads + tid < vecs) store(u * kRowThreads + tid, kept[u]);
-    for (uint32_t i = KEEP * kRowThreads + tid; i < vecs; i += kRowThreads) store(i, weigh(x[i], weight_at(i)));
+        if (u * kRowThreads + tid < padded) store(u * kRowThreads + tid, u * kRowThreads + tid < vecs ? kept[u] : zero);
+    for (uint32_t i = KEEP * kRowThreads + tid; i < padded; i += kRowThreads) store(i, i < vecs ? weigh(x[i], weight_at(i)) : zero);
     if (tid == 0) {
         const float inv = weight ? 1.0f / sqrtf(__fadd_rn(__fdiv_rn(ss, (float)p.k), p.eps)) : 1.0f;
-        p.row_scale[row] = inv * pow2(-e);
+        p.row_scale[row] = {inv, undo_exponent(top)};
     }
 }
 
 template <uint32_t BN>
-int launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_split_weight &w, const wr_f32_gemm_args &a)
+int launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_f32_gemm_args &a)
 {
     constexpr uint32_t flag = BN == 128 ? 1u << 17 : 1u << 18;
     if (!(ctx->attr_flags & flag)) {
@@ -449,10 +482,9 @@ int launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_split_weight &w, con
     }
     GemmParams p;
     p.a = a;
-    p.w = w;
     p.m_tiles = (a.m + kBM - 1) / kBM;
-    p.n_tiles = (w.n + BN - 1) / BN;
-    p.k_blocks = wr_weight_blocks(w.k);
+    p.n_tiles = (a.source.to.n + BN - 1) / BN;
+    p.k_blocks = wr_weight_blocks(a.source.to.k);
     p.part_blocks = (p.k_blocks + a.k_parts - 1) / a.k_parts;
     p.wait_limit = ctx->wait_limit;
     p.err = ctx->dev_err;
@@ -488,7 +520,7 @@ int wr_split_weights_launch(wr_cuda_ctx *ctx, const wr_split_source *list, uint3
 
 int wr_split_rows_launch(wr_cuda_ctx *ctx, const wr_split_rows_args &a)
 {
-    if (a.rows == 0 || a.k == 0 || (a.k & 3u) || (a.x_stride & 3u) || (a.ld & 7u)) return WR_CUDA_ERR_INVAL;
+    if (a.rows == 0 || a.k == 0 || (a.k & 3u) || (a.x_stride & 3u) || a.ld < wr_split_ld(a.k) || (a.ld & 63u)) return WR_CUDA_ERR_INVAL;
     if (a.parts && (a.n_parts == 0 || a.n_parts > kMaxParts)) return WR_CUDA_ERR_INVAL;
     const dim3 grid(a.rows), block(kRowThreads);
     if (a.k <= 4 * kRowThreads) WR_CUDA_TRY(wr_launch_pdl(split_rows_kernel<1>, grid, block, 0, ctx->stream, a));
@@ -507,24 +539,27 @@ uint32_t wr_f32_gemm_k_parts(uint32_t n, uint32_t k)
     return parts;
 }
 
-int wr_f32_gemm_launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_split_weight &w, const wr_f32_gemm_args &a)
+bool wr_f32_gemm_covers(uint32_t k, uint32_t k_parts)
 {
-    if (a.m == 0 || w.n == 0 || w.k == 0 || a.n_seg == 0 || a.n_seg > 3 || a.k_parts == 0 || (a.k_parts > 1 && a.pair))
+    return (wr_weight_blocks(k) + k_parts - 1) / k_parts * kBK <= kPartMost;
+}
+
+int wr_f32_gemm_launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_f32_gemm_args &a)
+{
+    const wr_split_weight &w = a.source.to;
+    if (a.m == 0 || w.n == 0 || w.k == 0 || a.n_seg == 0 || a.n_seg > 3 || a.k_parts == 0 || (a.k_parts > 1 && a.source.pair))
         return WR_CUDA_ERR_INVAL;
+    if (!wr_f32_gemm_covers(w.k, a.k_parts)) return WR_CUDA_ERR_UNSUPPORTED;
     for (uint32_t s = 0; s < a.n_seg; ++s)
         if ((a.seg[s].n & 3u) || (a.seg[s].ld & 3u)) return WR_CUDA_ERR_INVAL;
-    // The tile width that finishes first: rounds over the device times a unit's time, which goes by shared memory: 64
-    // K-values are 12 products that read 4 KB of x and 32 BN bytes of W each, and 32 KB + 256 BN that arrive.
-    uint32_t best = 0;
-    uint64_t best_cost = ~0ull;
-    for (uint32_t bn : {128u, 64u}) {
+    // The tile width that finishes first: rounds over the device times a unit's time, in hundredths of a microsecond as measured
+    // (16 to 64 blocks of K).  128 columns fill the accumulators, so nothing overlaps their filling and fetch; 64 columns have
+    // two sets of them, but read x twice as often.  700 rows, us with 64 and 128 columns: 4096 x 1024 30.7, 34.8; 24576 x 4096 593, 504.
+    const uint32_t blocks = (wr_weight_blocks(w.k) + a.k_parts - 1) / a.k_parts;
+    auto rounds = [&](uint32_t bn) {
         const uint64_t units = (uint64_t)((a.m + kBM - 1) / kBM) * ((w.n + bn - 1) / bn) * a.k_parts;
-        const uint64_t cost = ((units + ctx->sm_count - 1) / ctx->sm_count) * (bn + 128u);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = bn;
-        }
-    }
-    if (best == 128) return launch<128>(ctx, x, w, a);
-    return launch<64>(ctx, x, w, a);
+        return (units + ctx->sm_count - 1) / ctx->sm_count;
+    };
+    if (rounds(128) * (blocks * 76u + 390u) <= rounds(64) * (blocks * 55u + 10u) + 300u) return launch<128>(ctx, x, a);
+    return launch<64>(ctx, x, a);
 }

@@ -639,32 +639,34 @@ int launch_wide(wr_cuda_ctx *ctx, GemvParams &p)
         src.n[s] = p.seg[s].n;
     }
     src.pair = p.swiglu;
-    const uint32_t parts = direct ? 1u : wr_f32_gemm_k_parts(w.n, w.k), ld = (p.k + 7u) & ~7u;
-    const size_t b_blocks = up256(wr_split_weight_bytes(w.n, w.k)), b_unscale = up256((size_t)w.n * 4);
-    const size_t b_rows = up256((size_t)2 * p.rows * ld * 2), b_scale = up256((size_t)p.rows * 4);
+    const uint32_t parts = direct ? 1u : wr_f32_gemm_k_parts(w.n, w.k), ld = wr_split_ld(p.k);
+    if (!wr_f32_gemm_covers(p.k, parts)) return WR_CUDA_ERR_UNSUPPORTED;
+    const size_t b_blocks = up256(wr_split_weight_bytes(w.n, w.k)), b_exponent = up256((size_t)w.n * 4);
+    const size_t b_rows = up256((size_t)2 * p.rows * ld * 2), b_scale = up256(p.rows * sizeof(wr_split_scale));
     const size_t b_parts = direct ? 0 : (size_t)parts * p.rows * w.n * 4;
-    int rc = wr_ctx_reserve_ws(ctx, b_blocks + b_unscale + b_rows + b_scale + b_parts, 0);
+    int rc = wr_ctx_reserve_ws(ctx, b_blocks + b_exponent + b_rows + b_scale + b_parts, 0);
     if (rc != WR_CUDA_OK) return rc;
     char *at = reinterpret_cast<char *>(ctx->ws);
     w.blocks = at;
-    w.unscale = reinterpret_cast<float *>(at += b_blocks);
+    w.exponent = reinterpret_cast<int *>(at += b_blocks);
     wr_split_rows_args r{};
     r.x = const_cast<float *>(p.x); r.x_stride = p.x_stride; r.k = p.k; r.rows = p.rows;      // (no parts: x is only read)
     r.norm_w = p.norm_w; r.eps = p.eps;
-    r.out = reinterpret_cast<__half *>(at += b_unscale); r.ld = ld; r.pad = p.rows;
-    r.row_scale = reinterpret_cast<float *>(at += b_rows);
+    r.out = reinterpret_cast<__half *>(at += b_exponent); r.ld = ld; r.pad = p.rows;
+    r.row_scale = reinterpret_cast<wr_split_scale *>(at += b_rows);
     float *sums = reinterpret_cast<float *>(at += b_scale);
     CUtensorMap map;
     if ((rc = wr_split_weights_launch(ctx, &src, 1)) != WR_CUDA_OK || (rc = wr_split_rows_launch(ctx, r)) != WR_CUDA_OK ||
-        (rc = wr_gemm_map_rows(&map, r.out, 2 * p.rows, p.k, ld)) != WR_CUDA_OK)
+        (rc = wr_gemm_map_rows(&map, r.out, 2 * p.rows, ld, ld)) != WR_CUDA_OK)
         return rc;
     wr_f32_gemm_args a{};
-    a.m = a.pad = p.rows; a.row_scale = r.row_scale; a.k_parts = parts; a.pair = p.swiglu; a.n_seg = p.swiglu ? 1u : p.n_seg;
+    a.source = src; a.x = p.x; a.x_stride = p.x_stride; a.norm_w = p.norm_w;
+    a.m = a.pad = p.rows; a.row_scale = r.row_scale; a.k_parts = parts; a.n_seg = p.swiglu ? 1u : p.n_seg;
     if (direct)
         for (uint32_t s = 0; s < a.n_seg; ++s) a.seg[s] = {p.seg[s].out, p.seg[s].n, p.seg[s].out_stride};
     else
         a.seg[0] = {sums, w.n, w.n};
-    if ((rc = wr_f32_gemm_launch(ctx, map, w, a)) != WR_CUDA_OK || direct) return rc;
+    if ((rc = wr_f32_gemm_launch(ctx, map, a)) != WR_CUDA_OK || direct) return rc;
     WR_CUDA_TRY(wr_launch_pdl(finish_rows_kernel, dim3((n + 255) / 256, p.rows), dim3(256), 0, ctx->stream, p, (const float *)sums,
                               parts, w.n));
     ctx->launches++;

@@ -31,7 +31,8 @@ struct wr_cuda_model {
     bool split_kept = false;             // every layer has split weights of its own (else all use the same memory in turn)
     std::vector<wr_split_weight> split;  // per layer: q | k | v, o, gate / up, down
     __half *split_rows = nullptr;
-    float *row_scale = nullptr, *parts = nullptr;
+    wr_split_scale *row_scale = nullptr;
+    float *parts = nullptr;
     uint32_t *h_tokens = nullptr;        // pinned: token ids in, arg-max ids out
     uint32_t ffn_max = 0;
     uint64_t launches = 0;

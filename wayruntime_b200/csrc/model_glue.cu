@@ -186,6 +186,7 @@ void take_prompt_memory(wr_cuda_model *m)
     size_t parts = 1, all = 0, most = 0;
     std::vector<size_t> at(n_layers);                    // a layer's split weights, from the first one's
     m->split.resize(4 * n_layers);
+    bool covered = true;
     for (size_t L = 0; L < n_layers; ++L) {
         const uint32_t ffn = m->layers[L].ffn, gate_up = (ffn + 7u) / 8u * 16u;
         const uint32_t n[4] = {nq + 2 * nkv, m->hidden, gate_up, m->hidden}, k[4] = {m->hidden, nq, m->hidden, ffn};
@@ -193,6 +194,7 @@ void take_prompt_memory(wr_cuda_model *m)
         for (int i = 0; i < 4; ++i) {
             m->split[4 * L + i].n = n[i];
             m->split[4 * L + i].k = k[i];
+            covered = covered && wr_f32_gemm_covers(k[i], i == 1 || i == 3 ? wr_f32_gemm_k_parts(n[i], k[i]) : 1);
             bytes += up256(wr_split_weight_bytes(n[i], k[i])) + up256((size_t)n[i] * 4);
         }
         parts = std::max<size_t>({parts, wr_f32_gemm_k_parts(m->hidden, nq), wr_f32_gemm_k_parts(m->hidden, ffn)});
@@ -200,8 +202,9 @@ void take_prompt_memory(wr_cuda_model *m)
         all += bytes;
         most = std::max(most, bytes);
     }
-    const size_t rows = up256(2 * R * ((widest + 7) & ~(size_t)7) * 2), sums = up256(parts * R * m->hidden * 4);
-    const size_t rest = rows + up256(R * 4) + sums;
+    if (!covered) return;
+    const size_t rows = up256(2 * R * wr_split_ld((uint32_t)widest) * 2), sums = up256(parts * R * m->hidden * 4);
+    const size_t rest = rows + up256(R * sizeof(wr_split_scale)) + sums;
     size_t free_bytes = 0, total_bytes = 0;
     if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) (void)cudaGetLastError();
     m->split_kept = all <= free_bytes / 16 && cudaMalloc((void **)&m->prompt, all + rest) == cudaSuccess;
@@ -216,43 +219,54 @@ void take_prompt_memory(wr_cuda_model *m)
             wr_split_weight &w = m->split[4 * L + i];
             w.blocks = cur;
             cur += up256(wr_split_weight_bytes(w.n, w.k));
-            w.unscale = reinterpret_cast<float *>(cur);
+            w.exponent = reinterpret_cast<int *>(cur);
             cur += up256((size_t)w.n * 4);
         }
     }
     cur = m->prompt + (m->split_kept ? all : most);
     m->split_rows = reinterpret_cast<__half *>(cur);
     cur += rows;
-    m->row_scale = reinterpret_cast<float *>(cur);
-    cur += up256(R * 4);
+    m->row_scale = reinterpret_cast<wr_split_scale *>(cur);
+    cur += up256(R * sizeof(wr_split_scale));
     m->parts = reinterpret_cast<float *>(cur);
+}
+
+// One of a layer's four split weights: q | k | v, o, gate / up, down
+wr_split_source split_source(const wr_cuda_model *m, uint32_t L, uint32_t which)
+{
+    const wr_cuda_layer_dev &l = m->layers[L];
+    const uint32_t hid = m->hidden, nq = m->n_q * m->hd, nkv = m->n_kv * m->hd;
+    const wr_split_weight &w = m->split[4 * L + which];
+    if (which == 0) return {w, {l.wq, l.wk, l.wv}, {nq, nkv, nkv}, 0};
+    if (which == 1) return {w, {l.wo, nullptr, nullptr}, {hid, 0, 0}, 0};
+    if (which == 2) return {w, {l.w_gate, l.w_up, nullptr}, {l.ffn, l.ffn, 0}, 1};
+    return {w, {l.w_down, nullptr, nullptr}, {hid, 0, 0}, 0};
 }
 
 int split_layer(wr_cuda_model *m, uint32_t L)
 {
-    const wr_cuda_layer_dev &l = m->layers[L];
-    const uint32_t hid = m->hidden, nq = m->n_q * m->hd, nkv = m->n_kv * m->hd;
-    const wr_split_weight *w = &m->split[4 * L];
-    const wr_split_source list[4] = {{w[0], {l.wq, l.wk, l.wv}, {nq, nkv, nkv}, 0},
-                                     {w[1], {l.wo, nullptr, nullptr}, {hid, 0, 0}, 0},
-                                     {w[2], {l.w_gate, l.w_up, nullptr}, {l.ffn, l.ffn, 0}, 1},
-                                     {w[3], {l.w_down, nullptr, nullptr}, {hid, 0, 0}, 0}};
+    const wr_split_source list[4] = {split_source(m, L, 0), split_source(m, L, 1), split_source(m, L, 2), split_source(m, L, 3)};
     return wr_split_weights_launch(m->ctx, list, 4);
 }
 
-// Split rows of x (the residual takes the parts of the product before first), and their tensor map.
+// Split rows of x (the residual takes the parts of the product before first), their tensor map, and what the product of
+// them with a split weight needs to know.
 int split_rows(wr_cuda_model *m, CUtensorMap *map, float *x, uint32_t x_stride, uint32_t k, uint32_t rows,
-               uint32_t n_parts, const float *norm_w)
+               uint32_t n_parts, const float *norm_w, wr_f32_gemm_args *g = nullptr)
 {
     wr_split_rows_args a{};
     a.x = x; a.x_stride = x_stride; a.k = k; a.rows = rows;
     a.parts = n_parts ? m->parts : nullptr; a.n_parts = n_parts;
     a.norm_w = norm_w; a.eps = m->eps;
-    a.out = map ? m->split_rows : nullptr; a.ld = (k + 7u) & ~7u; a.pad = rows;
+    a.out = map ? m->split_rows : nullptr; a.ld = wr_split_ld(k); a.pad = rows;
     a.row_scale = m->row_scale;
+    if (g) {
+        g->x = x; g->x_stride = x_stride; g->norm_w = norm_w;
+        g->m = g->pad = rows; g->row_scale = m->row_scale; g->k_parts = 1;
+    }
     ++m->launches;
     const int rc = wr_split_rows_launch(m->ctx, a);
-    return rc != WR_CUDA_OK || !map ? rc : wr_gemm_map_rows(map, m->split_rows, 2 * rows, k, a.ld);
+    return rc != WR_CUDA_OK || !map ? rc : wr_gemm_map_rows(map, m->split_rows, 2 * rows, a.ld, a.ld);
 }
 
 // The products of a layer for the rows of a prompt: before (q, k, v) and after (o, feed-forward) attention.  A product
@@ -267,40 +281,38 @@ int prompt_before(wr_cuda_model *m, uint32_t L, uint32_t rows, uint32_t *n_parts
         if ((rc = split_layer(m, L)) != WR_CUDA_OK) return rc;
     }
     CUtensorMap map;
-    rc = split_rows(m, &map, m->resid, hid, hid, rows, *n_parts, l.attn_norm);
+    wr_f32_gemm_args a{};
+    rc = split_rows(m, &map, m->resid, hid, hid, rows, *n_parts, l.attn_norm, &a);
     if (rc != WR_CUDA_OK) return rc;
     *n_parts = 0;
-    wr_f32_gemm_args a{};
-    a.m = a.pad = rows; a.row_scale = m->row_scale; a.k_parts = 1;
+    a.source = split_source(m, L, 0);
     a.seg[0] = {m->q, nq, nq}; a.seg[1] = {m->k, nkv, nkv}; a.seg[2] = {m->v, nkv, nkv}; a.n_seg = 3;
     ++m->launches;
-    return wr_f32_gemm_launch(m->ctx, map, m->split[4 * L], a);
+    return wr_f32_gemm_launch(m->ctx, map, a);
 }
 
 int prompt_after(wr_cuda_model *m, uint32_t L, uint32_t rows, uint32_t *n_parts)
 {
     const wr_cuda_layer_dev &l = m->layers[L];
-    const wr_split_weight *w4 = &m->split[4 * L];
     const uint32_t hid = m->hidden, nq = m->n_q * m->hd;
     CUtensorMap map;
-    auto to_residual = [&](const wr_split_weight &w) {
-        wr_f32_gemm_args a{};
-        a.m = a.pad = rows; a.row_scale = m->row_scale; a.k_parts = wr_f32_gemm_k_parts(w.n, w.k);
+    wr_f32_gemm_args a{};
+    auto to_residual = [&](uint32_t which) {
+        a.source = split_source(m, L, which);
+        a.k_parts = *n_parts = wr_f32_gemm_k_parts(a.source.to.n, a.source.to.k);
         a.seg[0] = {m->parts, hid, hid}; a.n_seg = 1;
-        *n_parts = a.k_parts;
-        return wr_f32_gemm_launch(m->ctx, map, w, a);
+        return wr_f32_gemm_launch(m->ctx, map, a);
     };
     m->launches += 3;
-    int rc = split_rows(m, &map, m->attn, nq, nq, rows, 0, nullptr);
-    if (rc != WR_CUDA_OK || (rc = to_residual(w4[1])) != WR_CUDA_OK) return rc;
-    rc = split_rows(m, &map, m->resid, hid, hid, rows, *n_parts, l.ffn_norm);
+    int rc = split_rows(m, &map, m->attn, nq, nq, rows, 0, nullptr, &a);
+    if (rc != WR_CUDA_OK || (rc = to_residual(1)) != WR_CUDA_OK) return rc;
+    rc = split_rows(m, &map, m->resid, hid, hid, rows, *n_parts, l.ffn_norm, &a);
     if (rc != WR_CUDA_OK) return rc;
-    wr_f32_gemm_args a{};
-    a.m = a.pad = rows; a.row_scale = m->row_scale; a.k_parts = 1;
-    a.seg[0] = {m->gate, l.ffn, m->ffn_max}; a.n_seg = 1; a.pair = 1;
-    if ((rc = wr_f32_gemm_launch(m->ctx, map, w4[2], a)) != WR_CUDA_OK) return rc;
-    rc = split_rows(m, &map, m->gate, m->ffn_max, l.ffn, rows, 0, nullptr);
-    return rc != WR_CUDA_OK ? rc : to_residual(w4[3]);
+    a.source = split_source(m, L, 2);
+    a.seg[0] = {m->gate, l.ffn, m->ffn_max}; a.n_seg = 1;
+    if ((rc = wr_f32_gemm_launch(m->ctx, map, a)) != WR_CUDA_OK) return rc;
+    rc = split_rows(m, &map, m->gate, m->ffn_max, l.ffn, rows, 0, nullptr, &a);
+    return rc != WR_CUDA_OK ? rc : to_residual(3);
 }
 
 }  // namespace

@@ -31,6 +31,11 @@ __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t m, uint32_t n)
 }
 // ... and for F16 x F16 -> F32
 __host__ __device__ constexpr uint32_t idesc_f16(uint32_t m, uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24); }
+// ... and for signed bytes -> S32 (kind::i8; 32 K-values to an instruction)
+__host__ __device__ constexpr uint32_t idesc_i8(uint32_t m, uint32_t n)
+{
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
+}
 __device__ __forceinline__ bool elect_one()
 {
     uint32_t pred;
@@ -43,6 +48,15 @@ __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint64_t a, uint64_t b, 
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mma_i8_ss(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
