@@ -251,3 +251,32 @@ def test_mixed_short_and_long_sessions_in_one_batch_stay_byte_equal_to_serial():
         kv.close()
     dm.close()
     ctx.close()
+
+
+def test_a_pass_that_fails_leaves_none_of_its_work_in_flight():
+    """Attention is refused when the rows' products and cache rows are on their way already."""
+    import torch
+    import wayruntime_b200 as wr
+    ctx = wr.Context(0)
+    shape = dict(n_layers=1, hidden=256, n_q_heads=4, n_kv_heads=2, head_dim=128, vocab=64, ffn=64)
+    w = _weights(shape, 990)
+    dm = _model(ctx, w, shape, max_rows=2048)
+    kv = dm.kv_create(4096)
+    for rows in (2000, 16):                          # (a kernel's first use waits for the device)
+        dm.forward(dm.FWD_PREFILL, [kv], [0], [1] * rows)
+    ctx.set_attn_max_seq(1024)
+    stream = torch.cuda.ExternalStream(ctx.stream)
+    big = torch.ones((4096, 4096), device="cuda")
+    torch.cuda.synchronize()
+    for rows in (2000, 16):
+        with torch.cuda.stream(stream):              # something for the pass to be queued behind
+            for _ in range(20):
+                big = big @ big * 0.0
+        with pytest.raises(wr.WrCudaError):
+            dm.forward(dm.FWD_PREFILL, [kv], [1020], [1] * rows, logits=False)
+        assert stream.query()
+    res = dm.forward(dm.FWD_PREFILL, [kv], [0], list(range(64)), out_from=63, logits=True)      # the model goes on
+    assert np.isfinite(res["logits"]).all()
+    kv.close()
+    dm.close()
+    ctx.close()

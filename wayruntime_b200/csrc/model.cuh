@@ -52,3 +52,17 @@ int  wr_mixed_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mode, uint32_t n_r
                       const uint32_t *positions, const uint32_t *tokens, uint32_t out_from, float *hidden_out,
                       float *normed_out, float *const *logits_out, uint32_t *argmax_out);
 void wr_mixed_destroy(wr_mixed *x);      // caller holds ctx->lock, device current, stream idle
+
+// A forward pass that returns early leaves none of its work in flight, on either stream: what it was given to fill may be
+// gone the moment it has returned.
+struct wr_settle {
+    wr_cuda_model *m;
+    bool done = false;                   // the pass has waited for its work itself
+    ~wr_settle()
+    {
+        if (done) return;
+        if (m->side) (void)cudaStreamSynchronize(m->side);
+        (void)cudaStreamSynchronize(m->ctx->stream);
+        (void)cudaGetLastError();
+    }
+};

@@ -521,6 +521,7 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
             if (pos_p[i] >= kv_p[i]->max_ctx) return WR_CUDA_ERR_CTX_FULL;
         }
     }
+    wr_settle settle{m};
     {
         std::lock_guard<std::mutex> g(ctx->lock);
         WR_CUDA_TRY(cudaSetDevice(ctx->device));
@@ -578,11 +579,8 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
                     a.side = m->side;
                 }
                 rc = wr_step_small_launch(ctx, n_short, kv_p, L, pos_p, a);
-                if (both) {                              // whatever comes of the launches between, the streams meet again
-                    WR_CUDA_TRY(cudaEventRecord(m->join, m->side));
-                    if (rc != WR_CUDA_OK) (void)cudaStreamWaitEvent(st, m->join, 0);
-                }
                 if (rc != WR_CUDA_OK) return rc;
+                if (both) WR_CUDA_TRY(cudaEventRecord(m->join, m->side));
             }
             if (l.q_norm && r_lo < n_rows && !fused) {
                 const uint32_t n_a = (n_rows - r_lo) * m->n_q, n_b = (n_rows - r_lo) * m->n_kv;
@@ -601,8 +599,8 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
                                          m->q + (size_t)n_short * nq, m->k + (size_t)n_short * nkv,
                                          m->v + (size_t)n_short * nkv, m->attn + (size_t)n_short * nq, m->n_q,
                                          m->theta, m->n_rot, WR_CUDA_APPEND_ROPE, m->scale, 0, WR_CUDA_MEM_DEVICE);
-                if (n_short && m->side) WR_CUDA_TRY(cudaStreamWaitEvent(st, m->join, 0));
                 if (rc != WR_CUDA_OK) return rc;
+                if (n_short && m->side) WR_CUDA_TRY(cudaStreamWaitEvent(st, m->join, 0));
             }
         } else {
             if (!fused) {
@@ -727,6 +725,7 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
     }
     m->last_enqueue_ns = (uint64_t)std::chrono::duration_cast<std::chrono::nanoseconds>(
                              std::chrono::steady_clock::now() - t_begin).count();
+    settle.done = true;
     int rc = wr_ctx_sync_checked(ctx);
     if (rc != WR_CUDA_OK) return rc;
     if (argmax_out)

@@ -1127,6 +1127,7 @@ int wr_mixed_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mode, uint32_t n_ro
         if (positions[s] == 0) kv[s]->state_len[1 - slot_out[s]] = -1;
     }
     cudaStream_t st = ctx->stream;
+    wr_settle settle{m};
     memcpy(x->h_tokens, tokens, n_rows * sizeof(uint32_t));
     WR_CUDA_TRY(cudaMemcpyAsync(x->tokens, x->h_tokens, n_rows * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     WR_CUDA_TRY(cudaMemcpyAsync(x->seqs, x->h_seqs, n_seq * sizeof(wr_seq_dev), cudaMemcpyHostToDevice, st));
@@ -1198,6 +1199,7 @@ int wr_mixed_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mode, uint32_t n_ro
     }
     m->last_enqueue_ns = (uint64_t)std::chrono::duration_cast<std::chrono::nanoseconds>(
                              std::chrono::steady_clock::now() - t_begin).count();
+    settle.done = true;
     TRY(wr_ctx_sync_checked(ctx));
     for (uint32_t s = 0; s < n_seq; ++s) kv[s]->state_len[slot_out[s]] = (int64_t)positions[s] + per_seq;
     if (argmax_out)
