@@ -280,3 +280,26 @@ def test_a_pass_that_fails_leaves_none_of_its_work_in_flight():
     kv.close()
     dm.close()
     ctx.close()
+
+
+def test_caches_whose_layers_differ_are_refused_before_anything_runs():
+    import ctypes as C
+
+    import wayruntime_b200 as wr
+    from wayruntime_b200.binding import F16, CacheLayer, KVCache
+    ctx = wr.Context(0)
+    shape = dict(SHAPE, n_layers=2)
+    dm = _model(ctx, _weights(shape, 980), shape, max_rows=64)
+    before = ctx.launch_count
+    for heads, dim in ((4, 128), (1, 128), (2, 64)):
+        layers = (CacheLayer * 2)(CacheLayer(2, 128, 128, F16, 0), CacheLayer(heads, dim, dim, F16, 0))
+        h = C.c_void_p()
+        assert ctx._lib.wr_cuda_kv_create_layout(ctx._h, 2, layers, C.c_uint32(64), C.byref(h)) == 0
+        kv = KVCache._of_handle(ctx, h, 64)
+        for mode, rows in ((dm.FWD_DECODE, 1), (dm.FWD_PREFILL, 5), (dm.FWD_PREFILL, 40)):
+            with pytest.raises(wr.WrCudaError):
+                dm.forward(mode, [kv], [0], [1] * rows)
+        kv.close()
+    assert ctx.launch_count == before
+    dm.close()
+    ctx.close()

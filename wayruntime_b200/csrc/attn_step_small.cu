@@ -156,34 +156,34 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
         const uint32_t tok = key % kPageTokens;
 #pragma unroll
         for (uint32_t c0 = 0; c0 < kHd / 8; c0 += kRaw) {
-        uint4 raw[kRaw];
+            uint4 raw[kRaw];
 #pragma unroll
-        for (uint32_t i = 0; i < kRaw; ++i) {
-            if (key == pos) raw[i] = *reinterpret_cast<const uint4 *>(&nk[8 * (c0 + i)]);
-            else raw[i] = __ldg(reinterpret_cast<const uint4 *>(row_chunk(kb, tok, c0 + i)));
-        }
-#pragma unroll
-        for (uint32_t c = c0; c < c0 + kRaw; ++c) {
-            const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw[c - c0]);
-            float kf[8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 f = __half22float2(h2[i]);
-                kf[2 * i] = f.x;
-                kf[2 * i + 1] = f.y;
+            for (uint32_t i = 0; i < kRaw; ++i) {
+                if (key == pos) raw[i] = *reinterpret_cast<const uint4 *>(&nk[8 * (c0 + i)]);
+                else raw[i] = __ldg(reinterpret_cast<const uint4 *>(row_chunk(kb, tok, c0 + i)));
             }
 #pragma unroll
-            for (uint32_t g = 0; g < (uint32_t)GM; ++g) {
-                if (g < G) {
-                    const float4 qa = *reinterpret_cast<const float4 *>(&sq[g][8 * c]);
-                    const float4 qb = *reinterpret_cast<const float4 *>(&sq[g][8 * c + 4]);
-                    float d = dot[g];
-                    d = fmaf(qa.x, kf[0], d); d = fmaf(qa.y, kf[1], d); d = fmaf(qa.z, kf[2], d); d = fmaf(qa.w, kf[3], d);
-                    d = fmaf(qb.x, kf[4], d); d = fmaf(qb.y, kf[5], d); d = fmaf(qb.z, kf[6], d); d = fmaf(qb.w, kf[7], d);
-                    dot[g] = d;
+            for (uint32_t c = c0; c < c0 + kRaw; ++c) {
+                const __half2 *h2 = reinterpret_cast<const __half2 *>(&raw[c - c0]);
+                float kf[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 f = __half22float2(h2[i]);
+                    kf[2 * i] = f.x;
+                    kf[2 * i + 1] = f.y;
+                }
+#pragma unroll
+                for (uint32_t g = 0; g < (uint32_t)GM; ++g) {
+                    if (g < G) {
+                        const float4 qa = *reinterpret_cast<const float4 *>(&sq[g][8 * c]);
+                        const float4 qb = *reinterpret_cast<const float4 *>(&sq[g][8 * c + 4]);
+                        float d = dot[g];
+                        d = fmaf(qa.x, kf[0], d); d = fmaf(qa.y, kf[1], d); d = fmaf(qa.z, kf[2], d); d = fmaf(qa.w, kf[3], d);
+                        d = fmaf(qb.x, kf[4], d); d = fmaf(qb.y, kf[5], d); d = fmaf(qb.z, kf[6], d); d = fmaf(qb.w, kf[7], d);
+                        dot[g] = d;
+                    }
                 }
             }
-        }
         }
 #pragma unroll
         for (uint32_t g = 0; g < (uint32_t)GM; ++g)
@@ -300,10 +300,10 @@ cudaError_t launch_small(uint32_t sets, uint32_t grid, cudaStream_t st, bool sid
 
 }  // namespace
 
-bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t n_q_heads, uint32_t position)
+bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t layer, uint32_t n_q_heads, uint32_t position)
 {
-    return kv->hd_at(0) == kHd && kv->n_kv_at(0) > 0 && n_q_heads % kv->n_kv_at(0) == 0 &&
-           n_q_heads / kv->n_kv_at(0) <= kSmallMaxGroup && position + 1 <= kSmallMaxKeys;
+    const uint32_t n_kv = kv->hd_at(layer) == kHd ? kv->n_kv_at(layer) : 0u;
+    return n_kv > 0 && n_q_heads % n_kv == 0 && n_q_heads / n_kv <= kSmallMaxGroup && position + 1 <= kSmallMaxKeys;
 }
 
 // Enqueue on device-resident rows.  Caller holds ctx->lock; every session must pass wr_step_small_covers and
@@ -314,7 +314,7 @@ int wr_step_small_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *k
     if (n_sess == 0 || n_sess > WR_CUDA_BATCH_MAX) return WR_CUDA_ERR_LIMIT;
     step_small_params p;
     for (uint32_t s = 0; s < n_sess; ++s) {
-        if (!wr_step_small_covers(kv[s], a.n_q_heads, positions[s])) return WR_CUDA_ERR_UNSUPPORTED;
+        if (!wr_step_small_covers(kv[s], layer, a.n_q_heads, positions[s])) return WR_CUDA_ERR_UNSUPPORTED;
         if (positions[s] >= kv[s]->max_ctx) return WR_CUDA_ERR_CTX_FULL;
         p.b.pages[s] = kv[s]->d_pages + (size_t)layer * kv[s]->n_pages;
         p.b.seq_len[s] = positions[s];

@@ -490,9 +490,11 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
     for (uint32_t r = 0; r < n_rows; ++r)
         if (tokens[r] >= m->vocab) return WR_CUDA_ERR_INVAL;      // refused before anything runs
     const uint32_t n_sess = (mode == WR_CUDA_FWD_DECODE) ? n_rows : 1;
-    for (uint32_t s = 0; s < n_sess; ++s)
-        if (!kv[s] || kv[s]->n_layers != m->n_layers || kv[s]->n_kv_at(0) != m->n_kv || kv[s]->hd_at(0) != m->hd)
-            return WR_CUDA_ERR_INVAL;
+    for (uint32_t s = 0; s < n_sess; ++s) {
+        if (!kv[s] || kv[s]->n_layers != m->n_layers) return WR_CUDA_ERR_INVAL;
+        for (uint32_t L = 0; L < m->n_layers; ++L)
+            if (kv[s]->n_kv_at(L) != m->n_kv || kv[s]->hd_at(L) != m->hd) return WR_CUDA_ERR_INVAL;
+    }
 
     std::lock_guard<std::mutex> fg(m->fwd);
     const auto t_begin = std::chrono::steady_clock::now();
@@ -510,14 +512,14 @@ extern "C" int wr_cuda_model_forward(wr_cuda_ctx *ctx, wr_cuda_model *m, int mod
         uint32_t n = 0;
         for (int pass = 0; pass < 2; ++pass)
             for (uint32_t r = 0; r < n_rows; ++r) {
-                const bool small = use_small && wr_step_small_covers(kv[r], m->n_q, positions[r]);
+                const bool small = use_small && wr_step_small_covers(kv[r], 0, m->n_q, positions[r]);
                 if (small == (pass == 0)) perm[n++] = r;
             }
         for (uint32_t i = 0; i < n_rows; ++i) {
             if (perm[i] != i) permuted = true;
             kv_p[i] = kv[perm[i]];
             pos_p[i] = positions[perm[i]];
-            if (use_small && wr_step_small_covers(kv_p[i], m->n_q, pos_p[i])) n_short = i + 1;
+            if (use_small && wr_step_small_covers(kv_p[i], 0, m->n_q, pos_p[i])) n_short = i + 1;
             if (pos_p[i] >= kv_p[i]->max_ctx) return WR_CUDA_ERR_CTX_FULL;
         }
     }

@@ -230,7 +230,7 @@ struct wr_append_extra {
 // One-kernel layer-step for short contexts (attn_step_small.cu): QK-norm, RoPE, append and the
 // new token's attention, for sessions of head_dim 128 with at most WR_STEP_SMALL_MAX_KEYS keys.
 #define WR_STEP_SMALL_MAX_KEYS 1024u
-bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t n_q_heads, uint32_t position);
+bool wr_step_small_covers(const wr_cuda_kv *kv, uint32_t layer, uint32_t n_q_heads, uint32_t position);
 struct wr_step_small_args {
     float *q;                        // [n_sess][n_q_heads][128]: raw rows in, normed and rotated ones out
     const float *k, *v;              // [n_sess][n_kv][128] new rows
