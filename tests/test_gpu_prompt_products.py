@@ -205,3 +205,28 @@ def test_weights_are_split_for_each_call_where_memory_is_short():
     del hold
     torch.cuda.empty_cache()
     assert np.array_equal(kept["hidden"], short["hidden"])
+
+
+@pytest.mark.parametrize("qk_norm", [True, False])
+def test_prompt_rows_agree_with_those_of_small_portions(qk_norm):
+    """The append of a prompt's rows (head norms or none, F16 queries) against the kernels for up to sixteen rows, two layers, a
+    portion behind a past.  Keys and values are cut to F16 and queries rounded to it: an F16 step of the largest."""
+    import wayruntime_b200 as wr
+    ctx = wr.Context(0)
+    shape = dict(n_layers=2, hidden=256, n_q_heads=6, n_kv_heads=2, head_dim=128, vocab=300, ffn=512)
+    w = _weights(shape, 1310, qk_norm=qk_norm)
+    dm = _model(ctx, w, shape, max_rows=256)
+    tokens = [(7 * r + 1) % 300 for r in range(230)]
+    got = []
+    for portions in ([130, 100], [16] * 14 + [6]):
+        kv, at, rows = ctx.kv_create(2, 2, 128, 230), 0, []
+        for n in portions:
+            rows.append(dm.forward(dm.FWD_PREFILL, [kv], [at], tokens[at:at + n], hidden=True)["hidden"])
+            at += n
+        got.append([np.concatenate(rows)] + [kv.read_rows(i, which, 0, 230).view(np.float16).astype(np.float64)
+                                             for i in range(2) for which in range(2)])
+        kv.close()
+    for a, b in zip(*got):
+        assert np.abs(a - b).max() <= 2.0 ** -9 * np.abs(b).max()
+    dm.close()
+    ctx.close()

@@ -44,3 +44,39 @@ def test_lengths_around_the_divisions(monkeypatch, n_q, n_kv):
         kv.close()
     dm.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("qk_norm", [True, False])
+def test_short_and_long_sessions_in_one_batch_over_three_layers(qk_norm):
+    """Two streams per layer that meet before the next product: every step of every session has the bits it has alone."""
+    import wayruntime_b200 as wr
+    ctx = wr.Context(0)
+    shape = dict(n_layers=3, hidden=256, n_q_heads=8, n_kv_heads=4, head_dim=128, vocab=515, ffn=128)
+    w = _weights(shape, 1520, qk_norm=qk_norm)
+    dm = _model(ctx, w, shape, max_rows=1024)
+    lens = [60, 1500, 300, 2100, 1022, 1023, 1024, 5, 3000, 700]
+    steps = 4                                        # (1022 and 1023 go from one kind to the other on the way)
+
+    def sessions():
+        kvs = [ctx.kv_create(3, 4, 128, n + steps) for n in lens]
+        for kv, n in zip(kvs, lens):
+            _prefill(dm, kv, [(11 * i + n) % shape["vocab"] for i in range(n)], chunk=1024)
+        return kvs
+
+    a, b = sessions(), sessions()
+    for t in range(steps):
+        pos, toks = [n + t for n in lens], [(31 * i + 7 * t) % shape["vocab"] for i in range(len(lens))]
+        alone = [dm.forward(dm.FWD_DECODE, [kv], [p], [x], logits=True, attn_tap=True) for kv, p, x in zip(a, pos, toks)]
+        batch = dm.forward(dm.FWD_DECODE, b, pos, toks, logits=True, attn_tap=True)
+        for i, n in enumerate(lens):
+            assert np.array_equal(batch["attn"][:, i].view(np.uint32), alone[i]["attn"][:, 0].view(np.uint32)), (t, n)
+            assert np.array_equal(batch["logits"][i].view(np.uint32), alone[i]["logits"][0].view(np.uint32)), (t, n)
+    for x, y in zip(a, b):
+        n = lens[a.index(x)] + steps
+        for layer in range(3):
+            for which in (0, 1):
+                assert np.array_equal(x.read_rows(layer, which, 0, n), y.read_rows(layer, which, 0, n))
+    for kv in a + b:
+        kv.close()
+    dm.close()
+    ctx.close()

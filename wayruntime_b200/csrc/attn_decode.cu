@@ -354,11 +354,9 @@ static int decode_common(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *k
 // K and Q), then attend over rows [0, positions[s]] of every session.  With
 // host buffers the inputs cross the bus once and only the attention rows come
 // back.
-extern "C" int wr_cuda_decode_step(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv,
-                                   uint32_t layer, const uint32_t *positions, float *q,
-                                   const float *k_rows, const float *v_rows, float *out,
-                                   uint32_t n_q_heads, float theta_base, uint32_t n_rot_pairs,
-                                   uint32_t flags, float scale_override, uint32_t window, int mem)
+int wr_decode_step(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer, const uint32_t *positions, float *q,
+                   const float *k_rows, const float *v_rows, float *out, uint32_t n_q_heads, float theta_base,
+                   uint32_t n_rot_pairs, uint32_t flags, float scale_override, uint32_t window, int mem, bool dependent)
 {
     if (!ctx) return WR_CUDA_ERR_INVAL;
     int rc = wr_append_validate(ctx, n_sess, kv, layer, positions, 1, k_rows, v_rows, q, n_q_heads,
@@ -415,7 +413,7 @@ extern "C" int wr_cuda_decode_step(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv
     const int prev = (ctx->pdl_index == ctx->launches) ? ctx->pdl_kind : WR_PDL_NONE;
     const bool early = prev == WR_PDL_NONE || prev == WR_PDL_DECODE_FULL;
     rc = wr_append_launch(ctx, n_sess, kv, layer, positions, 1, dk, dv, dq, n_q_heads, theta_base,
-                          n_rot_pairs, flags, dq_in);
+                          n_rot_pairs, flags, dq_in, nullptr, dependent);
     if (rc != WR_CUDA_OK) return rc;
     rc = wr_decode_launch(ctx, n_sess, kv, layer, seq_lens, dq, dout, n_q_heads, scale_override,
                           window, 0, nullptr, early);
@@ -426,6 +424,16 @@ extern "C" int wr_cuda_decode_step(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv
         return wr_ctx_sync_checked(ctx);
     }
     return WR_CUDA_OK;
+}
+
+extern "C" int wr_cuda_decode_step(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv,
+                                   uint32_t layer, const uint32_t *positions, float *q,
+                                   const float *k_rows, const float *v_rows, float *out,
+                                   uint32_t n_q_heads, float theta_base, uint32_t n_rot_pairs,
+                                   uint32_t flags, float scale_override, uint32_t window, int mem)
+{
+    return wr_decode_step(ctx, n_sess, kv, layer, positions, q, k_rows, v_rows, out, n_q_heads, theta_base, n_rot_pairs, flags,
+                          scale_override, window, mem, true);
 }
 
 extern "C" int wr_cuda_attn_decode(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv,

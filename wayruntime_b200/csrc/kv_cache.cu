@@ -809,7 +809,7 @@ int wr_append_validate(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv,
 int wr_append_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
                      const uint32_t *positions, uint32_t n_tokens, const float *dk,
                      const float *dv, float *dq, uint32_t n_q_heads, float theta_base,
-                     uint32_t n_rot_pairs, uint32_t flags, const float *dq_in, const wr_append_extra *extra)
+                     uint32_t n_rot_pairs, uint32_t flags, const float *dq_in, const wr_append_extra *extra, bool dependent)
 {
     append_params p;
     for (uint32_t s = 0; s < n_sess; ++s) {
@@ -845,7 +845,7 @@ int wr_append_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
             pp.q16 = extra->q16;
         }
         pp.per_cta = std::min(std::max(n_tok / (2u * (uint32_t)ctx->sm_count), 1u), kPromptTokens);
-        WR_CUDA_TRY(wr_launch_pdl(rope_prompt_append_kernel, dim3((n_tok + pp.per_cta - 1) / pp.per_cta), dim3(kAppendThreads), 0,
+        WR_CUDA_TRY(wr_launch(dependent, rope_prompt_append_kernel, dim3((n_tok + pp.per_cta - 1) / pp.per_cta), dim3(kAppendThreads), 0,
                                   ctx->stream, pp));
         ctx->launches++;
         ctx->pdl_kind = WR_PDL_APPEND;
@@ -855,7 +855,7 @@ int wr_append_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
     }
     const uint32_t q_ctas = (dq && p.rope) ? (n_q_heads + kAppendQHeads - 1) / kAppendQHeads : 0u;
     const dim3 grid(n_sess * n_tokens, 1 + q_ctas);
-    WR_CUDA_TRY(wr_launch_pdl(rope_kv_append_kernel, grid, dim3(kAppendThreads), hd * sizeof(float), ctx->stream, p));
+    WR_CUDA_TRY(wr_launch(dependent, rope_kv_append_kernel, grid, dim3(kAppendThreads), hd * sizeof(float), ctx->stream, p));
     ctx->launches++;
     ctx->pdl_kind = WR_PDL_APPEND;
     ctx->pdl_index = ctx->launches;

@@ -204,6 +204,11 @@ int wr_decode_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
                      float scale_override, uint32_t window, int emit_triples, wr_decode_xchg *xchg,
                      bool early_tiles = false);
 
+// wr_cuda_decode_step; dependent: the append may start while the kernel before it is finishing (wr_launch_pdl)
+int wr_decode_step(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer, const uint32_t *positions, float *q,
+                   const float *k_rows, const float *v_rows, float *out, uint32_t n_q_heads, float theta_base,
+                   uint32_t n_rot_pairs, uint32_t flags, float scale_override, uint32_t window, int mem, bool dependent);
+
 int wr_ctx_reserve_stage(wr_cuda_ctx *ctx, size_t dev_bytes, size_t host_bytes);
 // Wait for the context's stream and report (and clear) the device-side error
 // word: WR_CUDA_ERR_INTERNAL when a kernel gave up on a bounded wait.  Every
@@ -218,7 +223,8 @@ int wr_append_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
                      const uint32_t *positions, uint32_t n_tokens, const float *dk,
                      const float *dv, float *dq, uint32_t n_q_heads, float theta_base,
                      uint32_t n_rot_pairs, uint32_t flags,
-                     const float *dq_in /* null: rotate dq in place */, const struct wr_append_extra *extra = nullptr);
+                     const float *dq_in /* null: rotate dq in place */, const struct wr_append_extra *extra = nullptr,
+                     bool dependent = true /* may start while the kernel before it is finishing */);
 // What the append of a prompt's rows (head_dim 128, rows 16-byte aligned) can do on the way: RMSNorm of every Q and K
 // head first, and the rotated queries as F16 rows elsewhere (dq then stays as it is).
 struct wr_append_extra {
@@ -265,8 +271,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... Params>
-inline cudaError_t wr_launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                 const Params &...p)
+inline cudaError_t wr_launch(bool dependent, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                             const Params &...p)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -277,8 +283,14 @@ inline cudaError_t wr_launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 bloc
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, p...);
+}
+template <typename... Params>
+inline cudaError_t wr_launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                 const Params &...p)
+{
+    return wr_launch(true, kernel, grid, block, smem, stream, p...);
 }
 
 // Reference sentinel for "no score yet" / masked keys (src/core/kernels.c:1480).
