@@ -1,7 +1,7 @@
-"""GPU: the append kernel of prompts (64 tokens and more, head_dim 128, 16-byte aligned rows) leaves the cache bytes and
+"""GPU: the append kernel of prompts (many tokens or heads, head_dim 128, 16-byte aligned rows) leaves the cache bytes and
 rotated rows of the kernel that takes a token at a time, which test_gpu_kv_append.py checks against the oracle: blocks of one, two
 and four tokens with remainders, several sessions in one call, heads that leave a thread's batch half full, partial and
-no rotation, page borders; rows that are not aligned take the other kernel."""
+no rotation, page borders, both sides of each line between the kernels; rows that are not aligned take the other kernel."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,10 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n_sess,n,hq,hkv,n_rot,rope,first", [
     (1, 64, 4, 4, 0, True, 0), (1, 63, 4, 4, 0, True, 2), (1, 130, 5, 1, 20, True, 61), (3, 200, 10, 2, 0, True, 30), (2, 600, 0, 3, 63, True, 5),
-    (16, 5, 8, 8, 0, True, 127), (1, 1201, 16, 8, 1, True, 700), (1, 70, 4, 2, 0, False, 3)])
+    (16, 5, 8, 8, 0, True, 127), (1, 1201, 16, 8, 1, True, 700), (1, 70, 4, 2, 0, False, 3),
+    # 32 heads and more, from 64 tokens; fewer, from 8192 rows of heads or 1536 small CTAs
+    (1, 64, 16, 8, 0, True, 0), (1, 63, 16, 8, 0, True, 2), (3, 50, 40, 1, 20, True, 61), (16, 5, 32, 8, 0, True, 127), (1, 130, 36, 2, 0, False, 3),
+    (2, 683, 0, 3, 63, True, 5), (1, 1170, 5, 1, 7, True, 0), (1, 1535, 0, 1, 0, True, 3), (1, 1537, 0, 1, 0, True, 3), (1, 768, 2, 1, 64, True, 63)])
 @pytest.mark.parametrize("aligned", [True, False])
 def test_rows_and_bytes_of_the_token_kernel(n_sess, n, hq, hkv, n_rot, rope, first, aligned):
     import torch

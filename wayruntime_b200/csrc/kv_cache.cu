@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(kAppendThreads) rope_kv_append_kernel(const ap
     }
 }
 
-// The same for 64 tokens and more (head_dim 128).  rope_kv_append_kernel spends a prompt's time on starting
+// The same for many rows (head_dim 128).  rope_kv_append_kernel spends a prompt's time on starting
 // 256 threads per token and eight Q heads, each with a table of angles of its own, and moves two and four bytes at a
 // time.  Here a CTA has up to four tokens, their angles are worked out once, and a thread moves sixteen values of a head
 // (eight and the eight that they pair with): 64 bytes in, 32 or 64 out.  HBM bounds it from there.  2048 tokens of 8 K
@@ -680,7 +680,7 @@ struct prompt_append_params {
     __half *q16;                     // rotated Q rows as F16 instead of back into a.q_rows, or null
     uint32_t per_cta;                // tokens
 };
-constexpr uint32_t kPromptLeast = 64, kPromptTokens = 4, kPromptHd = 128, kPromptHalf = kPromptHd / 2;
+constexpr uint32_t kPromptTokens = 4, kPromptHd = 128, kPromptHalf = kPromptHd / 2;
 
 __global__ void __launch_bounds__(kAppendThreads) rope_prompt_append_kernel(const prompt_append_params p)
 {
@@ -829,13 +829,19 @@ int wr_append_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
     p.n_rot = (n_rot_pairs >= 1 && n_rot_pairs < half) ? n_rot_pairs : half;  // kernels.c:1381-1383
     p.theta = (theta_base < 1.0f) ? 10000.0f : theta_base;                    // kernels.c:1374
     p.rope = (flags & WR_CUDA_APPEND_ROPE) ? 1u : 0u;
-    // Many tokens: the prompt kernel, where its 16-byte pieces are aligned; cache bytes and rotated rows are the same in both.  The
-    // line: an append and attention of 17 tokens take 52.7 us (one kv head) and 21.9 (8, with 32 Q heads) with the kernel
-    // above, 53.5 and 21.9 with this one; of 64 tokens with 40 Q heads 25.2 and 24.1.
+    // Many rows: the prompt kernel, where its 16-byte pieces are aligned; cache bytes and rotated rows are the same in both.  It
+    // costs 2.3 us to begin with, the other 1.5 and what its small CTAs add up to: where the line lies hangs on the heads.  us, the
+    // kernel above / this one, in a graph of appends, for kv heads + rotated q heads:
+    //     1 + 0   512 tokens 1.8 / 3.4   1024 2.8 / 3.4   2048 5.7 / 4.3        8 + 0   384 tokens 3.0 / 3.3   512 4.6 / 3.6
+    //     1 + 2   512 tokens 2.8 / 3.5   1024 5.5 / 3.6                          4 + 16  192 tokens 2.7 / 2.7   384 4.4 / 3.4
+    //     8 + 16   48 tokens 2.3 / 2.3     64 2.7 / 2.4                          8 + 32   48 tokens 2.4 / 2.4    64 3.4 / 2.8
     const uint32_t n_tok = n_sess * n_tokens;
     const bool vectors = hd == kPromptHd && p.q_in == p.q_rows && (((uintptr_t)dk | (uintptr_t)dv | (uintptr_t)dq) & 15u) == 0;
     if (extra && !vectors) return WR_CUDA_ERR_UNSUPPORTED;
-    if (vectors && (n_tok >= kPromptLeast || extra)) {
+    const uint32_t q_ctas = (dq && p.rope) ? (n_q_heads + kAppendQHeads - 1) / kAppendQHeads : 0u;
+    const uint32_t heads = 2 * p.n_kv + (q_ctas ? n_q_heads : 0u);
+    const bool many = heads >= 32 ? n_tok >= 64 : (uint64_t)n_tok * heads >= 8192 || (uint64_t)n_tok * (1 + q_ctas) >= 1536;
+    if (vectors && (many || extra)) {
         prompt_append_params pp{};
         pp.a = p;
         if (extra) {
@@ -853,7 +859,6 @@ int wr_append_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
         WR_CUDA_TRY(cudaGetLastError());
         return WR_CUDA_OK;
     }
-    const uint32_t q_ctas = (dq && p.rope) ? (n_q_heads + kAppendQHeads - 1) / kAppendQHeads : 0u;
     const dim3 grid(n_sess * n_tokens, 1 + q_ctas);
     WR_CUDA_TRY(wr_launch(dependent, rope_kv_append_kernel, grid, dim3(kAppendThreads), hd * sizeof(float), ctx->stream, p));
     ctx->launches++;
