@@ -349,7 +349,9 @@ typedef struct wr_cuda_model_desc {
 } wr_cuda_model_desc;
 
 /* Uploads every weight (one device allocation) and takes the row scratch; the
- * host copies are not referenced after the call returns. */
+ * host copies are not referenced after the call returns.  With max_rows above WR_CUDA_BATCH_MAX the layers' weights are
+ * kept a second time, as the tensor cores read them, where that takes at most a sixteenth of the device's memory; room for one
+ * layer otherwise.  (wr_cuda_model_bytes counts both.) */
 int  wr_cuda_model_create(wr_cuda_ctx *ctx, const wr_cuda_model_desc *desc, wr_cuda_model **out);
 void wr_cuda_model_destroy(wr_cuda_model *m);
 uint64_t wr_cuda_model_bytes(const wr_cuda_model *m);      /* device bytes held */

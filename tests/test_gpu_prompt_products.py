@@ -192,19 +192,115 @@ def test_a_rows_bits_do_not_depend_on_how_many_follow():
     assert np.array_equal(many["hidden"][:128], few["hidden"][:128])
 
 
-def test_weights_are_split_for_each_call_where_memory_is_short():
-    """Split weights are kept when they take a sixteenth of the free memory or less; the results are the same."""
+def _like_normal(shape, seed, scale):
+    """Large weights quickly: a period of normal values that no dimension here divides."""
+    n = int(np.prod(shape))
+    return np.resize(_gen.normal(seed, (1000003,), scale), n).reshape(shape)
+
+
+def _run_in_portions(dm, kv, tokens, portion):
+    res = [dm.forward(dm.FWD_PREFILL, [kv], [at], tokens[at:at + portion], hidden=True, attn_tap=True)
+           for at in range(0, len(tokens), portion)]
+    return np.concatenate([r["hidden"] for r in res]), np.concatenate([r["attn"] for r in res], axis=1)
+
+
+def test_weights_are_split_for_each_call_in_models_too_large_to_keep_them():
+    """Split weights are kept when they take a sixteenth of the device's memory or less; here they would take more, and the
+    layers (all of the same weights) use one layer's memory in turn."""
     import torch
-    shape = dict(n_layers=2, hidden=1024, n_q_heads=8, n_kv_heads=4, head_dim=128, vocab=300, ffn=4096)
-    w = _weights(shape, 1303)
-    tokens = [(7 * r + 1) % 300 for r in range(150)]
-    kept, v = _run(shape, 150, w, 256, tokens)
+    import wayruntime_b200 as wr
+    limit = torch.cuda.mem_get_info()[1] // 16
+    one = dict(hidden=8192, n_q_heads=2, n_kv_heads=1, head_dim=128, vocab=64, ffn=24576)
+    layer = 4 * 8192 * (6 * 128 + 3 * 24576)
+    shape = dict(one, n_layers=limit // layer + 1)
+    big = {n: _like_normal(s, 1320 + i, s[1] ** -0.5) for i, (n, s) in enumerate(
+        dict(w_gate=(24576, 8192), w_up=(24576, 8192), w_down=(8192, 24576), wq=(256, 8192), wk=(128, 8192), wv=(128, 8192), wo=(8192, 256)).items())}
+    w = {"embed": _gen.normal(1327, (64, 8192)), "final_norm": np.ones(8192, np.float32)}
+    w["lm_head"] = w["embed"]
+    for i in range(shape["n_layers"]):
+        w.update({f"l{i}.{n}": a for n, a in big.items()})
+        w.update({f"l{i}.{n}": np.ones(8192, np.float32) for n in ("attn_norm", "ffn_norm")})
+    ctx = wr.Context(0)
+    dm = _model(ctx, w, shape, max_rows=64)
+    assert shape["n_layers"] * layer < dm.device_bytes < (shape["n_layers"] + 2) * layer
+    tokens, got = [(7 * r + 1) % 64 for r in range(40)], []
+    for portion in (40, 10):
+        kv = ctx.kv_create(shape["n_layers"], 1, 128, 40)
+        got.append(_run_in_portions(dm, kv, tokens, portion)[0])
+        kv.close()
+    assert np.abs(got[0] - got[1]).max() <= 2.0 ** -9 * np.abs(got[1]).max()        # (F16 keys and values)
+    dm.close()
+    ctx.close()
+
+
+def test_products_that_split_their_weights_in_slices():
+    """A feed-forward too wide for the digit sums (its down product takes the F32 kernels): no memory for prompts at all, and every other
+    product splits its weights through a workspace that stays small.  q | k | v in two slices, gate and up in five."""
+    import torch
+    import wayruntime_b200 as wr
+    hid, n_q, n_kv, ffn = 4096, 90, 30, 32772
+    shape = dict(n_layers=1, hidden=hid, n_q_heads=n_q, n_kv_heads=n_kv, head_dim=128, vocab=64, ffn=ffn)
+    w = {f"l0.{n}": _like_normal(s, 1330 + i, s[1] ** -0.5) for i, (n, s) in enumerate(
+        dict(w_gate=(ffn, hid), w_up=(ffn, hid), w_down=(hid, ffn), wq=(n_q * 128, hid), wk=(n_kv * 128, hid), wv=(n_kv * 128, hid),
+             wo=(hid, n_q * 128)).items())}
+    w.update({"embed": _gen.normal(1338, (64, hid)), "final_norm": np.ones(hid, np.float32),
+              "l0.attn_norm": 1 + _gen.normal(1339, (hid,), 0.1), "l0.ffn_norm": 1 + _gen.normal(1340, (hid,), 0.1)})
+    w["lm_head"] = w["embed"]
+    tokens = [(5 * r + 1) % 64 for r in range(24)]
+    ctx = wr.Context(0)
+    dm = _model(ctx, w, shape, max_rows=64)
+    kv = ctx.kv_create(1, n_kv, 128, 24)
     free = torch.cuda.mem_get_info()[0]
-    hold = torch.empty(free - (3 << 29), dtype=torch.uint8, device="cuda")       # 1.5 GB stay free, the weights are 128 MB
-    short, _ = _run(shape, 150, w, 256, tokens)
+    hidden, attn = _run_in_portions(dm, kv, tokens, 24)
+    assert free - torch.cuda.mem_get_info()[0] <= 320 << 20
+    v = kv.read_rows(0, 1, 0, 24).reshape(24, -1).view(np.float16).astype(np.float64)
+    kv.close()
+    dm.close()
+    ctx.close()
+    _check({"hidden": hidden, "attn": attn}, v, w, tokens)
+
+
+def test_head_columns_in_slices_and_without_the_memory_for_them():
+    """Mixed stack in F32, a head of 70003 columns for more rows than a decode batch: two slices through sums of their own.  A context
+    without the memory takes the F32 kernels."""
+    import torch
+    import wayruntime_b200 as wr
+    from _tumadra_models import attn, config, weights, with_mlp
+    from test_gpu_tumadra import build
+    cfg = config([with_mlp(attn(), 64)], width=1024, vocab=70003, groups=4)
+    rng = np.random.default_rng(1350)
+    w = weights(dict(cfg, vocab=8), 1351)
+    w["embed"], w["head"] = _like_normal((70003, 1024), 1352, 1.0), _like_normal((70003, 1024), 1353, 1024 ** -0.5)
+    tokens = [int(t) for t in rng.integers(0, 70003, 40)]
+
+    def logits(ctx, m, places):
+        kv = m.kv_create(64)
+        out = m.forward(m.FWD_PREFILL, [kv], [0], tokens, logits=places)["logits"]
+        kv.close()
+        return out
+
+    ctx = wr.Context(0)
+    m = build(ctx, cfg, w, "float32", max_rows=64)
+    few = np.concatenate([logits(ctx, m, list(range(lo, lo + 10))) for lo in range(0, 40, 10)])
+    free = torch.cuda.mem_get_info()[0]
+    many = logits(ctx, m, list(range(40)))
+    assert free - torch.cuda.mem_get_info()[0] <= 320 << 20
+    tol = 16 * 2.0 ** -24 * np.linalg.norm(few, axis=1, keepdims=True)
+    assert (np.linalg.norm(many - few, axis=1, keepdims=True) <= tol).all()
+    m.close()
+    ctx.close()
+    ctx = wr.Context(0)
+    m = build(ctx, cfg, w, "float32", max_rows=64)
+    logits(ctx, m, [0])
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (96 << 20), dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        short = logits(ctx, m, list(range(40)))
+        assert (np.linalg.norm(short - few, axis=1, keepdims=True) <= tol).all()
     del hold
     torch.cuda.empty_cache()
-    assert np.array_equal(kept["hidden"], short["hidden"])
+    m.close()
+    ctx.close()
 
 
 @pytest.mark.parametrize("qk_norm", [True, False])

@@ -600,53 +600,55 @@ int launch_batch(wr_cuda_ctx *ctx, GemvParams &p)
     return WR_CUDA_OK;
 }
 
-}  // namespace
-
-namespace {
-
-// out = act(sum of the parts + bias) mul + add for one product of many rows
-__global__ void __launch_bounds__(256) finish_rows_kernel(const GemvParams p, const float *parts, uint32_t n_parts, uint32_t ld)
+// out = act(sum of the parts + bias) mul + add for columns n0 on of one product of many rows
+__global__ void __launch_bounds__(256) finish_rows_kernel(const GemvParams p, const float *parts, uint32_t n_parts, uint32_t ld,
+                                                          uint32_t n0)
 {
     pdl_trigger();
     pdl_wait();
-    const uint32_t row = blockIdx.y, n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= p.seg[0].n) return;
-    float y = parts[(size_t)row * ld + n];
-    for (uint32_t j = 1; j < n_parts; ++j) y = __fadd_rn(y, parts[((size_t)j * p.rows + row) * ld + n]);
+    const uint32_t row = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x, n = n0 + c;
+    if (c >= ld || n >= p.seg[0].n) return;
+    float y = parts[(size_t)row * ld + c];
+    for (uint32_t j = 1; j < n_parts; ++j) y = __fadd_rn(y, parts[((size_t)j * p.rows + row) * ld + c]);
     p.seg[0].out[(size_t)row * p.seg[0].out_stride + n] = finish(p, 0, n, row, y);
 }
 
 // More rows than a decode batch: the tensor-core product of gemm_f32.cu, weights and rows split into the context's
 // workspace on the way.  17 rows are two passes of the GEMV over the weights; this is three (in, out and in again, the
-// last two in L2) whatever the rows, and the products at the tensor cores' rate.  Two layers of the mixed stack in F32, the whole
-// call: 17 rows of width 4096 2459 -> 1464 us, 40 of 2048 1268 -> 661, 700 of 1024 4568 -> 1172.  WR_CUDA_ERR_NOMEM: no
-// workspace.
+// last two in L2 where they fit) whatever the rows, and the products at the tensor cores' rate.  Two layers of the mixed stack in
+// F32, the whole call: 17 rows of width 4096 2459 -> 1464 us, 40 of 2048 1268 -> 661, 700 of 1024 4568 -> 1172.
+// Split weights take kWideBytes at most: larger ones go in slices of output columns, one after the other through the same memory
+// (a 151936 x 4096 head would keep 2.5 GB; with half of it 17 rows through two layers of width 4096, whose 4096 x 12288 products
+// then have too few tiles for the device, take 1799 us instead of 1440).  Columns are products of their own, so slices change no bits.  The split rows take what
+// F32 rows would.  WR_CUDA_ERR_NOMEM: no workspace.
+constexpr size_t kWideBytes = (size_t)256 << 20;
+
 int launch_wide(wr_cuda_ctx *ctx, GemvParams &p)
 {
     auto up256 = [](size_t n) { return (n + 255u) & ~(size_t)255u; };
-    uint32_t n = 0;
-    for (uint32_t s = 0; s < p.n_seg; ++s) n += p.seg[s].n;
     bool direct = !p.bias && p.act == WR_GEMV_ACT_NONE && p.mul == 1.f && !p.add;
-    for (uint32_t s = 0; s < (p.swiglu ? 1u : p.n_seg); ++s)
+    const uint32_t n_out = p.swiglu ? 1u : p.n_seg;
+    for (uint32_t s = 0; s < n_out; ++s)
         direct = direct && !(p.seg[s].n & 3u) && !(p.seg[s].out_stride & 3u) && !((uintptr_t)p.seg[s].out & 15u);
     if (!direct && (p.swiglu || p.n_seg > 1)) return WR_CUDA_ERR_UNSUPPORTED;
-    wr_split_source src{};
-    wr_split_weight &w = src.to;
-    w.n = p.swiglu ? (p.seg[0].n + 7u) / 8u * 16u : (n + 3u) & ~3u;
-    w.k = p.k;
-    for (uint32_t s = 0; s < p.n_seg; ++s) {
-        src.src[s] = p.seg[s].w;
-        src.n[s] = p.seg[s].n;
-    }
-    src.pair = p.swiglu;
-    const uint32_t parts = direct ? 1u : wr_f32_gemm_k_parts(w.n, w.k), ld = wr_split_ld(p.k);
+    // columns: of all segments one after the other, or of gate and up
+    uint32_t n = 0;
+    for (uint32_t s = 0; s < n_out; ++s) n += p.seg[s].n;
+    const uint32_t parts = direct ? 1u : wr_f32_gemm_k_parts((n + 3u) & ~3u, p.k), ld = wr_split_ld(p.k);
     if (!wr_f32_gemm_covers(p.k, parts)) return WR_CUDA_ERR_UNSUPPORTED;
-    const size_t b_blocks = up256(wr_split_weight_bytes(w.n, w.k)), b_exponent = up256((size_t)w.n * 4);
+    auto weight_rows_of = [&](uint32_t cols) { return p.swiglu ? (cols + 7u) / 8u * 16u : (cols + 3u) & ~3u; };
+    const size_t col_bytes = std::max((size_t)(p.swiglu ? 2 : 1) * ld * 4, direct ? 0 : (size_t)parts * p.rows * 4);
+    const uint32_t slice = (uint32_t)std::min<size_t>(n, std::max<size_t>(kWideBytes / col_bytes / kWBlock, 1) * kWBlock);
+    const uint32_t most = weight_rows_of(slice);
+    const size_t b_blocks = up256(wr_split_weight_bytes(most, p.k)), b_exponent = up256((size_t)most * 4);
     const size_t b_rows = up256((size_t)2 * p.rows * ld * 2), b_scale = up256(p.rows * sizeof(wr_split_scale));
-    const size_t b_parts = direct ? 0 : (size_t)parts * p.rows * w.n * 4;
-    int rc = wr_ctx_reserve_ws(ctx, b_blocks + b_exponent + b_rows + b_scale + b_parts, 0);
+    const size_t b_parts = direct ? 0 : (size_t)parts * p.rows * most * 4;
+    int rc = wr_ctx_try_ws(ctx, b_blocks + b_exponent + b_rows + b_scale + b_parts);
     if (rc != WR_CUDA_OK) return rc;
     char *at = reinterpret_cast<char *>(ctx->ws);
+    wr_f32_gemm_args a{};
+    wr_split_weight &w = a.source.to;
+    w.k = p.k;
     w.blocks = at;
     w.exponent = reinterpret_cast<int *>(at += b_blocks);
     wr_split_rows_args r{};
@@ -656,21 +658,39 @@ int launch_wide(wr_cuda_ctx *ctx, GemvParams &p)
     r.row_scale = reinterpret_cast<wr_split_scale *>(at += b_rows);
     float *sums = reinterpret_cast<float *>(at += b_scale);
     CUtensorMap map;
-    if ((rc = wr_split_weights_launch(ctx, &src, 1)) != WR_CUDA_OK || (rc = wr_split_rows_launch(ctx, r)) != WR_CUDA_OK ||
-        (rc = wr_gemm_map_rows(&map, r.out, 2 * p.rows, ld, ld)) != WR_CUDA_OK)
-        return rc;
-    wr_f32_gemm_args a{};
-    a.source = src; a.x = p.x; a.x_stride = p.x_stride; a.norm_w = p.norm_w;
-    a.m = a.pad = p.rows; a.row_scale = r.row_scale; a.k_parts = parts; a.n_seg = p.swiglu ? 1u : p.n_seg;
-    if (direct)
-        for (uint32_t s = 0; s < a.n_seg; ++s) a.seg[s] = {p.seg[s].out, p.seg[s].n, p.seg[s].out_stride};
-    else
-        a.seg[0] = {sums, w.n, w.n};
-    if ((rc = wr_f32_gemm_launch(ctx, map, a)) != WR_CUDA_OK || direct) return rc;
-    WR_CUDA_TRY(wr_launch_pdl(finish_rows_kernel, dim3((n + 255) / 256, p.rows), dim3(256), 0, ctx->stream, p, (const float *)sums,
-                              parts, w.n));
-    ctx->launches++;
-    WR_CUDA_TRY(cudaGetLastError());
+    if ((rc = wr_gemm_map_rows(&map, r.out, 2 * p.rows, ld, ld)) != WR_CUDA_OK) return rc;
+    a.source.pair = p.swiglu; a.x = p.x; a.x_stride = p.x_stride; a.norm_w = p.norm_w;
+    a.m = a.pad = p.rows; a.row_scale = r.row_scale; a.k_parts = parts;
+    for (uint32_t c0 = 0; c0 < n; c0 += slice) {
+        const uint32_t c1 = std::min(n, c0 + slice);
+        w.n = weight_rows_of(c1 - c0);
+        a.n_seg = 0;
+        uint32_t at_col = 0, k = 0;
+        for (uint32_t s = 0; s < n_out; ++s, at_col += p.seg[s - 1].n) {      // what of each segment lies in the slice
+            const uint32_t lo = std::max(c0, at_col), hi = std::min(c1, at_col + p.seg[s].n);
+            if (lo >= hi) continue;
+            a.source.src[k] = p.seg[s].w + (size_t)(lo - at_col) * p.k;
+            a.source.n[k++] = hi - lo;
+            a.seg[a.n_seg++] = {p.seg[s].out + (lo - at_col), hi - lo, p.seg[s].out_stride};
+            if (p.swiglu) {
+                a.source.src[k] = p.seg[1].w + (size_t)lo * p.k;
+                a.source.n[k++] = hi - lo;
+            }
+        }
+        for (; k < 3; ++k) {
+            a.source.src[k] = nullptr;
+            a.source.n[k] = 0;
+        }
+        if (!direct) a.seg[0] = {sums, w.n, w.n};
+        if ((rc = wr_split_weights_launch(ctx, &a.source, 1)) != WR_CUDA_OK) return rc;
+        if (c0 == 0 && (rc = wr_split_rows_launch(ctx, r)) != WR_CUDA_OK) return rc;
+        if ((rc = wr_f32_gemm_launch(ctx, map, a)) != WR_CUDA_OK) return rc;
+        if (direct) continue;
+        WR_CUDA_TRY(wr_launch_pdl(finish_rows_kernel, dim3((c1 - c0 + 255) / 256, p.rows), dim3(256), 0, ctx->stream, p,
+                                  (const float *)sums, parts, w.n, c0));
+        ctx->launches++;
+        WR_CUDA_TRY(cudaGetLastError());
+    }
     return WR_CUDA_OK;
 }
 

@@ -227,6 +227,28 @@ int wr_ctx_reserve_ws(wr_cuda_ctx *ctx, size_t ws_bytes, size_t tickets)
     return WR_CUDA_OK;
 }
 
+int wr_ctx_try_ws(wr_cuda_ctx *ctx, size_t ws_bytes)
+{
+    if (ws_bytes <= ctx->ws_bytes) return WR_CUDA_OK;
+    if (ws_bytes >= ctx->ws_refused) return WR_CUDA_ERR_NOMEM;
+    const size_t want = std::max(ws_bytes, (size_t)8 << 20);
+    float *ws = nullptr;
+    if (cudaMalloc((void **)&ws, want) != cudaSuccess) {
+        (void)cudaGetLastError();
+        ctx->ws_refused = ws_bytes;
+        return WR_CUDA_ERR_NOMEM;
+    }
+    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        (void)cudaFree(ws);
+        return WR_CUDA_ERR_INTERNAL;
+    }
+    if (ctx->ws) (void)cudaFree(ctx->ws);
+    ctx->ws = ws;
+    ctx->ws_bytes = want;
+    return WR_CUDA_OK;
+}
+
 // -------------------------------------------------------------- page pool
 
 static int pool_take(wr_cuda_ctx *ctx, uint64_t page_bytes, size_t n, size_t *pool_index,

@@ -748,7 +748,7 @@ template <typename T, typename TO, int LG> int scan_pieces(wr_cuda_ctx *ctx, con
 {
     const uint32_t pieces = (rw.n_rows + kScanPiece - 1) / kScanPiece;
     const size_t held = 4u << LG, n_ends = (size_t)(pieces - 1) * wr_ld(a.inner) * held, n_steps = (size_t)(pieces - 1) * wr_ld(a.inner);
-    const int rc = wr_ctx_reserve_ws(ctx, (n_ends + n_steps) * 4, 0);
+    const int rc = wr_ctx_try_ws(ctx, (n_ends + n_steps) * 4);
     if (rc != WR_CUDA_OK) return rc;
     float *ends = ctx->ws, *steps = ends + n_ends;
     const int first = scan_one<T, TO, 4, LG, SCAN_ENDS>(ctx, rw, a, pieces - 1, ends, steps);

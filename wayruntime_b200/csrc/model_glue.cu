@@ -176,8 +176,8 @@ size_t up256(size_t n) { return (n + 255u) & ~(size_t)255u; }
 
 // What the rows of a prompt need beside the weights.  Splitting a layer's weights for each call moves them three times (a
 // prompt of 1000 rows of the Qwen3-0.6B shape: 0.6 of 6.6 ms; of 17 rows most of its time), so split weights are kept where
-// they take little: a sixteenth of the memory that is free.  Otherwise all layers use the same memory in turn.  A model that
-// cannot have even that keeps the GEMV for prompts.
+// they take little: a sixteenth of the device's memory for a model, whatever else is on it.  Otherwise all layers use the same
+// memory in turn.  A model that cannot have even that splits every product's weights through the context's workspace (gemv.cu).
 void take_prompt_memory(wr_cuda_model *m)
 {
     if (m->max_rows <= WR_CUDA_BATCH_MAX) return;
@@ -207,7 +207,7 @@ void take_prompt_memory(wr_cuda_model *m)
     const size_t rest = rows + up256(R * sizeof(wr_split_scale)) + sums;
     size_t free_bytes = 0, total_bytes = 0;
     if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) (void)cudaGetLastError();
-    m->split_kept = all <= free_bytes / 16 && cudaMalloc((void **)&m->prompt, all + rest) == cudaSuccess;
+    m->split_kept = all <= total_bytes / 16 && cudaMalloc((void **)&m->prompt, all + rest) == cudaSuccess;
     if (!m->split_kept && cudaMalloc((void **)&m->prompt, most + rest) != cudaSuccess) m->prompt = nullptr;
     (void)cudaGetLastError();
     if (!m->prompt) return;
@@ -459,6 +459,7 @@ extern "C" void wr_cuda_model_destroy(wr_cuda_model *m)
         if (m->mixed) wr_mixed_destroy(m->mixed);
         cudaFree(m->slab);
         cudaFree(m->prompt);
+        m->ctx->ws_refused = ~(size_t)0;
         drop_side(m);
         cudaFreeHost(m->h_tokens);
     }
