@@ -88,3 +88,48 @@ def test_threads_take_and_give_back():
     for t in threads:
         t.join()
     assert not bad and lib.made <= 3 * 8 * 2           # (three size classes, an old and a new array per thread)
+
+
+def test_arrays_made_together_go_one_by_one():
+    lib = FakeLib()
+    rows = _ResultRows(lib, 1)
+    some, at = rows.many(16, (1, 40000))
+    assert at == [a.ctypes.data for a in some]
+    for i, a in enumerate(some):
+        a[:] = i
+    assert lib.made == 16 and len({a.ctypes.data for a in some}) == 16
+    kept = some[5]
+    del some, a
+    gc.collect()
+    more, _ = rows.many(16, (1, 40000))                  # fifteen blocks are free again, the kept row's is not
+    for a in more:
+        a[:] = -1
+    assert lib.made == 17 and (kept == 5).all()
+    rows.LIMIT = lib.made << 18
+    del more, a
+    assert [a.base is None for a in rows.many(18, (1, 40000))[0]] == [False] * 16 + [True] * 2
+
+
+def test_an_engine_gives_every_session_a_row_of_its_own():
+    from wayruntime_b200.engine import Engine
+
+    class Model:
+        FWD_DECODE, FWD_PREFILL, ROWS_APART, vocab, max_rows = 0, 1, True, 40000, 64
+        rows = _ResultRows(FakeLib(), 1)
+
+        def kv_create(self, n):
+            return None
+
+        def forward(self, mode, kvs, positions, tokens, out_from=0, *, logits=False, argmax=False, apart=False):
+            assert apart and mode == self.FWD_DECODE
+            out, _ = self.rows.many(len(logits), (1, self.vocab))
+            for a, i in zip(out, logits):
+                a[:] = tokens[i]
+            return {"logits": out}
+
+    e = Engine(Model())
+    got = e.advance([e.session(8) for _ in range(6)], [[i] for i in range(6)], [[0], [], [0], [0, 0], [0], [0]])
+    for i, g in enumerate(got):
+        assert g.shape == (([1, 0, 1, 2, 1, 1][i]), 40000) and (g == i).all()
+    assert not any(np.shares_memory(a, b) for i, a in enumerate(got) for b in got[:i])
+    assert Model.rows._bytes == 5 << 18

@@ -12,7 +12,6 @@ import ctypes as C
 import math
 import os
 import threading
-import weakref
 from collections import deque
 
 import numpy as np
@@ -235,34 +234,52 @@ class _ResultRows:
         self._lock = threading.Lock()
         self._back = deque()             # (size, address) of arrays that are gone: their finalizers may run anywhere
         self._idle = {}                  # size -> addresses
+        self._types = {}                 # size -> type of its blocks
         self._bytes = 0
 
     def empty(self, shape):
-        n = 4 * math.prod(shape)
-        p = self._take(1 << (n - 1).bit_length()) if n >= self.LEAST else None
-        if p is None:
-            return np.empty(shape, np.float32)
-        size, address = p
-        block = (C.c_char * n).from_address(address)
-        weakref.finalize(block, self._give_back, p).atexit = False
-        return np.frombuffer(block, np.float32).reshape(shape)
+        return self.many(1, shape)[0][0]
+
+    def many(self, count, shape):
+        """`count` arrays, each with a block of its own (one that is kept costs no more than itself), and their addresses."""
+        n, places = 4 * math.prod(shape), []
+        if n >= self.LEAST:
+            size = 1 << (n - 1).bit_length()
+            with self._lock:
+                self._collect()
+                while len(places) < count and (place := self._take(size)):
+                    places.append(place)
+        arrays = [np.ndarray(shape, np.float32, self._block(place)) for place in places]
+        at = [place[1] for place in places]
+        for _ in range(count - len(places)):
+            arrays.append(np.empty(shape, np.float32))
+            at.append(arrays[-1].ctypes.data)
+        return arrays, at
+
+    def _block(self, place):
+        """What an array keeps as its base: gone, the memory goes back."""
+        of = self._types.get(place[0])
+        if of is None:
+            back = self._give_back
+            of = self._types[place[0]] = type("Block", (C.c_char * place[0],), {"__del__": lambda block: back(block.place)})
+        block = of.from_address(place[1])
+        block.place = place
+        return block
 
     def _take(self, size):
-        with self._lock:
-            self._collect()
-            if self._idle.get(size):
-                return size, self._idle[size].pop()
-            if size > self.LIMIT or self._handle is None:
-                return None
+        if self._idle.get(size):
+            return size, self._idle[size].pop()
+        if size > self.LIMIT or self._handle is None:
+            return None
+        if self._bytes + size > self.LIMIT:
+            self._release()
             if self._bytes + size > self.LIMIT:
-                self._release()
-                if self._bytes + size > self.LIMIT:
-                    return None
-            p = C.c_void_p()
-            if self._lib.wr_cuda_host_alloc(self._handle, size, C.byref(p)) != 0:
                 return None
-            self._bytes += size
-            return size, p.value
+        p = C.c_void_p()
+        if self._lib.wr_cuda_host_alloc(self._handle, size, C.byref(p)) != 0:
+            return None
+        self._bytes += size
+        return size, p.value
 
     def _collect(self):
         while self._back:
@@ -526,6 +543,7 @@ class DeviceModel:
     `l{i}.attn_norm|wq|wk|wv|q_norm|k_norm|wo|ffn_norm|w_gate|w_up|w_down`."""
 
     FWD_DECODE, FWD_PREFILL = 0, 1
+    ROWS_APART = True                    # forward takes `apart`
 
     def __init__(self, ctx: "Context", weights: dict, *, n_layers, hidden, n_q_heads, n_kv_heads, head_dim,
                  vocab, ffn, rms_eps=1e-6, rope_theta=10000.0, n_rot_pairs=0, attn_scale=0.0, max_rows=256):
@@ -583,10 +601,11 @@ class DeviceModel:
         return KVCache._of_handle(self._ctx, h, max_ctx)
 
     def forward(self, mode, kvs, positions, tokens, out_from=0, *, hidden=False, normed=False, logits=False,
-                argmax=False, attn_tap=False) -> dict:
+                argmax=False, attn_tap=False, apart=False) -> dict:
         """One forward pass; returns the requested results for rows [out_from, n) as numpy arrays.
         logits may be a list of places among those rows (the others are skipped): the result then has
-        one row per place, in the list's order."""
+        one row per place, in the list's order.  apart: the rows of logits come as a list of arrays [1, vocab]
+        that share no memory, for callers that give them to different owners."""
         n = len(tokens)
         n_out = n - out_from
         res = {}
@@ -594,17 +613,22 @@ class DeviceModel:
         nrm = np.empty((n_out, self.hidden), np.float32) if normed else None
         some = None if isinstance(logits, bool) else [int(i) for i in logits]
         logits = bool(some) if some is not None else logits
-        lg = self._ctx._rows.empty((len(some) if some is not None else n_out, self.vocab)) if logits else None
+        asked = some if some is not None else range(n_out)
+        lg = None
+        if logits and apart:
+            lg, at = self._ctx._rows.many(len(asked), (1, self.vocab))
+        elif logits:
+            (lg,), (at,) = self._ctx._rows.many(1, (len(asked), self.vocab))
+            at = range(at, at + lg.nbytes, 4 * self.vocab)
         am = (C.c_uint32 * max(n_out, 1))() if argmax else None
         tap = np.empty((self.n_layers, n, self.n_q * self.hd), np.float32) if attn_tap else None
         lptrs = None
         if logits:
             lptrs = (C.c_void_p * max(n_out, 1))()
-            base, row = lg.ctypes.data, lg.strides[0]
-            for j, i in enumerate(some if some is not None else range(n_out)):
+            for i, to in zip(asked, at):
                 if not 0 <= i < n_out or lptrs[i]:
                     raise ValueError("places out of range or named twice")
-                lptrs[i] = base + j * row
+                lptrs[i] = to
         _check(self._lib.wr_cuda_model_forward(
             self._ctx._h, self._h, mode, n, Context._handles(kvs), Context._u32s(positions),
             Context._u32s(tokens), out_from, hid.ctypes.data if hidden else None,

@@ -96,15 +96,16 @@ class Engine:
     def _decode(self, rows, sessions, tokens, want, argmax, out):
         m = self.model
         asked = [j for j, i in enumerate(rows) if len(want[i])]
+        own = {"apart": True} if asked and not argmax and getattr(m, "ROWS_APART", False) else {}
         res = m.forward(m.FWD_DECODE, [sessions[i].kv for i in rows], [sessions[i].pos for i in rows],
-                        [tokens[i][0] for i in rows], logits=False if argmax else asked, argmax=argmax)
+                        [tokens[i][0] for i in rows], logits=False if argmax else asked, argmax=argmax, **own)
         for j, i in enumerate(rows):
             sessions[i].pos += 1
             if argmax:
                 out[i] = int(res["argmax"][j])
             elif j in asked:
                 at = asked.index(j)
-                row = res["logits"][at:at + 1]           # (its own row: nothing is copied for one place)
+                row = res["logits"][at] if own else res["logits"][at:at + 1]
                 out[i] = row if len(want[i]) == 1 else row.repeat(len(want[i]), axis=0)
             else:
                 out[i] = np.empty((0, m.vocab), np.float32)
