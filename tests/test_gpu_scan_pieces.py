@@ -1,4 +1,4 @@
-"""GPU: selective scan of portions that are cut into pieces (more than 512 tokens), against the float64 restatement:
+"""GPU: selective scan of portions that are cut into pieces (more than 768 tokens here), against the float64 restatement:
 state sizes around those that two, four and eight threads hold, pieces with remainders, a portion that goes on from a
 state, and the decode step behind it.  Tolerances as for the mixer alone (test_gpu_tumadra.py)."""
 import numpy as np
@@ -22,7 +22,7 @@ def test_portions_of_several_pieces(dtype, inner, state):
     want = []
     plain.forward(cfg, w, toks, want)
     m = build(ctx, cfg, w, dtype, max_rows=2048)
-    for cuts in ([1109, 1], [513, 596, 1], [300, 768, 41, 1]):
+    for cuts in ([1109, 1], [513, 596, 1], [300, 768, 41, 1], [300, 769, 40, 1], [20, 1089, 1]):
         kv, pos = m.kv_create(1200), 0
         for n in cuts:
             tap = np.zeros((1, n, 48), np.float32)

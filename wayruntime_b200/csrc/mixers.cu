@@ -521,7 +521,11 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, co
         for (uint32_t i = 0; i < piece; ++i) {
             e.decay(steps[(size_t)i * ld + c], A2);
             b.load(ends + ((size_t)i * ld + c) * HELD + part * NS);
+            States<NS> before = S;
             S.advance(e, b);
+#pragma unroll
+            for (int j = 0; j < NS; ++j)                         // (token by token an infinite state stays what it is)
+                if (isinf(before.get(j))) S.set(j, before.get(j) + b.get(j));
         }
     }
     __syncthreads();
@@ -747,27 +751,39 @@ int scan_one(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a, uint32_
 template <typename T, typename TO, int LG> int scan_pieces(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a)
 {
     const uint32_t pieces = (rw.n_rows + kScanPiece - 1) / kScanPiece;
-    const size_t held = 4u << LG, n_ends = (size_t)(pieces - 1) * wr_ld(a.inner) * held, n_steps = (size_t)(pieces - 1) * wr_ld(a.inner);
-    const int rc = wr_ctx_try_ws(ctx, (n_ends + n_steps) * 4);
+    const int rc = wr_ctx_try_ws(ctx, wr_scan_ws_bytes(rw.n_rows, a.inner, a.state));
     if (rc != WR_CUDA_OK) return rc;
-    float *ends = ctx->ws, *steps = ends + n_ends;
+    float *ends = ctx->ws, *steps = ends + (size_t)(pieces - 1) * wr_ld(a.inner) * (4u << LG);
     const int first = scan_one<T, TO, 4, LG, SCAN_ENDS>(ctx, rw, a, pieces - 1, ends, steps);
     return first != WR_CUDA_OK ? first : scan_one<T, TO, 4, LG, SCAN_PIECE>(ctx, rw, a, pieces, ends, steps);
 }
 
-// One state per thread while that is what it takes to fill the device, two above; a choice by the model's sizes
-// alone, so that a session's sums are added in one order whatever the step looks like.
+// One state per thread while that is what it takes to fill the device, two above.
+inline bool scan_few(uint32_t inner, uint32_t state) { return (uint64_t)inner * state < 131072; }
+
+// The line to pieces: where what four states per thread save outweighs the second pass over the decays: where the whole chain has
+// one state per thread, from four pieces on.  A prompt through four layers, us whole / in pieces:
+//     2048 channels of 16   640 tokens 660 / 695    769  775 / 753    1024  929 / 765    2048 1669 / 1025
+//     4096 channels of 16   640 tokens 947 / 1003   769 1020 / 993    1024 1189 / 1043   2048 2082 / 1613
+//     8192 channels of 8                            769 1839 / 1645   1024 2052 / 1697   2048 3709 / 2811
+// and with two states per thread  8192 channels of 16  1300 tokens 2462 / 2444  2048 3285 / 3209;  of 32  1281 2638 / 2920  2048 3585 / 3933.
+// A portion's states are therefore summed in one order or another by its length (not by what else is in the step or in memory: the model
+// takes the workspace when it is created): portions of other lengths agree to rounding.  Error of a layer of 512 channels against
+// float64, 2000 tokens at once / as four portions of one chain each: 8.5e-7 / 1.0e-6 in F32, the same in BF16.
+inline bool scan_in_pieces(uint32_t rows, uint32_t inner, uint32_t state)
+{
+    return state > 4 && state <= 32 && scan_few(inner, state) && rows > 3 * kScanPiece;
+}
+
 template <typename T, typename TO> int scan_launch(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a)
 {
-    // The line to pieces: from three of them on the second pass over the decays is less than what four states per thread save
-    // (and the last sum of a session's state is formed piece by piece, whatever else is in the step).
-    if (!rw.decode && rw.n_seq == 1 && rw.n_rows > 2 * kScanPiece && a.state > 4 && a.state <= 32) {
+    if (!rw.decode && rw.n_seq == 1 && scan_in_pieces(rw.n_rows, a.inner, a.state)) {
         const int rc = a.state <= 8    ? scan_pieces<T, TO, 1>(ctx, rw, a)
                        : a.state <= 16 ? scan_pieces<T, TO, 2>(ctx, rw, a)
                                        : scan_pieces<T, TO, 3>(ctx, rw, a);
         if (rc != WR_CUDA_ERR_NOMEM) return rc;
     }
-    const bool few = (uint64_t)a.inner * a.state < 131072;
+    const bool few = scan_few(a.inner, a.state);
     if (a.state <= 1) return scan_one<T, TO, 1, 0>(ctx, rw, a);
     if (a.state <= 2) return scan_one<T, TO, 1, 1>(ctx, rw, a);
     if (a.state <= 4) return scan_one<T, TO, 1, 2>(ctx, rw, a);
@@ -1169,6 +1185,13 @@ int wr_conv_silu_launch(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_conv_args 
 {
     WR_CUDA_TRY(a.type == WR_ACT_BF16 ? conv_launch<__nv_bfloat16>(ctx, rw, a) : conv_launch<float>(ctx, rw, a));
     return finish_launch(ctx);
+}
+
+size_t wr_scan_ws_bytes(uint32_t rows, uint32_t inner, uint32_t state)
+{
+    if (!scan_in_pieces(rows, inner, state)) return 0;
+    const size_t held = state <= 8 ? 8 : state <= 16 ? 16 : 32;
+    return (size_t)((rows + kScanPiece - 1) / kScanPiece - 1) * wr_ld(inner) * (held + 1) * 4;
 }
 
 int wr_scan_launch(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a)

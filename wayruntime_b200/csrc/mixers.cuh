@@ -72,6 +72,8 @@ struct wr_scan_args {
     void *out; int out_type;         // [rows][wr_ld(inner)]
 };
 int wr_scan_launch(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a);
+// Workspace of a portion that is scanned in pieces (0: of one that is not); without it the portion is scanned as a whole.
+size_t wr_scan_ws_bytes(uint32_t rows, uint32_t inner, uint32_t state);
 
 struct wr_attn_geom {
     uint32_t n_q, n_kv, maps, kd, vd;    // query heads, kv heads, maps per head, query/key size per map, value size

@@ -724,6 +724,9 @@ extern "C" int wr_cuda_model_create_mixed(wr_cuda_ctx *ctx, const wr_cuda_mixed_
         if (rc == WR_CUDA_OK) rc = fix_mat(l.down, *x, x->mid, rows, wr_ld(l.down.k));
     }
     if (rc != WR_CUDA_OK) return fail(rc);
+    // now, so that which form a scan takes does not hang on the memory there is later
+    for (const Layer &l : x->layers)
+        if (l.mixer == WR_CUDA_MIXER_MAMBA1) (void)wr_ctx_try_ws(ctx, wr_scan_ws_bytes(m->max_rows, l.inner, l.state));
     *out = m;
     return WR_CUDA_OK;
 }
