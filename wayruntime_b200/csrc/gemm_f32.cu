@@ -81,7 +81,7 @@ __device__ __forceinline__ void put16(const GemmParams &p, const float (&y)[16],
 }
 
 // The same where a power of two is not a normal F32 number, or an infinity or a NaN is among the factors.  The latter is what
-// plain F32 arithmetic makes of it (kNotFinite is no exponent's size, and no two exponents' sum).
+// plain F32 arithmetic makes of it.
 __device__ __noinline__ void put16_rare(const GemmParams &p, const float *raw, const wr_split_scale rs, uint32_t part, uint32_t row,
                                         uint32_t n_at, uint32_t k_lo, uint32_t k_hi)
 {
@@ -95,10 +95,20 @@ __device__ __noinline__ void put16_rare(const GemmParams &p, const float *raw, c
         if (e < kNotFinite / 2) {
             const int first = min(max(e, -126), 127);
             y[i] = raw[i] * pow2(first) * pow2(min(max(e - first, -126), 127));
-        } else {
-            const float *w = wr_split_row(a.source, n_at + i), *x = a.x + (size_t)row * a.x_stride;
-            for (uint32_t k = k_lo; k < min(k_hi, a.source.to.k); ++k)
-                y[i] = fmaf(a.norm_w ? __fmul_rn(x[k], a.norm_w[k]) : x[k], w ? w[k] : 0.f, y[i]);
+        } else if (e >= kNotNumbers / 2 + kNotFinite) {
+            y[i] = __int_as_float(0x7fffffff);
+        } else if (const float *w = wr_split_row(a.source, n_at + i)) {
+            const float *x = a.x + (size_t)row * a.x_stride;
+#pragma unroll 4
+            for (uint32_t k = k_lo; k < min(k_hi, a.source.to.k); k += 4) {           // (K is a multiple of 4)
+                float4 v = *reinterpret_cast<const float4 *>(x + k);
+                const float4 u = *reinterpret_cast<const float4 *>(w + k);
+                if (a.norm_w) {
+                    const float4 nw = *reinterpret_cast<const float4 *>(a.norm_w + k);
+                    v = make_float4(__fmul_rn(v.x, nw.x), __fmul_rn(v.y, nw.y), __fmul_rn(v.z, nw.z), __fmul_rn(v.w, nw.w));
+                }
+                y[i] = fmaf(v.w, u.w, fmaf(v.z, u.z, fmaf(v.y, u.y, fmaf(v.x, u.x, y[i]))));
+            }
         }
         y[i] = __fmul_rn(y[i], rs.factor);
     }
@@ -286,7 +296,7 @@ __device__ __forceinline__ int scale_exponent(uint32_t max_bits)
 // The exponent that undoes it; infinities and NaNs are marked.
 __device__ __forceinline__ int undo_exponent(uint32_t max_bits)
 {
-    return max_bits >= 0x7f800000u ? kNotFinite : max_bits == 0 ? 0 : -scale_exponent(max_bits);
+    return max_bits > 0x7f800000u ? kNotNumbers : max_bits == 0x7f800000u ? kNotFinite : max_bits == 0 ? 0 : -scale_exponent(max_bits);
 }
 struct Scale {
     float a, b;                                           // two factors: together up to 2^156

@@ -15,10 +15,12 @@
 // Weights: digits 0 and 1 in wr_weight's blocks of 128-byte rows (gemm_bf16.cuh), then digits 2 and 3 likewise.
 struct wr_split_weight {
     char *blocks = nullptr;
-    int *exponent = nullptr;             // [n]: of the power of two that undoes the row's scale and the digits' unit; or kNotFinite
+    int *exponent = nullptr;             // [n]: of the power of two that undoes the row's scale and the digits' unit; or one of the next two
     uint32_t n = 0, k = 0;
 };
-constexpr int kNotFinite = 1 << 20;      // a row with infinities or NaNs: products are worked out from the F32 rows instead
+// A row with infinities, products with which are worked out from the F32 rows; a row with NaNs, products with which are NaN.  (No sum of
+// two exponents comes near either, nor two of the first to the second.)
+constexpr int kNotFinite = 1 << 20, kNotNumbers = 1 << 22;
 size_t wr_split_weight_bytes(uint32_t n, uint32_t k);
 // byte offset of a row's digit 0 or 1 (digits 2 and 3: half the bytes on) of value i
 __host__ __device__ inline size_t wr_split_off(uint32_t k, uint32_t row, uint32_t digit, uint32_t i)
@@ -55,7 +57,7 @@ int wr_split_weights_launch(wr_cuda_ctx *ctx, const wr_split_source *list, uint3
 inline uint32_t wr_split_ld(uint32_t k) { return (k + kWBlock - 1) / kWBlock * kWBlock; }
 struct wr_split_scale {
     float factor;                        // what a product of the row is multiplied by last (1 / rms)
-    int exponent;                        // of the power of two that undoes the row's scale, or kNotFinite
+    int exponent;                        // of the power of two that undoes the row's scale, or as for weights
 };
 struct wr_split_rows_args {
     float *x;                            // [rows][x_stride]; gets the partial sums added when there are any
