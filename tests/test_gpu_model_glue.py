@@ -10,7 +10,7 @@ on its own, in float64 numpy, using the attention rows the call itself reports
     logits     = normed_out @ lm_head^T,  argmax = first maximum
 and the K rows that reach the cache are RMSNorm(embed) @ wk^T with QK-norm and
 RoPE (the reference's rotation, through the CPU restatement).  Row-count
-independence — a row's bits do not depend on how many rows share the call — is
+independence — a decode row's bits do not depend on how many rows share the call — is
 what keeps a batched step byte-equal to serial ones (src/core/batch.c).
 """
 import numpy as np
@@ -122,8 +122,8 @@ def test_a_rows_bits_do_not_depend_on_the_batch():
 
 
 def test_prefill_rows_match_token_by_token_decode():
-    """40 prompt rows in one pass (three row groups of the GEMV, the tensor-core
-    prefill kernel) against the same tokens fed one at a time (decode kernel)."""
+    """40 prompt rows in one pass (the tensor-core products and prefill
+    kernel) against the same tokens fed one at a time (GEMV, decode kernel)."""
     import wayruntime_b200 as wr
     ctx = wr.Context(0)
     shape = dict(SHAPE, n_layers=2)

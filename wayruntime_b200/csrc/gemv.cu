@@ -37,8 +37,8 @@ __device__ __forceinline__ float4 ldg_stream(const float *p)
 // multiplies x by the norm weight first and the finished sum by
 // 1/sqrt(mean(x^2)+eps) last, the sum of squares following the same quarter /
 // lane / butterfly order.  Because all kernels compute every output by exactly
-// this recipe, a row's bits do not depend on how many rows share the call or on
-// which kernel served it.
+// this recipe, a row's bits do not depend on how many rows share the call (up to
+// sixteen: more take gemm_f32.cu's arithmetic) or on which kernel served it.
 //
 //   gemv_splitk_kernel (<= 4 activation rows): a CTA owns C weight rows and
 //     its four warps take one quarter each, so every lane has all its loads in
