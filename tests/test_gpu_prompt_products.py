@@ -206,7 +206,7 @@ def _run_in_portions(dm, kv, tokens, portion):
 
 def test_weights_are_split_for_each_call_in_models_too_large_to_keep_them():
     """Split weights are kept when they take a sixteenth of the device's memory or less; here they would take more, and the
-    layers (all of the same weights) use one layer's memory in turn."""
+    layers use one layer's memory in turn."""
     import torch
     import wayruntime_b200 as wr
     limit = torch.cuda.mem_get_info()[1] // 16
@@ -219,6 +219,9 @@ def test_weights_are_split_for_each_call_in_models_too_large_to_keep_them():
     w["lm_head"] = w["embed"]
     for i in range(shape["n_layers"]):
         w.update({f"l{i}.{n}": a for n, a in big.items()})
+        w[f"l{i}.wv"], w[f"l{i}.wo"] = big["wv"] * np.float32(2.0 ** (i % 3)), big["wo"] * np.float32(3.0 ** -(i % 3))
+        if i % 2:
+            w[f"l{i}.w_gate"], w[f"l{i}.w_up"] = big["w_up"], big["w_gate"]
         w.update({f"l{i}.{n}": np.ones(8192, np.float32) for n in ("attn_norm", "ffn_norm")})
     ctx = wr.Context(0)
     dm = _model(ctx, w, shape, max_rows=64)

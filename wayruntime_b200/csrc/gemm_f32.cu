@@ -254,7 +254,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
                 bool odd = false;
 #pragma unroll
                 for (uint32_t i = 0; i < 16; i += 4) {
-                    const int4 we = __ldg(reinterpret_cast<const int4 *>(w.exponent + n0 + c + i));
+                    const int4 we = *reinterpret_cast<const int4 *>(w.exponent + n0 + c + i);      // (written while this kernel may be waiting)
                     const int es[4] = {we.x, we.y, we.z, we.w};
 #pragma unroll
                     for (uint32_t j = i; j < i + 4; ++j) {
