@@ -230,12 +230,12 @@ int wr_ctx_reserve_ws(wr_cuda_ctx *ctx, size_t ws_bytes, size_t tickets)
 int wr_ctx_try_ws(wr_cuda_ctx *ctx, size_t ws_bytes)
 {
     if (ws_bytes <= ctx->ws_bytes) return WR_CUDA_OK;
-    if (ws_bytes >= ctx->ws_refused) return WR_CUDA_ERR_NOMEM;
     const size_t want = std::max(ws_bytes, (size_t)8 << 20);
+    size_t free_bytes = 0, total_bytes = 0;
     float *ws = nullptr;
-    if (cudaMalloc((void **)&ws, want) != cudaSuccess) {
+    if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess || free_bytes < want ||
+        cudaMalloc((void **)&ws, want) != cudaSuccess) {
         (void)cudaGetLastError();
-        ctx->ws_refused = ws_bytes;
         return WR_CUDA_ERR_NOMEM;
     }
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {

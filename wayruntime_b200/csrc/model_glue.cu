@@ -459,7 +459,6 @@ extern "C" void wr_cuda_model_destroy(wr_cuda_model *m)
         if (m->mixed) wr_mixed_destroy(m->mixed);
         cudaFree(m->slab);
         cudaFree(m->prompt);
-        m->ctx->ws_refused = ~(size_t)0;
         drop_side(m);
         cudaFreeHost(m->h_tokens);
     }

@@ -99,7 +99,6 @@ struct wr_cuda_ctx {
     // split-KV scratch: per-chunk partial triples and per-group arrival tickets
     float *ws = nullptr;
     size_t ws_bytes = 0;
-    size_t ws_refused = ~(size_t)0;  // wr_ctx_try_ws
     int *tickets = nullptr;
     size_t ticket_count = 0;
     int *prefill_sched = nullptr;    // prefill kernel: next work tile, CTAs that have left
@@ -216,8 +215,7 @@ int wr_ctx_reserve_stage(wr_cuda_ctx *ctx, size_t dev_bytes, size_t host_bytes);
 // call that synchronises ends with this.  Caller holds ctx->lock.
 int wr_ctx_sync_checked(wr_cuda_ctx *ctx);
 int wr_ctx_reserve_ws(wr_cuda_ctx *ctx, size_t ws_bytes, size_t tickets);
-// The workspace for callers that can do without: it stays as it is where memory does not suffice, and what was refused once is
-// not asked for again until a model has given memory back.
+// The workspace for callers that can do without: where memory does not suffice it stays as it is, and nothing waits.
 int wr_ctx_try_ws(wr_cuda_ctx *ctx, size_t ws_bytes);
 int wr_kv_batch_check(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer);
 int wr_append_validate(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer,
