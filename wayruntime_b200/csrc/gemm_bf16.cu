@@ -1,13 +1,16 @@
 // gemm_bf16.cu — out[m][n] = act(x . w^T + bias) + add on the 5th-generation tensor cores.
 //
-// Persistent CTAs (one per SM) walk output tiles of 128 rows x BN columns, m fastest so that the
-// tiles in flight share weight rows in L2.  Warp 0 feeds a ring of shared-memory stages with TMA
-// (64 K-values of both operands per stage: activations through a tensor map, weights as linear copies
-// of blocks stored in the operand's layout; what lies beyond K arrives as zeros), warp 1 issues tcgen05.mma into one of two TMEM accumulators, warps 2-5 read the other one
-// back and write the finished rows (bias, softplus, residual; F32, BF16 or saturated F16), so that a
-// tile's output overlaps the next tile's products.  Columns may be gate / up pairs, of which the activation leaves
-// (wr_pair_args), row tiles may have weights of their own (wr_group_args), and activations may come from a cache's pages.  Every wait is bounded by the context's wait
-// limit; a warp that gives up records an error word and all of them leave.
+// Persistent workers walk output tiles, m fastest so that the tiles in flight share weight rows in L2.  A worker is a
+// pair of CTAs (cta_group::2, tiles of 256 rows: each rank holds its 128 rows of activations and half of the tile's
+// weight rows) or one CTA (tiles of 128 rows: few rows, or row tiles with weights of their own).  Warp 0 feeds a ring of
+// shared-memory stages with TMA (64 K-values of both operands per stage: activations through a tensor map, weights as
+// linear copies out of blocks stored in the operand's layout; what lies beyond K arrives as zeros), warp 1 issues
+// tcgen05.mma into one of two TMEM accumulators (in a pair the even rank's; the odd rank's tells it of stages that have
+// arrived there), warps 2-9 read the other one back and write the finished rows (bias, softplus, residual; F32, BF16 or
+// saturated F16), so that a tile's output overlaps the next tile's products.  Columns may be gate / up pairs, of which the
+// activation leaves (wr_pair_args), row tiles may have weights of their own (wr_group_args), and activations may come from
+// a cache's pages.  Every wait is bounded by the context's wait limit; a warp that gives up records an error word and all
+// of them leave.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -17,22 +20,21 @@
 
 namespace {
 
-constexpr uint32_t kBM = 128, kBK = 64;
-constexpr uint32_t kThreads = 192;
-constexpr uint32_t kABytes = kBM * kBK * 2;
-constexpr uint32_t kStageBudget = 196608;
-
-template <uint32_t BN> struct Tile {
-    static constexpr uint32_t kBBytes = BN * kBK * 2;
-    static constexpr uint32_t kStages = kStageBudget / (kABytes + kBBytes);
-    static constexpr uint32_t kSmem = kStages * (kABytes + kBBytes) + 1024;
-    static constexpr uint32_t kTmemCols = 2 * BN;        // two accumulators
-};
+constexpr uint32_t kBM = 128, kBK = 64;                  // rows of one CTA, K-values of a stage
+constexpr uint32_t kMaxN = 256;                          // columns of a tile, and of one accumulator of two
+constexpr uint32_t kMapRows = 32;                        // a pair's rank takes a multiple of these of a tile's weight rows
+constexpr uint32_t kOutWarps = 8, kThreads = 64 + 32 * kOutWarps;
+constexpr uint32_t kABytes = kBM * kBK * 2, kRowBytes = kBK * 2;
+constexpr uint32_t kMaxStages = 8, kStageBudget = 196608;
+constexpr uint32_t kOutBytes = 4096;                     // a warp's 32 x 32 results on their way out
+constexpr uint32_t kSmem = kStageBudget + kOutWarps * kOutBytes + 1024;
 
 struct GemmParams {
     wr_gemm_args a;
     wr_weight w;
     uint32_t m_tiles, n_tiles, k_blocks;
+    uint32_t wide, bn0, bn1;                             // the first `wide` column tiles have bn0 columns, the others bn1
+    uint32_t stages, stage_bytes;
     long long wait_limit;
     int *err;
 };
@@ -50,31 +52,159 @@ __device__ __forceinline__ uint32_t pack_f16(float a, float b)
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-template <uint32_t BN>
-__global__ void __launch_bounds__(kThreads, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
+struct TileAt {
+    uint32_t strip, n0, bn;
+    bool wide;
+};
+__device__ __forceinline__ TileAt tile_at(const GemmParams &p, uint32_t m_tiles, uint32_t tile)
 {
-    using T = Tile<BN>;
+    const uint32_t j = tile / m_tiles;
+    const bool wide = j < p.wide;
+    return {tile - j * m_tiles, wide ? j * p.bn0 : p.wide * p.bn0 + (j - p.wide) * p.bn1, wide ? p.bn0 : p.bn1, wide};
+}
+
+// Residual i of a 32 x 32 piece as finish() adds it: lane l has columns 4 (l % 8) .. + 3 of rows l / 8, l / 8 + 4, ...
+__device__ __forceinline__ void fetch_add(const GemmParams &p, uint32_t row0, uint32_t col0, uint32_t lane, uint32_t i, float4 &r)
+{
+    const uint32_t col = col0 + 4 * (lane & 7u), row = row0 + (lane >> 3) + 4 * i;
+    if (p.a.add && col < ((p.w.n + 7u) & ~7u) && (col & ~15u) < p.a.pair.from && row < p.a.m)
+        r = *reinterpret_cast<const float4 *>(p.a.add + (size_t)row * p.a.add_ld + col);
+}
+
+// four gate values of a row and the up values that belong to them
+__device__ __forceinline__ void put_pair(const GemmParams &p, uint32_t row, uint32_t at, const float4 &g, const float4 &u)
+{
+    const float y0 = wr_pair_act(p.a.pair.act, p.a.pair.alpha, p.a.pair.limit, g.x, u.x);
+    const float y1 = wr_pair_act(p.a.pair.act, p.a.pair.alpha, p.a.pair.limit, g.y, u.y);
+    const float y2 = wr_pair_act(p.a.pair.act, p.a.pair.alpha, p.a.pair.limit, g.z, u.z);
+    const float y3 = wr_pair_act(p.a.pair.act, p.a.pair.alpha, p.a.pair.limit, g.w, u.w);
+    *reinterpret_cast<uint2 *>((__nv_bfloat16 *)p.a.pair.out + (size_t)row * p.a.pair.ld + at) =
+        make_uint2(pack_bf16(y0, y1), pack_bf16(y2, y3));
+}
+
+// A 32 x 32 piece of finished sums, a row to a lane as the tensor core leaves them, on through shared memory: eight lanes
+// write (and read the residual of) 128 bytes of one row instead of each lane sixteen bytes of a row of its own.
+__device__ __forceinline__ void lay_out(uint8_t *buf, const float (&v)[32], uint32_t lane)
+{
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c)
+        *reinterpret_cast<float4 *>(buf + lane * 128u + ((c ^ (lane & 7u)) << 4)) =
+            make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+    __syncwarp();
+}
+// where lane l finds its four columns of row l / 8 + 4 i
+__device__ __forceinline__ uint8_t *piece(uint8_t *buf, uint32_t lane, uint32_t i)
+{
+    const uint32_t rr = (lane >> 3) + 4 * i;
+    return buf + rr * 128u + (((lane & 7u) ^ (rr & 7u)) << 4);
+}
+
+// The piece's plain columns.  A worker's last tile runs this alone, with two warps to a scheduler: reads, sums and writes
+// of all rows go together, without a branch between them.
+template <uint32_t TYPE>
+__device__ __forceinline__ void finish(const GemmParams &p, uint8_t *buf, uint32_t row0, uint32_t col0, uint32_t lane,
+                                       const float4 &bias, float4 (&r)[8], bool more, uint32_t next_col)
+{
+    const uint32_t col = col0 + 4 * (lane & 7u), row1 = row0 + (lane >> 3);
+    const bool mine = col < ((p.w.n + 7u) & ~7u) && (col & ~15u) < p.a.pair.from;
+    const uint32_t rows = mine && row1 < p.a.m ? (p.a.m - row1 + 3) / 4 : 0u;           // rows i < rows are there
+    float4 u[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) u[i] = *reinterpret_cast<const float4 *>(piece(buf, lane, i));
+    const bool add = p.a.add != nullptr;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        u[i].x = (u[i].x + bias.x) * p.a.mul; u[i].y = (u[i].y + bias.y) * p.a.mul;
+        u[i].z = (u[i].z + bias.z) * p.a.mul; u[i].w = (u[i].w + bias.w) * p.a.mul;
+        u[i].x = add ? u[i].x + r[i].x : u[i].x; u[i].y = add ? u[i].y + r[i].y : u[i].y;
+        u[i].z = add ? u[i].z + r[i].z : u[i].z; u[i].w = add ? u[i].w + r[i].w : u[i].w;
+    }
+    const size_t at = (size_t)row1 * p.a.out_ld + col, step = (size_t)4 * p.a.out_ld;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        if (TYPE == WR_GEMM_OUT_F32) {
+            if (i < rows) *reinterpret_cast<float4 *>((float *)p.a.out + at + i * step) = u[i];
+        } else {
+            const uint2 h = TYPE == WR_GEMM_OUT_BF16 ? make_uint2(pack_bf16(u[i].x, u[i].y), pack_bf16(u[i].z, u[i].w))
+                                                     : make_uint2(pack_f16(u[i].x, u[i].y), pack_f16(u[i].z, u[i].w));
+            if (i < rows) *reinterpret_cast<uint2 *>((uint16_t *)p.a.out + at + i * step) = h;
+        }
+    }
+    if (add && more) {                                   // the residual of this warp's next piece
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) fetch_add(p, row0, next_col, lane, i, r[i]);
+    }
+}
+
+// What a piece may need besides, a row at a time: gate / up pairs, softplus (in place), the BF16 copy.
+__device__ __forceinline__ void finish_pairs(const GemmParams &p, uint8_t *buf, uint32_t row0, uint32_t col0, uint32_t lane)
+{
+    const uint32_t c = lane & 7u, col = col0 + 4 * c, group = col & ~15u;
+    const bool gate = group >= p.a.pair.from && col < ((p.w.n + 7u) & ~7u) && !(c & 2u);
+#pragma unroll 2
+    for (uint32_t i = 0; i < 8; ++i) {
+        const uint32_t row = row0 + (lane >> 3) + 4 * i;
+        const float4 g = *reinterpret_cast<const float4 *>(piece(buf, lane, i));
+        const float4 up = *reinterpret_cast<const float4 *>(piece(buf, lane ^ 2u, i));   // two lanes on
+        if (gate && row < p.a.m) put_pair(p, row, (group - p.a.pair.from) / 2 + 4 * (c & 1u), g, up);
+    }
+}
+__device__ __forceinline__ void finish_softplus(uint8_t *buf, uint32_t lane, float4 &bias)
+{
+#pragma unroll 1
+    for (uint32_t i = 0; i < 8; ++i) {
+        float4 *u = reinterpret_cast<float4 *>(piece(buf, lane, i));
+        *u = make_float4(softplus(u->x + bias.x), softplus(u->y + bias.y), softplus(u->z + bias.z), softplus(u->w + bias.w));
+    }
+    bias = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ void finish_copy(const GemmParams &p, uint8_t *buf, uint32_t row0, uint32_t col0, uint32_t lane, const float4 &bias)
+{
+    const uint32_t col = col0 + 4 * (lane & 7u);
+    const bool mine = col < ((p.w.n + 7u) & ~7u) && (col & ~15u) < p.a.pair.from;
+#pragma unroll 2
+    for (uint32_t i = 0; i < 8; ++i) {
+        const uint32_t row = row0 + (lane >> 3) + 4 * i;
+        const float4 u = *reinterpret_cast<const float4 *>(piece(buf, lane, i));
+        if (mine && row < p.a.m)
+            *reinterpret_cast<uint2 *>((__nv_bfloat16 *)p.a.out_bf16 + (size_t)row * p.a.out_bf16_ld + col) =
+                make_uint2(pack_bf16(u.x + bias.x, u.y + bias.y), pack_bf16(u.z + bias.z, u.w + bias.w));
+    }
+}
+
+template <bool PAIR>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w0_map,
+                 const __grid_constant__ CUtensorMap w1_map, const GemmParams p)
+{
+    constexpr uint32_t kRanks = PAIR ? 2 : 1;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full[T::kStages], empty[T::kStages], acc_full[2], acc_empty[2];
+    // (a pair's full and acc_empty: those of the even rank)
+    __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     uint8_t *stages = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023u) & ~(uintptr_t)1023u);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = PAIR ? tc5::cluster_rank() : 0u;
+    const uint32_t worker = blockIdx.x / kRanks, workers = gridDim.x / kRanks;
     pdl_trigger();
     if (threadIdx.x == 0) {
-        for (uint32_t i = 0; i < T::kStages; ++i) {
+        for (uint32_t i = 0; i < p.stages; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], 4);
+            mbar_init(&acc_empty[i], kRanks * kOutWarps);
         }
         fence_barrier_init();
     }
-    if (warp == 1) tc5::alloc(&tmem_slot, T::kTmemCols);
+    if (warp == 1) {
+        if (PAIR) tc5::alloc2(&tmem_slot, 2 * kMaxN);
+        else tc5::alloc(&tmem_slot, 2 * kMaxN);
+    }
     tc5::fence_before();
-    __syncthreads();
+    if (PAIR) tc5::cluster_sync();                       // (the other rank's barriers too)
+    else __syncthreads();
     tc5::fence_after();
     const uint32_t tmem = tmem_slot;
     pdl_wait();
@@ -82,159 +212,153 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const GemmParams p)
 
     if (warp == 0) {
         if (lane == 0) {
-            uint32_t it = 0;
+            const uint32_t w_rows = wr_weight_blocks(p.w.n) * kWBlock;
+            uint32_t it = 0, st = 0, phase = 0;          // stage it % stages, round it / stages
             bool ok = true;
-            for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-                const uint32_t m0 = (tile % m_tiles) * kBM, n0 = (tile / m_tiles) * BN;
+            for (uint32_t tile = worker; tile < tiles && ok; tile += workers) {
+                const TileAt t = tile_at(p, m_tiles, tile);
+                const uint32_t m0 = (t.strip * kRanks + rank) * kBM;
+                const uint32_t share = t.bn / kRanks, r0 = t.n0 + rank * share;     // this rank's weight rows
+                const uint32_t rows = r0 < w_rows ? min(share, w_rows - r0) : 0u;
                 const char *blocks = static_cast<const char *>(p.w.blocks);
-                if (p.a.group.list) blocks += p.a.group.list[tile % m_tiles] * p.a.group.stride;
-                for (uint32_t kb = 0; kb < p.k_blocks; ++kb, ++it) {
-                    const uint32_t st = it % T::kStages;
-                    if (it >= T::kStages && !mbar_wait(&empty[st], (it / T::kStages - 1) & 1, p.wait_limit)) {
+                if (p.a.group.list) blocks += p.a.group.list[t.strip] * p.a.group.stride;
+                const uint32_t np = !p.a.pages || m0 >= p.a.m ? 0u : m0 + kPageTokens < p.a.m ? 2u : 1u;
+                // (a pair's boxes count whole; what they bring from beyond the weight's rows belongs to no column)
+                const uint32_t bytes = PAIR ? 2 * kABytes + t.bn * kRowBytes : (p.a.pages ? np * (kABytes / 2) : kABytes) + rows * kRowBytes;
+                const CUtensorMap *w_map = t.wide ? &w0_map : &w1_map;
+                for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                    if (it >= p.stages && !mbar_wait(&empty[st], phase ^ 1u, p.wait_limit)) {
                         ok = false;
                         break;
                     }
-                    uint8_t *a = stages + st * (kABytes + T::kBBytes), *b = a + kABytes;
-                    const uint32_t nb0 = n0 / kWBlock, nb = min(BN / kWBlock, wr_weight_blocks(p.w.n) - nb0);
-                    if (p.a.pages) {
-                        const uint32_t np = m0 + kPageTokens < p.a.m ? 2u : 1u;
-                        mbar_expect_tx(&full[st], np * kABytes / 2 + nb * kWBlockBytes);
-                        for (uint32_t i = 0; i < np; ++i)
-                            bulk_g2s(a + i * kABytes / 2, reinterpret_cast<const char *>(p.a.pages[m0 / kPageTokens + i]) + kb * kABytes / 2,
-                                     kABytes / 2, &full[st]);
+                    uint8_t *a = stages + st * p.stage_bytes, *b = a + kABytes;
+                    if (rank == 0) mbar_expect_tx(&full[st], bytes);
+                    if (PAIR) {
+                        tc5::tma_load_2d_pair(a, &x_map, (int)(kb * kBK), (int)m0, &full[st]);
+                        tc5::tma_load_2d_pair(b, w_map, 0, (int)(kb * w_rows + r0), &full[st]);
                     } else {
-                        mbar_expect_tx(&full[st], kABytes + nb * kWBlockBytes);
-                        tc5::tma_load_2d(a, &x_map, (int)(kb * kBK), (int)m0, &full[st]);
+                        if (p.a.pages) {
+                            for (uint32_t i = 0; i < np; ++i)
+                                bulk_g2s(a + i * kABytes / 2,
+                                         reinterpret_cast<const char *>(p.a.pages[m0 / kPageTokens + i]) + kb * kABytes / 2, kABytes / 2,
+                                         &full[st]);
+                        } else {
+                            tc5::tma_load_2d(a, &x_map, (int)(kb * kBK), (int)m0, &full[st]);
+                        }
+                        if (rows) bulk_g2s(b, blocks + wr_weight_row(p.w.n, r0, kb), rows * kRowBytes, &full[st]);
                     }
-                    const char *w = blocks + ((size_t)nb0 * p.k_blocks + kb) * kWBlockBytes;
-                    for (uint32_t i = 0; i < nb; ++i)
-                        bulk_g2s(b + i * kWBlockBytes, w + (size_t)i * p.k_blocks * kWBlockBytes, kWBlockBytes, &full[st]);
+                    ++it;
+                    if (++st == p.stages) {
+                        st = 0;
+                        phase ^= 1;
+                    }
                 }
             }
             if (!ok) atomicCAS(p.err, 0, 41);
             // nothing of this CTA's may be in flight when it leaves: the last loads have landed and (unless
-            // a wait ran out) the products that read them have completed
-            const uint32_t last = it < T::kStages ? it : T::kStages;
+            // a wait ran out) the products that read them have completed (a pair's odd rank waits the limit out then)
+            const uint32_t last = it < p.stages ? it : p.stages;
             for (uint32_t i = it - last; i < it; ++i)
-                (void)mbar_wait(ok ? &empty[i % T::kStages] : &full[i % T::kStages], (i / T::kStages) & 1, p.wait_limit);
+                (void)mbar_wait(ok ? &empty[i % p.stages] : &full[i % p.stages], (i / p.stages) & 1, p.wait_limit);
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 && rank == 0) {
         const bool lead = tc5::elect_one();
-        const uint32_t idesc = p.a.pages ? tc5::idesc_f16(kBM, BN) : tc5::idesc_bf16(kBM, BN);
-        uint32_t it = 0, n_tile = 0;
+        uint32_t st = 0, phase = 0, n_tile = 0;
         bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++n_tile) {
+        for (uint32_t tile = worker; tile < tiles && ok; tile += workers, ++n_tile) {
+            const uint32_t bn = tile_at(p, m_tiles, tile).bn;
+            const uint32_t idesc = p.a.pages ? tc5::idesc_f16(kRanks * kBM, bn) : tc5::idesc_bf16(kRanks * kBM, bn);
             const uint32_t acc = n_tile & 1;
             if (n_tile >= 2 && !mbar_wait(&acc_empty[acc], (n_tile / 2 - 1) & 1, p.wait_limit)) {
                 ok = false;
                 break;
             }
             tc5::fence_after();
-            for (uint32_t kb = 0; kb < p.k_blocks; ++kb, ++it) {
-                const uint32_t st = it % T::kStages;
-                if (!mbar_wait(&full[st], (it / T::kStages) & 1, p.wait_limit)) {
+            for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                if (!mbar_wait(&full[st], phase, p.wait_limit)) {
                     ok = false;
                     break;
                 }
                 tc5::fence_after();
-                const uint32_t a_addr = smem_u32(stages + st * (kABytes + T::kBBytes));
+                const uint32_t a_addr = smem_u32(stages + st * p.stage_bytes);
                 const uint64_t a = tc5::desc_kmajor(a_addr), b = tc5::desc_kmajor(a_addr + kABytes);
 #pragma unroll
                 for (uint32_t kk = 0; kk < kBK / 16; ++kk)
-                    if (lead) tc5::mma_ss(tmem + acc * BN, a + 2 * kk, b + 2 * kk, idesc, (kb | kk) != 0);
-                if (lead) tc5::commit(&empty[st]);
+                    if (lead) {
+                        if (PAIR) tc5::mma2_ss(tmem + acc * kMaxN, a + 2 * kk, b + 2 * kk, idesc, (kb | kk) != 0);
+                        else tc5::mma_ss(tmem + acc * kMaxN, a + 2 * kk, b + 2 * kk, idesc, (kb | kk) != 0);
+                    }
+                if (lead) {
+                    if (PAIR) tc5::commit2(&empty[st]);
+                    else tc5::commit(&empty[st]);
+                }
+                if (++st == p.stages) {
+                    st = 0;
+                    phase ^= 1;
+                }
             }
-            if (ok && lead) tc5::commit(&acc_full[acc]);
+            if (ok && lead) {
+                if (PAIR) tc5::commit2(&acc_full[acc]);
+                else tc5::commit(&acc_full[acc]);
+            }
         }
         if (!ok && lane == 0) atomicCAS(p.err, 0, 42);
-    } else {
-        const uint32_t quarter = warp & 3;                       // TMEM lanes this warp may read
+    } else if (warp >= 2) {
+        const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;       // TMEM lanes this warp may read; its pieces of 32 columns
+        uint8_t *buf = stages + kStageBudget + (warp - 2) * kOutBytes;
         uint32_t n_tile = 0;
         bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++n_tile) {
-            const uint32_t m0 = (tile % m_tiles) * kBM, n0 = (tile / m_tiles) * BN;
-            const uint32_t acc = n_tile & 1, row = m0 + quarter * 32 + lane;
+        for (uint32_t tile = worker; tile < tiles && ok; tile += workers, ++n_tile) {
+            const TileAt t = tile_at(p, m_tiles, tile);
+            const uint32_t row0 = (t.strip * kRanks + rank) * kBM + quarter * 32, acc = n_tile & 1;
+            const uint32_t end = min(t.bn, p.w.n > t.n0 ? p.w.n - t.n0 : 0u);
+            float4 r[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) fetch_add(p, row0, t.n0 + half * 32, lane, i, r[i]);
             if (!mbar_wait(&acc_full[acc], (n_tile / 2) & 1, p.wait_limit)) {
                 ok = false;
                 break;
             }
+            __syncwarp();
             tc5::fence_after();
-            const uint32_t n_pad = (p.w.n + 7u) & ~7u;
 #pragma unroll 1
-            for (uint32_t c0 = 0; c0 < BN && n0 + c0 < n_pad; c0 += 32) {
+            for (uint32_t c0 = half * 32; c0 < end; c0 += 64) {
                 float v[32];
-                tc5::ld32(tmem + ((quarter * 32) << 16) + acc * BN + c0, v);
+                tc5::ld32(tmem + ((quarter * 32) << 16) + acc * kMaxN + c0, v);
                 tc5::wait_ld();
-                if (row < p.a.m) {
-#pragma unroll
-                    for (uint32_t g = 0; g < 4; ++g) {
-                        const uint32_t col = n0 + c0 + 8 * g;
-                        if (col >= p.a.pair.from) {
-                            if ((g & 1u) || col >= n_pad) continue;
-                            float y[8];
-#pragma unroll
-                            for (int e = 0; e < 8; ++e)
-                                y[e] = wr_pair_act(p.a.pair.act, p.a.pair.alpha, p.a.pair.limit, v[8 * g + e],
-                                                   v[8 * ((g + 1) & 3u) + e]);
-                            *reinterpret_cast<uint4 *>((__nv_bfloat16 *)p.a.pair.out + (size_t)row * p.a.pair.ld +
-                                                       (col - p.a.pair.from) / 2) =
-                                make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]),
-                                           pack_bf16(y[6], y[7]));
-                        } else if (col < n_pad) {
-                            float *u = v + 8 * g;
-                            if (p.a.bias) {
-                                const float4 b0 = *reinterpret_cast<const float4 *>(p.a.bias + col);
-                                const float4 b1 = *reinterpret_cast<const float4 *>(p.a.bias + col + 4);
-                                u[0] += b0.x; u[1] += b0.y; u[2] += b0.z; u[3] += b0.w;
-                                u[4] += b1.x; u[5] += b1.y; u[6] += b1.z; u[7] += b1.w;
-                            }
-                            if (p.a.act == WR_GEMM_ACT_SOFTPLUS) {
-#pragma unroll
-                                for (int e = 0; e < 8; ++e) u[e] = softplus(u[e]);
-                            }
-                            if (p.a.out_bf16)
-                                *reinterpret_cast<uint4 *>((__nv_bfloat16 *)p.a.out_bf16 + (size_t)row * p.a.out_bf16_ld + col) =
-                                    make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]),
-                                               pack_bf16(u[6], u[7]));
-                            if (p.a.mul != 1.f) {
-#pragma unroll
-                                for (int e = 0; e < 8; ++e) u[e] *= p.a.mul;
-                            }
-                            if (p.a.add) {
-                                const float *r = p.a.add + (size_t)row * p.a.add_ld + col;
-                                const float4 r0 = *reinterpret_cast<const float4 *>(r);
-                                const float4 r1 = *reinterpret_cast<const float4 *>(r + 4);
-                                u[0] += r0.x; u[1] += r0.y; u[2] += r0.z; u[3] += r0.w;
-                                u[4] += r1.x; u[5] += r1.y; u[6] += r1.z; u[7] += r1.w;
-                            }
-                            const size_t at = (size_t)row * p.a.out_ld + col;
-                            if (p.a.out_type == WR_GEMM_OUT_F32) {
-                                float4 *o = reinterpret_cast<float4 *>((float *)p.a.out + at);
-                                o[0] = make_float4(u[0], u[1], u[2], u[3]);
-                                o[1] = make_float4(u[4], u[5], u[6], u[7]);
-                            } else if (p.a.out_type == WR_GEMM_OUT_BF16) {
-                                *reinterpret_cast<uint4 *>((__nv_bfloat16 *)p.a.out + at) =
-                                    make_uint4(pack_bf16(u[0], u[1]), pack_bf16(u[2], u[3]), pack_bf16(u[4], u[5]),
-                                               pack_bf16(u[6], u[7]));
-                            } else {
-                                *reinterpret_cast<uint4 *>((__half *)p.a.out + at) =
-                                    make_uint4(pack_f16(u[0], u[1]), pack_f16(u[2], u[3]), pack_f16(u[4], u[5]),
-                                               pack_f16(u[6], u[7]));
-                            }
-                        }
-                    }
+                lay_out(buf, v, lane);
+                const uint32_t col0 = t.n0 + c0, col = col0 + 4 * (lane & 7u);
+                const bool more = c0 + 64 < end;
+                if (col0 + 16 >= p.a.pair.from) finish_pairs(p, buf, row0, col0, lane);
+                if (col0 < p.a.pair.from) {
+                    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (p.a.bias && col < ((p.w.n + 7u) & ~7u)) bias = *reinterpret_cast<const float4 *>(p.a.bias + col);
+                    if (p.a.act == WR_GEMM_ACT_SOFTPLUS) finish_softplus(buf, lane, bias);
+                    if (p.a.out_bf16) finish_copy(p, buf, row0, col0, lane, bias);
+                    if (p.a.out_type == WR_GEMM_OUT_F32) finish<WR_GEMM_OUT_F32>(p, buf, row0, col0, lane, bias, r, more, col0 + 64);
+                    else if (p.a.out_type == WR_GEMM_OUT_BF16) finish<WR_GEMM_OUT_BF16>(p, buf, row0, col0, lane, bias, r, more, col0 + 64);
+                    else finish<WR_GEMM_OUT_F16>(p, buf, row0, col0, lane, bias, r, more, col0 + 64);
                 }
+                __syncwarp();                            // the next piece takes the buffer
             }
             tc5::fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[acc]);
+            if (lane == 0) {
+                if (PAIR) tc5::arrive_rank(&acc_empty[acc], 0);
+                else mbar_arrive(&acc_empty[acc]);
+            }
         }
         if (!ok && lane == 0) atomicCAS(p.err, 0, 43);
     }
+    __syncwarp();
     tc5::fence_before();
-    __syncthreads();
+    if (PAIR) tc5::cluster_sync();                       // nobody leaves while its barriers or operands are still used
+    else __syncthreads();
     tc5::fence_after();
-    if (warp == 1) tc5::dealloc(tmem, T::kTmemCols);
+    if (warp == 1) {
+        if (PAIR) tc5::dealloc2(tmem, 2 * kMaxN);
+        else tc5::dealloc(tmem, 2 * kMaxN);
+    }
 }
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -242,7 +366,8 @@ typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32
                                     CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                                     CUtensorMapFloatOOBfill);
 
-int map_2d(CUtensorMap *map, const void *base, uint32_t rows, uint32_t k, uint32_t ld, uint32_t box_rows)
+int map_2d(CUtensorMap *map, const void *base, uint32_t rows, uint32_t k, uint32_t ld, uint32_t box_rows,
+           CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B)
 {
     static encode_tiled_fn fn = nullptr;
     if (!fn) {
@@ -260,31 +385,89 @@ int map_2d(CUtensorMap *map, const void *base, uint32_t rows, uint32_t k, uint32
     const cuuint32_t box[2] = {kBK, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
                ? WR_CUDA_OK
                : WR_CUDA_ERR_INTERNAL;
 }
 
-template <uint32_t BN>
-int launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_weight &w, const wr_gemm_args &a)
+
+struct Plan {
+    uint64_t cost = ~0ull;
+    uint32_t wide = 0, bn0 = kMaxN, bn1 = kMaxN;
+};
+
+// A worker's clocks per 64 K-values of a tile: the products, or the operands on their way out of L2.
+uint64_t tile_cost(uint32_t ranks, uint32_t bn) { return std::max(2u * bn, ranks == 2 ? 350u : 150u + (kBM + bn) * 5u / 4u) + 24u; }
+
+// The cut of n columns into tiles that the workers finish first: tiles of 256 columns, and behind them (so that the last
+// round is a full one) narrower tiles for the rest.
+Plan plan(uint32_t ranks, uint32_t m_tiles, uint32_t n, uint32_t workers, bool one_width)
 {
-    constexpr uint32_t flag = BN == 256 ? 16u : BN == 128 ? 32u : 64u;
+    Plan best;
+    const uint32_t most = (n + kMaxN - 1) / kMaxN, rounds = (uint32_t)(((uint64_t)most * m_tiles + workers - 1) / workers);
+    for (uint32_t k = 0; k < rounds && k < 9; ++k) {
+        // wide tiles fill the first rounds but k (none at all: every tile has the narrow width)
+        const uint64_t full = k + 1 == rounds || k == 8 ? 0 : (uint64_t)(rounds - 1 - k) * workers / m_tiles;
+        const uint32_t wide = (uint32_t)std::min<uint64_t>(full, most);
+        if (one_width && wide) continue;
+        for (uint32_t bn = kMapRows * ranks; bn <= std::min(kMaxN, wr_weight_blocks(n) * kWBlock); bn += kMapRows * ranks) {
+            const uint32_t left = n > wide * kMaxN ? (n - wide * kMaxN + bn - 1) / bn : 0u;
+            const uint64_t t0 = (uint64_t)wide * m_tiles, tiles = t0 + (uint64_t)left * m_tiles;
+            uint64_t cost = 0;                           // tiles go round: the workers differ at two places only
+            for (uint64_t w : {(uint64_t)0, t0 % workers}) {
+                const uint64_t all = (tiles - std::min(w, tiles) + workers - 1) / workers, a = (t0 - std::min(w, t0) + workers - 1) / workers;
+                cost = std::max(cost, a * tile_cost(ranks, kMaxN) + (all - a) * tile_cost(ranks, bn));
+            }
+            if (cost < best.cost) {
+                best.cost = cost;
+                best.wide = wide;
+                best.bn1 = bn;
+            }
+        }
+    }
+    return best;
+}
+
+template <bool PAIR>
+int launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_weight &w, const wr_gemm_args &a, uint32_t m_tiles,
+           uint32_t workers, const Plan &pl)
+{
+    constexpr uint32_t ranks = PAIR ? 2 : 1, flag = PAIR ? 16u : 32u;
     if (!(ctx->attr_flags & flag)) {
-        WR_CUDA_TRY(cudaFuncSetAttribute(gemm_bf16_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)Tile<BN>::kSmem));
+        WR_CUDA_TRY(cudaFuncSetAttribute(gemm_bf16_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
         ctx->attr_flags |= flag;
     }
     GemmParams p;
     p.a = a;
     p.w = w;
-    p.m_tiles = (a.m + kBM - 1) / kBM;
-    p.n_tiles = (w.n + BN - 1) / BN;
+    p.m_tiles = m_tiles;
+    p.wide = pl.wide;
+    p.bn0 = pl.bn0;
+    p.bn1 = pl.bn1;
+    p.n_tiles = pl.wide + (w.n > pl.wide * pl.bn0 ? (w.n - pl.wide * pl.bn0 + pl.bn1 - 1) / pl.bn1 : 0u);
     p.k_blocks = wr_weight_blocks(w.k);
+    p.stage_bytes = kABytes + (pl.wide ? pl.bn0 : pl.bn1) / ranks * kRowBytes;
+    p.stages = std::min(kMaxStages, kStageBudget / p.stage_bytes);
     p.wait_limit = ctx->wait_limit;
     p.err = ctx->dev_err;
-    const uint32_t grid = std::min<uint32_t>((a.group.list ? a.group.max : p.m_tiles) * p.n_tiles, (uint32_t)ctx->sm_count);
-    WR_CUDA_TRY(wr_launch_pdl(gemm_bf16_kernel<BN>, dim3(grid), dim3(kThreads), Tile<BN>::kSmem, ctx->stream, x, p));
+    const uint32_t grid = ranks * (uint32_t)std::min<uint64_t>((uint64_t)m_tiles * p.n_tiles, workers);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = ranks;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = PAIR ? 2 : 1;
+    WR_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_bf16_kernel<PAIR>, x, PAIR ? w.maps->box[pl.bn0 / 2 / kMapRows - 1] : x,
+                                   PAIR ? w.maps->box[pl.bn1 / 2 / kMapRows - 1] : x, p));
     ctx->launches++;
     WR_CUDA_TRY(cudaGetLastError());
     return WR_CUDA_OK;
@@ -297,6 +480,16 @@ int wr_gemm_map_rows(CUtensorMap *map, const void *x, uint32_t rows, uint32_t k,
     return map_2d(map, x, rows, k, ld, kBM);
 }
 
+int wr_gemm_map_weight(wr_weight_maps *maps, const void *blocks, uint32_t n, uint32_t k)
+{
+    const uint32_t rows = wr_weight_blocks(n) * wr_weight_blocks(k) * kWBlock;
+    for (uint32_t i = 0; i < 4; ++i) {                   // (no box has more rows than there are: plan() takes no such tiles)
+        const int rc = map_2d(&maps->box[i], blocks, rows, kBK, kBK, std::min((i + 1) * kMapRows, rows), CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (rc != WR_CUDA_OK) return rc;
+    }
+    return WR_CUDA_OK;
+}
+
 int wr_skinny_map_rows(CUtensorMap *map, const void *split_rows, uint32_t k, uint32_t ld, uint32_t groups)
 {
     return map_2d(map, split_rows, groups * 2 * WR_CUDA_BATCH_MAX, k, ld, 2 * WR_CUDA_BATCH_MAX);
@@ -307,19 +500,11 @@ int wr_gemm_launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_weight &w, c
     if (a.m == 0 || w.n == 0 || w.k == 0 || (a.out_ld & 7u) || (a.out_bf16_ld & 7u) || (a.add_ld & 7u) ||
         (a.pair.from != ~0u && ((a.pair.from & 15u) || (a.pair.ld & 7u))))
         return WR_CUDA_ERR_INVAL;
-    // the tile width that finishes first: rounds over the device times the width's share of the work
-    const uint32_t m_tiles = a.group.list ? a.group.max : (a.m + kBM - 1) / kBM;
-    uint32_t best = 0;
-    uint64_t best_cost = ~0ull;
-    for (uint32_t bn : {256u, 128u, 64u}) {
-        const uint64_t tiles = (uint64_t)m_tiles * ((w.n + bn - 1) / bn);
-        const uint64_t cost = ((tiles + ctx->sm_count - 1) / ctx->sm_count) * (bn + 48u);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = bn;
-        }
+    const uint32_t sms = (uint32_t)ctx->sm_count, m_one = a.group.list ? a.group.max : (a.m + kBM - 1) / kBM, m_two = (m_one + 1) / 2;
+    const Plan one = plan(1, m_one, w.n, sms, a.group.list != nullptr);
+    if (w.maps && !a.group.list && !a.pages && a.m > kBM && sms >= 2) {
+        const Plan two = plan(2, m_two, w.n, sms / 2, false);
+        if (two.cost <= one.cost) return launch<true>(ctx, x, w, a, m_two, sms / 2, two);
     }
-    if (best == 256) return launch<256>(ctx, x, w, a);
-    if (best == 128) return launch<128>(ctx, x, w, a);
-    return launch<64>(ctx, x, w, a);
+    return launch<false>(ctx, x, w, a, m_one, sms, one);
 }

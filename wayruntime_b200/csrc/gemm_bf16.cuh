@@ -48,28 +48,39 @@ struct wr_gemm_args {
     const uint64_t *pages = nullptr;
 };
 
-// A BF16 weight [n][k] as the tensor core reads it: blocks of 64 rows x 64 K-values, each the 8 KB image of a
-// 128-byte-swizzled operand (row r at r * 128, its 16-byte piece c at c ^ (r & 7)), K-blocks of a row block one
-// after the other.  A block is one linear bulk copy, and a CTA's walk along K is one contiguous read.  Rows and
-// K-values beyond n and k are zeros.
+// A BF16 weight [n][k] as the tensor core reads it: for every 64 K-values the 128-byte pieces of all rows, one after the
+// other, each the image of a 128-byte-swizzled operand's row (its 16-byte piece c at c ^ (r & 7)).  So any run of rows
+// (from a multiple of eight on) is one copy.  That counts: issuing a copy takes a thread about 50 ns, and with blocks of
+// 64 rows (a copy per block) the products of a prompt waited for their weights (128 rows of weights and 64 K-values per
+// 0.42 us in four copies, 0.32 in two, 0.25 in one).  Rows and K-values beyond n and k are zeros.
 constexpr uint32_t kWBlock = 64, kWBlockBytes = kWBlock * kWBlock * 2;
 struct wr_weight {
     const void *blocks;
     uint32_t n, k;
+    const struct wr_weight_maps *maps = nullptr;     // (host memory) products of many rows may use pairs of CTAs
 };
 __host__ __device__ inline uint32_t wr_weight_blocks(uint32_t n) { return (n + kWBlock - 1) / kWBlock; }
 inline size_t wr_weight_bytes(uint32_t n, uint32_t k) { return (size_t)wr_weight_blocks(n) * wr_weight_blocks(k) * kWBlockBytes; }
-// byte offset of element (r, i)
-__host__ __device__ inline size_t wr_weight_off(uint32_t k, uint32_t r, uint32_t i)
+// byte offset of row r of the 64 K-values kb (its pieces swizzled by r & 7), of element (r, i)
+__host__ __device__ inline size_t wr_weight_row(uint32_t n, uint32_t r, uint32_t kb)
 {
-    const size_t block = (size_t)(r / kWBlock) * wr_weight_blocks(k) + i / kWBlock;
-    const uint32_t rr = r % kWBlock, ii = i % kWBlock;
-    return block * kWBlockBytes + rr * 128u + (((ii >> 3) ^ (rr & 7u)) << 4) + (ii & 7u) * 2u;
+    return ((size_t)kb * wr_weight_blocks(n) * kWBlock + r) * 128u;
+}
+__host__ __device__ inline size_t wr_weight_off(uint32_t n, uint32_t r, uint32_t i)
+{
+    const uint32_t ii = i % kWBlock;
+    return wr_weight_row(n, r, i / kWBlock) + (((ii >> 3) ^ (r & 7u)) << 4) + (ii & 7u) * 2u;
 }
 
 // Tensor map of activation rows [rows][k], ld elements apart (a multiple of 8; base 16-byte aligned).
 // WR_CUDA_ERR_INTERNAL when the driver refuses the map.
 int wr_gemm_map_rows(CUtensorMap *map, const void *x, uint32_t rows, uint32_t k, uint32_t ld);
+
+// ... and of a weight, in boxes of 32, 64, 96 and 128 rows.
+struct wr_weight_maps {
+    CUtensorMap box[4];
+};
+int wr_gemm_map_weight(wr_weight_maps *maps, const void *blocks, uint32_t n, uint32_t k);
 
 // Enqueue out[m][n] = act(x . w^T + bias) + add on the context's stream.
 int wr_gemm_launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_weight &w, const wr_gemm_args &args);

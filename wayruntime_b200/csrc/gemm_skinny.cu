@@ -111,17 +111,15 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const SkinnyParams
     if (warp == 0) {
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&x_map) : "memory");
-            // the row tile's one or two blocks of weights
-            const uint32_t nb = min(kM / kWBlock, wr_weight_blocks(p.w.n) - n0 / kWBlock);
-            const char *w = blocks + ((size_t)(n0 / kWBlock) * p.k_blocks + kb0) * kWBlockBytes;
+            const uint32_t bytes = min(kM, wr_weight_blocks(p.w.n) * kWBlock - n0) * kBK * 2;    // the row tile's weights per stage
+            const char *w = blocks + wr_weight_row(p.w.n, n0, kb0);
+            const size_t next = wr_weight_row(p.w.n, 0, 1);
             const uint64_t policy = l2_policy_evict_first();         // streamed once
             auto weights = [&](uint32_t it) {
                 const uint32_t st = it % kStages;
                 uint8_t *a = stages + st * kStageBytes;
-                mbar_expect_tx(&full[st], nb * kWBlockBytes + kBBytes);
-                for (uint32_t i = 0; i < nb; ++i)
-                    bulk_g2s_hint(a + i * kWBlockBytes, w + ((size_t)i * p.k_blocks + it) * kWBlockBytes, kWBlockBytes, &full[st],
-                                  policy);
+                mbar_expect_tx(&full[st], bytes + kBBytes);
+                bulk_g2s_hint(a, w + it * next, bytes, &full[st], policy);
             };
             auto rows = [&](uint32_t it) {
                 const uint32_t st = it % kStages;

@@ -117,22 +117,22 @@ __global__ void __launch_bounds__(256) latent_rotate_kernel(const wr_rows rw, co
 }
 
 // element pairs / quads of a weight row in either layout
-__device__ __forceinline__ float2 weight2(const float *w, uint32_t k, uint32_t r, uint32_t i)
+__device__ __forceinline__ float2 weight2(const float *w, uint32_t, uint32_t k, uint32_t r, uint32_t i)
 {
     if (i >= wr_ld(k)) return make_float2(0.f, 0.f);
     return *reinterpret_cast<const float2 *>(w + (size_t)r * wr_ld(k) + i);
 }
-__device__ __forceinline__ float2 weight2(const __half *w, uint32_t k, uint32_t r, uint32_t i)
+__device__ __forceinline__ float2 weight2(const __half *w, uint32_t n, uint32_t, uint32_t r, uint32_t i)
 {
-    return __half22float2(*reinterpret_cast<const __half2 *>(reinterpret_cast<const char *>(w) + wr_weight_off(k, r, i)));
+    return __half22float2(*reinterpret_cast<const __half2 *>(reinterpret_cast<const char *>(w) + wr_weight_off(n, r, i)));
 }
-__device__ __forceinline__ float4 weight4(const float *w, uint32_t k, uint32_t r, uint32_t i)
+__device__ __forceinline__ float4 weight4(const float *w, uint32_t, uint32_t k, uint32_t r, uint32_t i)
 {
     return load4(w + (size_t)r * wr_ld(k) + i);
 }
-__device__ __forceinline__ float4 weight4(const __half *w, uint32_t k, uint32_t r, uint32_t i)
+__device__ __forceinline__ float4 weight4(const __half *w, uint32_t n, uint32_t, uint32_t r, uint32_t i)
 {
-    return load4(reinterpret_cast<const __half *>(reinterpret_cast<const char *>(w) + wr_weight_off(k, r, i)));
+    return load4(reinterpret_cast<const __half *>(reinterpret_cast<const char *>(w) + wr_weight_off(n, r, i)));
 }
 
 // A block is one head, 64 columns of the cached row and RT rows; its four warps take a quarter of the head's dimensions
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(128) latent_query_kernel(const wr_rows rw, con
     for (int r = 0; r < RT; ++r) acc[r][0] = acc[r][1] = 0.f;
 #pragma unroll 8
     for (uint32_t d = lo; d < hi; ++d) {
-        const float2 w = weight2(static_cast<const TW *>(a.w_ukv), g.kv_rank, head * g.dim_pad() + d, c0 + 2 * lane);
+        const float2 w = weight2(static_cast<const TW *>(a.w_ukv), g.ukv_rows(), g.kv_rank, head * g.dim_pad() + d, c0 + 2 * lane);
 #pragma unroll
         for (int r = 0; r < RT; ++r) {
             acc[r][0] = fmaf(Q[r * g.dim + d], w.x, acc[r][0]);
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(128) latent_value_kernel(const wr_rows rw, con
         for (int r = 0; r < RT; ++r) acc[r] = 0.f;
 #pragma unroll 4
         for (uint32_t c = 4 * lane; c < ld; c += 128) {
-            const float4 w = weight4(static_cast<const TW *>(a.w_ukv), g.kv_rank,
+            const float4 w = weight4(static_cast<const TW *>(a.w_ukv), g.ukv_rows(), g.kv_rank,
                                        g.heads * g.dim_pad() + head * g.vdim_pad() + v, c);
 #pragma unroll
             for (int r = 0; r < RT; ++r) {
@@ -302,8 +302,7 @@ __global__ void __launch_bounds__(128) latent_query_mma_kernel(const wr_rows rw,
     __half *Q = reinterpret_cast<__half *>(W + dp * 128);        // [hi | lo][16][ld]
     for (uint32_t i = threadIdx.x; i < dp * 8; i += 128) {
         const uint32_t r = i / 8, at = head * dp + r;
-        const char *src = static_cast<const char *>(a.w_ukv) +
-                          ((size_t)(at / kWBlock) * wr_weight_blocks(g.kv_rank) + blockIdx.y) * kWBlockBytes + at % kWBlock * 128;
+        const char *src = static_cast<const char *>(a.w_ukv) + wr_weight_row(g.ukv_rows(), at, blockIdx.y);
         *reinterpret_cast<uint4 *>(W + r * 128 + i % 8 * 16) = *reinterpret_cast<const uint4 *>(src + i % 8 * 16);
     }
     pdl_wait();
@@ -354,13 +353,14 @@ __global__ void __launch_bounds__(128) latent_value_mma_kernel(const wr_rows rw,
     const uint32_t head = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3u, blocks = g.rank_pad() / 64;
     const uint32_t v0 = blockIdx.y * kValueCols + 8 * warp, row = min(v0 + (lane >> 2), g.vdim_pad() - 1);
     const uint32_t at = g.heads * g.dim_pad() + head * g.vdim_pad() + row, sw = at & 7u;
-    const char *src = static_cast<const char *>(a.w_ukv) + (size_t)(at / kWBlock) * blocks * kWBlockBytes + at % kWBlock * 128;
+    const char *src = static_cast<const char *>(a.w_ukv) + wr_weight_row(g.ukv_rows(), at, 0);
+    const size_t next = wr_weight_row(g.ukv_rows(), 0, 1);
     uint4 w[kMaxBlocks][2];
 #pragma unroll
     for (uint32_t b = 0; b < kMaxBlocks; ++b)
         if (b < blocks) {
-            w[b][0] = *reinterpret_cast<const uint4 *>(src + (size_t)b * kWBlockBytes + ((t ^ sw) << 4));
-            w[b][1] = *reinterpret_cast<const uint4 *>(src + (size_t)b * kWBlockBytes + (((t + 4) ^ sw) << 4));
+            w[b][0] = *reinterpret_cast<const uint4 *>(src + b * next + ((t ^ sw) << 4));
+            w[b][1] = *reinterpret_cast<const uint4 *>(src + b * next + (((t + 4) ^ sw) << 4));
         }
     pdl_wait();
     const uint32_t rp = g.rank_pad(), ld = rp + 32;

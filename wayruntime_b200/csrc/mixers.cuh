@@ -140,6 +140,7 @@ struct wr_latent_geom {
     __host__ __device__ uint32_t dim_pad() const { return (dim + 15u) & ~15u; }
     __host__ __device__ uint32_t rot_pad() const { return (rot + 15u) & ~15u; }
     __host__ __device__ uint32_t vdim_pad() const { return (vdim + 15u) & ~15u; }
+    __host__ __device__ uint32_t ukv_rows() const { return heads * (dim_pad() + vdim_pad()); }
     __host__ __device__ uint32_t q_head() const { return dim_pad() + rot_pad(); }
     __host__ __device__ uint32_t rank_pad() const { return (kv_rank + 63u) & ~63u; }
     __host__ __device__ uint32_t row() const { return rank_pad() + ((rot + 63u) & ~63u); }

@@ -35,6 +35,7 @@ struct Mat {                             // [n][k]: F32 rows wr_ld(k) apart, or 
     const void *w = nullptr;
     uint32_t n = 0, k = 0;
     CUtensorMap x_map{}, xs_map{};       // BF16 models: its input rows, and its input as split rows
+    wr_weight_maps w_maps{};             // ... and itself
     wr_pair_args pair;                   // BF16 models: gate and up rows side by side (where they lie, act)
 };
 
@@ -219,7 +220,7 @@ struct Packer {
                 const uint32_t pk = p.k ? p.k : k;
                 const size_t src = (size_t)(p.row0 + r) * pk;
                 for (uint32_t i = 0; i < pk; i += 8) {           // pieces of eight stay together (col: a multiple of 8)
-                    uint16_t *dst = reinterpret_cast<uint16_t *>(buf.data() + o + wr_weight_off(k, p.dst(r), p.col + i));
+                    uint16_t *dst = reinterpret_cast<uint16_t *>(buf.data() + o + wr_weight_off(rows, p.dst(r), p.col + i));
                     const uint32_t n = std::min(8u, pk - i);
                     if (type == WR_CUDA_F16)
                         for (uint32_t e = 0; e < n; ++e) dst[e] = f32_to_f16(elem(*p.t, src + i + e));
@@ -387,7 +388,7 @@ void pack_layer(Packer &pk, const wr_cuda_mixed_layer &l, Layer &o, uint32_t wid
         mat(o.uq, {Part{&l.w_uq, 0, g.heads * (g.dim + g.rot), 0}.in_groups(g.dim + g.rot, g.q_head(), g.dim, g.dim_pad())},
             g.heads * g.q_head(), g.q_rank);
         const int half = bf ? WR_CUDA_F16 : WR_CUDA_F32;
-        o.ukv.n = g.heads * (g.dim_pad() + g.vdim_pad());
+        o.ukv.n = g.ukv_rows();
         o.ukv.k = g.kv_rank;
         set_off(o.ukv.w, pk.mat({Part{&l.w_uk, 0, g.heads * g.dim, 0}.in_groups(g.dim, g.dim_pad()),
                                  Part{&l.w_uv, 0, g.heads * g.vdim, g.heads * g.dim_pad()}.in_groups(g.vdim, g.vdim_pad())},
@@ -504,6 +505,7 @@ int fix_mat(Mat &m, const wr_mixed &x, const void *input, uint32_t input_rows, u
     fix(m.w, x.weights);
     if (x.compute != WR_CUDA_BF16) return WR_CUDA_OK;
     int rc = wr_gemm_map_rows(&m.x_map, input, input_rows, m.k, input_ld);
+    if (rc == WR_CUDA_OK) rc = wr_gemm_map_weight(&m.w_maps, m.w, m.n, m.k);
     if (rc == WR_CUDA_OK) rc = wr_skinny_map_rows(&m.xs_map, few_input ? few_input : input, m.k, input_ld, groups);
     return rc;
 }
@@ -792,7 +794,7 @@ struct Step {
             a.mul = mul;
             a.pair = pair;
             ++m->launches;
-            return wr_gemm_launch(ctx, mat.x_map, {mat.w, mat.n, mat.k}, a);
+            return wr_gemm_launch(ctx, mat.x_map, {mat.w, mat.n, mat.k, &mat.w_maps}, a);
         }
         ++m->launches;
         if (x->compute == WR_CUDA_BF16) {
