@@ -10,8 +10,11 @@
 // the two rows' largest values, and 2^-31 of it in the mean square.
 // Error of one product against float64 (2-norm; rounding the exact result to F32 is 2.5e-8), K of 1024 / 2048 / 4096 and Gaussian
 // rows: the GEMV 9.5e-8 / 1.1e-7 / 1.3e-7, this 4.5e-8 / 3.6e-8 / 3.6e-8 (with the rounding of the residual that it is added to).
-// 1000 rows, us: 4096 x 1024 35.6, gate / up of 2 x 3072 x 1024 53.9, 1024 x 3072 26.2: 2300 to 2450 TOP/s of digit products, 230 to
-// 245 TFLOP/s of F32 ones.  Sixteen warps fetch: with eight the gate / up product takes 63.2.
+// 1000 rows, us: 4096 x 1024 35.0, gate / up of 2 x 3072 x 1024 50.2, 1024 x 3072 25.7: 2400 to 2500 TOP/s of digit products, 240 to
+// 250 TFLOP/s of F32 ones (37.4, 54.8, 26.1 with each sixteen sums finished and written before the next were fetched, and
+// weights in 64-row blocks).  Sixteen warps fetch: with eight the gate / up product takes 63.2.  Back to back these products
+// draw what the device may (980 of 1000 W): tiles of 256 x 64 on pairs of CTAs (gemm_bf16.cu), whose output overlaps the next
+// tile's products, took 33.9 and 47.2 us alone and not a microsecond off a whole prompt, as they move more per product.
 // Stages: 64 K-values, all digits of both operands.  Persistent CTAs, tiles of 128 x BN, m fastest: the tiles in flight
 // share weight rows in L2.
 #include <math.h>
@@ -39,9 +42,6 @@ template <uint32_t BN> struct Tile {
     static constexpr uint32_t kTmemCols = 512;
     static constexpr uint32_t kCols = BN / 4;                        // columns a warp finishes
 };
-// Sums of i + j = 0, 2, 1, 3 lie side by side in this order: digits q and q + 2 of a weight lie BN rows apart in shared
-// memory, and one instruction of twice the width takes a digit of x with both.
-__host__ __device__ constexpr uint32_t diag_at(uint32_t d) { return d == 1 ? 2u : d == 2 ? 1u : d; }
 
 struct GemmParams {
     wr_f32_gemm_args a;
@@ -149,14 +149,14 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
 
     if (warp == 0) {
         if (lane == 0) {
-            const size_t lo_off = (size_t)wr_weight_blocks(w.n) * p.k_blocks * kWBlockBytes;
+            const uint32_t w_rows = wr_weight_blocks(w.n) * kWBlock;
             uint32_t it = 0;
             bool ok = true;
             for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
                 const uint32_t tile = unit % tiles, k_lo = unit / tiles * p.part_blocks;
                 const uint32_t k_hi = min(k_lo + p.part_blocks, p.k_blocks);
-                const uint32_t m0 = (tile % p.m_tiles) * kBM, nb0 = (tile / p.m_tiles) * (BN / kWBlock);
-                const uint32_t nb = min(BN / kWBlock, wr_weight_blocks(w.n) - nb0);
+                const uint32_t m0 = (tile % p.m_tiles) * kBM, n0 = (tile / p.m_tiles) * BN;
+                const uint32_t rows = min(BN, w_rows - n0);
                 for (uint32_t kb = k_lo; kb < k_hi; ++kb, ++it) {
                     const uint32_t st = it % T::kStages;
                     if (it >= T::kStages && !mbar_wait(&empty[st], (it / T::kStages - 1) & 1, p.wait_limit)) {
@@ -164,14 +164,11 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
                         break;
                     }
                     uint8_t *a = stages + st * T::kStageBytes, *b = a + 2 * kABytes;
-                    mbar_expect_tx(&full[st], 2 * (kABytes + nb * kWBlockBytes));
+                    mbar_expect_tx(&full[st], 2 * (kABytes + rows * 128));
                     tc5::tma_load_2d(a, &x_map, (int)(kb * kBK), (int)m0, &full[st]);
                     tc5::tma_load_2d(a + kABytes, &x_map, (int)(kb * kBK), (int)(p.a.pad + m0), &full[st]);
-                    const char *from = w.blocks + ((size_t)nb0 * p.k_blocks + kb) * kWBlockBytes;
-                    for (uint32_t i = 0; i < nb; ++i, from += (size_t)p.k_blocks * kWBlockBytes) {
-                        bulk_g2s(b + i * kWBlockBytes, from, kWBlockBytes, &full[st]);
-                        bulk_g2s(b + T::kBBytes + i * kWBlockBytes, from + lo_off, kWBlockBytes, &full[st]);
-                    }
+                    bulk_g2s(b, w.blocks + wr_weight_row(w.n, n0, kb), rows * 128, &full[st]);
+                    bulk_g2s(b + T::kBBytes, w.blocks + wr_weight_row(w.n, n0, p.k_blocks + kb), rows * 128, &full[st]);
                 }
             }
             if (!ok) atomicCAS(p.err, 0, 71);
@@ -200,20 +197,20 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
                 }
                 tc5::fence_after();
                 const uint32_t a_addr = smem_u32(stages + st * T::kStageBytes), b_addr = a_addr + 2 * kABytes;
-                // digit i of 32 K-values: 64 bytes in a row for an odd one, the second half of the stage from 2 on
+                // digit i of 32 K-values of x: 64 bytes in a row for an odd one, the second half from 2 on; digits i and i + 1 of the
+                // weights (i even: digits of one kind lie BN rows behind the other), or of half the rows digit i alone
                 auto a_of = [&](uint32_t i, uint32_t kk) { return tc5::desc_kmajor(a_addr + (i >> 1) * kABytes) + 4 * (i & 1) + 2 * kk; };
-                auto b_of = [&](uint32_t i, uint32_t kk) { return tc5::desc_kmajor(b_addr) + 4 * (i & 1) + 2 * kk; };
+                auto b_of = [&](uint32_t i, uint32_t kk) { return tc5::desc_kmajor(b_addr) + 2 * i + 2 * kk; };
                 if (lead) {
 #pragma unroll
                     for (uint32_t kk = 0; kk < kBK / 32; ++kk) {
                         const uint32_t more = kb != k_lo || kk != 0;
-                        tc5::mma_i8_ss(d + diag_at(0) * BN, a_of(0, kk), b_of(0, kk), two, more);      // 0 0, 0 2
-                        tc5::mma_i8_ss(d + diag_at(1) * BN, a_of(0, kk), b_of(1, kk), two, more);      // 0 1, 0 3
-                        tc5::mma_i8_ss(d + diag_at(1) * BN, a_of(1, kk), b_of(0, kk), two, 1);         // 1 0, 1 2
-                        tc5::mma_i8_ss(d + diag_at(2) * BN, a_of(1, kk), b_of(1, kk), one, 1);
-                        tc5::mma_i8_ss(d + diag_at(2) * BN, a_of(2, kk), b_of(0, kk), one, 1);
-                        tc5::mma_i8_ss(d + diag_at(3) * BN, a_of(2, kk), b_of(1, kk), one, 1);
-                        tc5::mma_i8_ss(d + diag_at(3) * BN, a_of(3, kk), b_of(0, kk), one, 1);
+                        tc5::mma_i8_ss(d, a_of(0, kk), b_of(0, kk), two, more);                  // 0 0, 0 1
+                        tc5::mma_i8_ss(d + 2 * BN, a_of(0, kk), b_of(2, kk), two, more);         // 0 2, 0 3
+                        tc5::mma_i8_ss(d + BN, a_of(1, kk), b_of(0, kk), two, 1);                // 1 0, 1 1
+                        tc5::mma_i8_ss(d + 3 * BN, a_of(1, kk), b_of(2, kk), one, 1);            // 1 2
+                        tc5::mma_i8_ss(d + 2 * BN, a_of(2, kk), b_of(0, kk), two, 1);            // 2 0, 2 1
+                        tc5::mma_i8_ss(d + 3 * BN, a_of(3, kk), b_of(0, kk), one, 1);            // 3 0
                     }
                     tc5::commit(&empty[st]);
                     if (kb + 1 == k_hi) tc5::commit(&acc_full[acc]);
@@ -237,18 +234,24 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
                 break;
             }
             tc5::fence_after();
-#pragma unroll 1
-            for (uint32_t c = 0; c < T::kCols; c += 16) {
-                int v[kDiags][16];
+            // all of the warp's sums first: with 128 columns the next tile's products wait for the accumulators
+            float raw[T::kCols];
+#pragma unroll
+            for (uint32_t c = 0; c < T::kCols; c += 8) {
+                int v[kDiags][8];
 #pragma unroll
                 for (uint32_t d = 0; d < kDiags; ++d)
-                    tc5::ld16(tmem + ((quarter * 32) << 16) + (acc * kDiags + diag_at(d)) * BN + c_lo + c, reinterpret_cast<float *>(v[d]));
+                    tc5::ld8(tmem + ((quarter * 32) << 16) + (acc * kDiags + d) * BN + c_lo + c, reinterpret_cast<float *>(v[d]));
                 tc5::wait_ld();
-                if (c + 16 == T::kCols) {                        // the next tile may have the accumulators
-                    tc5::fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[acc]);
-                }
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j)
+                    raw[c + j] = __ll2float_rn((long long)v[0][j] * (1 << 24) + (long long)v[1][j] * (1 << 16) + (long long)v[2][j] * 256 + v[3][j]);
+            }
+            tc5::fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[acc]);
+#pragma unroll
+            for (uint32_t c = 0; c < T::kCols; c += 16) {
                 if (!in || n0 + c >= w.n) continue;
                 float y[16];
                 bool odd = false;
@@ -258,20 +261,18 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
                     const int es[4] = {we.x, we.y, we.z, we.w};
 #pragma unroll
                     for (uint32_t j = i; j < i + 4; ++j) {
-                        const long long t = (long long)v[0][j] * (1 << 24) + (long long)v[1][j] * (1 << 16) + (long long)v[2][j] * 256 + v[3][j];
                         const int e = rs.exponent + es[j - i];
                         odd = odd || (uint32_t)(e + 126) > 253u;
-                        v[0][j] = __float_as_int(__ll2float_rn(t));
-                        y[j] = __fmul_rn(__int_as_float(v[0][j]) * pow2(e), rs.factor);
+                        y[j] = __fmul_rn(raw[c + j] * pow2(e), rs.factor);
                     }
                 }
                 if (!odd) {
                     put16(p, y, part, row, n0 + c);
                 } else {
-                    float raw[16];
+                    float z[16];
 #pragma unroll
-                    for (uint32_t i = 0; i < 16; ++i) raw[i] = __int_as_float(v[0][i]);
-                    put16_rare(p, raw, rs, part, row, n0 + c, k_lo, k_hi);
+                    for (uint32_t i = 0; i < 16; ++i) z[i] = raw[c + i];
+                    put16_rare(p, z, rs, part, row, n0 + c, k_lo, k_hi);
                 }
             }
             __syncwarp();
@@ -369,14 +370,13 @@ __global__ void __launch_bounds__(32 * kSplitWarps) split_weights_kernel(const S
     const Scale scale(top);
     pdl_wait();                                          // the blocks are read by the product before
     if (row >= wr_weight_blocks(s.to.n) * kWBlock) return;
-    const size_t lo_off = (size_t)wr_weight_blocks(s.to.n) * (k_pad / kWBlock) * kWBlockBytes;
     auto store = [&](uint32_t at, const float4 (&v)[2]) {
         uint32_t a[4], b[4];
         digits4(v[0], scale, a);
         digits4(v[1], scale, b);
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i)
-            *reinterpret_cast<uint2 *>(s.to.blocks + (i >> 1) * lo_off + wr_split_off(k, row, i & 1, at)) = make_uint2(a[i], b[i]);
+            *reinterpret_cast<uint2 *>(s.to.blocks + wr_split_off(s.to.n, k, row, i, at)) = make_uint2(a[i], b[i]);
     };
 #pragma unroll
     for (uint32_t u = 0; u < kKeep; ++u)

@@ -11,8 +11,9 @@
 // within 2^-31 of the row's largest value: all of its 24 bits are there down to 2^-7 of it, and the row as a vector is off by less
 // than sqrt(k) 2^-31 of its length.
 //
-// Digits of 64 values take 256 bytes: 64 of the highest, 64 of the next, and, elsewhere, 64 of each of the other two.
-// Weights: digits 0 and 1 in wr_weight's blocks of 128-byte rows (gemm_bf16.cuh), then digits 2 and 3 likewise.
+// Digits of 64 values take 256 bytes: 64 of each of two digits, and, elsewhere, 64 of each of the other two.
+// Weights: digits 0 and 2 in wr_weight's 128-byte pieces (gemm_bf16.cuh), then digits 1 and 3 likewise, so that digits 0 and 1
+// (2 and 3) of a tile's rows are one operand of twice the rows.
 struct wr_split_weight {
     char *blocks = nullptr;
     int *exponent = nullptr;             // [n]: of the power of two that undoes the row's scale and the digits' unit; or one of the next two
@@ -22,12 +23,11 @@ struct wr_split_weight {
 // two exponents comes near either, nor two of the first to the second.)
 constexpr int kNotFinite = 1 << 20, kNotNumbers = 1 << 22;
 size_t wr_split_weight_bytes(uint32_t n, uint32_t k);
-// byte offset of a row's digit 0 or 1 (digits 2 and 3: half the bytes on) of value i
-__host__ __device__ inline size_t wr_split_off(uint32_t k, uint32_t row, uint32_t digit, uint32_t i)
+// byte offset of digit `digit` of value i of a row
+__host__ __device__ inline size_t wr_split_off(uint32_t n, uint32_t k, uint32_t row, uint32_t digit, uint32_t i)
 {
-    const size_t block = (size_t)(row / kWBlock) * wr_weight_blocks(k) + i / kWBlock;
-    const uint32_t r = row % kWBlock, piece = digit * 4 + i % kWBlock / 16;
-    return block * kWBlockBytes + r * 128u + ((piece ^ (r & 7u)) << 4) + i % 16;
+    const uint32_t piece = (digit >> 1) * 4 + i % kWBlock / 16, kb = (digit & 1u) * wr_weight_blocks(k) + i / kWBlock;
+    return wr_weight_row(n, row, kb) + ((piece ^ (row & 7u)) << 4) + i % 16;
 }
 
 // Rows of one split weight, from up to three F32 matrices [n_i][k] one below the other, or (pair) from gate and up
