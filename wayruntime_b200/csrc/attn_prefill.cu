@@ -359,7 +359,7 @@ __host__ __device__ inline uint32_t prefill_tile_count(uint32_t n_qtiles, uint32
     if (n_qtiles & 1u) n += n_kv * ((group & 1u) + group / 2u);      // the first query tile on its own
     return n;
 }
-__device__ inline tile_info decode_tile(const prefill_params &p, uint32_t idx)
+__host__ __device__ inline tile_info decode_tile(const prefill_params &p, uint32_t idx)
 {
     tile_info t;
     t.valid = 0; t.nblk = 0; t.kvh = 0; t.pad = 0;
@@ -368,8 +368,9 @@ __device__ inline tile_info decode_tile(const prefill_params &p, uint32_t idx)
     t.valid = 1;
     if (p.single) {
         t.nblk = 1;
-        t.kvh = t.head[0] = idx % p.n_kv;
-        t.qt[0] = p.n_qtiles - 1 - idx / p.n_kv;
+        t.head[0] = idx % p.n_q;
+        t.kvh = t.head[0] / p.group;
+        t.qt[0] = p.n_qtiles - 1 - idx / p.n_q;
         return t;
     }
     const uint32_t per = tiles_per_qpair(p.n_kv, p.group), pairs = p.group / 2u, odd = p.group & 1u;
@@ -399,17 +400,48 @@ __device__ inline tile_info decode_tile(const prefill_params &p, uint32_t idx)
 struct block_range {
     uint32_t tok0, rows, key_end, lo, hi;
 };
-__device__ __forceinline__ block_range range_of(const prefill_params &p, uint32_t qt)
+__host__ __device__ __forceinline__ block_range range_of(const prefill_params &p, uint32_t qt)
 {
     block_range b;
     b.tok0 = qt * kBM;
-    b.rows = min((uint32_t)kBM, p.n - b.tok0);
+    b.rows = p.n - b.tok0 < (uint32_t)kBM ? p.n - b.tok0 : (uint32_t)kBM;
     b.key_end = p.p0 + b.tok0 + b.rows;
     uint32_t key_first = 0;
     if (p.window > 0 && p.p0 + b.tok0 + 1 > p.window) key_first = p.p0 + b.tok0 + 1 - p.window;
     b.lo = key_first / kBN;
     b.hi = (b.key_end + kBN - 1) / kBN;
     return b;
+}
+
+// When the CTAs would be done with p's tiles, in hundredths of a microsecond: a step (128 keys) of one block takes 1.87 us, of two
+// blocks 2.03 (they share the chain of scores, softmax and values), a tile that follows another 1.4 more.  Tiles are
+// numbered longest first, so a CTA's second tile is as far from the middle as its first.
+inline uint32_t tiles_time(const prefill_params &p, uint32_t ctas)
+{
+    uint32_t worst = 0;
+    for (uint32_t i = 0; i < ctas && i < p.n_tiles; ++i) {
+        uint32_t t = 0;
+        for (uint32_t round = 0; round * ctas < p.n_tiles; ++round) {
+            const tile_info ti = decode_tile(p, round * ctas + ((round & 1u) ? ctas - 1 - i : i));
+            if (!ti.valid) continue;
+            const block_range a = range_of(p, ti.qt[0]), b = range_of(p, ti.qt[ti.nblk - 1]);
+            t += (std::max(a.hi, b.hi) - std::min(a.lo, b.lo)) * (ti.nblk > 1 ? 203u : 187u) + (round ? 140u : ti.nblk > 1 ? 145u : 0u);
+        }
+        worst = std::max(worst, t);
+    }
+    return worst;
+}
+// Tiles of one block each instead of two: always where they all go round at once (us, two blocks / one: 100 rows of 32 heads
+// 11.1 / 9.3, 1000 rows of 16 heads 24.8 / 22.5), never where two blocks go round several times; in between the lengths decide
+// (513 rows of 32 heads 21.1 / 14.6; behind 6000 keys 1700 rows of 16 heads 129 / 147).  A block's arithmetic is the same.
+inline void tiles_of_one(prefill_params &p, uint32_t ctas)
+{
+    const uint32_t singles = p.n_qtiles * p.n_q;
+    if (singles > 3 * ctas) return;
+    prefill_params one = p;
+    one.single = 1;
+    one.n_tiles = singles;
+    if (singles <= ctas || tiles_time(one, ctas) < tiles_time(p, ctas)) p = one;
 }
 
 // ---- the kernel ------------------------------------------------------------
@@ -1195,6 +1227,7 @@ extern "C" int wr_cuda_attn_prefill(wr_cuda_ctx *ctx, wr_cuda_kv *kv, uint32_t l
     p.window = window;
     p.n_qtiles = (n + kBM - 1) / kBM;
     p.n_tiles = prefill_tile_count(p.n_qtiles, p.n_kv, p.group);
+    tiles_of_one(p, (uint32_t)ctx->sm_count);
     const float scale = (scale_override > 0.0f) ? scale_override : 1.0f / sqrtf((float)kHd);   // kernels.c:1457-1459
     p.scale_log2 = scale * kLog2e;
     if (!(ctx->attr_flags & 2u)) {
