@@ -221,7 +221,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
                 const uint32_t share = t.bn / kRanks, r0 = t.n0 + rank * share;     // this rank's weight rows
                 const uint32_t rows = r0 < w_rows ? min(share, w_rows - r0) : 0u;
                 const char *blocks = static_cast<const char *>(p.w.blocks);
-                if (p.a.group.list) blocks += p.a.group.list[t.strip] * p.a.group.stride;
+                uint32_t y0 = r0;                        // (in the weights' maps)
+                if (p.a.group.list) {
+                    const uint32_t e = p.a.group.list[t.strip];
+                    blocks += e * p.a.group.stride;
+                    y0 += e * (uint32_t)(p.a.group.stride / kRowBytes);
+                }
                 const uint32_t np = !p.a.pages || m0 >= p.a.m ? 0u : m0 + kPageTokens < p.a.m ? 2u : 1u;
                 // (a pair's boxes count whole; what they bring from beyond the weight's rows belongs to no column)
                 const uint32_t bytes = PAIR ? 2 * kABytes + t.bn * kRowBytes : (p.a.pages ? np * (kABytes / 2) : kABytes) + rows * kRowBytes;
@@ -235,7 +240,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
                     if (rank == 0) mbar_expect_tx(&full[st], bytes);
                     if (PAIR) {
                         tc5::tma_load_2d_pair(a, &x_map, (int)(kb * kBK), (int)m0, &full[st]);
-                        tc5::tma_load_2d_pair(b, w_map, 0, (int)(kb * w_rows + r0), &full[st]);
+                        tc5::tma_load_2d_pair(b, w_map, 0, (int)(kb * w_rows + y0), &full[st]);
                     } else {
                         if (p.a.pages) {
                             for (uint32_t i = 0; i < np; ++i)
@@ -480,9 +485,9 @@ int wr_gemm_map_rows(CUtensorMap *map, const void *x, uint32_t rows, uint32_t k,
     return map_2d(map, x, rows, k, ld, kBM);
 }
 
-int wr_gemm_map_weight(wr_weight_maps *maps, const void *blocks, uint32_t n, uint32_t k)
+int wr_gemm_map_weight(wr_weight_maps *maps, const void *blocks, uint32_t n, uint32_t k, uint32_t count, size_t stride)
 {
-    const uint32_t rows = wr_weight_blocks(n) * wr_weight_blocks(k) * kWBlock;
+    const uint32_t rows = wr_weight_blocks(n) * wr_weight_blocks(k) * kWBlock + (uint32_t)((count - 1) * (stride / kRowBytes));
     for (uint32_t i = 0; i < 4; ++i) {                   // (no box has more rows than there are: plan() takes no such tiles)
         const int rc = map_2d(&maps->box[i], blocks, rows, kBK, kBK, std::min((i + 1) * kMapRows, rows), CU_TENSOR_MAP_SWIZZLE_NONE);
         if (rc != WR_CUDA_OK) return rc;
@@ -500,9 +505,16 @@ int wr_gemm_launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_weight &w, c
     if (a.m == 0 || w.n == 0 || w.k == 0 || (a.out_ld & 7u) || (a.out_bf16_ld & 7u) || (a.add_ld & 7u) ||
         (a.pair.from != ~0u && ((a.pair.from & 15u) || (a.pair.ld & 7u))))
         return WR_CUDA_ERR_INVAL;
-    const uint32_t sms = (uint32_t)ctx->sm_count, m_one = a.group.list ? a.group.max : (a.m + kBM - 1) / kBM, m_two = (m_one + 1) / 2;
-    const Plan one = plan(1, m_one, w.n, sms, a.group.list != nullptr);
-    if (w.maps && !a.group.list && !a.pages && a.m > kBM && sms >= 2) {
+    const uint32_t sms = (uint32_t)ctx->sm_count;
+    if (a.group.list) {
+        const uint32_t likely = a.group.likely ? std::min(a.group.likely, a.group.max) : a.group.max;
+        if (a.group.tile == kBM) return launch<false>(ctx, x, w, a, a.group.max, sms, plan(1, likely, w.n, sms, true));
+        if (a.group.tile != 2 * kBM || !w.maps || a.group.stride % kRowBytes || sms < 2) return WR_CUDA_ERR_INVAL;
+        return launch<true>(ctx, x, w, a, a.group.max, sms / 2, plan(2, likely, w.n, sms / 2, true));
+    }
+    const uint32_t m_one = (a.m + kBM - 1) / kBM, m_two = (m_one + 1) / 2;
+    const Plan one = plan(1, m_one, w.n, sms, false);
+    if (w.maps && !a.pages && a.m > kBM && sms >= 2) {
         const Plan two = plan(2, m_two, w.n, sms / 2, false);
         if (two.cost <= one.cost) return launch<true>(ctx, x, w, a, m_two, sms / 2, two);
     }

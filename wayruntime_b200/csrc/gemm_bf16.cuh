@@ -19,7 +19,7 @@ struct wr_pair_args {
     uint32_t ld = 0;
 };
 // One product per group of rows, each with a weight of its own (experts), `stride` bytes apart.  `list` names the
-// weight of every 128-row tile of the activations (many rows), or of every group (few rows: group g's results are
+// weight of every tile of `tile` rows of the activations (many rows), or of every group (few rows: group g's results are
 // rows 16 g .. of out, split rows 32 g .. of pair.out, and its input the split rows x_rows * g ..).
 struct wr_group_args {
     const uint32_t *list = nullptr;      // device memory, as is:
@@ -28,6 +28,8 @@ struct wr_group_args {
     uint32_t usual = 1;                  // few rows: how many a single row has
     uint32_t x_rows = 0;
     size_t stride = 0;
+    uint32_t tile = 128;                 // many rows: 128, or 256 (a tile of a pair of CTAs; the weights need their maps)
+    uint32_t likely = 0;                 // many rows: how many tiles there will be, about
 };
 
 struct wr_gemm_args {
@@ -76,11 +78,11 @@ __host__ __device__ inline size_t wr_weight_off(uint32_t n, uint32_t r, uint32_t
 // WR_CUDA_ERR_INTERNAL when the driver refuses the map.
 int wr_gemm_map_rows(CUtensorMap *map, const void *x, uint32_t rows, uint32_t k, uint32_t ld);
 
-// ... and of a weight, in boxes of 32, 64, 96 and 128 rows.
+// ... and of a weight (or `count` of them, `stride` bytes apart, a multiple of 128), in boxes of 32, 64, 96 and 128 rows.
 struct wr_weight_maps {
     CUtensorMap box[4];
 };
-int wr_gemm_map_weight(wr_weight_maps *maps, const void *blocks, uint32_t n, uint32_t k);
+int wr_gemm_map_weight(wr_weight_maps *maps, const void *blocks, uint32_t n, uint32_t k, uint32_t count = 1, size_t stride = 0);
 
 // Enqueue out[m][n] = act(x . w^T + bias) + add on the context's stream.
 int wr_gemm_launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_weight &w, const wr_gemm_args &args);

@@ -30,6 +30,15 @@ constexpr double kLog2e = 1.4426950408889634;
 size_t up256(size_t n) { return (n + 255u) & ~(size_t)255u; }
 
 constexpr uint32_t kMoeTile = 128;       // rows of a tile of gemm_bf16.cu
+// Tiles of pairs of CTAs where the experts have that many rows each on average: a pair takes about half the time of one CTA for
+// a tile twice as high, so it pays from where most experts' rows fill more than a quarter of it.
+constexpr uint32_t kMoePairRows = 96;
+inline uint32_t moe_tile(uint32_t rows, uint32_t experts, uint32_t top) { return (uint64_t)rows * top >= (uint64_t)experts * kMoePairRows ? 2 * kMoeTile : kMoeTile; }
+// places that up to `rows` rows may take
+inline size_t moe_places(uint32_t rows, uint32_t experts, uint32_t top)
+{
+    return std::max((size_t)wr_route_tiles(rows, experts, top, kMoeTile) * kMoeTile, (size_t)wr_route_tiles(rows, experts, top, 2 * kMoeTile) * 2 * kMoeTile);
+}
 
 struct Mat {                             // [n][k]: F32 rows wr_ld(k) apart, or BF16 blocks (wr_weight)
     const void *w = nullptr;
@@ -499,13 +508,13 @@ template <typename P> void fix(P *&p, const char *base)
 }
 
 int fix_mat(Mat &m, const wr_mixed &x, const void *input, uint32_t input_rows, uint32_t input_ld, const void *few_input = nullptr,
-            uint32_t groups = 1)
+            uint32_t groups = 1, uint32_t count = 1, size_t stride = 0)
 {
     if (!m.w) return WR_CUDA_OK;
     fix(m.w, x.weights);
     if (x.compute != WR_CUDA_BF16) return WR_CUDA_OK;
     int rc = wr_gemm_map_rows(&m.x_map, input, input_rows, m.k, input_ld);
-    if (rc == WR_CUDA_OK) rc = wr_gemm_map_weight(&m.w_maps, m.w, m.n, m.k);
+    if (rc == WR_CUDA_OK) rc = wr_gemm_map_weight(&m.w_maps, m.w, m.n, m.k, count, stride);
     if (rc == WR_CUDA_OK) rc = wr_skinny_map_rows(&m.xs_map, few_input ? few_input : input, m.k, input_ld, groups);
     return rc;
 }
@@ -637,7 +646,7 @@ extern "C" int wr_cuda_model_create_mixed(wr_cuda_ctx *ctx, const wr_cuda_mixed_
         }
         if (l.experts) {
             const uint32_t tile = bf ? kMoeTile : kMoeTileF32, tiles = wr_route_tiles((uint32_t)R, l.experts, l.top, tile);
-            const size_t places = (size_t)tiles * tile, groups = wr_route_tiles((uint32_t)few, l.experts, l.top, 0);
+            const size_t places = bf ? moe_places((uint32_t)R, l.experts, l.top) : (size_t)tiles * tile, groups = wr_route_tiles((uint32_t)few, l.experts, l.top, 0);
             const size_t es = bf ? 2 : 4, lf = wr_ld(l.ff);
             lat = std::max<size_t>(lat, wr_ld(l.experts));
             e_top = std::max<size_t>(e_top, l.top);
@@ -710,11 +719,11 @@ extern "C" int wr_cuda_model_create_mixed(wr_cuda_ctx *ctx, const wr_cuda_mixed_
         if (rc == WR_CUDA_OK) rc = fix_mat(l.gate, *x, x->xin, rows, x->ldw);
         if (rc == WR_CUDA_OK) rc = fix_mat(l.router, *x, x->xin, rows, x->ldw);
         if (rc == WR_CUDA_OK && l.experts) {
-            const uint32_t places = wr_route_tiles(rows, l.experts, l.top, kMoeTile) * kMoeTile;
-            rc = fix_mat(l.e_up, *x, x->e_in, places, x->ldw, x->xin);
+            const uint32_t places = (uint32_t)moe_places(rows, l.experts, l.top);
+            rc = fix_mat(l.e_up, *x, x->e_in, places, x->ldw, x->xin, 1, l.experts, l.up_stride);
             if (rc == WR_CUDA_OK)
                 rc = fix_mat(l.e_down, *x, x->e_act, places, wr_ld(l.ff), x->e_act,
-                             wr_route_tiles((uint32_t)few, l.experts, l.top, 0));
+                             wr_route_tiles((uint32_t)few, l.experts, l.top, 0), l.experts, l.down_stride);
         }
         if (rc == WR_CUDA_OK) rc = fix_mat(l.qkvg, *x, x->xin, rows, x->ldw);
         if (rc == WR_CUDA_OK) rc = fix_mat(l.o, *x, x->mid, rows, wr_ld(l.o.k));
@@ -1005,7 +1014,7 @@ struct Step {
     {
         wr_route_args r{};
         r.logits = x->lat + off; r.ld = ld; r.bias = l.router_b; r.experts = l.experts; r.top = l.top;
-        r.tile = split() ? 0 : x->compute == WR_CUDA_BF16 ? kMoeTile : kMoeTileF32;
+        r.tile = split() ? 0 : x->compute == WR_CUDA_BF16 ? moe_tile(rw.n_rows, l.experts, l.top) : kMoeTileF32;
         r.weight = x->e_weight; r.expert = x->e_expert; r.place = x->e_place; r.row_of = x->e_row_of;
         r.list = x->e_list; r.count = x->e_count;
         return r;
@@ -1040,17 +1049,19 @@ struct Step {
             c.type = WR_ACT_F32;
             c.few = true;
         } else if (bf) {
-            TRY(wr_moe_gather_launch(ctx, x->xin, x->e_in, x->ldw, x->e_row_of, x->e_count, groups, kMoeTile));
+            TRY(wr_moe_gather_launch(ctx, x->xin, x->e_in, x->ldw, x->e_row_of, x->e_count, groups, r.tile));
+            gr.tile = r.tile;
+            gr.likely = rw.n_rows * l.top / r.tile + std::min(l.experts, rw.n_rows * l.top) / 2;
             wr_gemm_args a{};
-            a.m = groups * kMoeTile;
+            a.m = groups * r.tile;
             a.pair = l.e_up.pair; a.pair.out = x->e_act; a.pair.ld = lf;
             a.group = gr; a.group.stride = l.up_stride;
-            TRY(wr_gemm_launch(ctx, l.e_up.x_map, {l.e_up.w, l.e_up.n, l.e_up.k}, a));
+            TRY(wr_gemm_launch(ctx, l.e_up.x_map, {l.e_up.w, l.e_up.n, l.e_up.k, &l.e_up.w_maps}, a));
             wr_gemm_args b{};
-            b.m = groups * kMoeTile;
+            b.m = groups * r.tile;
             b.out = x->e_out; b.out_ld = x->ldw; b.out_type = WR_GEMM_OUT_BF16;
             b.group = gr; b.group.stride = l.down_stride;
-            TRY(wr_gemm_launch(ctx, l.e_down.x_map, {l.e_down.w, l.e_down.n, l.e_down.k}, b));
+            TRY(wr_gemm_launch(ctx, l.e_down.x_map, {l.e_down.w, l.e_down.n, l.e_down.k, &l.e_down.w_maps}, b));
             c.type = WR_ACT_BF16;
             ++m->launches;
         } else {
