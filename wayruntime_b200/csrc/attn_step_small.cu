@@ -96,6 +96,18 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
         cs_tab[tid] = cs;
         sn_tab[tid] = sn;
     }
+    // Short sessions: the K and V lines on their way into L2 (between two steps the weights have pushed them out): a hint, whatever
+    // is still being written.  (28 layers, 64 to 192 keys: 1030 -> 1023 us a step.  With more keys, and beside another stream's kernel,
+    // the hints cost more than they bring: 16 sessions of 200 to 2000 keys 2973 -> 3001.)
+    if constexpr (SETS == 1) {
+        __syncthreads();
+        for (uint32_t i = tid; i < pos * 4; i += kSmallThreads) {
+            const uint32_t key = i >> 2, which = (i >> 1) & 1u, line = i & 1u;
+            const char *at = s_page[key / kPageTokens] + wr_block_off(kvh, which, kHd) + line * (kPageTokens * 128u) +
+                             key % kPageTokens * 128u;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+        }
+    }
     pdl_wait();
     // ---- rows in
     const size_t q_at = ((size_t)s * p.n_q + (size_t)kvh * G) * kHd;

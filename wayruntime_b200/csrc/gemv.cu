@@ -96,6 +96,15 @@ __device__ __forceinline__ float finish(const GemvParams &p, uint32_t s, uint32_
     return y;
 }
 
+// ... the residual at hand
+__device__ __forceinline__ float finish(const GemvParams &p, uint32_t s, uint32_t n, float y, float resid)
+{
+    if (p.bias && s == 0) y = __fadd_rn(y, p.bias[n]);
+    if (p.act == WR_GEMV_ACT_SOFTPLUS) y = softplus(y);
+    y = __fmul_rn(y, p.mul);
+    return p.add ? __fadd_rn(resid, y) : y;
+}
+
 // weight rows of a CTA / warp: plain, or swiglu (first half gate rows, second half the same rows of up)
 template <int NR>
 __device__ __forceinline__ void weight_rows(const GemvParams &p, const GemvSeg &seg, uint32_t n0,
@@ -161,6 +170,13 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_splitk_kernel(const GemvPar
         }
     }
     pdl_wait();
+    // the residual that a finishing thread adds: on its way while the sums are worked out
+    constexpr int kOut = C * RG;
+    float resid = 0.f;
+    if (!p.swiglu && p.add && tid < kOut) {
+        const uint32_t n = n0 + tid / RG, row = r0 + tid % RG;
+        if (n < seg.n && row < p.rows) resid = p.add[(size_t)row * p.add_stride + n];
+    }
     auto step = [&](uint32_t v, const float4 (&w)[C]) {
         float4 nw = make_float4(1.f, 1.f, 1.f, 1.f);
         if (p.norm_w) nw = *reinterpret_cast<const float4 *>(p.norm_w + 4 * v);
@@ -216,7 +232,7 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_splitk_kernel(const GemvPar
                 const float u = __fmul_rn(red[(c + H) * RG + r], inv);
                 seg.out[(size_t)row * seg.out_stride + n] = silu_mul(y, u);
             } else {
-                seg.out[(size_t)row * seg.out_stride + n] = finish(p, s, n, row, y);
+                seg.out[(size_t)row * seg.out_stride + n] = finish(p, s, n, y, resid);
             }
         }
     }
