@@ -71,6 +71,8 @@ constexpr uint32_t kTmemS = 0;                   // S (then P) of block b at col
 constexpr uint32_t kTmemO = 256;                 // O of block b at columns 256 + 128*b
 constexpr float kRescaleLog2 = 8.0f;             // move the reference max when it is 2^8 behind
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr uint32_t kLeastPiece = 3, kMostParts = 16; // steps of a piece, pieces of a tile
+constexpr uint32_t kMergeTime = 1000;            // what pieces have to bring at least, in hundredths of a microsecond
 constexpr int kTileSlots = 4;                    // ring of published work tiles
 // Of every kPolyPeriod pairs of exponentials one pair is evaluated on the FMA pipe (0: none).
 #ifndef WR_PREFILL_POLY_PERIOD
@@ -125,14 +127,19 @@ struct prefill_params {
     uint32_t q_head, q_rot;                      // columns per head of the query rows; where the rotated ones start
     uint32_t k_head, v_at, v_head;               // columns per head of the K / V rows; where V starts
     uint32_t rot_block;                          // 64-wide block of a page where the rotated key part starts
-    uint32_t k_stages, v_stages, single; // single: work tiles of one block each
+    uint32_t k_stages, v_stages, single;         // single: work tiles of one block each
+    // The last tiles cut along the keys (not LATENT): work items n_whole on are `parts` pieces of tile n_whole, then of the next;
+    // n_tiles counts items.  What a piece leaves goes to part_rows (its tensor map: kv_map) and part_ml, [tile][piece][block][128 rows].
+    uint32_t n_whole, parts;
+    float2 *part_ml;             // reference maximum (log2) and sum
     uint32_t vdim, v_cols, out_ld;               // value size, rounded up to 16; row length of the output
     __nv_bfloat16 *out;
 };
 
 // A published work tile: up to two blocks over the same KV head.
 struct tile_info {
-    uint32_t valid, nblk, kvh, pad;
+    uint32_t valid, nblk, kvh;
+    uint32_t piece;              // 0: a whole tile; else 1 + its number among all pieces
     uint32_t head[2], qt[2];
 };
 
@@ -359,18 +366,26 @@ __host__ __device__ inline uint32_t prefill_tile_count(uint32_t n_qtiles, uint32
     if (n_qtiles & 1u) n += n_kv * ((group & 1u) + group / 2u);      // the first query tile on its own
     return n;
 }
-__host__ __device__ inline tile_info decode_tile(const prefill_params &p, uint32_t idx)
+// What tiles a launch has: blocks two by two, or by themselves in groups of one head (PLAIN); by themselves in any group (ONE); either
+// of these, whole or cut along the keys (CUT).  Every tile change waits for this arithmetic: with CUT's, tiles of one block took 1 us longer.
+enum { TILES_PLAIN, TILES_ONE, TILES_CUT };
+template <int TILES> __host__ __device__ inline tile_info decode_tile(const prefill_params &p, uint32_t idx)
 {
     tile_info t;
-    t.valid = 0; t.nblk = 0; t.kvh = 0; t.pad = 0;
+    t.valid = 0; t.nblk = 0; t.kvh = 0; t.piece = 0;
     t.head[0] = t.head[1] = 0; t.qt[0] = t.qt[1] = 0;
     if (idx >= p.n_tiles) return t;
     t.valid = 1;
+    if (TILES == TILES_CUT && p.parts && idx >= p.n_whole) {
+        t.piece = 1 + idx - p.n_whole;
+        idx = p.n_whole + (idx - p.n_whole) / p.parts;
+    }
     if (p.single) {
+        const uint32_t heads = TILES != TILES_PLAIN ? p.n_q : p.n_kv;
         t.nblk = 1;
-        t.head[0] = idx % p.n_q;
-        t.kvh = t.head[0] / p.group;
-        t.qt[0] = p.n_qtiles - 1 - idx / p.n_q;
+        t.kvh = t.head[0] = idx % heads;
+        if (TILES != TILES_PLAIN) t.kvh /= p.group;
+        t.qt[0] = p.n_qtiles - 1 - idx / heads;
         return t;
     }
     const uint32_t per = tiles_per_qpair(p.n_kv, p.group), pairs = p.group / 2u, odd = p.group & 1u;
@@ -413,8 +428,33 @@ __host__ __device__ __forceinline__ block_range range_of(const prefill_params &p
     return b;
 }
 
+// The steps of a tile's blocks, and of the tile: those of its piece, if it is one.  (A piece has two steps at least and the blocks'
+// ranges end at most one apart, so both blocks have steps in every piece.)
+struct tile_range {
+    block_range b0, b1;
+    uint32_t lo, hi;
+};
+template <int TILES> __host__ __device__ __forceinline__ tile_range ranges_of(const prefill_params &p, const tile_info &t)
+{
+    tile_range r;
+    r.b0 = range_of(p, t.qt[0]);
+    r.b1 = range_of(p, t.qt[t.nblk - 1]);
+    r.lo = r.b0.lo < r.b1.lo ? r.b0.lo : r.b1.lo;
+    r.hi = r.b0.hi > r.b1.hi ? r.b0.hi : r.b1.hi;
+    if (TILES == TILES_CUT && t.piece) {
+        const uint32_t part = (t.piece - 1) % p.parts, len = r.hi - r.lo, lo = r.lo + len * part / p.parts, hi = r.lo + len * (part + 1) / p.parts;
+        r.lo = lo;
+        r.hi = hi;
+        r.b0.lo = r.b0.lo > lo ? r.b0.lo : lo;
+        r.b1.lo = r.b1.lo > lo ? r.b1.lo : lo;
+        r.b0.hi = r.b0.hi < hi ? r.b0.hi : hi;
+        r.b1.hi = r.b1.hi < hi ? r.b1.hi : hi;
+    }
+    return r;
+}
+
 // When the CTAs would be done with p's tiles, in hundredths of a microsecond: a step (128 keys) of one block takes 1.87 us, of two
-// blocks 2.03 (they share the chain of scores, softmax and values), a tile that follows another 1.4 more.  Tiles are
+// blocks 2.03 (they share the chain of scores, softmax and values), a tile that follows another 2.2 more.  Tiles are
 // numbered longest first, so a CTA's second tile is as far from the middle as its first.
 inline uint32_t tiles_time(const prefill_params &p, uint32_t ctas)
 {
@@ -422,18 +462,31 @@ inline uint32_t tiles_time(const prefill_params &p, uint32_t ctas)
     for (uint32_t i = 0; i < ctas && i < p.n_tiles; ++i) {
         uint32_t t = 0;
         for (uint32_t round = 0; round * ctas < p.n_tiles; ++round) {
-            const tile_info ti = decode_tile(p, round * ctas + ((round & 1u) ? ctas - 1 - i : i));
+            const tile_info ti = decode_tile<TILES_CUT>(p, round * ctas + ((round & 1u) ? ctas - 1 - i : i));
             if (!ti.valid) continue;
-            const block_range a = range_of(p, ti.qt[0]), b = range_of(p, ti.qt[ti.nblk - 1]);
-            t += (std::max(a.hi, b.hi) - std::min(a.lo, b.lo)) * (ti.nblk > 1 ? 203u : 187u) + (round ? 140u : ti.nblk > 1 ? 145u : 0u);
+            const tile_range r = ranges_of<TILES_CUT>(p, ti);
+            t += (r.hi - r.lo) * (ti.nblk > 1 ? 203u : 187u) + (round ? 220u : ti.nblk > 1 ? 145u : 0u);
         }
         worst = std::max(worst, t);
     }
     return worst;
 }
-// Tiles of one block each instead of two: always where they all go round at once (us, two blocks / one: 100 rows of 32 heads
-// 11.1 / 9.3, 1000 rows of 16 heads 24.8 / 22.5), never where two blocks go round several times; in between the lengths decide
-// (513 rows of 32 heads 21.1 / 14.6; behind 6000 keys 1700 rows of 16 heads 129 / 147).  A block's arithmetic is the same.
+// The tiles that would be the CTAs' last round, cut along the keys into as many pieces as there are CTAs for them.
+inline void cut_last_tiles(prefill_params &p, uint32_t ctas)
+{
+    const uint32_t whole = p.n_tiles / ctas * ctas, rest = p.n_tiles - whole;
+    if (!rest || p.window) return;
+    const tile_range r = ranges_of<TILES_CUT>(p, decode_tile<TILES_CUT>(p, p.n_tiles - 1));    // the shortest
+    const uint32_t parts = std::min({ctas / rest, (r.hi - r.lo) / kLeastPiece, (uint32_t)kMostParts});
+    if (parts < 2) return;
+    p.n_whole = whole;
+    p.parts = parts;
+    p.n_tiles = whole + rest * parts;
+}
+// Tiles of one block each instead of two: always where they all go round at once (us with the append before it, two blocks / one:
+// 300 rows of 32 heads 19.8 / 18.6, 700 of 10 heads 23.6 / 21.5, 1000 of 16 heads 30.8 / 29.5), never where two blocks go round
+// several times; in between the lengths decide (513 rows of 32 heads 25.0 / 22.1, 1000 rows 31.8 / 31.6; behind 6000 keys 1600 rows
+// of 16 heads 128 / 192).  A block's arithmetic is the same.
 inline void tiles_of_one(prefill_params &p, uint32_t ctas)
 {
     const uint32_t singles = p.n_qtiles * p.n_q;
@@ -443,11 +496,22 @@ inline void tiles_of_one(prefill_params &p, uint32_t ctas)
     one.n_tiles = singles;
     if (singles <= ctas || tiles_time(one, ctas) < tiles_time(p, ctas)) p = one;
 }
+// ... with the last tiles cut along the keys where that is 10 us sooner or more (the merge takes 5 to 8), 20 us after whole tiles (they
+// end at different times, so whole last tiles start sooner than tiles_time says).  us with the append, whole / cut: 17 rows of 40
+// heads behind 6000 keys 97 / 44, 1000 rows 194 / 142, 700 rows of 8 heads on one kv head behind 1000 keys 34.3 / 26.9; 1999 rows of 40
+// heads behind 1000 keys 105.5 / 107.8 (24 tiles of 9 steps after two rounds: left whole).
+inline void tiles_in_pieces(prefill_params &p, uint32_t ctas)
+{
+    if (p.n_tiles > 4 * ctas) return;
+    prefill_params cut = p;
+    cut_last_tiles(cut, ctas);
+    if (cut.parts && tiles_time(cut, ctas) + (cut.n_whole ? 2 : 1) * kMergeTime < tiles_time(p, ctas)) p = cut;
+}
 
 // ---- the kernel ------------------------------------------------------------
 
 // (kv_map: LATENT's K and V rows; o_map: the other's output rows)
-template <bool LATENT>
+template <bool LATENT, int TILES>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
                     const __grid_constant__ CUtensorMap o_map, const prefill_params p)
@@ -545,9 +609,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         if (!p.early) pdl_wait();
         // The first tile's first loads (Q of block 0, the first K tile, Q of block 1) start
         // at once: they fly while TMEM is allocated and the other warps reach the barrier.
-        const tile_info ti = decode_tile(p, blockIdx.x);
-        const block_range r0 = range_of(p, ti.qt[0]), r1 = range_of(p, ti.qt[ti.nblk - 1]);
-        const uint32_t lo = min(r0.lo, r1.lo);
+        const tile_info ti = decode_tile<TILES>(p, blockIdx.x);
+        const uint32_t lo = ranges_of<TILES>(p, ti).lo;
         request_q(0, ti.head[0], ti.qt[0]);
         request_k(0, lo, ti.kvh);
         if (ti.nblk > 1) request_q(1, ti.head[1], ti.qt[1]);
@@ -565,10 +628,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     // Work tile number `it` of this CTA: the first one is the CTA's own number (every
     // role works it out for itself, nobody waits), later ones are published by the producer.
     auto tile_of = [&](uint32_t it, bool &ok) -> tile_info {
-        if (it == 0) return decode_tile(p, blockIdx.x);
+        if (it == 0) return decode_tile<TILES>(p, blockIdx.x);
         const uint32_t slot = it % kTileSlots;
         ok = mbar_wait(&sm.tile_ready[slot], ((it - 1) / kTileSlots) & 1, limit);
-        if (!ok) return decode_tile(p, p.n_tiles);                   // (invalid)
+        if (!ok) return decode_tile<TILES>(p, p.n_tiles);                   // (invalid)
         return sm.tile[slot];
     };
 
@@ -579,11 +642,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         if (lane == 0) {
             uint32_t kcount = 0;
             uint32_t q_loads[2] = {0, 0};                        // Q blocks requested per buffer
-            tile_info ti = decode_tile(p, blockIdx.x);
+            tile_info ti = decode_tile<TILES>(p, blockIdx.x);
             bool ok = true;
             for (uint32_t it = 0; ok && ti.valid; ++it) {
-                const block_range r0 = range_of(p, ti.qt[0]), r1 = range_of(p, ti.qt[ti.nblk - 1]);
-                const uint32_t lo = min(r0.lo, r1.lo), hi = max(r0.hi, r1.hi);
+                const tile_range tr = ranges_of<TILES>(p, ti);
+                const uint32_t lo = tr.lo, hi = tr.hi;
                 // (a block's buffer is free again when the block's last scores of the tile before have
                 // completed — block 0's come half a step before block 1's)
                 auto load_q = [&](uint32_t b, uint32_t head, uint32_t qt) -> bool {
@@ -629,7 +692,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                     pdl_wait();
                     next_tile = gridDim.x + (uint32_t)atomicAdd(p.sched, 1);
                 }
-                ti = decode_tile(p, next_tile);
+                ti = decode_tile<TILES>(p, next_tile);
                 const uint32_t slot = (it + 1) % kTileSlots;
                 sm.tile[slot] = ti;
                 mbar_arrive(&sm.tile_ready[slot]);               // (release: the tile is visible to the waiters)
@@ -645,8 +708,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             for (uint32_t it = 0; ok; ++it) {
                 const tile_info ti = tile_of(it, ok);
                 if (!ok || !ti.valid) break;
-                const block_range r0 = range_of(p, ti.qt[0]), r1 = range_of(p, ti.qt[ti.nblk - 1]);
-                const uint32_t lo = min(r0.lo, r1.lo), hi = max(r0.hi, r1.hi);
+                const tile_range tr = ranges_of<TILES>(p, ti);
+                const uint32_t lo = tr.lo, hi = tr.hi;
                 for (uint32_t j = lo; j < hi && ok; ++j, ++vcount) {
                     const uint32_t st = vcount % v_stages;
                     if (vcount >= v_stages) {
@@ -728,8 +791,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         for (uint32_t it = 0; ok; ++it) {
             const tile_info ti = tile_of(it, ok);
             if (!ok || !ti.valid) break;
-            const block_range rg0 = range_of(p, ti.qt[0]), rg1 = range_of(p, ti.qt[ti.nblk - 1]);
-            const uint32_t lo = min(rg0.lo, rg1.lo), hi = max(rg0.hi, rg1.hi);
+            const tile_range tr = ranges_of<TILES>(p, ti);
+            const block_range rg0 = tr.b0, rg1 = tr.b1;
+            const uint32_t lo = tr.lo, hi = tr.hi;
             const bool two = ti.nblk > 1;
             const uint32_t lo1 = two ? rg1.lo : hi, hi1 = two ? rg1.hi : hi;     // block 1's steps (none when absent)
             if (lane == 0) TLT(4, 1);                            // tile known
@@ -766,7 +830,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                         if (j == blo && o_uses > 0) good = mbar_wait(&sm.o_free[b], (o_uses - 1) & 1, limit);
                         const bool last = (j + 1 == bhi);
                         // steps of 16 keys; the last tile stops at the block's last key
-                        const uint32_t n_kk = last ? (key_end - j * kBN + 15u) / 16u : (uint32_t)(kBN / 16);
+                        const uint32_t n_kk = last ? (TILES == TILES_CUT ? min((key_end - j * kBN + 15u) / 16u, (uint32_t)(kBN / 16)) : (key_end - j * kBN + 15u) / 16u) : (uint32_t)(kBN / 16);
                         if (good) good = mbar_wait(&sm.p_full[b], p_uses & 1, limit);
                         ++p_uses;
                         if (!good) return false;
@@ -825,13 +889,13 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         for (uint32_t it = 0; ok; ++it) {
             const tile_info ti = tile_of(it, ok);
             if (!ok || !ti.valid) break;
-            const block_range rg0 = range_of(p, ti.qt[0]), rg1 = range_of(p, ti.qt[ti.nblk - 1]);
-            const uint32_t lo = min(rg0.lo, rg1.lo), hi = max(rg0.hi, rg1.hi);
+            const tile_range tr = ranges_of<TILES>(p, ti);
+            const uint32_t lo = tr.lo, hi = tr.hi;
             if (b >= ti.nblk) {                              // a lone block: this group sits the tile out
                 vc += hi - lo;
                 continue;
             }
-            const block_range me = (b == 0) ? rg0 : rg1;
+            const block_range me = (b == 0) ? tr.b0 : tr.b1;
             const uint32_t head = (b == 0) ? ti.head[0] : ti.head[1];
             TLST(1);                                             // tile known
             const uint32_t qpos = p.p0 + me.tok0 + row;      // absolute position of this query
@@ -1037,7 +1101,17 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                     }
                 }
             } else {
-                const float inv = (l > 0.f) ? 1.0f / l : 0.f;
+                float inv = (l > 0.f) ? 1.0f / l : 0.f;
+                uint32_t part_row = UINT32_MAX;
+                if constexpr (TILES == TILES_CUT) {                             // a piece leaves its sums as they are
+                    const uint32_t piece = p.parts ? tile_of(it, ok).piece : 0;      // (read again: no register kept)
+                    if (piece) {
+                        const uint32_t at = ((piece - 1) * 2 + b) * kBM;
+                        part_row = at + wq * 32u;
+                        inv = 1.0f;
+                        p.part_ml[at + row] = make_float2(m_ref, l);
+                    }
+                }
                 const bool send = (lane == 0) && (wq * 32u < me.rows);   // (a piece wholly past the prompt is not sent)
 #pragma unroll
                 for (int c = 0; c < kHd / 16; ++c) {
@@ -1051,7 +1125,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                                         o[16 * c + 4 * k + 3] * inv);
                     fence_proxy_async();                         // generic writes -> the TMA unit's reads
                     __syncwarp();
-                    if (send) tma_store_2d(&o_map, stage, (int)(head * kHd + 16 * c), (int)(me.tok0 + wq * 32u));
+                    if (TILES == TILES_CUT && send && part_row != UINT32_MAX) tma_store_2d(&kv_map, stage, 16 * c, (int)part_row);
+                    else if (send) tma_store_2d(&o_map, stage, (int)(head * kHd + 16 * c), (int)(me.tok0 + wq * 32u));
                 }
             }
             TLST(5);                                             // output rows issued
@@ -1078,6 +1153,34 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             __threadfence();
         }
     }
+}
+
+// The pieces of the tiles that were cut along the keys, put together in order: a warp per row, four values to a lane.
+constexpr uint32_t kMergeRows = 8;
+__global__ void __launch_bounds__(32 * kMergeRows) prefill_merge_kernel(const prefill_params p, const float *part_rows, float *out)
+{
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t lane = threadIdx.x & 31, at = blockIdx.x * kMergeRows + (threadIdx.x >> 5), row = at % kBM, b = at / kBM % 2;
+    const uint32_t tile = at / (2 * kBM);                        // among those that were cut
+    const tile_info ti = decode_tile<TILES_CUT>(p, p.n_whole + tile * p.parts);
+    if (!ti.valid || b >= ti.nblk) return;
+    const uint32_t tok = ti.qt[b] * kBM + row;
+    if (tok >= p.n) return;
+    float m = WR_NEG_SENTINEL, l = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t i = 0; i < p.parts; ++i) {
+        const size_t r = ((size_t)(tile * p.parts + i) * 2 + b) * kBM + row;
+        const float2 ml = p.part_ml[r];
+        const float4 v = reinterpret_cast<const float4 *>(part_rows + r * kHd)[lane];
+        if (ml.x == WR_NEG_SENTINEL) continue;                   // no key of this piece is visible to the row
+        const float top = fmaxf(m, ml.x), keep = m == WR_NEG_SENTINEL ? 0.f : ex2_approx(m - top), w = ex2_approx(ml.x - top);
+        l = fmaf(l, keep, ml.y * w);
+        o = make_float4(fmaf(o.x, keep, v.x * w), fmaf(o.y, keep, v.y * w), fmaf(o.z, keep, v.z * w), fmaf(o.w, keep, v.w * w));
+        m = top;
+    }
+    const float inv = l > 0.f ? 1.0f / l : 0.f;
+    reinterpret_cast<float4 *>(out + ((size_t)tok * p.n_q + ti.head[b]) * kHd)[lane] = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
 }
 
 // F32 -> F16 (round to nearest) copy of Q for callers that hold F32 queries.
@@ -1228,11 +1331,23 @@ extern "C" int wr_cuda_attn_prefill(wr_cuda_ctx *ctx, wr_cuda_kv *kv, uint32_t l
     p.n_qtiles = (n + kBM - 1) / kBM;
     p.n_tiles = prefill_tile_count(p.n_qtiles, p.n_kv, p.group);
     tiles_of_one(p, (uint32_t)ctx->sm_count);
+    CUtensorMap part_map = q_map;
+    if (ctx->prefill_parts) {
+        tiles_in_pieces(p, (uint32_t)ctx->sm_count);
+        const uint32_t rows = (uint32_t)ctx->sm_count * 2 * kBM;         // (no more pieces than CTAs)
+        const cuuint64_t p_dims[2] = {kHd, rows}, p_strides[1] = {kHd * 4};
+        p.part_ml = reinterpret_cast<float2 *>(ctx->prefill_parts + (size_t)rows * kHd);
+        if (p.parts && encode(&part_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void *)ctx->prefill_parts, p_dims, p_strides, o_box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return WR_CUDA_ERR_INTERNAL;
+    }
     const float scale = (scale_override > 0.0f) ? scale_override : 1.0f / sqrtf((float)kHd);   // kernels.c:1457-1459
     p.scale_log2 = scale * kLog2e;
     if (!(ctx->attr_flags & 2u)) {
-        WR_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kSmemBytes));
+        WR_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_kernel<false, TILES_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        WR_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_kernel<false, TILES_ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        WR_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_kernel<false, TILES_CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
         ctx->attr_flags |= 2u;
     }
     const uint32_t grid = std::min<uint32_t>(p.n_tiles, (uint32_t)ctx->sm_count);
@@ -1242,12 +1357,21 @@ extern "C" int wr_cuda_attn_prefill(wr_cuda_ctx *ctx, wr_cuda_kv *kv, uint32_t l
     const bool full = grid == (uint32_t)ctx->sm_count;
     p.early = (!convert && !host && full && ctx->pdl_index == ctx->launches &&
                ctx->pdl_kind == WR_PDL_PREFILL_FULL) ? 1u : 0u;
-    WR_CUDA_TRY(wr_launch_pdl(attn_prefill_kernel<false>, dim3(grid), dim3(kThreads), kSmemBytes, ctx->stream, q_map,
-                              q_map, o_map, p));
+    const auto kernel = p.parts ? attn_prefill_kernel<false, TILES_CUT> : p.single ? attn_prefill_kernel<false, TILES_ONE> : attn_prefill_kernel<false, TILES_PLAIN>;
+    WR_CUDA_TRY(wr_launch_pdl(kernel, dim3(grid), dim3(kThreads), kSmemBytes, ctx->stream, q_map, part_map, o_map, p));
     ctx->launches++;
     ctx->pdl_kind = full ? WR_PDL_PREFILL_FULL : WR_PDL_PREFILL_PART;
     ctx->pdl_index = ctx->launches;
     WR_CUDA_TRY(cudaGetLastError());
+    if (p.parts) {
+        const uint32_t rows = (p.n_tiles - p.n_whole) / p.parts * 2 * kBM;
+        WR_CUDA_TRY(wr_launch_pdl(prefill_merge_kernel, dim3(rows / kMergeRows), dim3(32 * kMergeRows), 0, ctx->stream, p,
+                                  (const float *)ctx->prefill_parts, dout));
+        ctx->launches++;
+        ctx->pdl_kind = WR_PDL_PREFILL_PART;             // (the append before the attention may still be running when this starts)
+        ctx->pdl_index = ctx->launches;
+        WR_CUDA_TRY(cudaGetLastError());
+    }
     if (host) {
         WR_CUDA_TRY(cudaMemcpyAsync(out, dout, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
         return wr_ctx_sync_checked(ctx);
@@ -1338,9 +1462,9 @@ int wr_latent_flash_launch(wr_cuda_ctx *ctx, const wr_latent_flash_args &a)
     p.v_cols = g.vdim_pad();
     p.out_ld = a.out_ld;
     p.out = static_cast<__nv_bfloat16 *>(a.out);
-    WR_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    WR_CUDA_TRY(cudaFuncSetAttribute(attn_prefill_kernel<true, TILES_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint32_t grid = std::min<uint32_t>(p.n_tiles, (uint32_t)ctx->sm_count);
-    WR_CUDA_TRY(wr_launch_pdl(attn_prefill_kernel<true>, dim3(grid), dim3(kThreads), (size_t)smem, ctx->stream, q_map, kv_map,
+    WR_CUDA_TRY(wr_launch_pdl(attn_prefill_kernel<true, TILES_PLAIN>, dim3(grid), dim3(kThreads), (size_t)smem, ctx->stream, q_map, kv_map,
                               q_map, p));
     ctx->launches++;
     WR_CUDA_TRY(cudaGetLastError());

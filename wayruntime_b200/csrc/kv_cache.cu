@@ -64,6 +64,11 @@ extern "C" int wr_cuda_ctx_create(int device, wr_cuda_ctx **out)
         wr_cuda_ctx_destroy(ctx);
         return rc;
     }
+    // Room for prompt attention in pieces (20 MB), for good: launches that a graph keeps may use it.  Without it tiles stay whole.
+    if (cudaMalloc((void **)&ctx->prefill_parts, (size_t)ctx->sm_count * 256 * (128 * sizeof(float) + sizeof(float2))) != cudaSuccess) {
+        (void)cudaGetLastError();
+        ctx->prefill_parts = nullptr;
+    }
     *out = ctx;
     return WR_CUDA_OK;
 }
@@ -78,6 +83,7 @@ extern "C" void wr_cuda_ctx_destroy(wr_cuda_ctx *ctx)
     if (ctx->ws) (void)cudaFree(ctx->ws);
     if (ctx->tickets) (void)cudaFree(ctx->tickets);
     if (ctx->prefill_sched) (void)cudaFree(ctx->prefill_sched);
+    if (ctx->prefill_parts) (void)cudaFree(ctx->prefill_parts);
     if (ctx->debug_buf) (void)cudaFree(ctx->debug_buf);
     if (ctx->host_err) (void)cudaFreeHost(ctx->host_err);       // (dev_err is its device-side alias)
     if (ctx->stage_dev) (void)cudaFree(ctx->stage_dev);

@@ -102,6 +102,7 @@ struct wr_cuda_ctx {
     int *tickets = nullptr;
     size_t ticket_count = 0;
     int *prefill_sched = nullptr;    // prefill kernel: next work tile, CTAs that have left
+    float *prefill_parts = nullptr;  // ... what the pieces of tiles leave: sm_count x 256 rows of 128 values, then (m, l) of each; or null
     void *debug_buf = nullptr;       // development builds only (kernel timelines)
     int *host_err = nullptr;         // error word: page-locked host memory, mapped into the device
     int *dev_err = nullptr;          // its device-side address (what kernels get)
