@@ -5,10 +5,12 @@
 // rows [0, p0+i] through wri_op_gqa_attention (src/core/kernels.c:1414-1527).
 // This kernel computes the same rows all at once as a dense contraction.
 //
-// Work is cut into BLOCKS of 128 query rows of one q head.  A CTA always holds
+// Work is cut into BLOCKS of 128 query rows of one q head.  A CTA usually holds
 // two blocks that read the same K/V tiles: two q heads of one GQA group over
 // the same 128 tokens, or — for the odd head of a group — the same head over
-// two consecutive 128-token ranges.  CTAs are persistent (one per SM): they
+// two consecutive 128-token ranges.  Where that would leave SMs idle a tile is
+// one block (tiles_of_one), and the last tiles are cut along the keys
+// (tiles_in_pieces; prefill_merge_kernel puts their sums together).  CTAs are persistent (one per SM): they
 // draw work tiles, longest first, from a counter in global memory, and the
 // next tile's queries and first scores are in flight while the previous
 // tile's output leaves.
@@ -39,7 +41,7 @@
 //     normalised, and sent out in pieces of 32 rows x 16 values through two swizzled
 //     shared-memory buffers as TMA tensor stores (a store instruction whose lanes each write a
 //     row of their own touches 32 cache lines for 512 bytes).
-// The kernel exists twice.  With LATENT = false it is what is described above, over a cache of head_dim 128.  With
+// The kernel has two forms.  With LATENT = false it is what is described above, over a cache of head_dim 128.  With
 // LATENT = true it serves layers whose heads share one cached latent row (wr_latent_flash_launch): every head has K
 // and V of its own, which a matrix product has written out for the step (rows of one buffer, loaded through a tensor
 // map), the key's rotated part is shared and comes from the cache's pages; sizes are arguments (query and key
