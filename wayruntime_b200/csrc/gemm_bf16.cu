@@ -2,22 +2,26 @@
 //
 // Persistent workers walk output tiles, m fastest so that the tiles in flight share weight rows in L2.  A worker is a
 // pair of CTAs (cta_group::2, tiles of 256 rows: each rank holds its 128 rows of activations and half of the tile's
-// weight rows) or one CTA (tiles of 128 rows: few rows, or row tiles with weights of their own).  Warp 0 feeds a ring of
-// shared-memory stages with TMA (64 K-values of both operands per stage: activations through a tensor map, weights as
-// linear copies out of blocks stored in the operand's layout; what lies beyond K arrives as zeros), warp 1 issues
-// tcgen05.mma into one of two TMEM accumulators (in a pair the even rank's; the odd rank's tells it of stages that have
-// arrived there), warps 2-9 read the other one back and write the finished rows (bias, softplus, residual; F32, BF16 or
-// saturated F16), so that a tile's output overlaps the next tile's products.  Columns may be gate / up pairs, of which the
-// activation leaves (wr_pair_args), row tiles may have weights of their own (wr_group_args), and activations may come from
-// a cache's pages.  Every wait is bounded by the context's wait limit; a warp that gives up records an error word and all
-// of them leave.
+// weight rows) or one CTA (tiles of 128 rows: few rows, or row tiles with weights of their own).  Warp 0 and the last warp
+// feed a ring of shared-memory stages with TMA, 64 K-values of both operands per stage: warp 0 the activations through a
+// tensor map (what lies beyond K arrives as zeros), the last warp the weights, copies out of blocks stored in the operand's
+// layout.  Warp 1 issues tcgen05.mma into one of two TMEM accumulators (in a pair the even rank's does; the odd rank's
+// copies count on the even rank's barriers), warps 2-9 read the other one back and write the finished rows (bias, softplus,
+// residual; F32, BF16 or saturated F16), so that a tile's output overlaps the next tile's products.  Columns may be gate /
+// up pairs, of which the activation leaves (wr_pair_args), row tiles may have weights of their own (wr_group_args), and
+// activations may come from a cache's pages.  Every wait is bounded by the context's wait limit; a warp that gives up
+// records an error word and all of them leave.
 //
 // What bounds it: the way of the operands from L2 into the SMs while tiles are narrow, the tensor cores' power on long runs.
 // Measured (us, one CTA per tile of 128 rows / pairs; rows x columns x K): 2048 x 8192 x 2048 68.8 / 49.1, 2048 x 2048 x 6144
-// with a residual 62.8 / 39.2 (cuBLAS without one: 52 and 37).  What the pair is made of: a pair reads two thirds of the
-// operands; a linear copy costs its thread about 50 ns to issue, so weights lie K-block by K-block and a stage's rows are one
-// copy (with one per 64 rows 61); the odd rank's copies count on the even rank's barrier (a warp that relayed them: 70 against
-// 61); eight warps bring a tile's last results out through shared memory in 7 us instead of four in 18.
+// with a residual 62.8 / 39.2 (cuBLAS without one: 52 and 37).  What the pair is made of:
+// - It reads two thirds of the operands.
+// - A linear copy costs its thread about 50 ns to issue, so weights lie K-block by K-block and a stage's rows are one copy
+//   (with one per 64 rows 61).
+// - The odd rank's copies count on the even rank's barrier (a warp that relayed them: 70 against 61).
+// - Eight warps bring a tile's last results out through shared memory in 7 us, four without it took 18.
+// - Weights have a warp of their own, which does not wait for the kernel ahead: a prompt of 2048 rows, 8 layers of width
+//   2048, 2614 -> 2597 us, one of 1501 rows, 4 layers with experts, 1300 -> 1286.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -30,7 +34,7 @@ namespace {
 constexpr uint32_t kBM = 128, kBK = 64;                  // rows of one CTA, K-values of a stage
 constexpr uint32_t kMaxN = 256;                          // columns of a tile, and of one accumulator of two
 constexpr uint32_t kMapRows = 32;                        // a pair's rank takes a multiple of these of a tile's weight rows
-constexpr uint32_t kOutWarps = 8, kThreads = 64 + 32 * kOutWarps;
+constexpr uint32_t kOutWarps = 8, kWeightWarp = 2 + kOutWarps, kThreads = 32 * (kWeightWarp + 1);
 constexpr uint32_t kABytes = kBM * kBK * 2, kRowBytes = kBK * 2;
 constexpr uint32_t kMaxStages = 8, kStageBudget = 196608;
 constexpr uint32_t kOutBytes = 4096;                     // a warp's 32 x 32 results on their way out
@@ -214,11 +218,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
     else __syncthreads();
     tc5::fence_after();
     const uint32_t tmem = tmem_slot;
-    pdl_wait();
+    if (warp != kWeightWarp || p.a.group.list) pdl_wait();       // (weights depend on nothing)
     const uint32_t m_tiles = p.a.group.list ? *p.a.group.count : p.m_tiles, tiles = m_tiles * p.n_tiles;
 
-    if (warp == 0) {
+    if (warp == 0 || warp == kWeightWarp) {
         if (lane == 0) {
+            const bool weights = warp != 0;
             const uint32_t w_rows = wr_weight_blocks(p.w.n) * kWBlock;
             uint32_t it = 0, st = 0, phase = 0;          // stage it % stages, round it / stages
             bool ok = true;
@@ -244,12 +249,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
                         break;
                     }
                     uint8_t *a = stages + st * p.stage_bytes, *b = a + kABytes;
-                    if (rank == 0) mbar_expect_tx(&full[st], bytes);
-                    if (PAIR) {
-                        tc5::tma_load_2d_pair(a, &x_map, (int)(kb * kBK), (int)m0, &full[st]);
-                        tc5::tma_load_2d_pair(b, w_map, 0, (int)(kb * w_rows + y0), &full[st]);
+                    // (a stage's bytes may come before they are expected: its barrier still waits for warp 0)
+                    if (weights) {
+                        if (PAIR) tc5::tma_load_2d_pair(b, w_map, 0, (int)(kb * w_rows + y0), &full[st]);
+                        else if (rows) bulk_g2s(b, blocks + wr_weight_row(p.w.n, r0, kb), rows * kRowBytes, &full[st]);
                     } else {
-                        if (p.a.pages) {
+                        if (rank == 0) mbar_expect_tx(&full[st], bytes);
+                        if (PAIR) {
+                            tc5::tma_load_2d_pair(a, &x_map, (int)(kb * kBK), (int)m0, &full[st]);
+                        } else if (p.a.pages) {
                             for (uint32_t i = 0; i < np; ++i)
                                 bulk_g2s(a + i * kABytes / 2,
                                          reinterpret_cast<const char *>(p.a.pages[m0 / kPageTokens + i]) + kb * kABytes / 2, kABytes / 2,
@@ -257,7 +265,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
                         } else {
                             tc5::tma_load_2d(a, &x_map, (int)(kb * kBK), (int)m0, &full[st]);
                         }
-                        if (rows) bulk_g2s(b, blocks + wr_weight_row(p.w.n, r0, kb), rows * kRowBytes, &full[st]);
                     }
                     ++it;
                     if (++st == p.stages) {
@@ -315,7 +322,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
             }
         }
         if (!ok && lane == 0) atomicCAS(p.err, 0, 42);
-    } else if (warp >= 2) {
+    } else if (warp >= 2) {                              // (not the weights' warp, see above)
         const uint32_t quarter = warp & 3, half = (warp - 2) >> 2;       // TMEM lanes this warp may read; its pieces of 32 columns
         uint8_t *buf = stages + kStageBudget + (warp - 2) * kOutBytes;
         uint32_t n_tile = 0;
@@ -409,8 +416,9 @@ struct Plan {
     uint32_t wide = 0, bn0 = kMaxN, bn1 = kMaxN;
 };
 
-// A worker's clocks per 64 K-values of a tile: the products, or the operands on their way out of L2.  A pair's 128 + bn / 2 rows
-// per rank take less than the issue of three copies (350 clocks, whatever bn); a CTA by itself gets about 100 bytes a clock.
+// A worker's clocks per 64 K-values of a tile: the products, or the operands on their way out of L2.  A pair takes 350 clocks
+// or more, however narrow its tile (with 180 or 230 here narrower tiles are chosen: a prompt of 1501 rows with experts 1284 us
+// -> 1295); a CTA by itself gets about 100 bytes a clock.
 uint64_t tile_cost(uint32_t ranks, uint32_t bn) { return std::max(2u * bn, ranks == 2 ? 350u : 150u + (kBM + bn) * 5u / 4u) + 24u; }
 
 // The cut of n columns into tiles that the workers finish first: tiles of 256 columns, and behind them (so that the last
