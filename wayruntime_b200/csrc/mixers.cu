@@ -411,12 +411,14 @@ __global__ void __launch_bounds__(kPolyThreads) polynorm_kernel(const wr_polynor
 
 // The same for a BF16 prompt's rows of up to 2048 NV values: a thread keeps its values, and eight blocks share an SM, so that the
 // rows' loads, sums and stores overlap (2048 rows of 6144: 18.8 -> 13.9 us; 512 threads that read their values twice, four blocks
-// to an SM, spent most of it waiting for each other).
+// to an SM, spent most of it waiting for each other).  Sums are those of the kernel above, bit for bit: a thread stands for threads t
+// and t + 256 of its 512 (values u = 0, 2, .. and 1, 3, ..), a warp for two of its sixteen.
 constexpr uint32_t kPolyRowThreads = 256;
 template <int NV>
 __global__ void __launch_bounds__(kPolyRowThreads) polynorm_rows_kernel(const wr_polynorm_args a)
 {
-    __shared__ float red[3][kPolyRowThreads / 32];
+    __shared__ float red[3][kPolyWarps];
+    static_assert(2 * kPolyRowThreads == kPolyThreads, "a thread's values are those of two threads above");
     pdl_trigger();
     pdl_wait();
     const uint32_t ld = wr_ld(a.ff), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -436,7 +438,8 @@ __global__ void __launch_bounds__(kPolyRowThreads) polynorm_rows_kernel(const wr
             v[2 * e + 1] = i + 2 * e + 1 < a.ff ? __uint_as_float(w[e] & 0xffff0000u) : 0.f;
         }
     };
-    float s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    constexpr int kSums = NV > 1 ? 2 : 1;
+    float s[3][2] = {};
 #pragma unroll
     for (int u = 0; u < NV; ++u) {
         float v[8];
@@ -444,22 +447,29 @@ __global__ void __launch_bounds__(kPolyRowThreads) polynorm_rows_kernel(const wr
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const float v2 = v[e] * v[e], v3 = v2 * v[e];
-            s1 = fmaf(v[e], v[e], s1);
-            s2 = fmaf(v2, v2, s2);
-            s3 = fmaf(v3, v3, s3);
+            s[0][u & 1] = fmaf(v[e], v[e], s[0][u & 1]);
+            s[1][u & 1] = fmaf(v2, v2, s[1][u & 1]);
+            s[2][u & 1] = fmaf(v3, v3, s[2][u & 1]);
         }
     }
-    s1 = warp_sum(s1);
-    s2 = warp_sum(s2);
-    s3 = warp_sum(s3);
-    if (lane == 0) { red[0][warp] = s1; red[1][warp] = s2; red[2][warp] = s3; }
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+#pragma unroll
+        for (int h = 0; h < kSums; ++h) s[p][h] = warp_sum(s[p][h]);
+    if (lane == 0) {
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            red[p][warp] = s[p][0];
+            red[p][warp + kPolyWarps / 2] = s[p][1];     // (zeros where NV is 1)
+        }
+    }
     __syncthreads();
     float k[3];
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
         float t = 0.f;
 #pragma unroll
-        for (uint32_t w = 0; w < kPolyRowThreads / 32; ++w) t += red[p][w];
+        for (uint32_t w = 0; w < kPolyWarps; ++w) t += red[p][w];
         k[p] = 1.0f / sqrtf(t / (float)a.ff + a.eps);
     }
     const float ka = a.a * k[0], kb = a.b * k[1], kc = a.c * k[2];
