@@ -1,5 +1,5 @@
-"""GPU: selective scan in pieces where the whole chain would have two states per thread, around the length from which portions are cut,
-against the float64 restatement.  Tolerances as for the mixer alone (test_gpu_tumadra.py)."""
+"""GPU: selective scan of portions of some hundred tokens that are not cut into pieces: two states per thread, one state per thread,
+and portions that go on from a state, against the float64 restatement.  Tolerances as for the mixer alone (test_gpu_tumadra.py)."""
 import numpy as np
 import pytest
 

@@ -630,6 +630,19 @@ template <int NS> struct States {
         unpack2(t, x, y);
         return x + y;
     }
+    // ... four states at a time, as threads of four states each would add them up
+    __device__ __forceinline__ float dot_by_fours(const States &c) const
+    {
+        static_assert(P == 2 || P == 4, "two fours at most");
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < P; j += 2) {
+            float x, y;
+            unpack2(fma2(v[j + 1], c.v[j + 1], mul2(v[j], c.v[j])), x, y);
+            sum = j == 0 ? x + y : sum + (x + y);
+        }
+        return sum;
+    }
     __device__ __forceinline__ void set(int j, float f)
     {
         float x, y;
@@ -659,14 +672,15 @@ template <> struct States<1> {
 //
 // A sequence is one chain, and with one state per thread the instructions around a state's four (addresses, loads, the sums'
 // exchange) are most of the work.  A long portion is therefore cut into pieces of kScanPiece tokens, which gives enough threads
-// for eight states each: SCAN_ENDS works out what every piece but the last leaves of nothing, and the sum of its step
+// for several states each (four in the first pass, eight in the second): SCAN_ENDS works out what every piece but the last leaves of nothing, and the sum of its step
 // sizes; SCAN_PIECE starts every piece from the state before the portion, brought forward over the pieces before it
 // (2^(a2 * their step sizes) times it, plus what they left).  The decays are worked out twice.
-// 2048 tokens x 4096 channels x 16 states: a chain 147 us; pieces of 256 tokens with four states per thread 45 + 86.  A prompt of
-// 2048 tokens through two such layers and two of attention, us by states per thread and tokens per piece: 4, 256 1507   4, 128 1466
-// 8, 256 1476   8, 128 1431   8, 64 1453   16, 128 1480.  What is left is latency: the exponentials alone would take some 60 us.
+// 2048 tokens x 4096 channels x 16 states: a chain 147 us; with four states per thread in both passes 45 + 86.  A prompt of 2048
+// tokens through eight layers, four of them such scans, us by states per thread in the first and the second pass: 4, 4 2696
+// 8, 4 2722   8, 8 2636   4, 8 2619.  All four give the same bits: a thread of eight adds its sums up as two threads of four do.
+// (Pieces of 128 tokens take 80 us less and give other ones.)  What is left is latency: the exponentials alone would take some 60 us.
 enum { SCAN_WHOLE = 0, SCAN_ENDS = 1, SCAN_PIECE = 2 };
-constexpr uint32_t kScanPiece = 128;
+constexpr uint32_t kScanPiece = 256;
 
 template <typename T, typename TO, int NS, int LG, int MODE>
 __global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, const wr_scan_args a, float *ends, float *steps)
@@ -764,7 +778,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const wr_rows rw, co
         float y[U];
         auto chain = [&](const Group &g, int i, int u) {
             S.advance(g.e[i], g.b[i]);
-            if (MODE != SCAN_ENDS) y[u] = S.dot(g.c[i]);
+            if constexpr (MODE == SCAN_PIECE) y[u] = S.dot_by_fours(g.c[i]);
+            else if (MODE == SCAN_WHOLE) y[u] = S.dot(g.c[i]);
         };
         // the channel's threads exchange their parts of U tokens' sums and finish some tokens each
         auto finish = [&](uint32_t tb) {
@@ -935,40 +950,41 @@ int scan_one(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a, uint32_
     return finish_launch(ctx);
 }
 
-template <typename T, typename TO, int NS, int LG> int scan_pieces(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a)
+// LG: log2 of the threads that share a channel in the second pass, eight states each (four in the first)
+template <typename T, typename TO, int LG> int scan_pieces(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a)
 {
     const uint32_t pieces = (rw.n_rows + kScanPiece - 1) / kScanPiece;
     const int rc = wr_ctx_try_ws(ctx, wr_scan_ws_bytes(rw.n_rows, a.inner, a.state));
     if (rc != WR_CUDA_OK) return rc;
-    float *ends = ctx->ws, *steps = ends + (size_t)(pieces - 1) * wr_ld(a.inner) * ((uint32_t)NS << LG);
-    const int first = scan_one<T, TO, NS, LG, SCAN_ENDS>(ctx, rw, a, pieces - 1, ends, steps);
-    return first != WR_CUDA_OK ? first : scan_one<T, TO, NS, LG, SCAN_PIECE>(ctx, rw, a, pieces, ends, steps);
+    float *ends = ctx->ws, *steps = ends + (size_t)(pieces - 1) * wr_ld(a.inner) * (8u << LG);
+    const int first = scan_one<T, TO, 4, LG + 1, SCAN_ENDS>(ctx, rw, a, pieces - 1, ends, steps);
+    return first != WR_CUDA_OK ? first : scan_one<T, TO, 8, LG, SCAN_PIECE>(ctx, rw, a, pieces, ends, steps);
 }
 
 // One state per thread while that is what it takes to fill the device, two above.
 inline bool scan_few(uint32_t inner, uint32_t state) { return (uint64_t)inner * state < 131072; }
 
-// The line to pieces: where what eight states per thread save outweighs the second pass over the decays.  A prompt through four
-// layers (two of them scans), us whole / in pieces:
-//     2048 channels of 16   300 tokens 500 / 533   400  544 / 520   513  602 / 585   769  775 / 621   2048 1669 / 924
-//     4096 channels of 16   300 tokens 694 / 700   400  740 / 728   513  837 / 810   769 1020 / 905   2048 2082 / 1431
-//     8192 channels of 16   300 tokens 1115 / 1147 400 1229 / 1237  513 1366 / 1352  769 1707 / 1688  2048 3533 / 3477
-//     2048 channels of 16, F32 rows                400 1424 / 1435  513 1732 / 1751  769 2342 / 2295
-// (8192 channels of 32 states lost with pieces of four states per thread: 2048 tokens 3585 / 3933.)
+// The line to pieces: where what several states per thread save outweighs the second pass over the decays: where the whole chain has
+// one state per thread, from four pieces on.  A prompt through four layers (two of them scans), us whole / in pieces:
+//     2048 channels of 16   513 tokens 594 / 633   640  638 / 656   700  671 / 669   769  711 / 671   1024  804 / 705   2048 1300 /  971
+//     4096 channels of 16   513 tokens 806 / 838   640  851 / 851   700  882 / 864   769  959 / 940   1024 1072 / 994   2048 1737 / 1433
+//     2048 channels of 16, F32 rows                640 1957 / 1992                   769 2296 / 2321  1024 2882 / 2885
+// and with two states per thread, in pieces of four states  8192 channels of 16  1300 tokens 2462 / 2444  2048 3285 / 3209;  of 32
+// 1281 2638 / 2920  2048 3585 / 3933.
 // A portion's states are therefore summed in one order or another by its length (not by what else is in the step or in memory: the model
 // takes the workspace when it is created): portions of other lengths agree to rounding.  Error of a layer of 512 channels against
 // float64, 2000 tokens at once / as four portions of one chain each: 8.5e-7 / 1.0e-6 in F32, the same in BF16.
 inline bool scan_in_pieces(uint32_t rows, uint32_t inner, uint32_t state)
 {
-    return state > 4 && (state <= 16 || (state <= 32 && scan_few(inner, state))) && rows > 5 * kScanPiece;
+    return state > 4 && state <= 32 && scan_few(inner, state) && rows > 3 * kScanPiece;
 }
 
 template <typename T, typename TO> int scan_launch(wr_cuda_ctx *ctx, const wr_rows &rw, const wr_scan_args &a)
 {
     if (!rw.decode && rw.n_seq == 1 && scan_in_pieces(rw.n_rows, a.inner, a.state)) {
-        const int rc = a.state <= 8    ? scan_pieces<T, TO, 8, 0>(ctx, rw, a)
-                       : a.state <= 16 ? scan_pieces<T, TO, 8, 1>(ctx, rw, a)
-                                       : scan_pieces<T, TO, 8, 2>(ctx, rw, a);
+        const int rc = a.state <= 8    ? scan_pieces<T, TO, 0>(ctx, rw, a)
+                       : a.state <= 16 ? scan_pieces<T, TO, 1>(ctx, rw, a)
+                                       : scan_pieces<T, TO, 2>(ctx, rw, a);
         if (rc != WR_CUDA_ERR_NOMEM) return rc;
     }
     const bool few = scan_few(a.inner, a.state);
