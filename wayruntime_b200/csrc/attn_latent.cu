@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const Latent
         bool ok = true;
         for (uint32_t i = blockIdx.x; i < p.items && ok; i += gridDim.x, ++n_item) {
             const Item it = item_of(p, i);
-            ok = mbar_wait(&sm.q_full, n_item & 1, p.wait_limit);
+            ok = mbar_wait_warp(&sm.q_full, n_item & 1, p.wait_limit);
             if (!ok) break;
             for (uint32_t t = 0; t < it.tiles && ok; ++t, ++n_tile) {
                 // S^T, box by box as they arrive
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const Latent
                 };
                 for (uint32_t u = 0; u < p.units && ok; ++u) {
                     const uint32_t j = n_unit + u, st = j % p.ring;
-                    ok = mbar_wait(&sm.full[st], (j / p.ring) & 1, p.wait_limit);
+                    ok = mbar_wait_warp(&sm.full[st], (j / p.ring) & 1, p.wait_limit);
                     if (!ok) break;
                     tc5::fence_after();
                     score(smem_u32(units + st * kUnit));
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const Latent
                 }
                 for (uint32_t r = 0; r < p.rot_boxes && ok; ++r, ++n_rot) {
                     const uint32_t st = n_rot % p.rot_ring;
-                    ok = mbar_wait(&sm.rot_full[st], (n_rot / p.rot_ring) & 1, p.wait_limit);
+                    ok = mbar_wait_warp(&sm.rot_full[st], (n_rot / p.rot_ring) & 1, p.wait_limit);
                     if (!ok) break;
                     tc5::fence_after();
                     score(smem_u32(rots + st * kBox));
@@ -247,9 +247,9 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const Latent
                     if (t + 1 == it.tiles) tc5::commit(&sm.q_empty);
                     tc5::commit(&sm.s_full);
                 }
-                ok = mbar_wait(&sm.p_full, n_tile & 1, p.wait_limit);
+                ok = mbar_wait_warp(&sm.p_full, n_tile & 1, p.wait_limit);
                 // the item's first product overwrites O: the one before must have left TMEM
-                if (ok && t == 0 && n_item > 0) ok = mbar_wait(&sm.o_free, (n_item - 1) & 1, p.wait_limit);
+                if (ok && t == 0 && n_item > 0) ok = mbar_wait_warp(&sm.o_free, (n_item - 1) & 1, p.wait_limit);
                 if (!ok) break;
                 tc5::fence_after();
                 // O^T: 128 latents of a unit at a time, 16 keys a step
@@ -283,8 +283,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const Latent
                 l[h] = 0.f;
             }
             for (uint32_t t = 0; t < it.tiles; ++t, ++n_tile, ++n_red) {
-                if (ok) ok = mbar_wait(&sm.s_full, n_tile & 1, p.wait_limit);    // (the tile before has been multiplied: P is quiet)
-                ok = __all_sync(0xffffffffu, ok);
+                if (ok) ok = mbar_wait_warp(&sm.s_full, n_tile & 1, p.wait_limit);       // (the tile before has been multiplied: P is quiet)
                 tc5::fence_after();
                 float v[32];
                 tc5::ld32(tmem_s + lanes, v);
@@ -337,8 +336,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const Latent
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.p_full);
             }
-            if (ok) ok = mbar_wait(&sm.o_full, n_item & 1, p.wait_limit);
-            ok = __all_sync(0xffffffffu, ok);
+            if (ok) ok = mbar_wait_warp(&sm.o_full, n_item & 1, p.wait_limit);
             tc5::fence_after();
             const size_t at = ((size_t)it.row * p.heads + head0) * p.chunks + it.chunk, stride = (size_t)p.chunks * p.rank_pad;
             float *out = p.o + at * p.rank_pad;

@@ -631,8 +631,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     // role works it out for itself, nobody waits), later ones are published by the producer.
     auto tile_of = [&](uint32_t it, bool &ok) -> tile_info {
         if (it == 0) return decode_tile<TILES>(p, blockIdx.x);
-        const uint32_t slot = it % kTileSlots;
-        ok = mbar_wait(&sm.tile_ready[slot], ((it - 1) / kTileSlots) & 1, limit);
+        const uint32_t slot = it % kTileSlots, parity = ((it - 1) / kTileSlots) & 1;
+        ok = warp == 8 ? mbar_wait(&sm.tile_ready[slot], parity, limit) : mbar_wait_warp(&sm.tile_ready[slot], parity, limit);    // (one lane / all)
         if (!ok) return decode_tile<TILES>(p, p.n_tiles);                   // (invalid)
         return sm.tile[slot];
     };
@@ -801,14 +801,14 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             if (lane == 0) TLT(4, 1);                            // tile known
 
             // first scores of the tile
-            ok = mbar_wait(&sm.k_full[k_st], k_par, limit);
-            if (ok && lo >= rg0.lo && lo < rg0.hi) ok = mbar_wait(&sm.q_full[0], (q_uses0++) & 1, limit);
+            ok = mbar_wait_warp(&sm.k_full[k_st], k_par, limit);
+            if (ok && lo >= rg0.lo && lo < rg0.hi) ok = mbar_wait_warp(&sm.q_full[0], (q_uses0++) & 1, limit);
             if (!ok) break;
             tc_fence_after();
             if (lo >= rg0.lo && lo < rg0.hi) issue_s(0, k_st);
             if (lead && rg0.hi == lo + 1) umma_commit(&sm.q_free[0]);        // block 0's Q is no longer read
             if (two) {
-                ok = mbar_wait(&sm.q_full[1], (q_uses1++) & 1, limit);
+                ok = mbar_wait_warp(&sm.q_full[1], (q_uses1++) & 1, limit);
                 if (!ok) break;
                 tc_fence_after();
                 if (lo >= lo1 && lo < hi1) issue_s(1, k_st);
@@ -820,8 +820,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             for (uint32_t j = lo; j < hi && ok; ++j) {
                 const bool more = j + 1 < hi;
                 // this step's V tile and the next step's K tile landed long ago
-                ok = mbar_wait(&sm.v_full[v_st], v_par, limit);
-                if (!LATENT && ok && more) ok = mbar_wait(&sm.k_full[k_st], k_par, limit);
+                ok = mbar_wait_warp(&sm.v_full[v_st], v_par, limit);
+                if (!LATENT && ok && more) ok = mbar_wait_warp(&sm.k_full[k_st], k_par, limit);
                 if (!ok) break;
                 // one block: wait for its P, issue its P.V, then its next scores
                 auto step_block = [&](uint32_t b, uint32_t blo, uint32_t bhi, uint32_t key_end, uint32_t &p_uses,
@@ -829,11 +829,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                     if (j >= blo && j < bhi) {
                         bool good = true;
                         // the first P.V of a tile overwrites O: the previous tile's rows must have left TMEM
-                        if (j == blo && o_uses > 0) good = mbar_wait(&sm.o_free[b], (o_uses - 1) & 1, limit);
+                        if (j == blo && o_uses > 0) good = mbar_wait_warp(&sm.o_free[b], (o_uses - 1) & 1, limit);
                         const bool last = (j + 1 == bhi);
                         // steps of 16 keys; the last tile stops at the block's last key
                         const uint32_t n_kk = last ? (TILES == TILES_CUT ? min((key_end - j * kBN + 15u) / 16u, (uint32_t)(kBN / 16)) : (key_end - j * kBN + 15u) / 16u) : (uint32_t)(kBN / 16);
-                        if (good) good = mbar_wait(&sm.p_full[b], p_uses & 1, limit);
+                        if (good) good = mbar_wait_warp(&sm.p_full[b], p_uses & 1, limit);
                         ++p_uses;
                         if (!good) return false;
                         if (lane == 0) TL(2);                    // P seen
@@ -846,7 +846,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                     }
                     if (more && j + 1 >= blo && j + 1 < bhi) {
                         if (LATENT) {                            // (its K ring may be one stage deep)
-                            if (!mbar_wait(&sm.k_full[k_st], k_par, limit)) return false;
+                            if (!mbar_wait_warp(&sm.k_full[k_st], k_par, limit)) return false;
                             tc_fence_after();
                         }
                         issue_s(b, k_st);                        // (P_b of step j was consumed just above)
@@ -906,7 +906,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             float m_ref = WR_NEG_SENTINEL;                   // reference max, log2 domain
             float l = 0.f;
             for (uint32_t j = me.lo; j < me.hi && ok; ++j) {
-                ok = mbar_wait(&sm.s_full[b], s_uses & 1, limit);
+                ok = mbar_wait_warp(&sm.s_full[b], s_uses & 1, limit);
                 ++s_uses;
                 if (!ok) break;
                 TLS();                                           // 0: scores ready
@@ -1010,7 +1010,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                     // tile so that 0 * garbage cannot make a NaN (both groups do it
                     // before releasing their own P.V; the writes are equal).
                     const uint32_t vn = vc + (j - lo), vst = vn % v_stages;
-                    ok = mbar_wait(&sm.v_full[vst], (vn / v_stages) & 1, limit);
+                    ok = mbar_wait_warp(&sm.v_full[vst], (vn / v_stages) & 1, limit);
                     if (!ok) break;
                     const uint32_t first_bad = p.p0 + p.n - key0;
                     if (row >= first_bad) {
@@ -1035,7 +1035,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             vc += hi - lo;
             if (!ok) break;
             // ---- the tile's last P.V has completed: O leaves TMEM, normalised
-            ok = mbar_wait(&sm.o_done[b], o_uses & 1, limit);
+            ok = mbar_wait_warp(&sm.o_done[b], o_uses & 1, limit);
             ++o_uses;
             if (!ok) break;
             tc_fence_after();

@@ -288,13 +288,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
             const uint32_t bn = tile_at(p, m_tiles, tile).bn;
             const uint32_t idesc = p.a.pages ? tc5::idesc_f16(kRanks * kBM, bn) : tc5::idesc_bf16(kRanks * kBM, bn);
             const uint32_t acc = n_tile & 1;
-            if (n_tile >= 2 && !mbar_wait(&acc_empty[acc], (n_tile / 2 - 1) & 1, p.wait_limit)) {
+            if (n_tile >= 2 && !mbar_wait_warp(&acc_empty[acc], (n_tile / 2 - 1) & 1, p.wait_limit)) {
                 ok = false;
                 break;
             }
             tc5::fence_after();
             for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
-                if (!mbar_wait(&full[st], phase, p.wait_limit)) {
+                if (!mbar_wait_warp(&full[st], phase, p.wait_limit)) {
                     ok = false;
                     break;
                 }
@@ -334,11 +334,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
             float4 r[8];
 #pragma unroll
             for (uint32_t i = 0; i < 8; ++i) fetch_add(p, row0, t.n0 + half * 32, lane, i, r[i]);
-            if (!mbar_wait(&acc_full[acc], (n_tile / 2) & 1, p.wait_limit)) {
+            if (!mbar_wait_warp(&acc_full[acc], (n_tile / 2) & 1, p.wait_limit)) {
                 ok = false;
                 break;
             }
-            __syncwarp();
             tc5::fence_after();
 #pragma unroll 1
             for (uint32_t c0 = half * 32; c0 < end; c0 += 64) {

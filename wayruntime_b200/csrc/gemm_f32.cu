@@ -185,13 +185,13 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
         for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x, ++turn) {
             const uint32_t k_lo = unit / tiles * p.part_blocks, k_hi = min(k_lo + p.part_blocks, p.k_blocks);
             const uint32_t acc = turn % T::kAccs, d = tmem + acc * kDiags * BN;
-            if (turn >= T::kAccs && !mbar_wait(&acc_empty[acc], (turn / T::kAccs - 1) & 1, p.wait_limit)) {
+            if (turn >= T::kAccs && !mbar_wait_warp(&acc_empty[acc], (turn / T::kAccs - 1) & 1, p.wait_limit)) {
                 ok = false;
                 break;
             }
             for (uint32_t kb = k_lo; kb < k_hi; ++kb, ++it) {
                 const uint32_t st = it % T::kStages;
-                if (!mbar_wait(&full[st], (it / T::kStages) & 1, p.wait_limit)) {
+                if (!mbar_wait_warp(&full[st], (it / T::kStages) & 1, p.wait_limit)) {
                     ok = false;
                     break;
                 }
@@ -229,7 +229,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
             const uint32_t row = (tile % p.m_tiles) * kBM + quarter * 32 + lane, n0 = (tile / p.m_tiles) * BN + c_lo;
             const bool in = row < p.a.m;
             const wr_split_scale rs = in ? p.a.row_scale[row] : wr_split_scale{0.f, 0};
-            if (!mbar_wait(&acc_full[acc], (turn / T::kAccs) & 1, p.wait_limit)) {
+            if (!mbar_wait_warp(&acc_full[acc], (turn / T::kAccs) & 1, p.wait_limit)) {
                 ok = false;
                 break;
             }

@@ -166,7 +166,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const SkinnyParams
         bool ok = true;
         for (uint32_t it = 0; it < nkb; ++it) {
             const uint32_t st = it % kStages;
-            if (!mbar_wait(&full[st], (it / kStages) & 1, p.wait_limit)) {
+            if (!mbar_wait_warp(&full[st], (it / kStages) & 1, p.wait_limit)) {
                 ok = false;
                 break;
             }
@@ -183,8 +183,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const SkinnyParams
         __syncwarp();
     } else {
         pdl_wait();
-        if (!mbar_wait(&acc_full, 0, p.wait_limit) && lane == 0) atomicCAS(p.err, 0, 53);
-        __syncwarp();
+        if (!mbar_wait_warp(&acc_full, 0, p.wait_limit) && lane == 0) atomicCAS(p.err, 0, 53);
         tc5::fence_after();
         float v[kN];
         tc5::ld32(tmem + (((warp & 3) * 32) << 16), v);  // lane: weight row; column: activation row
@@ -220,7 +219,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap x_map, const SkinnyParams
                     if (i < pitch) send4(to + 4 * i, s[i], s[i + 1], s[i + 2], s[i + 3], bar);
             }
             // (a rank that gave up on a wait of its own sends all the same, within two limits)
-            late = !mbar_wait(&sums, 0, 4 * p.wait_limit);
+            late = !mbar_wait_warp(&sums, 0, 4 * p.wait_limit);
             if (late && lane == 0) atomicCAS(p.err, 0, 54);
             for (uint32_t j = threadIdx.x - 64; !late && j < p.a.rows * share; j += kThreads - 64) {
                 const uint32_t i = j / share, mm = j % share;
