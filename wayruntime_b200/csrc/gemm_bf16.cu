@@ -31,9 +31,11 @@
 
 namespace {
 
-constexpr uint32_t kBM = 128, kBK = 64;                  // rows of one CTA, K-values of a stage
-constexpr uint32_t kMaxN = 256;                          // columns of a tile, and of one accumulator of two
-constexpr uint32_t kMapRows = 32;                        // a pair's rank takes a multiple of these of a tile's weight rows
+using wr_plan::kBM;
+using wr_plan::kMapRows;
+using wr_plan::kMaxN;
+using wr_plan::Plan;
+constexpr uint32_t kBK = 64;                             // K-values of a stage
 constexpr uint32_t kOutWarps = 8, kWeightWarp = 2 + kOutWarps, kThreads = 32 * (kWeightWarp + 1);
 constexpr uint32_t kABytes = kBM * kBK * 2, kRowBytes = kBK * 2;
 constexpr uint32_t kMaxStages = 8, kStageBudget = 196608;
@@ -409,46 +411,6 @@ int map_2d(CUtensorMap *map, const void *base, uint32_t rows, uint32_t k, uint32
                : WR_CUDA_ERR_INTERNAL;
 }
 
-
-struct Plan {
-    uint64_t cost = ~0ull;
-    uint32_t wide = 0, bn0 = kMaxN, bn1 = kMaxN;
-};
-
-// A worker's clocks per 64 K-values of a tile: the products, or the operands on their way out of L2.  A pair takes 350 clocks
-// or more, however narrow its tile (with 180 or 230 here narrower tiles are chosen: a prompt of 1501 rows with experts 1284 us
-// -> 1295); a CTA by itself gets about 100 bytes a clock.
-uint64_t tile_cost(uint32_t ranks, uint32_t bn) { return std::max(2u * bn, ranks == 2 ? 350u : 150u + (kBM + bn) * 5u / 4u) + 24u; }
-
-// The cut of n columns into tiles that the workers finish first: tiles of 256 columns, and behind them (so that the last
-// round is a full one) narrower tiles for the rest.
-Plan plan(uint32_t ranks, uint32_t m_tiles, uint32_t n, uint32_t workers, bool one_width)
-{
-    Plan best;
-    const uint32_t most = (n + kMaxN - 1) / kMaxN, rounds = (uint32_t)(((uint64_t)most * m_tiles + workers - 1) / workers);
-    for (uint32_t k = 0; k < rounds && k < 9; ++k) {
-        // wide tiles fill the first rounds but k (none at all: every tile has the narrow width)
-        const uint64_t full = k + 1 == rounds || k == 8 ? 0 : (uint64_t)(rounds - 1 - k) * workers / m_tiles;
-        const uint32_t wide = (uint32_t)std::min<uint64_t>(full, most);
-        if (one_width && wide) continue;
-        for (uint32_t bn = kMapRows * ranks; bn <= std::min(kMaxN, wr_weight_blocks(n) * kWBlock); bn += kMapRows * ranks) {
-            const uint32_t left = n > wide * kMaxN ? (n - wide * kMaxN + bn - 1) / bn : 0u;
-            const uint64_t t0 = (uint64_t)wide * m_tiles, tiles = t0 + (uint64_t)left * m_tiles;
-            uint64_t cost = 0;                           // tiles go round: the workers differ at two places only
-            for (uint64_t w : {(uint64_t)0, t0 % workers}) {
-                const uint64_t all = (tiles - std::min(w, tiles) + workers - 1) / workers, a = (t0 - std::min(w, t0) + workers - 1) / workers;
-                cost = std::max(cost, a * tile_cost(ranks, kMaxN) + (all - a) * tile_cost(ranks, bn));
-            }
-            if (cost < best.cost) {
-                best.cost = cost;
-                best.wide = wide;
-                best.bn1 = bn;
-            }
-        }
-    }
-    return best;
-}
-
 template <bool PAIR>
 int launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_weight &w, const wr_gemm_args &a, uint32_t m_tiles,
            uint32_t workers, const Plan &pl)
@@ -517,20 +479,24 @@ int wr_skinny_map_rows(CUtensorMap *map, const void *split_rows, uint32_t k, uin
 
 int wr_gemm_launch(wr_cuda_ctx *ctx, const CUtensorMap &x, const wr_weight &w, const wr_gemm_args &a)
 {
+    auto plan = [&](uint32_t ranks, const auto &m_tiles, uint32_t workers) {
+        return wr_plan::plan(ranks, m_tiles, w.n, wr_weight_blocks(w.n) * kWBlock, workers);
+    };
     if (a.m == 0 || w.n == 0 || w.k == 0 || (a.out_ld & 7u) || (a.out_bf16_ld & 7u) || (a.add_ld & 7u) ||
         (a.pair.from != ~0u && ((a.pair.from & 15u) || (a.pair.ld & 7u))))
         return WR_CUDA_ERR_INVAL;
     const uint32_t sms = (uint32_t)ctx->sm_count;
     if (a.group.list) {
-        const uint32_t likely = a.group.likely ? std::min(a.group.likely, a.group.max) : a.group.max;
-        if (a.group.tile == kBM) return launch<false>(ctx, x, w, a, a.group.max, sms, plan(1, likely, w.n, sms, true));
+        wr_plan::Tiles likely = a.group.likely;
+        for (uint32_t *t : {&likely.few, &likely.usual, &likely.many}) *t = *t ? std::min(*t, a.group.max) : a.group.max;
+        if (a.group.tile == kBM) return launch<false>(ctx, x, w, a, a.group.max, sms, plan(1, likely, sms));
         if (a.group.tile != 2 * kBM || !w.maps || a.group.stride % kRowBytes || sms < 2) return WR_CUDA_ERR_INVAL;
-        return launch<true>(ctx, x, w, a, a.group.max, sms / 2, plan(2, likely, w.n, sms / 2, true));
+        return launch<true>(ctx, x, w, a, a.group.max, sms / 2, plan(2, likely, sms / 2));
     }
     const uint32_t m_one = (a.m + kBM - 1) / kBM, m_two = (m_one + 1) / 2;
-    const Plan one = plan(1, m_one, w.n, sms, false);
+    const Plan one = plan(1, m_one, sms);
     if (w.maps && !a.pages && a.m > kBM && sms >= 2) {
-        const Plan two = plan(2, m_two, w.n, sms / 2, false);
+        const Plan two = plan(2, m_two, sms / 2);
         if (two.cost <= one.cost) return launch<true>(ctx, x, w, a, m_two, sms / 2, two);
     }
     return launch<false>(ctx, x, w, a, m_one, sms, one);

@@ -3,6 +3,7 @@
 
 #include <cuda.h>
 
+#include "gemm_plan.h"
 #include "wr_internal.cuh"
 
 enum { WR_GEMM_OUT_F32 = 0, WR_GEMM_OUT_BF16 = 1, WR_GEMM_OUT_F16 = 2 };
@@ -29,7 +30,7 @@ struct wr_group_args {
     uint32_t x_rows = 0;
     size_t stride = 0;
     uint32_t tile = 128;                 // many rows: 128, or 256 (a tile of a pair of CTAs; the weights need their maps)
-    uint32_t likely = 0;                 // many rows: how many tiles there will be, about
+    wr_plan::Tiles likely;               // many rows: how many tiles there will be (not known: max)
 };
 
 struct wr_gemm_args {

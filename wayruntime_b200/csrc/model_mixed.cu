@@ -1052,7 +1052,7 @@ struct Step {
         } else if (bf) {
             TRY(wr_moe_gather_launch(ctx, x->xin, x->e_in, x->ldw, x->e_row_of, x->e_count, groups, r.tile));
             gr.tile = r.tile;
-            gr.likely = rw.n_rows * l.top / r.tile + std::min(l.experts, rw.n_rows * l.top) / 2;
+            gr.likely = wr_plan::likely_tiles(rw.n_rows, l.experts, l.top, r.tile);
             wr_gemm_args a{};
             a.m = groups * r.tile;
             a.pair = l.e_up.pair; a.pair.out = x->e_act; a.pair.ld = lf;
