@@ -105,4 +105,19 @@ inline Tiles likely_tiles(uint32_t rows, uint32_t experts, uint32_t top, uint32_
     return t;
 }
 
+// Rows of experts' tiles: 256, on pairs of CTAs, where nearly every tile of 256 stands for two of 128, else 128.  32 experts, top 4, us a
+// prompt with tiles of 128 / 256 (4 layers of width 1024 and 2048, 2 of 4096), and how many of 128 one of 256 stands for:
+//      768 rows 1.00   598 /  632   913 /  977   1121 / 1297        2048 rows 1.67  1022 / 1021  1546 / 1551   2194 / 2301
+//     1024 rows 1.48   678 /  699  1036 / 1064   1329 / 1454        1152 rows 1.92   742 /  739  1152 / 1132   1476 / 1553
+//     1280 rows 2.00   777 /  774  1206 / 1174   1716 / 1689        1501 rows 2.00   844 /  841  1285 / 1270   1768 / 1755
+// and 2 layers   2560 rows 1.50  769 / 787  1150 / 1199    3584 rows 2.00  997 / 981  1494 / 1473    4096 rows 1.80  1095 / 1115  1682 / 1690
+//     6000 rows 1.93  1645 / 1634  2486 / 2469    8192 rows 1.89  2157 / 2160  3561 / 3556
+inline uint32_t expert_tile(uint32_t rows, uint32_t experts, uint32_t top)
+{
+    double one, two, dev;
+    expert_tiles(rows, experts, top, kBM, one, dev);
+    expert_tiles(rows, experts, top, 2 * kBM, two, dev);
+    return one >= 1.9 * two ? 2 * kBM : kBM;
+}
+
 }  // namespace wr_plan

@@ -30,11 +30,6 @@ constexpr double kLog2e = 1.4426950408889634;
 size_t up256(size_t n) { return (n + 255u) & ~(size_t)255u; }
 
 constexpr uint32_t kMoeTile = 128;       // rows of a tile of gemm_bf16.cu
-// Tiles of pairs of CTAs where the experts have that many rows each on average: a pair takes about half the time of one CTA for
-// a tile twice as high, so it pays from where most experts' rows fill more than a quarter of it.  (1501 rows, 32 experts, top 4,
-// width 2048: gate and up 144 -> 108 us, down 75 -> 55; their weights' bytes alone 62 and 31.)
-constexpr uint32_t kMoePairRows = 96;
-inline uint32_t moe_tile(uint32_t rows, uint32_t experts, uint32_t top) { return (uint64_t)rows * top >= (uint64_t)experts * kMoePairRows ? 2 * kMoeTile : kMoeTile; }
 // places that up to `rows` rows may take
 inline size_t moe_places(uint32_t rows, uint32_t experts, uint32_t top)
 {
@@ -1015,7 +1010,7 @@ struct Step {
     {
         wr_route_args r{};
         r.logits = x->lat + off; r.ld = ld; r.bias = l.router_b; r.experts = l.experts; r.top = l.top;
-        r.tile = split() ? 0 : x->compute == WR_CUDA_BF16 ? moe_tile(rw.n_rows, l.experts, l.top) : kMoeTileF32;
+        r.tile = split() ? 0 : x->compute == WR_CUDA_BF16 ? wr_plan::expert_tile(rw.n_rows, l.experts, l.top) : kMoeTileF32;
         r.weight = x->e_weight; r.expert = x->e_expert; r.place = x->e_place; r.row_of = x->e_row_of;
         r.list = x->e_list; r.count = x->e_count;
         return r;
