@@ -166,7 +166,7 @@ int wr_decode_validate(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv,
 // the kernel, so that they all give the same bits.  Fills everything of `p`
 // that depends on the batch; the caller adds buffers, scale and flags.
 void wr_decode_plan(uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer, const uint32_t *seq_lens,
-                    uint32_t n_q, uint32_t window, wr_decode::params &p, uint32_t &nt, uint32_t &items)
+                    uint32_t n_q, uint32_t window, bool shard, wr_decode::params &p, uint32_t &nt, uint32_t &items)
 {
     using namespace wr_decode;
     const uint32_t n_kv = kv[0]->n_kv_at(layer), hd = kv[0]->hd_at(layer);
@@ -185,7 +185,7 @@ void wr_decode_plan(uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer, cons
         const uint32_t n_tiles = (len + kTile - 1) / kTile;
         const uint32_t tile_lo = key_lo / kTile;
         const uint32_t span = n_tiles - tile_lo;
-        const uint32_t ct = chunk_tiles_for(span, n_kv, qsubs); // chunk length: this session and the cache geometry alone
+        const uint32_t ct = chunk_tiles_for(span, n_kv, qsubs, shard); // chunk length: this session and the cache geometry alone
         const uint32_t nc = (span + ct - 1) / ct;              // 0 for an empty shard
         p.b.pages[i] = kv[s]->d_pages + (size_t)layer * kv[s]->n_pages;
         p.b.seq_len[i] = len;
@@ -227,7 +227,7 @@ int wr_decode_launch(wr_cuda_ctx *ctx, uint32_t n_sess, wr_cuda_kv *const *kv, u
         using namespace wr_decode;
         params p;
         uint32_t nt = 1, items = 0;
-        wr_decode_plan(n_sess, kv, layer, seq_lens, n_q, window, p, nt, items);
+        wr_decode_plan(n_sess, kv, layer, seq_lens, n_q, window, emit_triples != 0, p, nt, items);
         int rc = wr_ctx_reserve_ws(ctx, (size_t)std::max(items, 1u) * 8 * kTripleStride * sizeof(float),
                                    (size_t)p.n_groups * kTicketsPerGroup + kTicketExtra);
         if (rc != WR_CUDA_OK) return rc;

@@ -73,11 +73,13 @@ constexpr int kItemsPerSessionTarget = WR_DECODE_ITEMS_TARGET;   // work items o
 // reaches every engine of the machine.  Sessions longer than 64 tiles use at
 // least 32 chunks, which keeps items short enough to balance a few long
 // sessions.  A chunk is never shorter than kMinChunkTiles, and a session of up to kOneChunkTiles is one chunk: a further tile takes
-// its engine 0.6 to 1 us, handing chunks to a merge warp 5 (one session of 16 q and 8 kv heads, device rows, us a call: 128 keys 20.9,
-// 192 keys in two chunks 25.4, in one 22.4, 256 keys 25.6 and 23.5).
-__host__ __device__ inline uint32_t chunk_tiles_for(uint32_t span_tiles, uint32_t n_kv, uint32_t qsubs)
+// its engine 0.6 to 1 us, handing chunks to a merge warp 5 (decode steps alone, us with 192 / 256 keys, one chunk and two: 8 kv heads with
+// 2 q heads each, one session 26.4 / 27.2 and 28.9 / 28.2, 16 sessions 28.0 / 29.5 and 31.3 / 31.1; one kv head with 8, one session 27.8 / 29.5
+// and 30.0 / 30.8, 16 sessions 29.6 / 31.5 and 33.2 / 32.9).  A shard of the keys (`shard`) keeps its two chunks: rows that go through merge
+// warps can be received and finished there (wr_decode_xchg), one launch instead of two.
+__host__ __device__ inline uint32_t chunk_tiles_for(uint32_t span_tiles, uint32_t n_kv, uint32_t qsubs, bool shard)
 {
-    if (span_tiles <= (uint32_t)kOneChunkTiles) return (uint32_t)kOneChunkTiles;
+    if (!shard && span_tiles <= (uint32_t)kOneChunkTiles) return (uint32_t)kOneChunkTiles;
     const uint32_t per_chunk = n_kv * qsubs;
     uint32_t max_chunks = ((uint32_t)kItemsPerSessionTarget + per_chunk - 1) / per_chunk;
     if (max_chunks < 16u) max_chunks = 16u;
@@ -155,7 +157,7 @@ __device__ __forceinline__ void xchg_rows_done(const params &p, uint32_t row_fir
 
 // Host side (attn_decode.cu): the batch-dependent part of `params`.
 void wr_decode_plan(uint32_t n_sess, wr_cuda_kv *const *kv, uint32_t layer, const uint32_t *seq_lens,
-                    uint32_t n_q, uint32_t window, wr_decode::params &p, uint32_t &nt, uint32_t &items);
+                    uint32_t n_q, uint32_t window, bool shard, wr_decode::params &p, uint32_t &nt, uint32_t &items);
 
 namespace wr_decode {
 

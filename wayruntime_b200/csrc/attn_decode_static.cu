@@ -134,7 +134,7 @@ extern "C" int wr_cuda_attn_decode_static(wr_cuda_ctx *ctx, uint32_t n_sess, wr_
     // The work decomposition is wr_cuda_attn_decode's own, so the result is the same.
     params p;
     uint32_t nt = 1, items = 0;
-    wr_decode_plan(n_sess, kv, layer, seq_lens, n_q_heads, window, p, nt, items);
+    wr_decode_plan(n_sess, kv, layer, seq_lens, n_q_heads, window, false, p, nt, items);
     if (items > WR_CUDA_STATIC_MAX_ITEMS || p.n_groups > WR_CUDA_STATIC_MAX_GROUPS)
         return WR_CUDA_ERR_LIMIT;           // the fixed scratch area cannot hold this call
     p.q = q;
