@@ -97,8 +97,9 @@ __global__ void __launch_bounds__(kSetThreads * SETS) attn_step_small_kernel(con
         sn_tab[tid] = sn;
     }
     // Short sessions: the K and V lines on their way into L2 (between two steps the weights have pushed them out): a hint, whatever
-    // is still being written.  (28 layers, 64 to 192 keys: 1030 -> 1023 us a step.  With more keys, and beside another stream's kernel,
-    // the hints cost more than they bring: 16 sessions of 200 to 2000 keys 2973 -> 3001.)
+    // is still being written.  (28 layers, 64 to 192 keys: 1030 -> 1023 us a step.  With more keys they cost more than they bring: 16
+    // sessions of 200 to 2000 keys 2973 -> 3001.  On the stream beside long sessions' kernels they make no difference: without / with
+    // them, 15 sessions of 60 to 228 keys and one of 2000 2380 / 2384, 8 and 8 of 1200 to 1900 2471 / 2461, one and one 1455 / 1459.)
     if constexpr (SETS == 1) {
         __syncthreads();
         for (uint32_t i = tid; i < pos * 4; i += kSmallThreads) {
