@@ -1175,7 +1175,8 @@ __global__ void __launch_bounds__(32 * kMergeRows) prefill_merge_kernel(const pr
         const size_t r = ((size_t)(tile * p.parts + i) * 2 + b) * kBM + row;
         const float2 ml = p.part_ml[r];
         const float4 v = reinterpret_cast<const float4 *>(part_rows + r * kHd)[lane];
-        if (ml.x == WR_NEG_SENTINEL) continue;                   // no key of this piece is visible to the row
+        // no key of this piece is visible to the row (the sums of scores that are not numbers are NaN, not zero, and stay)
+        if (ml.x == WR_NEG_SENTINEL && ml.y == 0.f) continue;
         const float top = fmaxf(m, ml.x), keep = m == WR_NEG_SENTINEL ? 0.f : ex2_approx(m - top), w = ex2_approx(ml.x - top);
         l = fmaf(l, keep, ml.y * w);
         o = make_float4(fmaf(o.x, keep, v.x * w), fmaf(o.y, keep, v.y * w), fmaf(o.z, keep, v.z * w), fmaf(o.w, keep, v.w * w));
