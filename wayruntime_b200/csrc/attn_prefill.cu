@@ -73,7 +73,10 @@ constexpr uint32_t kTmemS = 0;                   // S (then P) of block b at col
 constexpr uint32_t kTmemO = 256;                 // O of block b at columns 256 + 128*b
 constexpr float kRescaleLog2 = 8.0f;             // move the reference max when it is 2^8 behind
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr uint32_t kLeastPiece = 3, kMostParts = 16; // steps of a piece, pieces of a tile
+// Steps of a piece, pieces of a tile.  17 rows, us with the append: shortest pieces of 2 / 3 / 6 steps, 8 heads behind 1000 keys 20.7 / 23.7 /
+// 23.8, behind 2000 keys 21.1 / 22.3 / 27.4, 4 heads behind 1000 keys 29.0 / 24.9 / 24.6, behind 2000 keys 27.8 / 21.1 / 26.4; at most 8 / 16 / 32
+// pieces, 4 heads behind 8000 keys 28.2 / 23.4 / 25.1, behind 30000 keys 64.5 / 41.9 / 36.3.
+constexpr uint32_t kLeastPiece = 3, kMostParts = 16;
 constexpr uint32_t kMergeTime = 1000;            // what pieces have to bring at least, in hundredths of a microsecond
 constexpr int kTileSlots = 4;                    // ring of published work tiles
 // Of every kPolyPeriod pairs of exponentials one pair is evaluated on the FMA pipe (0: none).
