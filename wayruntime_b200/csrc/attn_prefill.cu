@@ -635,7 +635,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     auto tile_of = [&](uint32_t it, bool &ok) -> tile_info {
         if (it == 0) return decode_tile<TILES>(p, blockIdx.x);
         const uint32_t slot = it % kTileSlots, parity = ((it - 1) / kTileSlots) & 1;
-        ok = warp == 8 ? mbar_wait(&sm.tile_ready[slot], parity, limit) : mbar_wait_warp(&sm.tile_ready[slot], parity, limit);    // (one lane / all)
+        ok = warp == 9 ? mbar_wait_warp(&sm.tile_ready[slot], parity, limit) : mbar_wait(&sm.tile_ready[slot], parity, limit);
         if (!ok) return decode_tile<TILES>(p, p.n_tiles);                   // (invalid)
         return sm.tile[slot];
     };
@@ -873,6 +873,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         if (!ok && lane == 0) atomicCAS(p.err, 0, 12);
     } else {
         // ----------------------------- softmax warpgroup b: one thread per query row
+        // (A wait here needs no vote: what it waits for does not come again before the warp has met at a __syncwarp and its lane 0
+        // has handed something on.)
         const uint32_t b = warp >> 2;
         const uint32_t row = tid & (kGroupThreads - 1);     // TMEM lane
         const uint32_t wq = warp & 3u;
@@ -898,6 +900,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             const uint32_t lo = tr.lo, hi = tr.hi;
             if (b >= ti.nblk) {                              // a lone block: this group sits the tile out
                 vc += hi - lo;
+                __syncwarp();                                // (together: tiles' slots are used again)
                 continue;
             }
             const block_range me = (b == 0) ? tr.b0 : tr.b1;
@@ -909,7 +912,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             float m_ref = WR_NEG_SENTINEL;                   // reference max, log2 domain
             float l = 0.f;
             for (uint32_t j = me.lo; j < me.hi && ok; ++j) {
-                ok = mbar_wait_warp(&sm.s_full[b], s_uses & 1, limit);
+                ok = mbar_wait(&sm.s_full[b], s_uses & 1, limit);
                 ++s_uses;
                 if (!ok) break;
                 TLS();                                           // 0: scores ready
@@ -1013,7 +1016,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                     // tile so that 0 * garbage cannot make a NaN (both groups do it
                     // before releasing their own P.V; the writes are equal).
                     const uint32_t vn = vc + (j - lo), vst = vn % v_stages;
-                    ok = mbar_wait_warp(&sm.v_full[vst], (vn / v_stages) & 1, limit);
+                    ok = mbar_wait(&sm.v_full[vst], (vn / v_stages) & 1, limit);
                     if (!ok) break;
                     const uint32_t first_bad = p.p0 + p.n - key0;
                     if (row >= first_bad) {
@@ -1038,7 +1041,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             vc += hi - lo;
             if (!ok) break;
             // ---- the tile's last P.V has completed: O leaves TMEM, normalised
-            ok = mbar_wait_warp(&sm.o_done[b], o_uses & 1, limit);
+            ok = mbar_wait(&sm.o_done[b], o_uses & 1, limit);
             ++o_uses;
             if (!ok) break;
             tc_fence_after();

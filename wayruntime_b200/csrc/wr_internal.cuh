@@ -352,7 +352,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long l
 // seconds longer: a lane without work of its own had been left behind, and nobody asked whether its wait had run out.)
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, long long limit)
 {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
+    const uint32_t addr = smem_u32(bar);
+    long long t0 = 0;
+    for (bool first = true;; first = false) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (__all_sync(0xffffffffu, done)) return true;
+        if (first) t0 = clock64();
+        else if (__any_sync(0xffffffffu, clock64() - t0 > limit)) return false;
+    }
 }
 // One non-blocking look at a barrier phase.
 __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity)
