@@ -20,9 +20,11 @@
 //   (with one per 64 rows 61).
 // - The odd rank's copies count on the even rank's barrier (a warp that relayed them: 70 against 61).
 // - Eight warps bring a tile's last results out through shared memory in 7 us, four without it took 18.
-// - Experts' weights are read by a tile or two and go out of L2 first; else they push out what every prompt reads (dense weights,
-//   activations).  Nurosun prompts without / with, us: 4 layers of width 1024, 17 rows 419 / 396, 300 rows 488 / 470, 1024 rows 680 / 674;
-//   width 2048, 40 rows 680 / 663, 682 rows 895 / 872, 2048 rows 1547 / 1502; 2 layers of width 4096, 100 rows 837 / 809, 500 rows 974 / 931.
+// - Experts' weights that are read by a tile or two go out of L2 first (wr_group_args::once); else they push out what every prompt
+//   reads, dense weights and activations.  Nurosun prompts without / with, us, tiles of 128 rows: 4 layers of width 1024, 17 rows
+//   419 / 396, 300 rows 488 / 470; width 2048, 40 rows 680 / 663, 682 rows 895 / 872; 2 layers of width 4096, 100 rows 837 / 809, 500 rows
+//   974 / 931.  Tiles of 256: width 2048, 1280 rows 1181 / 1135, 1792 rows 1385 / 1341; width 4096 1675 / 1593, 1978 / 1913.  Where an expert
+//   has more rows its other tiles miss them: width 4096, tiles of 256, 2560 rows 2916 / 3045, 6000 rows 6463 / 6786.
 // - Weights have a warp of their own, which does not wait for the kernel ahead: a prompt of 2048 rows, 8 layers of width
 //   2048, 2614 -> 2597 us, one of 1501 rows, 4 layers with experts, 1300 -> 1286.
 #include <cuda_bf16.h>
@@ -257,8 +259,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
                     uint8_t *a = stages + st * p.stage_bytes, *b = a + kABytes;
                     // (a stage's bytes may come before they are expected: its barrier still waits for warp 0)
                     if (weights) {
-                        if (PAIR) tc5::tma_load_2d_pair(b, w_map, 0, (int)(kb * w_rows + y0), &full[st]);
-                        else if (rows && p.a.group.list) bulk_g2s_hint(b, blocks + wr_weight_row(p.w.n, r0, kb), rows * kRowBytes, &full[st], first_out);
+                        if (PAIR && p.a.group.once) tc5::tma_load_2d_pair_hint(b, w_map, 0, (int)(kb * w_rows + y0), &full[st], first_out);
+                        else if (PAIR) tc5::tma_load_2d_pair(b, w_map, 0, (int)(kb * w_rows + y0), &full[st]);
+                        else if (rows && p.a.group.once) bulk_g2s_hint(b, blocks + wr_weight_row(p.w.n, r0, kb), rows * kRowBytes, &full[st], first_out);
                         else if (rows) bulk_g2s(b, blocks + wr_weight_row(p.w.n, r0, kb), rows * kRowBytes, &full[st]);
                     } else {
                         if (rank == 0) mbar_expect_tx(&full[st], bytes);

@@ -31,6 +31,7 @@ struct wr_group_args {
     size_t stride = 0;
     uint32_t tile = 128;                 // many rows: 128, or 256 (a tile of a pair of CTAs; the weights need their maps)
     wr_plan::Tiles likely;               // many rows: how many tiles there will be (not known: max)
+    bool once = false;                   // many rows: a weight is read by a tile or two, and not kept in L2 for more
 };
 
 struct wr_gemm_args {

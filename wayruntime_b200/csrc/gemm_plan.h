@@ -107,11 +107,11 @@ inline Tiles likely_tiles(uint32_t rows, uint32_t experts, uint32_t top, uint32_
 
 // Rows of experts' tiles: 256, on pairs of CTAs, where nearly every tile of 256 stands for two of 128, else 128.  32 experts, top 4, us a
 // prompt with tiles of 128 / 256 (4 layers of width 1024 and 2048, 2 of 4096), and how many of 128 one of 256 stands for:
-//      768 rows 1.00   598 /  632   913 /  977   1121 / 1297        2048 rows 1.67  1022 / 1021  1546 / 1551   2194 / 2301
-//     1024 rows 1.48   678 /  699  1036 / 1064   1329 / 1454        1152 rows 1.92   742 /  739  1152 / 1132   1476 / 1553
-//     1280 rows 2.00   777 /  774  1206 / 1174   1716 / 1689        1501 rows 2.00   844 /  841  1285 / 1270   1768 / 1755
-// and 2 layers   2560 rows 1.50  769 / 787  1150 / 1199    3584 rows 2.00  997 / 981  1494 / 1473    4096 rows 1.80  1095 / 1115  1682 / 1690
-//     6000 rows 1.93  1645 / 1634  2486 / 2469    8192 rows 1.89  2157 / 2160  3561 / 3556
+//      768 rows 1.00   591 /  633   894 /  932   1033 / 1234        2048 rows 1.67  1017 / 1019  1514 / 1513   2211 / 2281
+//     1024 rows 1.48   677 /  695  1009 / 1021   1315 / 1380        1152 rows 1.92   739 /  735  1113 / 1089   1631 / 1468
+//     1280 rows 2.00   778 /  774  1171 / 1135   1733 / 1593        1501 rows 2.00   846 /  840  1251 / 1218   1772 / 1723
+// and 2 layers   2560 rows 1.50  783 / 787  1160 / 1219    3584 rows 2.00  994 / 988  1518 / 1546    4096 rows 1.80  1097 / 1117  1714 / 1714
+//     6000 rows 1.93  1676 / 1671  2609 / 2529    8192 rows 1.89  2157 / 2160  3561 / 3556
 inline uint32_t expert_tile(uint32_t rows, uint32_t experts, uint32_t top)
 {
     double one, two, dev;

@@ -1048,6 +1048,7 @@ struct Step {
             TRY(wr_moe_gather_launch(ctx, x->xin, x->e_in, x->ldw, x->e_row_of, x->e_count, groups, r.tile));
             gr.tile = r.tile;
             gr.likely = wr_plan::likely_tiles(rw.n_rows, l.experts, l.top, r.tile);
+            gr.once = (uint64_t)rw.n_rows * l.top <= (uint64_t)l.experts * 2 * kMoeTile;
             wr_gemm_args a{};
             a.m = groups * r.tile;
             a.pair = l.e_up.pair; a.pair.out = x->e_act; a.pair.ld = lf;

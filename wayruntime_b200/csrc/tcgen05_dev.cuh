@@ -184,7 +184,17 @@ __device__ __forceinline__ void tma_load_2d(void *dst_smem, const CUtensorMap *m
         : "memory");
 }
 
-// ... of a pair's rank into its own shared memory, counted by the even rank's barrier at this offset
+// ... of a pair's rank into its own shared memory, counted by the even rank's barrier at this offset; with a policy for L2
+__device__ __forceinline__ void tma_load_2d_pair_hint(void *dst_smem, const CUtensorMap *map, int x, int y, uint64_t *bar, uint64_t policy)
+{
+    asm volatile(
+        "{\n\t.reg .b32 r;\n\t"
+        "mapa.shared::cluster.u32 r, %4, 0;\n\t"
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint "
+        "[%0], [%1, {%2, %3}], [r], %5;\n\t}"
+        ::"r"(smem_u32(dst_smem)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy)
+        : "memory");
+}
 __device__ __forceinline__ void tma_load_2d_pair(void *dst_smem, const CUtensorMap *map, int x, int y, uint64_t *bar)
 {
     asm volatile(
