@@ -30,6 +30,10 @@ constexpr double kLog2e = 1.4426950408889634;
 size_t up256(size_t n) { return (n + 255u) & ~(size_t)255u; }
 
 constexpr uint32_t kMoeTile = 128;       // rows of a tile of gemm_bf16.cu
+// Experts' weights go out of L2 first (wr_group_args::once) up to that many rows of an expert on average.  32 experts, top 4, us a prompt
+// without / with: 1792 rows (224 of an expert) of width 2048 1385 / 1341, of 4096 1944 / 1885; 2048 rows (256) of width 2048 1558 / 1500,
+// but of 4096 2200 / 2315 (gate and up 474 / 580).
+constexpr uint32_t kMoeOnceRows = 224;
 // places that up to `rows` rows may take
 inline size_t moe_places(uint32_t rows, uint32_t experts, uint32_t top)
 {
@@ -1048,7 +1052,7 @@ struct Step {
             TRY(wr_moe_gather_launch(ctx, x->xin, x->e_in, x->ldw, x->e_row_of, x->e_count, groups, r.tile));
             gr.tile = r.tile;
             gr.likely = wr_plan::likely_tiles(rw.n_rows, l.experts, l.top, r.tile);
-            gr.once = (uint64_t)rw.n_rows * l.top <= (uint64_t)l.experts * 2 * kMoeTile;
+            gr.once = (uint64_t)rw.n_rows * l.top <= (uint64_t)l.experts * kMoeOnceRows;
             wr_gemm_args a{};
             a.m = groups * r.tile;
             a.pair = l.e_up.pair; a.pair.out = x->e_act; a.pair.ld = lf;
