@@ -409,13 +409,13 @@ __global__ void __launch_bounds__(kPolyThreads) polynorm_kernel(const wr_polynor
     }
 }
 
-// The same for a BF16 prompt's rows of up to 2048 NV values: a thread keeps its values, and eight blocks share an SM, so that the
-// rows' loads, sums and stores overlap (2048 rows of 6144: 18.8 -> 13.9 us; 512 threads that read their values twice, four blocks
-// to an SM, spent most of it waiting for each other).  Sums are those of the kernel above, bit for bit: a thread stands for threads t
+// The same for a BF16 prompt's rows of up to 2048 NV values: a thread keeps its values, and at least four blocks share an SM (two of
+// the longest rows), so that the rows' loads, sums and stores overlap (2048 rows of 6144: 18.8 -> 14.5 us, with three blocks
+// 15.8; 512 threads that read their values twice spent most of it waiting for each other).  Sums are those of the kernel above, bit for bit: a thread stands for threads t
 // and t + 256 of its 512 (values u = 0, 2, .. and 1, 3, ..), a warp for two of its sixteen.
 constexpr uint32_t kPolyRowThreads = 256;
 template <int NV>
-__global__ void __launch_bounds__(kPolyRowThreads) polynorm_rows_kernel(const wr_polynorm_args a)
+__global__ void __launch_bounds__(kPolyRowThreads, NV <= 3 ? 4 : 2) polynorm_rows_kernel(const wr_polynorm_args a)
 {
     __shared__ float red[3][kPolyWarps];
     static_assert(2 * kPolyRowThreads == kPolyThreads, "a thread's values are those of two threads above");
