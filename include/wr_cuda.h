@@ -69,6 +69,9 @@ typedef struct wr_cuda_kv  wr_cuda_kv;   /* one session's paged F16 K/V cache   
  * (src/core/engine.c:130): no B200 bound -> WR_ERR_UNSUPPORTED. */
 int wr_cuda_device_check(int device);
 
+/* Keeps 20 MB of device memory for prompts whose attention is cut along the
+ * keys.  A context that does not get them works without: such prompts take
+ * longer, and their rows agree with the others' to rounding. */
 int  wr_cuda_ctx_create(int device, wr_cuda_ctx **out);
 void wr_cuda_ctx_destroy(wr_cuda_ctx *ctx);
 
